@@ -8,15 +8,18 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <future>
 #include <initializer_list>
 #include <mutex>
 #include <new>
+#include <system_error>
 #include <vector>
 
 #include "pdf.h"
 #include "pdf_inject.h"
 #include "pdf_internal.h"
 #include "pdf_kernels.cuh"
+#include "pdf_plan.h"
 
 #include <atomic>
 
@@ -136,12 +139,10 @@ struct Workspace {
     DevBuf over_list, spill;  // pairs for the spill cover and its per-net (h, c) slots
     DevBuf nzb_fine, maxlvl_fine;  // lane circuits: the cover's bitmaps per quarter column block
     DevBuf pi_counts;         // pdf_cover_counts: paths per (primary input, pair)
-    uint32_t spill_slots = 0;
     DevBuf seg_first;  // (net, pair) hash set of the cover with segments
     uint64_t seg_first_mask = 0;
     DevBuf planes;   // internal V, T, M planes when the caller gives none
     DevBuf pi;       // staged host pairs
-    uint64_t plane_ld = 0, plane_words = 0;
     void release() {
         nzb.release();
         maxlvl.release();
@@ -152,7 +153,6 @@ struct Workspace {
         nzb_fine.release();
         maxlvl_fine.release();
         pi_counts.release();
-        spill_slots = 0;
         seg_first.release();
         seg_first_mask = 0;
         planes.release();
@@ -160,20 +160,90 @@ struct Workspace {
     }
 };
 
+namespace {
+
+// One walk over a netlist, on the device.
+struct Plan : PlanShape {
+    DevCircuit dc{};
+    const Piece *pieces = nullptr;
+    const uint32_t *far_ids = nullptr;
+    void bind(const LaunchPlan &l, const NetPlan &n, const unsigned char *base, const struct PlanOffsets &o);
+};
+
+struct PlanOffsets {
+    size_t rec = 0, edges = 0, level_off = 0, pieces = 0, far = 0, orig = 0;
+};
+
+void Plan::bind(const LaunchPlan &l, const NetPlan &n, const unsigned char *base, const PlanOffsets &o) {
+    static_cast<PlanShape &>(*this) = l;
+    dc.rec = reinterpret_cast<const GateRec *>(base + o.rec);
+    dc.edges = reinterpret_cast<const uint32_t *>(base + o.edges);
+    dc.level_off = reinterpret_cast<const uint32_t *>(base + o.level_off);
+    dc.orig = n.orig.empty() ? nullptr : reinterpret_cast<const uint32_t *>(base + o.orig);
+    dc.n_gates = n_gates;
+    dc.n_levels = n_levels;
+    dc.nfo_mask = nfo_mask;
+    pieces = reinterpret_cast<const Piece *>(base + o.pieces);
+    far_ids = reinterpret_cast<const uint32_t *>(base + o.far);
+}
+
+// Arrays of a circuit on their way into one device block: small circuits go
+// in one copy through a host image, large ones array by array.
+struct PlanUpload {
+    struct Part {
+        const void *src;
+        size_t off, bytes;
+    };
+    std::vector<Part> parts;
+    size_t bytes = 0;
+    size_t add(const void *src, size_t n) {
+        const size_t off = bytes;
+        parts.push_back({src, off, n});
+        bytes = (off + n + 255) & ~(size_t)255;
+        return off;
+    }
+    PlanOffsets add_plan(const NetPlan &n, const LaunchPlan &l) {
+        PlanOffsets o;
+        o.rec = add(l.recs.data(), l.recs.size() * sizeof(GateRec));
+        o.edges = add(n.edges.data(), n.edges.size() * 4);
+        bytes += 256;  // bulk copies of edge slices are rounded up to 16 bytes
+        o.level_off = add(n.level_off.data(), n.level_off.size() * 4);
+        o.pieces = add(l.pieces.data(), l.pieces.size() * sizeof(Piece));
+        o.far = add(l.far_ids.data(), l.far_ids.size() * 4);
+        o.orig = add(n.orig.data(), n.orig.size() * 4);
+        return o;
+    }
+    bool copy(unsigned char *dst) const {
+        if (bytes <= (1u << 20)) {
+            std::vector<unsigned char> img(bytes, 0);
+            for (const Part &p : parts)
+                if (p.src && p.bytes) std::memcpy(img.data() + p.off, p.src, p.bytes);
+            return cudaMemcpy(dst, img.data(), bytes, cudaMemcpyHostToDevice) == cudaSuccess;
+        }
+        for (const Part &p : parts) {
+            if (!p.bytes) continue;
+            const cudaError_t e = p.src ? cudaMemcpy(dst + p.off, p.src, p.bytes, cudaMemcpyHostToDevice)
+                                        : cudaMemset(dst + p.off, 0, p.bytes);
+            if (e != cudaSuccess) return false;
+        }
+        return true;
+    }
+};
+
+}  // namespace
+
 struct pdf_circuit {
     int device = 0;
     int mark_mode = PDF_MARK_DEFAULT;
     pdf_circuit_info info{};
-    DevBuf rec, edges, level_off, pieces, far, err;
-    DevCircuit dc{};
-    uint32_t bw = 4, threads = 512, ring = 0, ring2 = 0, farcap = 0;
-    uint32_t cap = 512, ecap = 2048, n_pieces = 0, bm_shared = 0;
-    uint32_t off_ring = 0, off_rec = 0, off_edge = 0, off_fid = 0, off_bm = 0, off_pbits = 0, off_mbar = 0;
-    size_t fwd_smem = 0;
+    DevBuf mem;  // the error word and both plans' arrays
+    uint32_t *err = nullptr;
+    uint32_t bw = 4;  // the tile: column block of the full walk, divisor of the device planes' pitch
+    Plan full, red;   // every gate; the reduced netlist (n_gates 0: none)
+    // the plan of grading calls that ask for no plane
+    const Plan &lean() const { return red.n_gates ? red : full; }
     uint32_t hash_cap = 4096, cover_threads = 256, cover_grid = 0;
     uint32_t wait_polls = 0;  // bound of the forward kernels' waits (0 = the default)
-    uint32_t occ = 1;  // forward CTAs per SM its registers and shared memory are sized for
-    uint64_t chain = 0;  // length of one CTA's walk (pieces, or gates for the lane kernel)
     Workspace stage;  // scratch of the stage calls
     std::mutex mu;    // serialises the stage scratch
     // segments longer than one net
@@ -212,6 +282,7 @@ struct pdf_state {
     ProfEvents *pe = nullptr;       // events of the call in progress
     // the batch marked by pdf_grade_mark_async and not yet counted
     bool pending = false;
+    const Plan *pend_plan = nullptr;
     const uint32_t *pend_M = nullptr;
     uint64_t pend_ld = 0, pend_n = 0, pend_base = 0;
 };
@@ -275,76 +346,80 @@ extern "C" pdf_status pdf_netlist_check(const pdf_netlist *nl, char *msg, size_t
         set_msg(msg, len, "level 0 (primary inputs) is empty");
         return PDF_EINVAL;
     }
-    std::vector<uint32_t> level(G);
-    for (uint32_t l = 0; l < L; l++)
-        for (uint32_t g = nl->level_offsets[l]; g < nl->level_offsets[l + 1]; g++) level[g] = l;
-    for (uint32_t g = 0; g < G; g++) {
-        const uint32_t t = nl->type[g];
-        if (t >= PDF_NTYPES) {
-            set_msg(msg, len, "gate %llu: unknown type code %llu", g, t);
-            return PDF_EINVAL;
-        }
-        if (nl->po[g] > 1) {
-            set_msg(msg, len, "gate %llu: po must be 0 or 1", g);
-            return PDF_EINVAL;
-        }
-        if ((t == PDF_INPT) != (g < npi)) {
-            set_msg(msg, len, "gate %llu: INPT gates must be exactly level 0", g);
-            return PDF_EINVAL;
-        }
-        if (t == PDF_INPT ? nl->nfi[g] != 0 : (nl->nfi[g] == 0 || nl->nfi[g] > 255)) {
-            set_msg(msg, len, "gate %llu: bad fan-in count %llu", g, nl->nfi[g]);
-            return PDF_EINVAL;
-        }
-        const uint64_t end = nl->edge_offset[g] + (uint64_t)nl->nfi[g] + nl->nfo[g];
-        if (end > nl->n_edges || end < nl->edge_offset[g]) {
-            set_msg(msg, len, "gate %llu: edge range out of bounds", g);
-            return PDF_EINVAL;
-        }
-        for (uint32_t j = 0; j < nl->nfi[g]; j++) {
-            const uint32_t f = nl->edges[nl->edge_offset[g] + j];
-            if (f >= G || level[f] >= level[g]) {
-                set_msg(msg, len, "gate %llu: fan-in %llu not on a lower level", g, f);
+    // A gate's fan-ins lie below its level's first gate, its fan-outs at or
+    // past the next level's.  Fan-in uses are counted on the way.
+    std::vector<uint32_t> start((size_t)G + 1, 0);  // [g + 1]: fan-in uses of g
+    uint64_t uses = 0;
+    for (uint32_t l = 0; l < L; l++) {
+        const uint32_t lo = nl->level_offsets[l], hi = nl->level_offsets[l + 1];
+        for (uint32_t g = lo; g < hi; g++) {
+            const uint32_t t = nl->type[g], nfi = nl->nfi[g], nfo = nl->nfo[g];
+            if (t >= PDF_NTYPES) {
+                set_msg(msg, len, "gate %llu: unknown type code %llu", g, t);
                 return PDF_EINVAL;
             }
-        }
-        for (uint32_t k = 0; k < nl->nfo[g]; k++) {
-            const uint32_t f = nl->edges[nl->edge_offset[g] + nl->nfi[g] + k];
-            if (f >= G || level[f] <= level[g]) {
-                set_msg(msg, len, "gate %llu: fan-out %llu not on a higher level", g, f);
+            if (nl->po[g] > 1) {
+                set_msg(msg, len, "gate %llu: po must be 0 or 1", g);
                 return PDF_EINVAL;
+            }
+            if ((t == PDF_INPT) != (g < npi)) {
+                set_msg(msg, len, "gate %llu: INPT gates must be exactly level 0", g);
+                return PDF_EINVAL;
+            }
+            if (t == PDF_INPT ? nfi != 0 : (nfi == 0 || nfi > 255)) {
+                set_msg(msg, len, "gate %llu: bad fan-in count %llu", g, nfi);
+                return PDF_EINVAL;
+            }
+            const uint64_t end = nl->edge_offset[g] + (uint64_t)nfi + nfo;
+            if (end > nl->n_edges || end < nl->edge_offset[g]) {
+                set_msg(msg, len, "gate %llu: edge range out of bounds", g);
+                return PDF_EINVAL;
+            }
+            if ((uses += (uint64_t)nfi + nfo) >= 0xFFFFFFFFull) {  // lists that overlap can add up to more than n_edges
+                set_msg(msg, len, "too many edges (%llu)", uses);
+                return PDF_EINVAL;
+            }
+            const uint32_t *e = nl->edges + nl->edge_offset[g];
+            for (uint32_t j = 0; j < nfi; j++) {
+                if (e[j] >= lo) {
+                    set_msg(msg, len, "gate %llu: fan-in %llu not on a lower level", g, e[j]);
+                    return PDF_EINVAL;
+                }
+                start[e[j] + 1]++;
+            }
+            for (uint32_t k = 0; k < nfo; k++) {
+                const uint32_t f = e[nfi + k];
+                if (f >= G || f < hi) {
+                    set_msg(msg, len, "gate %llu: fan-out %llu not on a higher level", g, f);
+                    return PDF_EINVAL;
+                }
             }
         }
     }
     // Fan-out lists must be the transpose of the fan-in lists (as multisets).
-    std::vector<uint64_t> cnt(G, 0);
     for (uint32_t g = 0; g < G; g++)
-        for (uint32_t j = 0; j < nl->nfi[g]; j++) cnt[nl->edges[nl->edge_offset[g] + j]]++;
-    for (uint32_t g = 0; g < G; g++)
-        if (cnt[g] != nl->nfo[g]) {
+        if (start[g + 1] != nl->nfo[g]) {
             set_msg(msg, len, "gate %llu: fan-out count %llu differs from its fan-in uses", g,
                     nl->nfo[g]);
             return PDF_EINVAL;
         }
     // Multiset comparison: the consumers of each gate (transposed from the
     // fan-in lists by a counting sort, hence ascending) against its fan-out
-    // list, sorted.  Linear in the edges apart from sorting each list.
-    {
-        std::vector<uint64_t> start(G + 1, 0);
-        for (uint32_t g = 0; g < G; g++) start[g + 1] = start[g] + cnt[g];
-        std::vector<uint32_t> cons(start[G]);
-        std::vector<uint64_t> fill(start.begin(), start.end() - 1);
-        for (uint32_t g = 0; g < G; g++)
-            for (uint32_t j = 0; j < nl->nfi[g]; j++) cons[fill[nl->edges[nl->edge_offset[g] + j]]++] = g;
-        std::vector<uint32_t> fo;
-        for (uint32_t g = 0; g < G; g++) {
-            const uint32_t *e = nl->edges + nl->edge_offset[g] + nl->nfi[g];
-            fo.assign(e, e + nl->nfo[g]);
-            std::sort(fo.begin(), fo.end());
-            if (!std::equal(fo.begin(), fo.end(), cons.begin() + start[g])) {
-                set_msg(msg, len, "fan-out lists are not the transpose of the fan-in lists (gate %llu)", g);
-                return PDF_EINVAL;
-            }
+    // list, sorted when it does not ascend already.
+    for (uint32_t g = 0; g < G; g++) start[g + 1] += start[g];
+    std::vector<uint32_t> cons(start[G]), fill(start.begin(), start.end() - 1), fo;
+    for (uint32_t g = 0; g < G; g++) {
+        const uint32_t *e = nl->edges + nl->edge_offset[g];
+        for (uint32_t j = 0; j < nl->nfi[g]; j++) cons[fill[e[j]]++] = g;
+    }
+    for (uint32_t g = 0; g < G; g++) {
+        const uint32_t *e = nl->edges + nl->edge_offset[g] + nl->nfi[g], *want = cons.data() + start[g];
+        if (std::equal(e, e + nl->nfo[g], want)) continue;
+        fo.assign(e, e + nl->nfo[g]);
+        std::sort(fo.begin(), fo.end());
+        if (!std::equal(fo.begin(), fo.end(), want)) {
+            set_msg(msg, len, "fan-out lists are not the transpose of the fan-in lists (gate %llu)", g);
+            return PDF_EINVAL;
         }
     }
     set_msg(msg, len, "ok");
@@ -421,6 +496,18 @@ pdf_status build_segments(pdf_circuit *c, const pdf_netlist *nl, uint32_t N) {
 
 }  // namespace
 
+namespace {
+
+// Column block of the reduced walk of a circuit whose tile is bw words, by
+// the mean width of its levels above the inputs.  Narrow levels leave most
+// warps of the lane kernel without a gate.
+uint32_t reduced_tile(uint32_t bw, uint64_t mean_width) {
+    if (lane_tile(bw) && mean_width < 512) return 4;
+    return bw;
+}
+
+}  // namespace
+
 extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circuit_opts *opts,
                                          pdf_circuit **out) {
     if (!out) return PDF_EINVAL;
@@ -464,31 +551,6 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     }
     for (uint32_t l = 0; l < L; l++)
         inf.max_level_width = std::max(inf.max_level_width, nl->level_offsets[l + 1] - nl->level_offsets[l]);
-
-    // Canonical edge array: each gate's fan-ins then fan-outs, gates in id
-    // order, so that a run of gates owns one contiguous slice (staged into
-    // shared memory by a bulk copy).  Padded so 16-byte rounding stays inside.
-    std::vector<uint32_t> edges;
-    std::vector<uint64_t> eoff(G + 1);
-    edges.reserve(nl->n_edges + 8);
-    for (uint32_t g = 0; g < G; g++) {
-        eoff[g] = edges.size();
-        const uint32_t *e = nl->edges + nl->edge_offset[g];
-        edges.insert(edges.end(), e, e + nl->nfi[g] + nl->nfo[g]);
-    }
-    eoff[G] = edges.size();
-    while (edges.size() % 4) edges.push_back(0);
-    for (int i = 0; i < 4; i++) edges.push_back(0);
-
-    std::vector<GateRec> recs(G);
-    for (uint32_t g = 0; g < G; g++) {
-        GateRec &r = recs[g];
-        std::memset(&r, 0, sizeof r);
-        r.w[0] = make_rec_header(nl->type[g], nl->po[g], nl->nfi[g], o.mark_mode >= PDF_MARK_FIXED_ROBUST);
-        r.w[1] = nl->nfo[g];
-        r.w[2] = (uint32_t)eoff[g];  // w[3..6]: source words, set with the launch plan below
-        r.w[7] = nl->nfi[g] ? edges[eoff[g]] : 0;
-    }
 
     // Launch plan: CTAs of `threads` threads own `bw` words of pairs; two
     // CTAs per SM share its shared memory.
@@ -535,226 +597,49 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     } else {
         c->bw = max_words / 8 >= 2ull * sms ? 8u : 4u;
     }
-    const bool lanes = lane_tile(c->bw);
-    if (lanes) {
-        // The lane kernel reads every fan-in from its plane row: source words
-        // are the fan-in ids themselves, flagged SRC_ZERO when the fan-in is
-        // a killed gate (S0 whatever its inputs); a gate writes its rows
-        // (RF_SPILL) only when some gate reads them.
-        std::vector<uint8_t> read(G, 0);
-        for (uint32_t g = 0; g < G; g++)
-            for (uint32_t q = 0; q < nl->nfi[g]; q++) {
-                const uint32_t f = edges[eoff[g] + q];
-                const bool zero = q < kInlineFanins && (recs[f].w[0] & RF_KILL);
-                if (q < kInlineFanins) recs[g].w[3 + q] = f | (zero ? SRC_ZERO : 0u);
-                if (!zero) read[f] = 1;
-            }
-        for (uint32_t g = 0; g < G; g++)
-            if (read[g]) recs[g].w[0] |= RF_SPILL;
+    const bool fixed = o.mark_mode >= PDF_MARK_FIXED_ROBUST;
+    PlanOpts po;
+    po.bw = c->bw;
+    po.threads = o.threads;
+    po.regs = forward_kernel_regs((int)po.bw, o.mark_mode);
+    po.smem_block = prop.sharedMemPerBlockOptin;
+    po.smem_sm = prop.sharedMemPerMultiprocessor;
+    // Canonical edge array: each gate's fan-ins then fan-outs, gates in id
+    // order, so that a run of gates owns one contiguous slice (staged into
+    // shared memory by a bulk copy).
+    const NetPlan net = net_plan(nl, fixed);
+    LaunchPlan full, red;
+    // The plan of the whole netlist is built on a second thread where there
+    // is enough of it, beside the reduced netlist and its plan here.
+    std::future<pdf_status> other;
+    if (G >= 16384 && o.seg_len <= 1) {
+        try {
+            other = std::async(std::launch::async, [&net, po, &full] { return build_plan(net, po, full); });
+        } catch (const std::system_error &) {  // no thread to be had
+        }
     }
-    const uint32_t max_threads = lanes ? lane_threads(c->bw) : (c->bw >= 8 ? 512 : 1024);
-    uint32_t threads_default = 512;  // set from the piece size below
-    auto al = [](size_t x) { return (x + 127) & ~(size_t)127; };
-    const uint32_t bm_words = (G + 31) / 32;
-    // Pieces (the kernels' unit of staging and of synchronisation), sized
-    // from the widest level above the inputs (the inputs' level, often the
-    // widest, just splits into more pieces): runs of one level, <= cap gates,
-    // edge slice <= ecap words.
-    uint32_t widest = 1;
-    for (uint32_t l = 1; l < L; l++) widest = std::max(widest, nl->level_offsets[l + 1] - nl->level_offsets[l]);
-    if (L == 1) widest = inf.max_level_width;
-    c->cap = lanes ? 0u : std::min<uint32_t>(512, (widest + 31) & ~31u);
-    // one thread per gate of a piece plus two warps that have none: they
-    // issue the next piece's far-row copies
-    threads_default = lanes ? lane_threads(c->bw) : std::min<uint32_t>(max_threads, c->cap + 64);
-    c->threads = o.threads ? std::min(o.threads, max_threads) : threads_default;
-    // a block size given by the caller also bounds the pieces: threads - 64
-    // gates, so two warps stay free for the far-row copies
-    if (!lanes && o.threads && c->threads >= 128) c->cap = std::min(c->cap, (c->threads - 64) & ~31u);
-    // CTAs per SM that the registers allow for this block size (at most 4);
-    // the dynamic shared memory of the forward kernels is then an equal share
-    // of the SM, less 1 KiB per CTA the system keeps and 1 KiB for the
-    // kernels' static variables (the batched kernel keeps its arguments there).
-    {
-        const int regs = forward_kernel_regs(c->bw, c->mark_mode);
-        if (regs <= 0) {
-            delete c;
-            return PDF_ECUDA;
+    pdf_status pst = PDF_OK;
+    if (!other.valid()) pst = build_plan(net, po, full);
+    // The reduced netlist (single nets; segments are listed over every net).
+    NetPlan rnet;
+    if (pst == PDF_OK && o.seg_len <= 1) {
+        const NetFacts facts = net_facts(net, fixed);
+        if (facts.n_needed <= (uint64_t)G * 9 / 10) {
+            rnet = reduce_net(net, facts);
+            const uint32_t rl = rnet.n_levels();
+            PlanOpts ro = po;
+            ro.bw = reduced_tile(c->bw, rl > 1 ? (rnet.n_gates() - rnet.level_off[1]) / (rl - 1) : 0);
+            if (ro.bw != po.bw) ro.regs = forward_kernel_regs((int)ro.bw, o.mark_mode);
+            pst = build_plan(rnet, ro, red);
         }
-        const uint32_t warps = (c->threads + 31) / 32;
-        const uint32_t warp_regs = ((uint32_t)regs * 32 + 255) & ~255u;
-        uint32_t occ = std::min<uint32_t>(65536 / (warps * warp_regs), 2048 / (warps * 32));
-        c->occ = std::max<uint32_t>(1, std::min<uint32_t>(occ, 4));
     }
-    const size_t budget = std::min<size_t>((size_t)prop.sharedMemPerBlockOptin,
-                                           (size_t)prop.sharedMemPerMultiprocessor / c->occ - 1024) -
-                          1024;
-    c->ecap = 2048;
-    std::vector<Piece> pieces;
-    std::vector<uint32_t> far_ids;
-    if (lanes) {
-        // The lane kernel keeps on chip two buffers of staged gate records
-        // and the column block's mark bitmap (in global memory when it does
-        // not fit); its pieces are runs of one level of <= cap gates: 2 x
-        // kLaneRecs when those buffers fit beside a shared-memory bitmap (a
-        // barrier per piece, so wide levels take half as many), else
-        // kLaneRecs.
-        const size_t bm_bytes = (size_t)bm_words * 4;
-        c->cap = kLaneRecs;
-        if (widest > kLaneRecs &&
-            2 * 2 * (size_t)kLaneRecs * sizeof(GateRec) + al(bm_bytes) + 2048 <= budget)
-            c->cap = 2 * kLaneRecs;
-        for (uint32_t l = 0; l < L; l++)
-            for (uint32_t a = nl->level_offsets[l]; a < nl->level_offsets[l + 1]; a += c->cap) {
-                Piece p{};
-                p.a = a;
-                p.b = std::min(a + c->cap, nl->level_offsets[l + 1]);
-                p.level = l;
-                pieces.push_back(p);
-            }
-        c->n_pieces = (uint32_t)pieces.size();
-        const size_t rec_bytes = 2 * (size_t)c->cap * sizeof(GateRec);
-        c->off_rec = 0;
-        c->off_bm = (uint32_t)rec_bytes;
-        c->bm_shared = rec_bytes + bm_bytes + 2048 <= budget ? 1u : 0u;
-        c->fwd_smem = rec_bytes + (c->bm_shared ? al(bm_bytes) : 0);
-        c->chain = G;
-        while (far_ids.size() < 4) far_ids.push_back(0);
-    } else {
-        auto f4 = [](uint64_t x) { return x & ~(uint64_t)3; };
-        auto c4 = [](uint64_t x) { return (x + 3) & ~(uint64_t)3; };
-        for (uint32_t l = 0; l < L; l++) {
-            const uint32_t s0 = nl->level_offsets[l], e0 = nl->level_offsets[l + 1];
-            for (uint32_t a = s0; a < e0;) {
-                uint32_t b = a + 1;
-                while (b < e0 && b - a < c->cap && c4(eoff[b + 1]) - f4(eoff[a]) <= c->ecap) b++;
-                Piece p{};
-                p.a = a;
-                p.b = b;
-                p.level = l;
-                if (c4(eoff[b]) - f4(eoff[a]) <= c->ecap) {
-                    p.ea = (uint32_t)f4(eoff[a]);
-                    p.eb = (uint32_t)c4(eoff[b]);
-                } else {
-                    p.ea = p.eb = 0xFFFFFFFFu;  // one gate with a huge edge list: read in place
-                }
-                pieces.push_back(p);
-                a = b;
-            }
-        }
-        c->n_pieces = (uint32_t)pieces.size();
-        if (c->n_pieces > 65536) {
-            delete c;
-            return PDF_ENOTSUP;
-        }
-        // Far fan-ins of piece i (ring of R slots): fan-ins 0..3 of its gates
-        // below b_i - R.  Those below a_{i-1} (complete when piece i - 1 starts)
-        // go to the piece's deduplicated far list, up to `limit` entries; the rest
-        // are read from their plane rows.  Fills the source words w[3..6].
-        auto far_lists = [&](uint32_t R, uint32_t limit) -> uint32_t {
-            uint32_t worst = 0;
-            far_ids.clear();
-            std::vector<uint32_t> seen(G, 0xFFFFFFFFu);  // gate -> slot in the current piece's list
-            std::vector<uint32_t> list;
-            for (size_t i = 0; i < pieces.size(); i++) {
-                Piece &p = pieces[i];
-                const uint32_t lo = p.b > R ? p.b - R : 0;
-                const uint32_t done = i ? pieces[i - 1].a : 0;
-                list.clear();
-                for (uint32_t g = p.a; g < p.b; g++) {
-                    const uint32_t nq = std::min<uint32_t>(nl->nfi[g], kInlineFanins);
-                    for (uint32_t q = 0; q < nq; q++) {
-                        const uint32_t f = edges[eoff[g] + q];
-                        uint32_t sw = f & (R - 1);
-                        if (f < lo) {
-                            sw = SRC_PLANE | f;
-                            if (f < done) {
-                                if (seen[f] == 0xFFFFFFFFu && list.size() < limit) {
-                                    seen[f] = (uint32_t)list.size();
-                                    list.push_back(f);
-                                }
-                                if (seen[f] != 0xFFFFFFFFu) sw = SRC_FAR | seen[f];
-                            }
-                        }
-                        recs[g].w[3 + q] = sw;
-                        if (sw & SRC_PLANE || sw & SRC_FAR) recs[f].w[0] |= RF_SPILL;
-                    }
-                    for (uint32_t q = kInlineFanins; q < nl->nfi[g]; q++) {  // read from edges[] at run time
-                        const uint32_t f = edges[eoff[g] + q];
-                        if (f < lo) recs[f].w[0] |= RF_SPILL;
-                    }
-                }
-                for (uint32_t f : list) seen[f] = 0xFFFFFFFFu;
-                worst = std::max<uint32_t>(worst, (uint32_t)list.size());
-                p.far_off = (uint32_t)far_ids.size();
-                p.far_n = (uint32_t)list.size();
-                far_ids.insert(far_ids.end(), list.begin(), list.end());
-                // lists start on 16-byte boundaries: the kernel stages the next
-                // piece's list by a bulk copy located from this piece's fields
-                while (far_ids.size() & 3) far_ids.push_back(0);
-            }
-            for (size_t i = 0; i < pieces.size(); i++) pieces[i].nfar_n = i + 1 < pieces.size() ? pieces[i + 1].far_n : 0;
-            return worst;
-        };
-        // Shared memory of k_forward: 2 record buffers; one region holding the
-        // reverse pass's 2 edge buffers or the forward pass's 2 far buffers;
-        // bitmap; piece bits; barriers; the ring.  The ring: the largest power of
-        // two (>= cap, <= 2 * n_gates) that leaves room for far lists of 64
-        // entries; the far lists then get the rest of the budget.
-        const size_t rec_bytes = al(2 * (size_t)c->cap * sizeof(GateRec));
-        const size_t bm_bytes = (size_t)bm_words * 4 <= 16384 ? al((size_t)bm_words * 4) : 0;
-        const size_t fixed = rec_bytes + bm_bytes + al(((size_t)c->n_pieces + 31) / 32 * 4) + 128;
-        const size_t edge_bytes = 2 * (size_t)c->ecap * 4;
-        const size_t far_entry = (size_t)2 * 3 * c->bw * 4;  // one far slot in both buffers, 3 planes
-        uint32_t rmin = 32;
-        while (rmin < c->cap) rmin *= 2;
-        uint32_t rmax = rmin;
-        while ((uint64_t)rmax < 2 * (uint64_t)G && fixed + (size_t)rmax * 2 * c->bw * 12 <= budget) rmax *= 2;
-        // the ring's memory also holds the reverse pass's row staging buffers
-        const size_t rows_bytes = (size_t)2 * c->cap * 2 * c->bw * 4;
-        auto ring_bytes = [&](size_t R) { return std::max(R * c->bw * 12, rows_bytes); };
-        // The largest ring that fits wins: a smaller ring with longer far lists
-        // was measured slower (1M gates, 5,000-gate levels: 116.8 against 109.9
-        // ms) although it leaves fewer fan-ins to plane-row reads.
-        // far region (far rows of two pieces, or the reverse pass's edges) and
-        // the two staged far-id lists, for lists of n entries
-        auto far_bytes = [&](size_t n) { return al(std::max(edge_bytes, n * far_entry)) + al(2 * n * 4); };
-        uint32_t ring = 0;
-        for (uint32_t R = rmax; R >= rmin && !ring; R /= 2)
-            if (fixed + far_bytes(64) + ring_bytes(R) <= budget) ring = R;
-        if (!ring) {
-            delete c;
-            return PDF_ENOTSUP;
-        }
-        const size_t far_room = budget - fixed - ring_bytes(ring);
-        uint32_t far_limit = (uint32_t)std::min<size_t>(kMaxFar, far_room / (far_entry + 8)) & ~3u;
-        while (far_limit > 64 && far_bytes(far_limit) > far_room) far_limit -= 4;
-        const uint32_t farcap = std::max<uint32_t>(4, (far_lists(ring, far_limit) + 3) & ~3u);
-        while (far_ids.size() < 4) far_ids.push_back(0);
-        c->ring = ring;
-        c->farcap = farcap;
-        size_t off = 0;
-        c->off_rec = (uint32_t)off;
-        off += rec_bytes;
-        c->off_edge = (uint32_t)off;
-        off += al(std::max(edge_bytes, farcap * far_entry));
-        c->off_fid = (uint32_t)off;
-        off += al(2 * (size_t)farcap * 4);
-        c->bm_shared = bm_bytes ? 1u : 0u;
-        c->off_bm = (uint32_t)off;
-        off += bm_bytes;
-        c->off_pbits = (uint32_t)off;
-        off += al(((size_t)c->n_pieces + 31) / 32 * 4);
-        c->off_mbar = (uint32_t)off;
-        off += 128;
-        c->off_ring = (uint32_t)off;
-        // reverse pass: ring2 and the row staging buffers [2][cap][2][bw] share
-        // the ring's memory
-        uint32_t ring2 = 0;
-        for (uint32_t r = 1; (size_t)r * c->bw * 4 + rows_bytes <= ring_bytes(ring); r *= 2) ring2 = r;
-        c->ring2 = ring2;
-        c->fwd_smem = off + ring_bytes(ring);
-        c->chain = c->n_pieces;
+    if (other.valid()) {
+        const pdf_status fst = other.get();
+        if (fst != PDF_OK) pst = fst;
+    }
+    if (pst != PDF_OK) {
+        delete c;
+        return pst;
     }
     // nets one pair may mark in the cover: as many as its shared memory holds
     c->hash_cap = 4096;
@@ -765,44 +650,30 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     auto fail = [&](pdf_status st2) {
         c->segs.release();
         c->seg_off.release();
-        c->rec.release();
-        c->edges.release();
-        c->level_off.release();
-        c->pieces.release();
-        c->far.release();
-        c->err.release();
+        c->mem.release();
         delete c;
         return st2;
     };
-    if (c->rec.ensure(sizeof(GateRec) * G) != cudaSuccess ||
-        c->edges.ensure(sizeof(uint32_t) * edges.size()) != cudaSuccess ||
-        c->level_off.ensure(sizeof(uint32_t) * (L + 1)) != cudaSuccess ||
-        c->pieces.ensure(sizeof(Piece) * pieces.size()) != cudaSuccess ||
-        c->far.ensure(sizeof(uint32_t) * far_ids.size()) != cudaSuccess || c->err.ensure(16) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return fail(PDF_ENOMEM);
+    // One device block: the error word, then both plans' arrays.
+    {
+        PlanUpload up;
+        up.add(nullptr, 16);
+        const PlanOffsets fo = up.add_plan(net, full);
+        const PlanOffsets ro = rnet.n_gates() ? up.add_plan(rnet, red) : PlanOffsets{};
+        if (c->mem.ensure(up.bytes) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return fail(PDF_ENOMEM);
+        }
+        if (!up.copy(c->mem.as<unsigned char>())) {
+            (void)cudaGetLastError();
+            return fail(PDF_ECUDA);
+        }
+        c->err = c->mem.as<uint32_t>();
+        c->full.bind(full, net, c->mem.as<unsigned char>(), fo);
+        if (rnet.n_gates()) c->red.bind(red, rnet, c->mem.as<unsigned char>(), ro);
     }
-    if (cudaMemcpy(c->rec.p, recs.data(), sizeof(GateRec) * G, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(c->edges.p, edges.data(), sizeof(uint32_t) * edges.size(), cudaMemcpyHostToDevice) !=
-            cudaSuccess ||
-        cudaMemcpy(c->level_off.p, nl->level_offsets, sizeof(uint32_t) * (L + 1), cudaMemcpyHostToDevice) !=
-            cudaSuccess ||
-        cudaMemcpy(c->pieces.p, pieces.data(), sizeof(Piece) * pieces.size(), cudaMemcpyHostToDevice) !=
-            cudaSuccess ||
-        cudaMemcpy(c->far.p, far_ids.data(), sizeof(uint32_t) * far_ids.size(), cudaMemcpyHostToDevice) !=
-            cudaSuccess ||
-        cudaMemset(c->err.p, 0, 16) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return fail(PDF_ECUDA);
-    }
-    c->dc.rec = c->rec.as<GateRec>();
-    c->dc.edges = c->edges.as<uint32_t>();
-    c->dc.level_off = c->level_off.as<uint32_t>();
-    c->dc.n_gates = G;
-    c->dc.n_levels = L;
-    c->dc.n_pi = inf.n_pi;
     inf.tile_words = c->bw;
-    inf.threads = c->threads;
+    inf.threads = c->full.threads;
     inf.max_pairs = o.max_pairs ? o.max_pairs : 65536;
     if (o.seg_len > 1) {
         const pdf_status sst = build_segments(c, nl, o.seg_len);
@@ -813,8 +684,7 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     }
     inf.seg_len = c->seg_len;
     inf.n_segments = c->n_first();
-    inf.device_bytes = c->rec.bytes + c->edges.bytes + c->level_off.bytes + c->pieces.bytes + c->far.bytes +
-                       c->segs.bytes + c->seg_off.bytes;
+    inf.device_bytes = c->mem.bytes + c->segs.bytes + c->seg_off.bytes;
     *out = c;
     return PDF_OK;
 }
@@ -834,12 +704,7 @@ extern "C" void pdf_circuit_destroy(pdf_circuit *c) {
     if (!c) return;
     DeviceGuard dg(c->device);
     c->stage.release();
-    c->rec.release();
-    c->edges.release();
-    c->level_off.release();
-    c->pieces.release();
-    c->far.release();
-    c->err.release();
+    c->mem.release();
     c->segs.release();
     c->seg_off.release();
     delete c;
@@ -1029,14 +894,21 @@ pdf_status check_pairs(const pdf_circuit *c, const pdf_pairs *pr, uint64_t pair_
     return PDF_OK;
 }
 
-// Sizes the workspace for W words of pairs.
-pdf_status ensure_ws(pdf_circuit *c, Workspace &ws, uint64_t W, bool need_planes) {
-    const uint64_t n_blocks = (W + c->bw - 1) / c->bw;
-    const uint64_t bm_words = (c->info.n_gates + 31) / 32;
+// Slots of the spill cover for circuits of n gates: 2 x n u128 each, up to
+// 16 MiB in all, at least one.
+uint32_t spill_slots(uint64_t n, uint64_t *slot) {
+    *slot = 2 * n * 16;
+    return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(16, (16ull << 20) / *slot));
+}
+
+// Sizes the workspace for a walk of plan p over W words of pairs.
+pdf_status ensure_ws(pdf_circuit *c, const Plan &p, Workspace &ws, uint64_t W, bool need_planes) {
+    const uint64_t n_blocks = (W + p.bw - 1) / p.bw;
+    const uint64_t bm_words = (p.n_gates + 31) / 32;
     PDF_CUDA(ws.nzb.ensure(n_blocks * bm_words * 4));
     PDF_CUDA(ws.maxlvl.ensure(n_blocks * 4));
-    if (lane_tile(c->bw)) {  // the cover's bitmaps per kLaneCoverWords words of a column block
-        const uint64_t nf = c->bw / kLaneCoverWords;
+    if (lane_tile(p.bw)) {  // the cover's bitmaps per kLaneCoverWords words of a column block
+        const uint64_t nf = p.bw / kLaneCoverWords;
         PDF_CUDA(ws.nzb_fine.ensure(nf * n_blocks * bm_words * 4));
         PDF_CUDA(ws.maxlvl_fine.ensure(nf * n_blocks * 4));
     }
@@ -1045,15 +917,13 @@ pdf_status ensure_ws(pdf_circuit *c, Workspace &ws, uint64_t W, bool need_planes
     const uint64_t list = std::min<uint64_t>(W * 32, 2 * std::max<uint64_t>(c->n_first(), c->info.n_gates));
     PDF_CUDA(ws.active_list.ensure(list * 4));
     // A pair can mark more nets than the cover's table holds only when the
-    // circuit has more gates than that; its count then goes through the
-    // spill cover, whose slots of 2 x n_gates u128 take up to 16 MiB (at
-    // least one slot).
-    if (c->info.n_gates > c->hash_cap) {
-        const uint64_t slot = 2 * (uint64_t)c->info.n_gates * 16;
-        const uint32_t slots = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(16, (16ull << 20) / slot));
+    // walk has more gates than that; its count then goes through the spill
+    // cover.
+    if (p.n_gates > c->hash_cap) {
+        uint64_t slot;
+        const uint32_t slots = spill_slots(p.n_gates, &slot);
         PDF_CUDA(ws.over_list.ensure(list * 4));
         PDF_CUDA(ws.spill.ensure(slots * slot));
-        ws.spill_slots = slots;
     }
     if (c->seg_len > 1) {
         // (net, pair) entries: at most N per first pair of a segment, two per
@@ -1066,40 +936,42 @@ pdf_status ensure_ws(pdf_circuit *c, Workspace &ws, uint64_t W, bool need_planes
             ws.seg_first_mask = cap - 1;
         }
     }
-    if (need_planes) {
-        const uint64_t ld = n_blocks * c->bw;
-        if (ws.plane_ld < ld || !ws.planes.p) {
-            PDF_CUDA(ws.planes.ensure(3 * (uint64_t)c->info.n_gates * ld * 4));
-            ws.plane_ld = ld;
-        }
-    }
+    if (need_planes) PDF_CUDA(ws.planes.ensure(3 * (uint64_t)p.n_gates * n_blocks * p.bw * 4));
     return PDF_OK;
 }
 
-FwdArgs base_fwd(pdf_circuit *c, uint64_t n_pairs) {
+// The workspace's planes for a walk of plan p over W words (after ensure_ws).
+void use_ws_planes(FwdArgs &a, const Plan &p, const Workspace &ws, uint64_t W) {
+    a.ld = (W + p.bw - 1) / p.bw * p.bw;
+    a.V = ws.planes.as<uint32_t>();
+    a.T = a.V + p.n_gates * a.ld;
+    a.M = a.T + p.n_gates * a.ld;
+}
+
+FwdArgs base_fwd(pdf_circuit *c, const Plan &p, uint64_t n_pairs) {
     FwdArgs a{};
-    a.c = c->dc;
-    a.pieces = c->pieces.as<Piece>();
-    a.n_pieces = c->n_pieces;
-    a.cap = c->cap;
-    a.ecap = c->ecap;
+    a.c = p.dc;
+    a.pieces = p.pieces;
+    a.n_pieces = p.n_pieces;
+    a.cap = p.cap;
+    a.ecap = p.ecap;
     a.n_pairs = n_pairs;
     a.W = (uint32_t)((n_pairs + 31) / 32);
     a.store_all = 1;
-    a.bm_words = (c->info.n_gates + 31) / 32;
-    a.bm_shared = c->bm_shared;
-    a.far_ids = c->far.as<uint32_t>();
-    a.farcap = c->farcap;
-    a.ring_gates = c->ring;
-    a.ring2_gates = c->ring2;
-    a.off_ring = c->off_ring;
-    a.off_rec = c->off_rec;
-    a.off_edge = c->off_edge;
-    a.off_fid = c->off_fid;
-    a.off_bm = c->off_bm;
-    a.off_pbits = c->off_pbits;
-    a.off_mbar = c->off_mbar;
-    a.err = c->err.as<uint32_t>();
+    a.bm_words = (p.n_gates + 31) / 32;
+    a.bm_shared = p.bm_shared;
+    a.far_ids = p.far_ids;
+    a.farcap = p.farcap;
+    a.ring_gates = p.ring;
+    a.ring2_gates = p.ring2;
+    a.off_ring = p.off_ring;
+    a.off_rec = p.off_rec;
+    a.off_edge = p.off_edge;
+    a.off_fid = p.off_fid;
+    a.off_bm = p.off_bm;
+    a.off_pbits = p.off_pbits;
+    a.off_mbar = p.off_mbar;
+    a.err = c->err;
     a.wait_polls = c->wait_polls;
     return a;
 }
@@ -1109,28 +981,28 @@ FwdArgs base_fwd(pdf_circuit *c, uint64_t n_pairs) {
 // is reported by the call that met it and by no later one.
 pdf_status take_circuit_err(pdf_circuit *c, cudaStream_t cs) {
     unsigned int e = 0;
-    PDF_CUDA(cudaMemcpyAsync(&e, c->err.p, sizeof e, cudaMemcpyDeviceToHost, cs));
+    PDF_CUDA(cudaMemcpyAsync(&e, c->err, sizeof e, cudaMemcpyDeviceToHost, cs));
     PDF_CUDA(cudaStreamSynchronize(cs));
     if (e) {
-        PDF_CUDA(cudaMemsetAsync(c->err.p, 0, sizeof e, cs));
+        PDF_CUDA(cudaMemsetAsync(c->err, 0, sizeof e, cs));
         PDF_CUDA(cudaStreamSynchronize(cs));
     }
     return err_status(e);
 }
 
-CoverArgs base_cover(pdf_circuit *c, Workspace &ws, const uint32_t *M, uint64_t ld, uint64_t n_pairs,
+CoverArgs base_cover(pdf_circuit *c, const Plan &p, Workspace &ws, const uint32_t *M, uint64_t ld, uint64_t n_pairs,
                      uint32_t pair_base, const uint32_t *fx, const uint32_t *fy, DevAcc *acc) {
     CoverArgs a{};
-    a.c = c->dc;
+    a.c = p.dc;
     a.M = M;
     a.ld = ld;
-    // a lane circuit's cover reads bitmaps per 8 words of its column blocks
+    // a lane walk's cover reads bitmaps per 8 words of its column blocks
     // (fewer candidate nets per pair than the whole block's)
-    const bool fine = lane_tile(c->bw);
+    const bool fine = lane_tile(p.bw);
     a.nzb = fine ? ws.nzb_fine.as<uint32_t>() : ws.nzb.as<uint32_t>();
     a.blk_maxlvl = fine ? ws.maxlvl_fine.as<uint32_t>() : ws.maxlvl.as<uint32_t>();
-    a.bm_words = (c->info.n_gates + 31) / 32;
-    a.bw = fine ? kLaneCoverWords : c->bw;
+    a.bm_words = (p.n_gates + 31) / 32;
+    a.bw = fine ? kLaneCoverWords : p.bw;
     a.first_x = fx;
     a.first_y = fy;
     a.n_pairs = n_pairs;
@@ -1142,7 +1014,8 @@ CoverArgs base_cover(pdf_circuit *c, Workspace &ws, const uint32_t *M, uint64_t 
     a.hash_cap = c->hash_cap;
     a.over_list = ws.over_list.as<uint32_t>();
     a.spill = ws.spill.as<unsigned char>();
-    a.spill_slots = ws.spill_slots;
+    uint64_t slot;
+    a.spill_slots = p.n_gates > c->hash_cap ? spill_slots(p.n_gates, &slot) : 0;
     a.seg = c->seg_args();
     if (c->seg_len > 1) {
         a.seg_first = ws.seg_first.as<unsigned long long>();
@@ -1210,30 +1083,31 @@ namespace {
 pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, uint64_t pair_base,
                              const pdf_outputs *out, cudaStream_t cs) {
     const uint64_t n = pr->n_pairs, W = (n + 31) / 32, G = c->info.n_gates;
+    // with no plane asked for, only what the marks depend on is evaluated,
+    // and only the rows read back are written
+    const bool planes = out && (out->sim_v || out->sim_t || out->mark);
+    const Plan &p = planes ? c->full : c->lean();
     const bool direct = out && out->on_device && planes_fit(c, W, out->ld, {out->sim_v, out->sim_t, out->mark});
-    pdf_status st = ensure_ws(c, s->ws, W, !direct);
+    pdf_status st = ensure_ws(c, p, s->ws, W, !direct);
     if (st != PDF_OK) return st;
     const uint32_t *pv, *pt;
     uint64_t pld;
     st = stage_pairs(c, s->ws, pr, &pv, &pt, &pld, cs);
     if (st != PDF_OK) return st;
 
-    FwdArgs a = base_fwd(c, n);
+    FwdArgs a = base_fwd(c, p, n);
     a.pi_v = pv;
     a.pi_t = pt;
     a.pi_ld = pld;
-    // with no plane asked for, only the rows read back are written
-    a.store_all = out && (out->sim_v || out->sim_t || out->mark) ? 1u : 0u;
+    a.store_all = planes ? 1u : 0u;
+    a.in_pieces = planes ? 0u : p.in_pieces;
     if (direct) {
         a.V = out->sim_v;
         a.T = out->sim_t;
         a.M = out->mark;
         a.ld = out->ld;
     } else {
-        a.ld = s->ws.plane_ld;
-        a.V = s->ws.planes.as<uint32_t>();
-        a.T = a.V + G * a.ld;
-        a.M = a.T + G * a.ld;
+        use_ws_planes(a, p, s->ws, W);
     }
     a.nzb = s->ws.nzb.as<uint32_t>();
     a.blk_maxlvl = s->ws.maxlvl.as<uint32_t>();
@@ -1247,21 +1121,21 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     a.err = &acc->err;
     s->pe = nullptr;
     if (s->profiling) {
-        ProfEvents p{};
+        ProfEvents pe{};
         if (!s->pool.empty()) {
-            p = s->pool.back();
+            pe = s->pool.back();
             s->pool.pop_back();
         } else {
-            for (auto &e : p.ev) PDF_CUDA(cudaEventCreate(&e));
+            for (auto &e : pe.ev) PDF_CUDA(cudaEventCreate(&e));
         }
-        s->prof.push_back(p);
+        s->prof.push_back(pe);
         s->pe = &s->prof.back();
         PDF_CUDA(cudaEventRecord(s->pe->ev[0], cs));
     }
     // the forward kernel also clears the batch count and the cover's active pairs
     a.acc = acc;
     a.active = s->ws.active.as<uint32_t>();
-    PDF_CUDA(launch_forward(a, FWD_FUSED, c->mark_mode, c->bw, c->threads, c->fwd_smem, cs));
+    PDF_CUDA(launch_forward(a, FWD_FUSED, c->mark_mode, p.bw, p.threads, p.fwd_smem, cs));
     if (c->seg_len > 1) {
         SegMergeArgs sm{};
         sm.seg = c->seg_args();
@@ -1270,12 +1144,12 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
         sm.ld = a.ld;
         sm.nzb = a.nzb;
         sm.bm_words = a.bm_words;
-        sm.bw = c->bw;
+        sm.bw = p.bw;
         sm.W = (uint32_t)W;
         sm.pair_base = (uint32_t)pair_base;
         sm.first_x = s->first_x.as<uint32_t>();
         sm.first_y = s->first_y.as<uint32_t>();
-        PDF_CUDA(launch_seg_merge(sm, (uint32_t)((W + c->bw - 1) / c->bw), cs));
+        PDF_CUDA(launch_seg_merge(sm, (uint32_t)((W + p.bw - 1) / p.bw), cs));
     }
     if (s->pe) PDF_CUDA(cudaEventRecord(s->pe->ev[1], cs));
     if (out && !direct) {
@@ -1284,6 +1158,7 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
         if (st == PDF_OK) st = copy_plane_out(out->mark, out->ld, out->on_device, a.M, a.ld, W, G, cs);
         if (st != PDF_OK) return st;
     }
+    s->pend_plan = &p;
     s->pend_M = a.M;
     s->pend_ld = a.ld;
     s->pend_n = n;
@@ -1299,7 +1174,7 @@ pdf_status grade_cover_locked(pdf_circuit *c, pdf_state *s, cudaStream_t cs) {
     s->pending = false;
     DevAcc *acc = s->acc.as<DevAcc>();
     const uint32_t base = (uint32_t)s->pend_base;
-    CoverArgs ca = base_cover(c, s->ws, s->pend_M, s->pend_ld, s->pend_n, base, s->first_x.as<uint32_t>(),
+    CoverArgs ca = base_cover(c, *s->pend_plan, s->ws, s->pend_M, s->pend_ld, s->pend_n, base, s->first_x.as<uint32_t>(),
                               s->first_y.as<uint32_t>(), acc);
     if (s->pe) PDF_CUDA(cudaEventRecord(s->pe->ev[2], cs));  // cover starts (after any exchange)
     PDF_CUDA(launch_cover(ca, c->cover_grid, c->cover_threads, false, cs));  // closes the batch
@@ -1393,13 +1268,13 @@ extern "C" pdf_status pdf_sim(pdf_circuit *c, const pdf_pairs *pr, uint32_t *sim
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     std::lock_guard<std::mutex> lk(c->mu);
     const bool direct = planes_fit(c, W, ld, {sim_v, sim_t});
-    st = ensure_ws(c, c->stage, W, !direct);
+    st = ensure_ws(c, c->full, c->stage, W, !direct);
     if (st != PDF_OK) return st;
     const uint32_t *pv, *pt;
     uint64_t pld;
     st = stage_pairs(c, c->stage, pr, &pv, &pt, &pld, cs);
     if (st != PDF_OK) return st;
-    FwdArgs a = base_fwd(c, pr->n_pairs);
+    FwdArgs a = base_fwd(c, c->full, pr->n_pairs);
     a.pi_v = pv;
     a.pi_t = pt;
     a.pi_ld = pld;
@@ -1408,11 +1283,9 @@ extern "C" pdf_status pdf_sim(pdf_circuit *c, const pdf_pairs *pr, uint32_t *sim
         a.T = sim_t;
         a.ld = ld;
     } else {
-        a.ld = c->stage.plane_ld;
-        a.V = c->stage.planes.as<uint32_t>();
-        a.T = a.V + G * a.ld;
+        use_ws_planes(a, c->full, c->stage, W);
     }
-    PDF_CUDA(launch_forward(a, FWD_SIM, c->mark_mode, c->bw, c->threads, c->fwd_smem, cs));
+    PDF_CUDA(launch_forward(a, FWD_SIM, c->mark_mode, c->bw, c->full.threads, c->full.fwd_smem, cs));
     if (!direct) {
         PDF_CUDA(cudaMemcpy2DAsync(sim_v, ld * 4, a.V, a.ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
         PDF_CUDA(cudaMemcpy2DAsync(sim_t, ld * 4, a.T, a.ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
@@ -1431,26 +1304,23 @@ pdf_status mark_planes(pdf_circuit *c, const uint32_t *sim_v, const uint32_t *si
     std::lock_guard<std::mutex> lk(c->mu);
     const uint64_t W = (n_pairs + 31) / 32, G = c->info.n_gates;
     const bool direct = planes_fit(c, W, ld, {sim_v, sim_t, mark});
-    pdf_status st = ensure_ws(c, c->stage, W, !direct);
+    pdf_status st = ensure_ws(c, c->full, c->stage, W, !direct);
     if (st != PDF_OK) return st;
-    FwdArgs a = base_fwd(c, n_pairs);
+    FwdArgs a = base_fwd(c, c->full, n_pairs);
     if (direct) {
         a.V = const_cast<uint32_t *>(sim_v);
         a.T = const_cast<uint32_t *>(sim_t);
         a.M = mark;
         a.ld = ld;
     } else {
-        a.ld = c->stage.plane_ld;
-        a.V = c->stage.planes.as<uint32_t>();
-        a.T = a.V + G * a.ld;
-        a.M = a.T + G * a.ld;
+        use_ws_planes(a, c->full, c->stage, W);
         PDF_CUDA(cudaMemcpy2DAsync(a.V, a.ld * 4, sim_v, ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
         PDF_CUDA(cudaMemcpy2DAsync(a.T, a.ld * 4, sim_t, ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
     }
     a.nzb = c->stage.nzb.as<uint32_t>();
     a.blk_maxlvl = c->stage.maxlvl.as<uint32_t>();
     a.no_prune = prune ? 0u : 1u;
-    PDF_CUDA(launch_forward(a, FWD_MARK, c->mark_mode, c->bw, c->threads, c->fwd_smem, cs));
+    PDF_CUDA(launch_forward(a, FWD_MARK, c->mark_mode, c->bw, c->full.threads, c->full.fwd_smem, cs));
     if (!direct)
         PDF_CUDA(cudaMemcpy2DAsync(mark, ld * 4, a.M, a.ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
     PDF_CUDA(cudaStreamSynchronize(cs));
@@ -1480,7 +1350,7 @@ extern "C" pdf_status pdf_merge(pdf_circuit *c, pdf_state *s, const uint32_t *si
         PDF_CUDA(launch_seg_merge_dense(c->seg_args(), sim_v, mark, ld, n_pairs, (uint32_t)pair_base,
                                         s->first_x.as<uint32_t>(), s->first_y.as<uint32_t>(), cs));
     else
-        PDF_CUDA(launch_merge_dense(c->dc, sim_v, mark, ld, n_pairs, (uint32_t)pair_base,
+        PDF_CUDA(launch_merge_dense(c->full.dc, sim_v, mark, ld, n_pairs, (uint32_t)pair_base,
                                     s->first_x.as<uint32_t>(), s->first_y.as<uint32_t>(), cs));
     return PDF_OK;
 }
@@ -1493,7 +1363,7 @@ pdf_status cover_chunk(pdf_circuit *c, pdf_state *s, const uint32_t *mark, uint6
                        uint64_t pair_base, uint64_t *counts, pdf_totals *chunk, cudaStream_t cs) {
     std::lock_guard<std::mutex> lk(s->mu);
     const uint64_t W = (n_pairs + 31) / 32;
-    pdf_status st = ensure_ws(c, s->ws, W, false);
+    pdf_status st = ensure_ws(c, c->full, s->ws, W, false);
     if (st != PDF_OK) return st;
     const size_t count_bytes = (size_t)c->info.n_pi * n_pairs * 16;
     if (counts) {
@@ -1502,10 +1372,10 @@ pdf_status cover_chunk(pdf_circuit *c, pdf_state *s, const uint32_t *mark, uint6
     }
     DevAcc *acc = s->acc.as<DevAcc>();
     PDF_CUDA(launch_batch_begin(acc, cs));
-    CoverArgs ca = base_cover(c, s->ws, mark, ld, n_pairs, (uint32_t)pair_base, s->first_x.as<uint32_t>(),
+    CoverArgs ca = base_cover(c, c->full, s->ws, mark, ld, n_pairs, (uint32_t)pair_base, s->first_x.as<uint32_t>(),
                               s->first_y.as<uint32_t>(), acc);
     // the bitmaps the cover reads, at its granularity, from the given marks
-    PDF_CUDA(launch_bitmap_from_marks(c->dc, mark, ld, n_pairs, ca.bw, const_cast<uint32_t *>(ca.nzb),
+    PDF_CUDA(launch_bitmap_from_marks(c->full.dc, mark, ld, n_pairs, ca.bw, const_cast<uint32_t *>(ca.nzb),
                                       const_cast<uint32_t *>(ca.blk_maxlvl), ca.bm_words, cs));
     if (counts) ca.pi_counts = s->ws.pi_counts.as<unsigned long long>();
     PDF_CUDA(launch_cover(ca, c->cover_grid, c->cover_threads, true, cs));  // closes the batch
@@ -1577,9 +1447,9 @@ extern "C" pdf_status pdf_cover_noalloc(pdf_circuit *c, const uint32_t *mark, ui
     // the array keeps the previous call's contents: clear the accumulator
     PDF_CUDA(cudaMemsetAsync(acc, 0, sizeof(DevAcc), cs));
     PDF_CUDA(launch_batch_begin(acc, cs));
-    PDF_CUDA(launch_bitmap_from_marks(c->dc, mark, ld, n_pairs, c->bw, nzb, maxlvl, (uint32_t)bm_words, cs));
+    PDF_CUDA(launch_bitmap_from_marks(c->full.dc, mark, ld, n_pairs, c->bw, nzb, maxlvl, (uint32_t)bm_words, cs));
     CoverArgs ca{};
-    ca.c = c->dc;
+    ca.c = c->full.dc;
     ca.M = mark;
     ca.ld = ld;
     ca.nzb = nzb;
@@ -1708,27 +1578,26 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
     std::vector<uint32_t> order(n_jobs);
     for (uint32_t i = 0; i < n_jobs; i++) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
-        const pdf_circuit *cx = jobs[x].circuit, *cy = jobs[y].circuit;
-        if (cx->bw != cy->bw) return cx->bw > cy->bw;
-        if (cx->occ != cy->occ) return cx->occ < cy->occ;
-        return cx->chain > cy->chain;
+        const Plan &px = jobs[x].circuit->lean(), &py = jobs[y].circuit->lean();
+        if (px.bw != py.bw) return px.bw > py.bw;
+        if (px.occ != py.occ) return px.occ < py.occ;
+        return px.chain > py.chain;
     });
     for (uint32_t k = 0; k < n_jobs; k++) {
         const pdf_batch_job &j = jobs[order[k]];
         const uint32_t i = k;
         pdf_circuit *c = j.circuit;
         pdf_state *s = j.state;
-        const uint64_t n = j.pairs.n_pairs, W = (n + 31) / 32, G = c->info.n_gates;
-        if (ensure_ws(c, s->ws, W, true) != PDF_OK) return PDF_ENOMEM;
-        FwdArgs a = base_fwd(c, n);
+        const Plan &p = c->lean();
+        const uint64_t n = j.pairs.n_pairs, W = (n + 31) / 32, G = p.n_gates;
+        if (ensure_ws(c, p, s->ws, W, true) != PDF_OK) return PDF_ENOMEM;
+        FwdArgs a = base_fwd(c, p, n);
         a.pi_v = j.pairs.v;
         a.pi_t = j.pairs.t;
         a.pi_ld = j.pairs.ld;
         a.store_all = 0;
-        a.ld = s->ws.plane_ld;
-        a.V = s->ws.planes.as<uint32_t>();
-        a.T = a.V + G * a.ld;
-        a.M = a.T + G * a.ld;
+        a.in_pieces = p.in_pieces;
+        use_ws_planes(a, p, s->ws, W);
         a.nzb = s->ws.nzb.as<uint32_t>();
         a.blk_maxlvl = s->ws.maxlvl.as<uint32_t>();
         a.nzb_fine = s->ws.nzb_fine.as<uint32_t>();
@@ -1741,26 +1610,27 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
         a.acc = acc;
         a.active = s->ws.active.as<uint32_t>();
         fa[i] = a;
-        ca[i] = base_cover(c, s->ws, a.M, a.ld, n, (uint32_t)j.pair_base, a.first_x, a.first_y, acc);
-        const uint64_t blocks = (W + c->bw - 1) / c->bw;
+        ca[i] = base_cover(c, p, s->ws, a.M, a.ld, n, (uint32_t)j.pair_base, a.first_x, a.first_y, acc);
+        const uint64_t blocks = (W + p.bw - 1) / p.bw;
         if (bp[i] + blocks > 0x7FFFFFFFull || gp[i] + G > 0xFFFFFFFFull) return PDF_ENOTSUP;
         bp[i + 1] = bp[i] + (uint32_t)blocks;
         gp[i + 1] = gp[i] + (uint32_t)G;
         items += std::min<uint64_t>(W * 32, 2 * G);
-        L.threads = std::max(L.threads, c->threads);
-        L.fwd_smem = std::max(L.fwd_smem, c->fwd_smem);
+        L.tile = std::max(L.tile, c->bw);
+        L.threads = std::max(L.threads, c->full.threads);
+        L.fwd_smem = std::max(L.fwd_smem, p.fwd_smem);
         L.cover_grid = std::max(L.cover_grid, c->cover_grid);
-        if (!L.n_class || L.cls[L.n_class - 1].occ != c->occ || L.cls[L.n_class - 1].bw != c->bw) {
+        if (!L.n_class || L.cls[L.n_class - 1].occ != p.occ || L.cls[L.n_class - 1].bw != p.bw) {
             if (L.n_class == kMaxBatchClasses) return PDF_ENOTSUP;
             BatchClass &k2 = L.cls[L.n_class++];
-            k2.bw = c->bw;
-            k2.occ = c->occ;
+            k2.bw = p.bw;
+            k2.occ = p.occ;
             k2.blk0 = bp[i];
         }
         BatchClass &cl = L.cls[L.n_class - 1];
-        cl.threads = std::max(cl.threads, c->threads);
-        cl.smem = std::max(cl.smem, c->fwd_smem);
-        b->gate_evals += G * n;
+        cl.threads = std::max(cl.threads, p.threads);
+        cl.smem = std::max(cl.smem, p.fwd_smem);
+        b->gate_evals += (uint64_t)c->info.n_gates * n;
         b->circuits.push_back(c);
         b->states.push_back(s);
     }
@@ -1893,7 +1763,7 @@ extern "C" void pdf_batch_destroy(pdf_batch *b) {
 extern "C" pdf_status pdf_batch_query(const pdf_batch *b, pdf_batch_info *info) {
     if (!b || !info) return PDF_EINVAL;
     info->n_jobs = b->L.n;
-    info->tile_words = b->L.n_class ? b->L.cls[0].bw : 0;  // of the first forward class
+    info->tile_words = b->L.tile;  // the widest circuit tile
     info->threads = b->L.threads;
     info->ctas = b->L.total_blocks;
     info->gate_evals = b->gate_evals;
@@ -2092,5 +1962,7 @@ extern "C" pdf_status pdf_state_reserve(pdf_state *s, uint64_t n_pairs) {
     DeviceGuard dg(s->c->device);
     if (!dg.ok) return PDF_ECUDA;
     std::lock_guard<std::mutex> lk(s->mu);
-    return ensure_ws(s->c, s->ws, (n_pairs + 31) / 32, true);
+    const uint64_t W = (n_pairs + 31) / 32;
+    const pdf_status st = ensure_ws(s->c, s->c->lean(), s->ws, W, true);
+    return st == PDF_OK ? ensure_ws(s->c, s->c->full, s->ws, W, true) : st;
 }

@@ -25,13 +25,14 @@ typedef unsigned __int128 pdf_u128;
 
 // Gate record, 32 bytes, one per gate, built at circuit upload.
 //   w[0] = type | po << 4 | RF_* flags (bits 5..7, 16..23) | nfi << 8 | nfold << 24
-//   w[1] = nfo
+//   w[1] = nfo; where counts and pieces fit 16 bits, above it the last piece that holds a
+//          gate whose mark this gate's can carry (its reach)
 //   w[2] = edge offset: fan-ins at edges[w2 + j], fan-outs at edges[w2 + nfi + k]
 //   w[3..6] = where the forward kernel reads fan-ins 0..3 (source words):
 //          SRC_PLANE | f   the plane row of gate f in global memory
 //          SRC_FAR | s     slot s of the piece's far buffer (prefetched)
 //          s               slot s of the shared-memory ring of recent gates
-//   w[7] = fan-in 0 (its gate id; 0 without fan-ins)
+//   w[7] = fan-in 0 (its gate id); of an input its row in the pair planes; else 0
 // Fan-ins past the fourth are read from edges[] (ring or plane row).
 struct __align__(16) GateRec {
     uint32_t w[8];
@@ -57,13 +58,15 @@ enum : uint32_t {
     RF_KILL = 1u << 19,    // the value is S0: a multi-input gate whose fold the
                            // coalesced simLUT sends to 0 (XOR, XNOR, NOT, others)
     RF_SENS = 1u << 20,    // the mark needs the side-input test (AND..XNOR, nfi >= 2)
-    RF_MARKF0 = 1u << 21,  // mark = transition & mark of fan-in 0
-    RF_INPT = 1u << 22,    // primary input: mark = transition
+    RF_MARKF0 = 1u << 21,  // mark = transition & mark of fan-in 0 (of an input: = transition)
+    RF_INPT = 1u << 22,    // primary input: mark = transition (RF_MARKF0 set too, unless the mark cannot
+                           // matter; its row in the pair planes is w[7])
     RF_SPILL = 1u << 23,   // a later gate reads this gate's plane rows from global memory
                            // (lane kernel: some gate reads its rows at all)
     // true n-input semantics (PDF_MARK_FIXED_*)
     RF_XOR = 1u << 5,      // fold steps are XOR (XOR, XNOR)
-    RF_OINV = 1u << 6,     // the folded value is inverted under both vectors (NAND, NOR, XNOR)
+    RF_OINV = 1u << 6,     // the folded value is inverted under both vectors (NAND, NOR, XNOR; with
+                           // RF_KILL in any mode: the constant S1)
     RF_MANY = 1u << 7,     // mark = transition & OR over fan-ins i of (mark(i) & side test for i)
 };
 
@@ -85,7 +88,7 @@ PDF_HD uint32_t make_rec_header(uint32_t type, uint32_t po, uint32_t nfi, bool f
         f |= nfi >= 2 ? (RF_SENS | RF_MANY) : RF_MARKF0;
         nfold = nfi - 1;
     } else if (type == PDF_INPT) {
-        f |= RF_INPT;
+        f |= RF_INPT | RF_MARKF0;
     } else if (copy) {
         f |= RF_MARKF0;  // :126-130 copy fan-in 0; mark follows fan-in 0 (:242-246)
     } else if (nfi >= 2 && !(type >= PDF_AND && type <= PDF_NOR)) {
@@ -132,8 +135,7 @@ template <bool FIX = false>
 PDF_HD void eval_finish(uint32_t h, uint32_t &V, uint32_t v1, uint32_t &T) {
     const uint32_t keep = ~flagmask(h, RF_KILL);
     T = (V ^ v1) & keep;
-    V &= keep;
-    if (FIX) V ^= flagmask(h, RF_OINV);  // inverting both vectors keeps the transition flag
+    V = (V & keep) ^ flagmask(h, RF_OINV);  // inverting both vectors keeps the transition flag
 }
 
 // Two-input fold step val = OP2(val, r) on bit-planes (simkernel.cuh:146 via

@@ -49,6 +49,10 @@ __device__ __forceinline__ void bitmap_set_aggregated(uint32_t *bm, uint32_t g) 
     if ((threadIdx.x & 31) == (uint32_t)(__ffs(grp) - 1)) atomicOr(bm + word, bits);
 }
 
+// The caller's id of gate g of a (possibly reduced) netlist, kEmpty for a
+// constant: the index of its first-detect ids.
+__device__ __forceinline__ uint32_t net_id(const DevCircuit &c, uint32_t g) { return c.orig ? __ldg(c.orig + g) : g; }
+
 __device__ __forceinline__ bool bit_test(const uint32_t *bm, uint32_t g) { return (bm[g >> 5] >> (g & 31)) & 1u; }
 
 // ---- TMA bulk copies and mbarriers (inline PTX, sm_90+ / sm_100a) ----
@@ -400,7 +404,7 @@ __device__ __forceinline__ void prune_and_merge(const FwdArgs &a, const FwdSmem 
 #pragma unroll
             for (int j = 0; j < BW; j++) keep.x[j] = rec_po(r) ? 0xFFFFFFFFu : 0u;
             if (!rec_po(r)) {
-                const uint32_t nfo = r.w[1], base = r.w[2] + rec_nfi(r);
+                const uint32_t nfo = r.w[1] & a.c.nfo_mask, base = r.w[2] + rec_nfi(r);
                 for (uint32_t k = 0; k < nfo; k++) {
                     const uint32_t fo = staged ? es[base + k - P.ea] : __ldg(edges + base + k);
                     if (!bit_test(S.bm, fo)) continue;
@@ -431,8 +435,9 @@ __device__ __forceinline__ void prune_and_merge(const FwdArgs &a, const FwdSmem 
                     if (x) cx = (w0 + j) * 32 + (__ffs(x) - 1);
                     if (y) cy = (w0 + j) * 32 + (__ffs(y) - 1);
                 }
-                if (cx != kEmpty) atomicMin(a.first_x + g, a.pair_base + cx);
-                if (cy != kEmpty) atomicMin(a.first_y + g, a.pair_base + cy);
+                const uint32_t id = net_id(a.c, g);
+                if (cx != kEmpty) atomicMin(a.first_x + id, a.pair_base + cx);
+                if (cy != kEmpty) atomicMin(a.first_y + id, a.pair_base + cy);
             }
             any |= nz;
         }
@@ -532,9 +537,14 @@ __device__ __forceinline__ void forward_cta(const FwdArgs &a, const uint32_t blk
             a.acc->done_over = 0;
         }
     }
-    __shared__ uint32_t s_fail;
+    // the last piece that can still hold a marked gate: the inputs' last, then
+    // as far as a marked gate reaches
+    __shared__ uint32_t s_fail, s_reach;
+    const bool early = MODE == FWD_FUSED && a.in_pieces;
+    uint32_t my_reach = 0;
     if (threadIdx.x == 0) {
         s_fail = 0;
+        s_reach = a.in_pieces - 1;
         mbar_init(S.mbar, 1);
         mbar_init(S.mbar + 1, 1);
         fence_mbar_init();
@@ -608,8 +618,8 @@ __device__ __forceinline__ void forward_cta(const FwdArgs &a, const uint32_t blk
                 V = vld<BW>(a.V + (size_t)g * a.ld + w0);
                 T = vld<BW>(a.T + (size_t)g * a.ld + w0);
             } else if (h & RF_INPT) {  // simkernel.cuh:112-125, pairs already formed
-                V = vldg<BW>(a.pi_v + (size_t)g * a.pi_ld + w0);
-                T = vldg<BW>(a.pi_t + (size_t)g * a.pi_ld + w0);
+                V = vldg<BW>(a.pi_v + (size_t)r.w[7] * a.pi_ld + w0);
+                T = vldg<BW>(a.pi_t + (size_t)r.w[7] * a.pi_ld + w0);
             }
             if (tail && (MODE == FWD_MARK || (h & RF_INPT))) {
 #pragma unroll
@@ -651,7 +661,7 @@ __device__ __forceinline__ void forward_cta(const FwdArgs &a, const uint32_t blk
             for (int j = 0; j < BW; j++) M.x[j] = 0;
             if (MODE != FWD_SIM) {  // markkernel.cuh:226-267
                 if (h & RF_INPT) {
-                    M = T;
+                    if (h & RF_MARKF0) M = T;
                 } else if ((h & RF_MARKF0) && vany(T) && bit_test(S.bm, r.w[7])) {
                     // fan-in 0 (gate w[7]) holds a mark: its bitmap bit is set
                     const Vec<BW> m0 = load(r.w[3], 2);
@@ -701,7 +711,12 @@ __device__ __forceinline__ void forward_cta(const FwdArgs &a, const uint32_t blk
             if (marked) {
                 bitmap_set_aggregated(S.bm, g);
                 any = true;
+                my_reach = max(my_reach, r.w[1] >> 16);
             }
+        }
+        if (early) {
+            const uint32_t wr = __reduce_max_sync(0xFFFFFFFFu, my_reach);
+            if ((threadIdx.x & 31) == 0 && wr > i) atomicMax(&s_reach, wr);
         }
         cp_async_wait_all();  // this thread's copies for piece i + 1
         if (__syncthreads_or(any) && threadIdx.x == 0) S.pbits[i >> 5] |= 1u << (i & 31);
@@ -713,6 +728,21 @@ __device__ __forceinline__ void forward_cta(const FwdArgs &a, const uint32_t blk
             if (MODE != FWD_SIM) empty_block(a, blk, gbm);
             if (threadIdx.x == 0) atomicOr(a.err, kErrTimeout);
             return;
+        }
+        // No gate past piece i can be marked (each needs a mark on its carrying
+        // fan-in, and no marked gate carries further), so with no plane asked
+        // for nothing past it can matter.  Every thread decides alike: s_reach
+        // only grows past i in threads that went on.
+        if (early && has_next && s_reach <= i) {
+            // piece i + 1's copy is on its way
+            const bool landed = mbar_wait(S.mbar + (buf ^ 1), (phase >> (buf ^ 1)) & 1u);
+            phase ^= 1u << (buf ^ 1);
+            if (__syncthreads_or(!landed)) {
+                empty_block(a, blk, gbm);
+                if (threadIdx.x == 0) atomicOr(a.err, kErrTimeout);
+                return;
+            }
+            break;
         }
     }
     if constexpr (MODE != FWD_SIM) {
@@ -856,8 +886,8 @@ __device__ __forceinline__ void lane_load(const FwdArgs &a, const LanePlanes &P,
             lload<LW>(lrow(P.T, g, P.ld4), x.ft[0]);
         } else {
             const uint32_t pld4 = (uint32_t)(a.pi_ld * 4);
-            lload_nc<LW>(lrow(reinterpret_cast<const char *>(a.pi_v + w), g, pld4), x.fv[0]);
-            lload_nc<LW>(lrow(reinterpret_cast<const char *>(a.pi_t + w), g, pld4), x.ft[0]);
+            lload_nc<LW>(lrow(reinterpret_cast<const char *>(a.pi_v + w), r1.w, pld4), x.fv[0]);
+            lload_nc<LW>(lrow(reinterpret_cast<const char *>(a.pi_t + w), r1.w, pld4), x.ft[0]);
         }
         return;
     }
@@ -935,7 +965,7 @@ __device__ __forceinline__ bool lane_gate(const FwdArgs &a, const LanePlanes &P,
     } else if ((h & RF_KILL) || !live) {
         lzero<LW>(V);
         lzero<LW>(T);
-        if (FIX && (h & RF_OINV)) {
+        if (h & RF_OINV) {
 #pragma unroll
             for (int j = 0; j < LW; j++) V[j] = wm[j];  // S0 inverted under both vectors: S1
         }
@@ -972,8 +1002,9 @@ __device__ __forceinline__ bool lane_gate(const FwdArgs &a, const LanePlanes &P,
     if (MODE != FWD_SIM) {  // markkernel.cuh:226-267
         const bool anyT = __any_sync(0xFFFFFFFFu, lany<LW>(T));
         if (h & RF_INPT) {
+            const uint32_t on = flagmask(h, RF_MARKF0);
 #pragma unroll
-            for (int j = 0; j < LW; j++) M[j] = T[j];
+            for (int j = 0; j < LW; j++) M[j] = T[j] & on;
         } else if ((h & RF_MARKF0) && x.bit0 && anyT) {
             // fan-in 0 (gate w[7]) holds a mark: its bitmap bit is set
 #pragma unroll
@@ -1082,6 +1113,11 @@ __device__ __forceinline__ void forward_lanes_cta(const FwdArgs &a, const uint32
             a.acc->done_over = 0;
         }
     }
+    // the last piece that can still hold a marked gate (as in forward_cta)
+    __shared__ uint32_t s_reach;
+    const bool early = MODE == FWD_FUSED && a.in_pieces;
+    uint32_t my_reach = 0;
+    if (threadIdx.x == 0) s_reach = a.in_pieces - 1;
     __syncthreads();
 
     // ------------------------------------------------------------- forward
@@ -1111,6 +1147,7 @@ __device__ __forceinline__ void forward_lanes_cta(const FwdArgs &a, const uint32
         cp_async_wait_all();  // this thread's copies of piece i's records
         if (__syncthreads_or(any) && i) top = max(top, prev_level + 1);
         any = false;
+        if (early && i && s_reach < i) break;  // nothing from piece i on can be marked
         if (i + 1 < a.n_pieces) stage(na, nb, (i + 1) & 1);  // into the buffer of piece i - 1, which every warp has left
         const uint32_t ga = pa, gb = pb;
         prev_level = pl;
@@ -1133,9 +1170,13 @@ __device__ __forceinline__ void forward_lanes_cta(const FwdArgs &a, const uint32
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 const uint32_t gu = g + u * NW;
-                if (gu < gb) any |= lane_gate<SEM, MODE, LW>(a, P, bm, rb + (gu - ga), gu, live, nw, wm, x[u]);
+                if (gu < gb && lane_gate<SEM, MODE, LW>(a, P, bm, rb + (gu - ga), gu, live, nw, wm, x[u])) {
+                    any = true;
+                    if (early) my_reach = max(my_reach, rb[gu - ga].w[1] >> 16);
+                }
             }
         }
+        if (early && lane == 0 && my_reach > i) atomicMax(&s_reach, my_reach);
     }
     if (__syncthreads_or(any)) top = max(top, prev_level + 1);
     if constexpr (MODE == FWD_SIM) {
@@ -1168,7 +1209,7 @@ __device__ __forceinline__ void forward_lanes_cta(const FwdArgs &a, const uint32
                         keep[j] = rec_po(r) ? 0xFFFFFFFFu : 0u;
                     }
                     if (!rec_po(r)) {
-                        const uint32_t nfo = r.w[1], base = r.w[2] + rec_nfi(r);
+                        const uint32_t nfo = r.w[1] & a.c.nfo_mask, base = r.w[2] + rec_nfi(r);
                         for (uint32_t k = 0; k < nfo; k += 4) {  // four fan-out rows in flight
                             uint32_t fo[4], m[4][LW];
 #pragma unroll
@@ -1210,8 +1251,9 @@ __device__ __forceinline__ void forward_lanes_cta(const FwdArgs &a, const uint32
                         cx = __reduce_min_sync(0xFFFFFFFFu, cx);
                         cy = __reduce_min_sync(0xFFFFFFFFu, cy);
                         if (lane == 0) {
-                            if (cx != kEmpty) atomicMin(a.first_x + g, a.pair_base + cx);
-                            if (cy != kEmpty) atomicMin(a.first_y + g, a.pair_base + cy);
+                            const uint32_t id = net_id(a.c, g);
+                            if (cx != kEmpty) atomicMin(a.first_x + id, a.pair_base + cx);
+                            if (cy != kEmpty) atomicMin(a.first_y + id, a.pair_base + cy);
                         }
                     }
                     any |= nz;
@@ -1252,7 +1294,9 @@ __global__ void __launch_bounds__(lane_threads(32 * LW), 1) k_forward_lanes(cons
 // whose bit it set.
 template <class Emit>
 __device__ __forceinline__ void active_gate(const CoverArgs &a, uint32_t g, Emit emit) {
-    const uint32_t f[2] = {a.first_x[g], a.first_y[g]};
+    const uint32_t id = net_id(a.c, g);
+    if (id == kEmpty) return;
+    const uint32_t f[2] = {a.first_x[id], a.first_y[id]};
 #pragma unroll
     for (int k = 0; k < 2; k++) {
         const uint32_t d = f[k] - a.pair_base;
@@ -1632,10 +1676,10 @@ __device__ __forceinline__ bool cover_pair(const CoverArgs &a, const uint32_t p,
         if (a.seg.N > 1) {
             first = first_set_find(a.seg_first, a.seg_first_mask, ((unsigned long long)g << 32) | p);
         } else {
-            const uint32_t fx = a.first_x[g], fy = a.first_y[g];
+            const uint32_t id = net_id(a.c, g), fx = a.first_x[id], fy = a.first_y[id];
             first = fx == pid || fy == pid;
         }
-        const uint32_t nfo = r.w[1], eb = r.w[2] + rec_nfi(r);
+        const uint32_t nfo = r.w[1] & a.c.nfo_mask, eb = r.w[2] + rec_nfi(r);
         uint32_t k = 0;
         for (uint32_t j = 0; j < nfo; j += 4) {  // four fan-out loads in flight
             uint32_t fo[4];
@@ -1766,7 +1810,7 @@ __device__ void spill_pair(const CoverArgs &a, const uint32_t p, pdf_u128 *Hs) {
             const GateRec r = load_rec(a.c.rec + g);
             pdf_u128 H = rec_po(r) ? 1 : 0, C = 0;
             bool dummy = false;
-            const uint32_t nfo = r.w[1], eb = r.w[2] + rec_nfi(r);
+            const uint32_t nfo = r.w[1] & a.c.nfo_mask, eb = r.w[2] + rec_nfi(r), id = net_id(a.c, g);
             for (uint32_t k = 0; k < nfo; k++) {
                 const uint32_t fo = __ldg(a.c.edges + eb + k);
                 if (!marks(fo)) continue;
@@ -1775,7 +1819,7 @@ __device__ void spill_pair(const CoverArgs &a, const uint32_t p, pdf_u128 *Hs) {
             }
             const bool first = a.seg.N > 1
                                    ? first_set_find(a.seg_first, a.seg_first_mask, ((unsigned long long)g << 32) | p)
-                                   : (a.first_x[g] == pid || a.first_y[g] == pid);
+                                   : (a.first_x[id] == pid || a.first_y[id] == pid);
             pdf_u128 c = C, h = H;
             if (first) {
                 c = add_sat(C, H, ovf);

@@ -12,7 +12,9 @@ struct DevCircuit {
     const GateRec *rec;         // [n_gates]
     const uint32_t *edges;      // fan-ins then fan-outs per gate
     const uint32_t *level_off;  // [n_levels + 1]
-    uint32_t n_gates, n_levels, n_pi;
+    const uint32_t *orig;       // reduced netlists: the caller's gate id per gate, or null
+    uint32_t n_gates, n_levels;
+    uint32_t nfo_mask;          // fan-out count bits of a record's w[1] (above them: its reach)
 };
 
 // Kernel stage selection for the forward kernel.
@@ -39,6 +41,8 @@ struct FwdArgs {
     DevCircuit c;
     const Piece *pieces;          // level-ordered runs of gates (the unit of staging and of sync)
     uint32_t n_pieces;
+    uint32_t in_pieces;           // pieces of level 0 when the walk may end before the last piece that
+                                  // can hold a mark (no plane asked for); 0: it never does
     uint32_t cap, ecap;           // gates / edge words per staging buffer
     const uint32_t *far_ids;      // per piece, the far fan-ins it reads (Piece::far_off / far_n),
                                   // each list padded to a multiple of 4 entries
@@ -158,7 +162,7 @@ constexpr uint32_t lane_threads(uint32_t bw) {
 constexpr uint32_t kLaneCoverWords = 8;
 // Forward launches of a batch at most: (tile width, CTAs per SM) classes of
 // the thread-per-gate kernel and the two lane tiles.
-constexpr uint32_t kMaxBatchClasses = 10;
+constexpr uint32_t kMaxBatchClasses = 20;
 
 // Batched grading (k_batch_forward, k_batch_active, k_batch_cover).
 struct BatchCtl {
@@ -188,6 +192,7 @@ struct BatchLaunch {
     BatchCtl *ctl;
     uint32_t n, total_blocks, total_gates;
     uint32_t sem, threads, cover_grid, hash_cap, append;  // sem: PDF_MARK_*
+    uint32_t tile;         // the widest circuit tile
     // the small-table cover that runs first: nets per pair, CTAs
     uint32_t small_cap, small_grid;
     size_t fwd_smem;

@@ -1,0 +1,253 @@
+// pdf_plan.cpp -- launch plans of the forward kernels (host code).
+#include "pdf_plan.h"
+
+#include <algorithm>
+
+#include "pdf_kernels.cuh"
+
+pdf_status build_plan(const NetPlan &n, const PlanOpts &o, LaunchPlan &pl) {
+    const uint32_t G = n.n_gates(), L = n.n_levels();
+    uint32_t widest_level = 0;
+    for (uint32_t l = 0; l < L; l++) widest_level = std::max(widest_level, n.level_off[l + 1] - n.level_off[l]);
+    pl.n_gates = G;
+    pl.n_levels = L;
+    pl.bw = o.bw;
+    pl.recs.assign(G, GateRec{});
+    for (uint32_t g = 0; g < G; g++) {
+        GateRec &r = pl.recs[g];
+        r.w[0] = n.hdr[g];
+        r.w[1] = n.nfo[g];
+        r.w[2] = (uint32_t)n.eoff[g];  // w[3..6]: source words, set below
+        // fan-in 0; of an input, its row in the pair planes
+        r.w[7] = n.nfi[g] ? n.edges[n.eoff[g]] : (n.hdr[g] & RF_INPT ? (n.orig.empty() ? g : n.orig[g]) : 0u);
+    }
+    const bool lanes = lane_tile(pl.bw);
+    if (lanes) {
+        // The lane kernel reads every fan-in from its plane row: source words
+        // are the fan-in ids themselves, flagged SRC_ZERO when the fan-in is
+        // a killed gate (S0 whatever its inputs); a gate writes its rows
+        // (RF_SPILL) only when some gate reads them.
+        std::vector<uint8_t> read(G, 0);
+        for (uint32_t g = 0; g < G; g++)
+            for (uint32_t q = 0; q < n.nfi[g]; q++) {
+                const uint32_t f = n.edges[n.eoff[g] + q];
+                const bool zero = q < kInlineFanins && (pl.recs[f].w[0] & RF_KILL) && !(pl.recs[f].w[0] & RF_OINV);
+                if (q < kInlineFanins) pl.recs[g].w[3 + q] = f | (zero ? SRC_ZERO : 0u);
+                if (!zero) read[f] = 1;
+            }
+        for (uint32_t g = 0; g < G; g++)
+            if (read[g]) pl.recs[g].w[0] |= RF_SPILL;
+    }
+    const uint32_t max_threads = lanes ? lane_threads(pl.bw) : (pl.bw >= 8 ? 512 : 1024);
+    uint32_t threads_default = 512;  // set from the piece size below
+    auto al = [](size_t x) { return (x + 127) & ~(size_t)127; };
+    const uint32_t bm_words = (G + 31) / 32;
+    // Pieces (the kernels' unit of staging and of synchronisation), sized
+    // from the widest level above the inputs (the inputs' level, often the
+    // widest, just splits into more pieces): runs of one level, <= cap gates,
+    // edge slice <= ecap words.
+    uint32_t widest = 1;
+    for (uint32_t l = 1; l < L; l++) widest = std::max(widest, n.level_off[l + 1] - n.level_off[l]);
+    if (L == 1) widest = widest_level;
+    pl.cap = lanes ? 0u : std::min<uint32_t>(512, (widest + 31) & ~31u);
+    // one thread per gate of a piece plus two warps that have none: they
+    // issue the next piece's far-row copies
+    threads_default = lanes ? lane_threads(pl.bw) : std::min<uint32_t>(max_threads, pl.cap + 64);
+    pl.threads = o.threads ? std::min(o.threads, max_threads) : threads_default;
+    // a block size given by the caller also bounds the pieces: threads - 64
+    // gates, so two warps stay free for the far-row copies
+    if (!lanes && o.threads && pl.threads >= 128) pl.cap = std::min(pl.cap, (pl.threads - 64) & ~31u);
+    // CTAs per SM that the registers allow for this block size (at most 4);
+    // the dynamic shared memory of the forward kernels is then an equal share
+    // of the SM, less 1 KiB per CTA the system keeps and 1 KiB for the
+    // kernels' static variables (the batched kernel keeps its arguments there).
+    {
+        if (o.regs <= 0) return PDF_ECUDA;
+        const uint32_t warps = (pl.threads + 31) / 32;
+        const uint32_t warp_regs = ((uint32_t)o.regs * 32 + 255) & ~255u;
+        uint32_t occ = std::min<uint32_t>(65536 / (warps * warp_regs), 2048 / (warps * 32));
+        pl.occ = std::max<uint32_t>(1, std::min<uint32_t>(occ, 4));
+    }
+    const size_t budget = std::min<size_t>((size_t)o.smem_block,
+                                           (size_t)o.smem_sm / pl.occ - 1024) -
+                          1024;
+    pl.ecap = 2048;
+    if (lanes) {
+        // The lane kernel keeps on chip two buffers of staged gate records
+        // and the column block's mark bitmap (in global memory when it does
+        // not fit); its pieces are runs of one level of <= cap gates: 2 x
+        // kLaneRecs when those buffers fit beside a shared-memory bitmap (a
+        // barrier per piece, so wide levels take half as many), else
+        // kLaneRecs.
+        const size_t bm_bytes = (size_t)bm_words * 4;
+        pl.cap = kLaneRecs;
+        if (widest > kLaneRecs &&
+            2 * 2 * (size_t)kLaneRecs * sizeof(GateRec) + al(bm_bytes) + 2048 <= budget)
+            pl.cap = 2 * kLaneRecs;
+        for (uint32_t l = 0; l < L; l++)
+            for (uint32_t a = n.level_off[l]; a < n.level_off[l + 1]; a += pl.cap) {
+                Piece p{};
+                p.a = a;
+                p.b = std::min(a + pl.cap, n.level_off[l + 1]);
+                p.level = l;
+                pl.pieces.push_back(p);
+            }
+        pl.n_pieces = (uint32_t)pl.pieces.size();
+        const size_t rec_bytes = 2 * (size_t)pl.cap * sizeof(GateRec);
+        pl.off_rec = 0;
+        pl.off_bm = (uint32_t)rec_bytes;
+        pl.bm_shared = rec_bytes + bm_bytes + 2048 <= budget ? 1u : 0u;
+        pl.fwd_smem = rec_bytes + (pl.bm_shared ? al(bm_bytes) : 0);
+        pl.chain = G;
+        while (pl.far_ids.size() < 4) pl.far_ids.push_back(0);
+    } else {
+        auto f4 = [](uint64_t x) { return x & ~(uint64_t)3; };
+        auto c4 = [](uint64_t x) { return (x + 3) & ~(uint64_t)3; };
+        for (uint32_t l = 0; l < L; l++) {
+            const uint32_t s0 = n.level_off[l], e0 = n.level_off[l + 1];
+            for (uint32_t a = s0; a < e0;) {
+                uint32_t b = a + 1;
+                while (b < e0 && b - a < pl.cap && c4(n.eoff[b + 1]) - f4(n.eoff[a]) <= pl.ecap) b++;
+                Piece p{};
+                p.a = a;
+                p.b = b;
+                p.level = l;
+                if (c4(n.eoff[b]) - f4(n.eoff[a]) <= pl.ecap) {
+                    p.ea = (uint32_t)f4(n.eoff[a]);
+                    p.eb = (uint32_t)c4(n.eoff[b]);
+                } else {
+                    p.ea = p.eb = 0xFFFFFFFFu;  // one gate with a huge edge list: read in place
+                }
+                pl.pieces.push_back(p);
+                a = b;
+            }
+        }
+        pl.n_pieces = (uint32_t)pl.pieces.size();
+        if (pl.n_pieces > 65536) return PDF_ENOTSUP;
+        // Far fan-ins of piece i (ring of R slots): fan-ins 0..3 of its gates
+        // below b_i - R.  Those below a_{i-1} (complete when piece i - 1 starts)
+        // go to the piece's deduplicated far list, up to `limit` entries; the rest
+        // are read from their plane rows.  Fills the source words w[3..6].
+        auto far_lists = [&](uint32_t R, uint32_t limit) -> uint32_t {
+            uint32_t worst = 0;
+            pl.far_ids.clear();
+            std::vector<uint32_t> seen(G, 0xFFFFFFFFu);  // gate -> slot in the current piece's list
+            std::vector<uint32_t> list;
+            for (size_t i = 0; i < pl.pieces.size(); i++) {
+                Piece &p = pl.pieces[i];
+                const uint32_t lo = p.b > R ? p.b - R : 0;
+                const uint32_t done = i ? pl.pieces[i - 1].a : 0;
+                list.clear();
+                for (uint32_t g = p.a; g < p.b; g++) {
+                    const uint32_t nq = std::min<uint32_t>(n.nfi[g], kInlineFanins);
+                    for (uint32_t q = 0; q < nq; q++) {
+                        const uint32_t f = n.edges[n.eoff[g] + q];
+                        uint32_t sw = f & (R - 1);
+                        if (f < lo) {
+                            sw = SRC_PLANE | f;
+                            if (f < done) {
+                                if (seen[f] == 0xFFFFFFFFu && list.size() < limit) {
+                                    seen[f] = (uint32_t)list.size();
+                                    list.push_back(f);
+                                }
+                                if (seen[f] != 0xFFFFFFFFu) sw = SRC_FAR | seen[f];
+                            }
+                        }
+                        pl.recs[g].w[3 + q] = sw;
+                        if (sw & SRC_PLANE || sw & SRC_FAR) pl.recs[f].w[0] |= RF_SPILL;
+                    }
+                    for (uint32_t q = kInlineFanins; q < n.nfi[g]; q++) {  // read from edges[] at run time
+                        const uint32_t f = n.edges[n.eoff[g] + q];
+                        if (f < lo) pl.recs[f].w[0] |= RF_SPILL;
+                    }
+                }
+                for (uint32_t f : list) seen[f] = 0xFFFFFFFFu;
+                worst = std::max<uint32_t>(worst, (uint32_t)list.size());
+                p.far_off = (uint32_t)pl.far_ids.size();
+                p.far_n = (uint32_t)list.size();
+                pl.far_ids.insert(pl.far_ids.end(), list.begin(), list.end());
+                // lists start on 16-byte boundaries: the kernel stages the next
+                // piece's list by a bulk copy located from this piece's fields
+                while (pl.far_ids.size() & 3) pl.far_ids.push_back(0);
+            }
+            for (size_t i = 0; i < pl.pieces.size(); i++) pl.pieces[i].nfar_n = i + 1 < pl.pieces.size() ? pl.pieces[i + 1].far_n : 0;
+            return worst;
+        };
+        // Shared memory of k_forward: 2 record buffers; one region holding the
+        // reverse pass's 2 edge buffers or the forward pass's 2 far buffers;
+        // bitmap; piece bits; barriers; the ring.  The ring: the largest power of
+        // two (>= cap, <= 2 * n_gates) that leaves room for far lists of 64
+        // entries; the far lists then get the rest of the budget.
+        const size_t rec_bytes = al(2 * (size_t)pl.cap * sizeof(GateRec));
+        const size_t bm_bytes = (size_t)bm_words * 4 <= 16384 ? al((size_t)bm_words * 4) : 0;
+        const size_t fixed = rec_bytes + bm_bytes + al(((size_t)pl.n_pieces + 31) / 32 * 4) + 128;
+        const size_t edge_bytes = 2 * (size_t)pl.ecap * 4;
+        const size_t far_entry = (size_t)2 * 3 * pl.bw * 4;  // one far slot in both buffers, 3 planes
+        uint32_t rmin = 32;
+        while (rmin < pl.cap) rmin *= 2;
+        uint32_t rmax = rmin;
+        while ((uint64_t)rmax < 2 * (uint64_t)G && fixed + (size_t)rmax * 2 * pl.bw * 12 <= budget) rmax *= 2;
+        // the ring's memory also holds the reverse pass's row staging buffers
+        const size_t rows_bytes = (size_t)2 * pl.cap * 2 * pl.bw * 4;
+        auto ring_bytes = [&](size_t R) { return std::max(R * pl.bw * 12, rows_bytes); };
+        // The largest ring that fits wins: a smaller ring with longer far lists
+        // was measured slower (1M gates, 5,000-gate levels: 116.8 against 109.9
+        // ms) although it leaves fewer fan-ins to plane-row reads.
+        // far region (far rows of two pieces, or the reverse pass's edges) and
+        // the two staged far-id lists, for lists of n entries
+        auto far_bytes = [&](size_t n) { return al(std::max(edge_bytes, n * far_entry)) + al(2 * n * 4); };
+        uint32_t ring = 0;
+        for (uint32_t R = rmax; R >= rmin && !ring; R /= 2)
+            if (fixed + far_bytes(64) + ring_bytes(R) <= budget) ring = R;
+        if (!ring) return PDF_ENOTSUP;
+        const size_t far_room = budget - fixed - ring_bytes(ring);
+        uint32_t far_limit = (uint32_t)std::min<size_t>(kMaxFar, far_room / (far_entry + 8)) & ~3u;
+        while (far_limit > 64 && far_bytes(far_limit) > far_room) far_limit -= 4;
+        const uint32_t farcap = std::max<uint32_t>(4, (far_lists(ring, far_limit) + 3) & ~3u);
+        while (pl.far_ids.size() < 4) pl.far_ids.push_back(0);
+        pl.ring = ring;
+        pl.farcap = farcap;
+        size_t off = 0;
+        pl.off_rec = (uint32_t)off;
+        off += rec_bytes;
+        pl.off_edge = (uint32_t)off;
+        off += al(std::max(edge_bytes, farcap * far_entry));
+        pl.off_fid = (uint32_t)off;
+        off += al(2 * (size_t)farcap * 4);
+        pl.bm_shared = bm_bytes ? 1u : 0u;
+        pl.off_bm = (uint32_t)off;
+        off += bm_bytes;
+        pl.off_pbits = (uint32_t)off;
+        off += al(((size_t)pl.n_pieces + 31) / 32 * 4);
+        pl.off_mbar = (uint32_t)off;
+        off += 128;
+        pl.off_ring = (uint32_t)off;
+        // reverse pass: ring2 and the row staging buffers [2][cap][2][bw] share
+        // the ring's memory
+        uint32_t ring2 = 0;
+        for (uint32_t r = 1; (size_t)r * pl.bw * 4 + rows_bytes <= ring_bytes(ring); r *= 2) ring2 = r;
+        pl.ring2 = ring2;
+        pl.fwd_smem = off + ring_bytes(ring);
+        pl.chain = pl.n_pieces;
+    }
+    // How far a gate's mark can reach: the last piece that holds a gate whose
+    // mark this one can carry.  Kept above the fan-out count in w[1] where
+    // both fit 16 bits; else the walk never ends early.
+    pl.nfo_mask = 0xFFFFFFFFu;
+    const uint32_t max_nfo = n.nfo.empty() ? 0 : *std::max_element(n.nfo.begin(), n.nfo.end());
+    if (max_nfo <= 0xFFFFu && pl.n_pieces <= 0xFFFFu) {
+        pl.nfo_mask = 0xFFFFu;
+        while (pl.in_pieces < pl.n_pieces && pl.pieces[pl.in_pieces].level == 0) pl.in_pieces++;
+        std::vector<uint16_t> reach(G, 0);
+        for (uint32_t i = 0; i < pl.n_pieces; i++)  // ascending: the last reader's piece stays
+            for (uint32_t g = pl.pieces[i].a; g < pl.pieces[i].b; g++) {
+                const uint32_t *fin = n.edges.data() + n.eoff[g];
+                if (n.hdr[g] & RF_MANY)
+                    for (uint32_t q = 0; q < n.nfi[g]; q++) reach[fin[q]] = (uint16_t)i;
+                else if ((n.hdr[g] & RF_MARKF0) && n.nfi[g])
+                    reach[fin[0]] = (uint16_t)i;
+            }
+        for (uint32_t g = 0; g < G; g++) pl.recs[g].w[1] |= (uint32_t)reach[g] << 16;
+    }
+    return PDF_OK;
+}

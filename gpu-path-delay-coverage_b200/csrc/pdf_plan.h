@@ -1,0 +1,42 @@
+// pdf_plan.h -- launch plans of the forward kernels: the gate records, pieces,
+// far lists and shared-memory layout of one walk over a netlist.  A circuit
+// has one for every gate (plane outputs, stage calls) and, when that leaves
+// gates out, one for its reduced netlist (pdf_reduce.h).
+#ifndef PDF_PLAN_H
+#define PDF_PLAN_H
+
+#include <cstddef>
+#include <vector>
+
+#include "pdf.h"
+#include "pdf_reduce.h"
+
+struct PlanOpts {
+    uint32_t bw = 4;         // words per column block
+    uint32_t threads = 0;    // the caller's block size (0: chosen)
+    int regs = 0;            // registers per thread of the forward kernel (forward_kernel_regs)
+    int smem_block = 0, smem_sm = 0;  // shared memory per block (opt-in) and per SM
+};
+
+// What a launch needs besides the device arrays.
+struct PlanShape {
+    uint32_t n_gates = 0, n_levels = 0;
+    uint32_t bw = 4, threads = 512, ring = 0, ring2 = 0, farcap = 0;
+    uint32_t cap = 512, ecap = 2048, n_pieces = 0, bm_shared = 0;
+    uint32_t off_ring = 0, off_rec = 0, off_edge = 0, off_fid = 0, off_bm = 0, off_pbits = 0, off_mbar = 0;
+    size_t fwd_smem = 0;
+    uint32_t occ = 1;    // forward CTAs per SM its registers and shared memory are sized for
+    uint32_t nfo_mask = 0xFFFFFFFFu;  // fan-out count bits of w[1]; the bits above: its reach (0: not kept)
+    uint32_t in_pieces = 0;  // pieces of level 0 (0 when the reach is not kept)
+    uint64_t chain = 0;  // length of one CTA's walk (pieces, or gates for the lane kernel)
+};
+
+struct LaunchPlan : PlanShape {
+    std::vector<GateRec> recs;
+    std::vector<Piece> pieces;
+    std::vector<uint32_t> far_ids;
+};
+
+pdf_status build_plan(const NetPlan &n, const PlanOpts &o, LaunchPlan &pl);
+
+#endif

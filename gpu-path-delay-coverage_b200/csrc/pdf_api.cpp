@@ -167,14 +167,29 @@ struct Plan : PlanShape {
     DevCircuit dc{};
     const Piece *pieces = nullptr;
     const uint32_t *far_ids = nullptr;
-    void bind(const LaunchPlan &l, const NetPlan &n, const unsigned char *base, const struct PlanOffsets &o);
+    // the resident kernel's image of the netlist (null: it does not fit)
+    const void *image = nullptr;
+    uint32_t off_edge_im = 0, off_lvl_im = 0;
+    ResidentSizes res;
+    void bind(const LaunchPlan &l, const NetPlan &n, const ResidentImage &im, const unsigned char *base,
+              const struct PlanOffsets &o);
+};
+
+// One call's walk over W words of pairs: the plan, the kernel and its column
+// block.
+struct Walk {
+    const Plan *p = nullptr;
+    uint32_t bw = 0;
+    bool resident = false;
+    ResidentShape rs;
 };
 
 struct PlanOffsets {
-    size_t rec = 0, edges = 0, level_off = 0, pieces = 0, far = 0, orig = 0;
+    size_t rec = 0, edges = 0, level_off = 0, pieces = 0, far = 0, orig = 0, image = 0;
 };
 
-void Plan::bind(const LaunchPlan &l, const NetPlan &n, const unsigned char *base, const PlanOffsets &o) {
+void Plan::bind(const LaunchPlan &l, const NetPlan &n, const ResidentImage &im, const unsigned char *base,
+                const PlanOffsets &o) {
     static_cast<PlanShape &>(*this) = l;
     dc.rec = reinterpret_cast<const GateRec *>(base + o.rec);
     dc.edges = reinterpret_cast<const uint32_t *>(base + o.edges);
@@ -185,6 +200,13 @@ void Plan::bind(const LaunchPlan &l, const NetPlan &n, const unsigned char *base
     dc.nfo_mask = nfo_mask;
     pieces = reinterpret_cast<const Piece *>(base + o.pieces);
     far_ids = reinterpret_cast<const uint32_t *>(base + o.far);
+    if (im.bytes.empty()) return;
+    image = base + o.image;
+    off_edge_im = im.off_edge;
+    off_lvl_im = im.off_lvl;
+    res.n_gates = n_gates;
+    res.n_levels = n_levels;
+    res.image_bytes = (uint32_t)im.bytes.size();
 }
 
 // Arrays of a circuit on their way into one device block: small circuits go
@@ -202,7 +224,7 @@ struct PlanUpload {
         bytes = (off + n + 255) & ~(size_t)255;
         return off;
     }
-    PlanOffsets add_plan(const NetPlan &n, const LaunchPlan &l) {
+    PlanOffsets add_plan(const NetPlan &n, const LaunchPlan &l, const ResidentImage &im) {
         PlanOffsets o;
         o.rec = add(l.recs.data(), l.recs.size() * sizeof(GateRec));
         o.edges = add(n.edges.data(), n.edges.size() * 4);
@@ -211,6 +233,7 @@ struct PlanUpload {
         o.pieces = add(l.pieces.data(), l.pieces.size() * sizeof(Piece));
         o.far = add(l.far_ids.data(), l.far_ids.size() * 4);
         o.orig = add(n.orig.data(), n.orig.size() * 4);
+        o.image = add(im.bytes.data(), im.bytes.size());
         return o;
     }
     bool copy(unsigned char *dst) const {
@@ -242,6 +265,13 @@ struct pdf_circuit {
     Plan full, red;   // every gate; the reduced netlist (n_gates 0: none)
     // the plan of grading calls that ask for no plane
     const Plan &lean() const { return red.n_gates ? red : full; }
+    Walk full_walk() const { return Walk{&full, full.bw, false, {}}; }
+    Walk lean_walk(uint64_t W) const {
+        const Plan &p = lean();
+        if (!p.image) return Walk{&p, p.bw, false, {}};
+        const ResidentShape r = resident_shape(p.res, W);
+        return Walk{&p, r.bw, true, r};
+    }
     uint32_t hash_cap = 4096, cover_threads = 256, cover_grid = 0;
     uint32_t wait_polls = 0;  // bound of the forward kernels' waits (0 = the default)
     Workspace stage;  // scratch of the stage calls
@@ -282,7 +312,7 @@ struct pdf_state {
     ProfEvents *pe = nullptr;       // events of the call in progress
     // the batch marked by pdf_grade_mark_async and not yet counted
     bool pending = false;
-    const Plan *pend_plan = nullptr;
+    Walk pend_walk;
     const uint32_t *pend_M = nullptr;
     uint64_t pend_ld = 0, pend_n = 0, pend_base = 0;
 };
@@ -620,12 +650,19 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     }
     pdf_status pst = PDF_OK;
     if (!other.valid()) pst = build_plan(net, po, full);
-    // The reduced netlist (single nets; segments are listed over every net).
+    // The reduced netlist (single nets; segments are listed over every net),
+    // and the resident kernel's image of what a lean call walks.
     NetPlan rnet;
+    ResidentImage image;
+    const size_t res_smem = (size_t)prop.sharedMemPerBlockOptin - 1024;
     if (pst == PDF_OK && o.seg_len <= 1) {
         const NetFacts facts = net_facts(net, fixed);
-        if (facts.n_needed <= (uint64_t)G * 9 / 10) {
-            rnet = reduce_net(net, facts);
+        const bool reduced = facts.n_needed <= (uint64_t)G * 9 / 10;
+        if (reduced) rnet = reduce_net(net, facts);
+        image = build_resident(reduced ? rnet : net, res_smem);
+        if (reduced && !image.bytes.empty()) {
+            build_records(rnet, red);
+        } else if (reduced) {
             const uint32_t rl = rnet.n_levels();
             PlanOpts ro = po;
             ro.bw = reduced_tile(c->bw, rl > 1 ? (rnet.n_gates() - rnet.level_off[1]) / (rl - 1) : 0);
@@ -658,8 +695,10 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     {
         PlanUpload up;
         up.add(nullptr, 16);
-        const PlanOffsets fo = up.add_plan(net, full);
-        const PlanOffsets ro = rnet.n_gates() ? up.add_plan(rnet, red) : PlanOffsets{};
+        const ResidentImage none;
+        const bool reduced = rnet.n_gates() != 0;
+        const PlanOffsets fo = up.add_plan(net, full, reduced ? none : image);
+        const PlanOffsets ro = reduced ? up.add_plan(rnet, red, image) : PlanOffsets{};
         if (c->mem.ensure(up.bytes) != cudaSuccess) {
             (void)cudaGetLastError();
             return fail(PDF_ENOMEM);
@@ -669,8 +708,14 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
             return fail(PDF_ECUDA);
         }
         c->err = c->mem.as<uint32_t>();
-        c->full.bind(full, net, c->mem.as<unsigned char>(), fo);
-        if (rnet.n_gates()) c->red.bind(red, rnet, c->mem.as<unsigned char>(), ro);
+        c->full.bind(full, net, reduced ? none : image, c->mem.as<unsigned char>(), fo);
+        if (reduced) c->red.bind(red, rnet, image, c->mem.as<unsigned char>(), ro);
+        for (Plan *p : {&c->full, &c->red}) {
+            p->res.sms = (uint32_t)prop.multiProcessorCount;
+            p->res.regs = 64;  // its launch bound's
+            p->res.smem_block = res_smem;
+            p->res.smem_sm = (size_t)prop.sharedMemPerMultiprocessor;
+        }
     }
     inf.tile_words = c->bw;
     inf.threads = c->full.threads;
@@ -901,14 +946,16 @@ uint32_t spill_slots(uint64_t n, uint64_t *slot) {
     return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(16, (16ull << 20) / *slot));
 }
 
-// Sizes the workspace for a walk of plan p over W words of pairs.
-pdf_status ensure_ws(pdf_circuit *c, const Plan &p, Workspace &ws, uint64_t W, bool need_planes) {
-    const uint64_t n_blocks = (W + p.bw - 1) / p.bw;
+// Sizes the workspace for a walk over W words of pairs.  A resident walk's
+// column block depends on W, so its share is sized for every smaller W too.
+pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, bool need_planes) {
+    const Plan &p = *k.p;
+    const uint64_t n_blocks = k.resident ? W : (W + k.bw - 1) / k.bw;
     const uint64_t bm_words = (p.n_gates + 31) / 32;
     PDF_CUDA(ws.nzb.ensure(n_blocks * bm_words * 4));
     PDF_CUDA(ws.maxlvl.ensure(n_blocks * 4));
-    if (lane_tile(p.bw)) {  // the cover's bitmaps per kLaneCoverWords words of a column block
-        const uint64_t nf = p.bw / kLaneCoverWords;
+    if (lane_tile(k.bw)) {  // the cover's bitmaps per kLaneCoverWords words of a column block
+        const uint64_t nf = k.bw / kLaneCoverWords;
         PDF_CUDA(ws.nzb_fine.ensure(nf * n_blocks * bm_words * 4));
         PDF_CUDA(ws.maxlvl_fine.ensure(nf * n_blocks * 4));
     }
@@ -936,19 +983,27 @@ pdf_status ensure_ws(pdf_circuit *c, const Plan &p, Workspace &ws, uint64_t W, b
             ws.seg_first_mask = cap - 1;
         }
     }
-    if (need_planes) PDF_CUDA(ws.planes.ensure(3 * (uint64_t)p.n_gates * n_blocks * p.bw * 4));
+    // a resident walk keeps V and T on chip: marks only
+    if (need_planes)
+        PDF_CUDA(ws.planes.ensure((k.resident ? 1 : 3) * (uint64_t)p.n_gates *
+                                  (k.resident ? (W + 7) / 8 * 8 : n_blocks * k.bw) * 4));
     return PDF_OK;
 }
 
-// The workspace's planes for a walk of plan p over W words (after ensure_ws).
-void use_ws_planes(FwdArgs &a, const Plan &p, const Workspace &ws, uint64_t W) {
-    a.ld = (W + p.bw - 1) / p.bw * p.bw;
+// The workspace's planes for a walk over W words (after ensure_ws).
+void use_ws_planes(FwdArgs &a, const Walk &k, const Workspace &ws, uint64_t W) {
+    a.ld = (W + k.bw - 1) / k.bw * k.bw;
+    if (k.resident) {
+        a.M = ws.planes.as<uint32_t>();
+        return;
+    }
     a.V = ws.planes.as<uint32_t>();
-    a.T = a.V + p.n_gates * a.ld;
-    a.M = a.T + p.n_gates * a.ld;
+    a.T = a.V + k.p->n_gates * a.ld;
+    a.M = a.T + k.p->n_gates * a.ld;
 }
 
-FwdArgs base_fwd(pdf_circuit *c, const Plan &p, uint64_t n_pairs) {
+FwdArgs base_fwd(pdf_circuit *c, const Walk &k, uint64_t n_pairs) {
+    const Plan &p = *k.p;
     FwdArgs a{};
     a.c = p.dc;
     a.pieces = p.pieces;
@@ -973,6 +1028,18 @@ FwdArgs base_fwd(pdf_circuit *c, const Plan &p, uint64_t n_pairs) {
     a.off_mbar = p.off_mbar;
     a.err = c->err;
     a.wait_polls = c->wait_polls;
+    if (k.resident) {
+        a.image = p.image;
+        a.image_bytes = p.res.image_bytes;
+        a.per = k.rs.per;
+        a.n_blocks = k.rs.blocks;
+        a.off_edge = p.off_edge_im;
+        a.off_fid = p.off_lvl_im;
+        a.off_ring = k.rs.off_vt;
+        a.off_rec = k.rs.off_m;
+        a.off_bm = k.rs.off_bm;
+        a.off_mbar = k.rs.off_mbar;
+    }
     return a;
 }
 
@@ -990,19 +1057,20 @@ pdf_status take_circuit_err(pdf_circuit *c, cudaStream_t cs) {
     return err_status(e);
 }
 
-CoverArgs base_cover(pdf_circuit *c, const Plan &p, Workspace &ws, const uint32_t *M, uint64_t ld, uint64_t n_pairs,
+CoverArgs base_cover(pdf_circuit *c, const Walk &k, Workspace &ws, const uint32_t *M, uint64_t ld, uint64_t n_pairs,
                      uint32_t pair_base, const uint32_t *fx, const uint32_t *fy, DevAcc *acc) {
+    const Plan &p = *k.p;
     CoverArgs a{};
     a.c = p.dc;
     a.M = M;
     a.ld = ld;
     // a lane walk's cover reads bitmaps per 8 words of its column blocks
     // (fewer candidate nets per pair than the whole block's)
-    const bool fine = lane_tile(p.bw);
+    const bool fine = lane_tile(k.bw);
     a.nzb = fine ? ws.nzb_fine.as<uint32_t>() : ws.nzb.as<uint32_t>();
     a.blk_maxlvl = fine ? ws.maxlvl_fine.as<uint32_t>() : ws.maxlvl.as<uint32_t>();
     a.bm_words = (p.n_gates + 31) / 32;
-    a.bw = fine ? kLaneCoverWords : p.bw;
+    a.bw = fine ? kLaneCoverWords : k.bw;
     a.first_x = fx;
     a.first_y = fy;
     a.n_pairs = n_pairs;
@@ -1039,25 +1107,27 @@ bool planes_fit(const pdf_circuit *c, uint64_t W, uint64_t ld, std::initializer_
 
 // Device pointers of the pairs, staging them through the workspace when
 // they are host memory or not in the kernels' layout.
-pdf_status stage_pairs(pdf_circuit *c, Workspace &ws, const pdf_pairs *pr, const uint32_t **v,
+// A resident walk reads them word by word, at any pitch.
+pdf_status stage_pairs(pdf_circuit *c, const Walk &k, Workspace &ws, const pdf_pairs *pr, const uint32_t **v,
                        const uint32_t **t, uint64_t *ld, cudaStream_t st) {
     const uint64_t W = (pr->n_pairs + 31) / 32, npi = c->info.n_pi;
-    if (pr->on_device && planes_fit(c, W, pr->ld, {pr->v, pr->t})) {
+    const bool words = ((reinterpret_cast<uintptr_t>(pr->v) | reinterpret_cast<uintptr_t>(pr->t)) & 3) == 0;
+    if (pr->on_device && (k.resident ? words : planes_fit(c, W, pr->ld, {pr->v, pr->t}))) {
         *v = pr->v;
         *t = pr->t;
         *ld = pr->ld;
         return PDF_OK;
     }
-    const uint64_t Wp = (W + c->bw - 1) / c->bw * c->bw;
-    PDF_CUDA(ws.pi.ensure(2 * npi * Wp * 4));
+    const uint64_t Wp = k.resident ? W : (W + c->bw - 1) / c->bw * c->bw;
+    PDF_CUDA(ws.pi.ensure(2 * npi * ((W + c->bw - 1) / c->bw * c->bw) * 4));
     uint32_t *dv = ws.pi.as<uint32_t>(), *dt = dv + npi * Wp;
-    const cudaMemcpyKind k = pr->on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+    const cudaMemcpyKind kind = pr->on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     if (pr->ld == Wp) {  // rows already at the device pitch: one contiguous copy per plane
-        PDF_CUDA(cudaMemcpyAsync(dv, pr->v, npi * Wp * 4, k, st));
-        PDF_CUDA(cudaMemcpyAsync(dt, pr->t, npi * Wp * 4, k, st));
+        PDF_CUDA(cudaMemcpyAsync(dv, pr->v, npi * Wp * 4, kind, st));
+        PDF_CUDA(cudaMemcpyAsync(dt, pr->t, npi * Wp * 4, kind, st));
     } else {
-        PDF_CUDA(cudaMemcpy2DAsync(dv, Wp * 4, pr->v, pr->ld * 4, W * 4, npi, k, st));
-        PDF_CUDA(cudaMemcpy2DAsync(dt, Wp * 4, pr->t, pr->ld * 4, W * 4, npi, k, st));
+        PDF_CUDA(cudaMemcpy2DAsync(dv, Wp * 4, pr->v, pr->ld * 4, W * 4, npi, kind, st));
+        PDF_CUDA(cudaMemcpy2DAsync(dt, Wp * 4, pr->t, pr->ld * 4, W * 4, npi, kind, st));
     }
     *v = dv;
     *t = dt;
@@ -1086,16 +1156,17 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     // with no plane asked for, only what the marks depend on is evaluated,
     // and only the rows read back are written
     const bool planes = out && (out->sim_v || out->sim_t || out->mark);
-    const Plan &p = planes ? c->full : c->lean();
+    const Walk k = planes ? c->full_walk() : c->lean_walk(W);
+    const Plan &p = *k.p;
     const bool direct = out && out->on_device && planes_fit(c, W, out->ld, {out->sim_v, out->sim_t, out->mark});
-    pdf_status st = ensure_ws(c, p, s->ws, W, !direct);
+    pdf_status st = ensure_ws(c, k, s->ws, W, !direct);
     if (st != PDF_OK) return st;
     const uint32_t *pv, *pt;
     uint64_t pld;
-    st = stage_pairs(c, s->ws, pr, &pv, &pt, &pld, cs);
+    st = stage_pairs(c, k, s->ws, pr, &pv, &pt, &pld, cs);
     if (st != PDF_OK) return st;
 
-    FwdArgs a = base_fwd(c, p, n);
+    FwdArgs a = base_fwd(c, k, n);
     a.pi_v = pv;
     a.pi_t = pt;
     a.pi_ld = pld;
@@ -1107,7 +1178,7 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
         a.M = out->mark;
         a.ld = out->ld;
     } else {
-        use_ws_planes(a, p, s->ws, W);
+        use_ws_planes(a, k, s->ws, W);
     }
     a.nzb = s->ws.nzb.as<uint32_t>();
     a.blk_maxlvl = s->ws.maxlvl.as<uint32_t>();
@@ -1135,7 +1206,10 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     // the forward kernel also clears the batch count and the cover's active pairs
     a.acc = acc;
     a.active = s->ws.active.as<uint32_t>();
-    PDF_CUDA(launch_forward(a, FWD_FUSED, c->mark_mode, p.bw, p.threads, p.fwd_smem, cs));
+    if (k.resident)
+        PDF_CUDA(launch_resident(a, c->mark_mode, k.bw, k.rs.ctas, k.rs.threads, k.rs.smem, cs));
+    else
+        PDF_CUDA(launch_forward(a, FWD_FUSED, c->mark_mode, p.bw, p.threads, p.fwd_smem, cs));
     if (c->seg_len > 1) {
         SegMergeArgs sm{};
         sm.seg = c->seg_args();
@@ -1158,7 +1232,7 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
         if (st == PDF_OK) st = copy_plane_out(out->mark, out->ld, out->on_device, a.M, a.ld, W, G, cs);
         if (st != PDF_OK) return st;
     }
-    s->pend_plan = &p;
+    s->pend_walk = k;
     s->pend_M = a.M;
     s->pend_ld = a.ld;
     s->pend_n = n;
@@ -1174,7 +1248,7 @@ pdf_status grade_cover_locked(pdf_circuit *c, pdf_state *s, cudaStream_t cs) {
     s->pending = false;
     DevAcc *acc = s->acc.as<DevAcc>();
     const uint32_t base = (uint32_t)s->pend_base;
-    CoverArgs ca = base_cover(c, *s->pend_plan, s->ws, s->pend_M, s->pend_ld, s->pend_n, base, s->first_x.as<uint32_t>(),
+    CoverArgs ca = base_cover(c, s->pend_walk, s->ws, s->pend_M, s->pend_ld, s->pend_n, base, s->first_x.as<uint32_t>(),
                               s->first_y.as<uint32_t>(), acc);
     if (s->pe) PDF_CUDA(cudaEventRecord(s->pe->ev[2], cs));  // cover starts (after any exchange)
     PDF_CUDA(launch_cover(ca, c->cover_grid, c->cover_threads, false, cs));  // closes the batch
@@ -1268,13 +1342,13 @@ extern "C" pdf_status pdf_sim(pdf_circuit *c, const pdf_pairs *pr, uint32_t *sim
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     std::lock_guard<std::mutex> lk(c->mu);
     const bool direct = planes_fit(c, W, ld, {sim_v, sim_t});
-    st = ensure_ws(c, c->full, c->stage, W, !direct);
+    st = ensure_ws(c, c->full_walk(), c->stage, W, !direct);
     if (st != PDF_OK) return st;
     const uint32_t *pv, *pt;
     uint64_t pld;
-    st = stage_pairs(c, c->stage, pr, &pv, &pt, &pld, cs);
+    st = stage_pairs(c, c->full_walk(), c->stage, pr, &pv, &pt, &pld, cs);
     if (st != PDF_OK) return st;
-    FwdArgs a = base_fwd(c, c->full, pr->n_pairs);
+    FwdArgs a = base_fwd(c, c->full_walk(), pr->n_pairs);
     a.pi_v = pv;
     a.pi_t = pt;
     a.pi_ld = pld;
@@ -1283,7 +1357,7 @@ extern "C" pdf_status pdf_sim(pdf_circuit *c, const pdf_pairs *pr, uint32_t *sim
         a.T = sim_t;
         a.ld = ld;
     } else {
-        use_ws_planes(a, c->full, c->stage, W);
+        use_ws_planes(a, c->full_walk(), c->stage, W);
     }
     PDF_CUDA(launch_forward(a, FWD_SIM, c->mark_mode, c->bw, c->full.threads, c->full.fwd_smem, cs));
     if (!direct) {
@@ -1304,16 +1378,16 @@ pdf_status mark_planes(pdf_circuit *c, const uint32_t *sim_v, const uint32_t *si
     std::lock_guard<std::mutex> lk(c->mu);
     const uint64_t W = (n_pairs + 31) / 32, G = c->info.n_gates;
     const bool direct = planes_fit(c, W, ld, {sim_v, sim_t, mark});
-    pdf_status st = ensure_ws(c, c->full, c->stage, W, !direct);
+    pdf_status st = ensure_ws(c, c->full_walk(), c->stage, W, !direct);
     if (st != PDF_OK) return st;
-    FwdArgs a = base_fwd(c, c->full, n_pairs);
+    FwdArgs a = base_fwd(c, c->full_walk(), n_pairs);
     if (direct) {
         a.V = const_cast<uint32_t *>(sim_v);
         a.T = const_cast<uint32_t *>(sim_t);
         a.M = mark;
         a.ld = ld;
     } else {
-        use_ws_planes(a, c->full, c->stage, W);
+        use_ws_planes(a, c->full_walk(), c->stage, W);
         PDF_CUDA(cudaMemcpy2DAsync(a.V, a.ld * 4, sim_v, ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
         PDF_CUDA(cudaMemcpy2DAsync(a.T, a.ld * 4, sim_t, ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
     }
@@ -1363,7 +1437,7 @@ pdf_status cover_chunk(pdf_circuit *c, pdf_state *s, const uint32_t *mark, uint6
                        uint64_t pair_base, uint64_t *counts, pdf_totals *chunk, cudaStream_t cs) {
     std::lock_guard<std::mutex> lk(s->mu);
     const uint64_t W = (n_pairs + 31) / 32;
-    pdf_status st = ensure_ws(c, c->full, s->ws, W, false);
+    pdf_status st = ensure_ws(c, c->full_walk(), s->ws, W, false);
     if (st != PDF_OK) return st;
     const size_t count_bytes = (size_t)c->info.n_pi * n_pairs * 16;
     if (counts) {
@@ -1372,7 +1446,7 @@ pdf_status cover_chunk(pdf_circuit *c, pdf_state *s, const uint32_t *mark, uint6
     }
     DevAcc *acc = s->acc.as<DevAcc>();
     PDF_CUDA(launch_batch_begin(acc, cs));
-    CoverArgs ca = base_cover(c, c->full, s->ws, mark, ld, n_pairs, (uint32_t)pair_base, s->first_x.as<uint32_t>(),
+    CoverArgs ca = base_cover(c, c->full_walk(), s->ws, mark, ld, n_pairs, (uint32_t)pair_base, s->first_x.as<uint32_t>(),
                               s->first_y.as<uint32_t>(), acc);
     // the bitmaps the cover reads, at its granularity, from the given marks
     PDF_CUDA(launch_bitmap_from_marks(c->full.dc, mark, ld, n_pairs, ca.bw, const_cast<uint32_t *>(ca.nzb),
@@ -1575,29 +1649,48 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
     // sized for its members), so the CTAs of narrow circuits share SMs
     // instead of holding the shared memory of the widest member; within a
     // class the longest CTA walks go first.
+    std::vector<Walk> walks(n_jobs);
+    uint64_t res_ctas = 0;
+    for (uint32_t i = 0; i < n_jobs; i++) {
+        Walk &k = walks[i] = jobs[i].circuit->lean_walk((jobs[i].pairs.n_pairs + 31) / 32);
+        if (!k.resident) continue;
+        // a CTA takes blocks worth about twice its copy of the image
+        const double load = 2.0 + k.p->res.image_bytes / 95e3;
+        k.rs.per = std::min(k.rs.blocks, 1 + (uint32_t)(2 * load / (k.rs.block_us * k.rs.occ)));
+        res_ctas += (k.rs.blocks + k.rs.per - 1) / k.rs.per;
+    }
+    // ... or fewer while that leaves SMs without a CTA
+    const uint64_t sms = c0->full.res.sms;
+    for (Walk &k : walks)
+        if (k.resident && res_ctas < 2 * sms)
+            k.rs.per = std::max<uint32_t>(1, (uint32_t)(k.rs.per * res_ctas / (2 * sms)));
+    const auto occ = [](const Walk &k) { return k.resident ? k.rs.occ : k.p->occ; };
     std::vector<uint32_t> order(n_jobs);
     for (uint32_t i = 0; i < n_jobs; i++) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
-        const Plan &px = jobs[x].circuit->lean(), &py = jobs[y].circuit->lean();
-        if (px.bw != py.bw) return px.bw > py.bw;
-        if (px.occ != py.occ) return px.occ < py.occ;
-        return px.chain > py.chain;
+        const Walk &kx = walks[x], &ky = walks[y];
+        if (kx.resident != ky.resident) return ky.resident;
+        if (kx.bw != ky.bw) return kx.bw > ky.bw;
+        if (occ(kx) != occ(ky)) return occ(kx) < occ(ky);
+        if (kx.resident) return kx.rs.per * kx.rs.block_us > ky.rs.per * ky.rs.block_us;
+        return kx.p->chain > ky.p->chain;
     });
     for (uint32_t k = 0; k < n_jobs; k++) {
         const pdf_batch_job &j = jobs[order[k]];
         const uint32_t i = k;
         pdf_circuit *c = j.circuit;
         pdf_state *s = j.state;
-        const Plan &p = c->lean();
+        const Walk &wk = walks[order[k]];
+        const Plan &p = *wk.p;
         const uint64_t n = j.pairs.n_pairs, W = (n + 31) / 32, G = p.n_gates;
-        if (ensure_ws(c, p, s->ws, W, true) != PDF_OK) return PDF_ENOMEM;
-        FwdArgs a = base_fwd(c, p, n);
+        if (ensure_ws(c, wk, s->ws, W, true) != PDF_OK) return PDF_ENOMEM;
+        FwdArgs a = base_fwd(c, wk, n);
         a.pi_v = j.pairs.v;
         a.pi_t = j.pairs.t;
         a.pi_ld = j.pairs.ld;
         a.store_all = 0;
         a.in_pieces = p.in_pieces;
-        use_ws_planes(a, p, s->ws, W);
+        use_ws_planes(a, wk, s->ws, W);
         a.nzb = s->ws.nzb.as<uint32_t>();
         a.blk_maxlvl = s->ws.maxlvl.as<uint32_t>();
         a.nzb_fine = s->ws.nzb_fine.as<uint32_t>();
@@ -1610,26 +1703,29 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
         a.acc = acc;
         a.active = s->ws.active.as<uint32_t>();
         fa[i] = a;
-        ca[i] = base_cover(c, p, s->ws, a.M, a.ld, n, (uint32_t)j.pair_base, a.first_x, a.first_y, acc);
-        const uint64_t blocks = (W + p.bw - 1) / p.bw;
+        ca[i] = base_cover(c, wk, s->ws, a.M, a.ld, n, (uint32_t)j.pair_base, a.first_x, a.first_y, acc);
+        const uint64_t blocks = wk.resident ? (wk.rs.blocks + wk.rs.per - 1) / wk.rs.per : (W + p.bw - 1) / p.bw;
         if (bp[i] + blocks > 0x7FFFFFFFull || gp[i] + G > 0xFFFFFFFFull) return PDF_ENOTSUP;
         bp[i + 1] = bp[i] + (uint32_t)blocks;
         gp[i + 1] = gp[i] + (uint32_t)G;
         items += std::min<uint64_t>(W * 32, 2 * G);
         L.tile = std::max(L.tile, c->bw);
         L.threads = std::max(L.threads, c->full.threads);
-        L.fwd_smem = std::max(L.fwd_smem, p.fwd_smem);
+        const size_t smem = wk.resident ? wk.rs.smem : p.fwd_smem;
+        L.fwd_smem = std::max(L.fwd_smem, smem);
         L.cover_grid = std::max(L.cover_grid, c->cover_grid);
-        if (!L.n_class || L.cls[L.n_class - 1].occ != p.occ || L.cls[L.n_class - 1].bw != p.bw) {
+        if (!L.n_class || L.cls[L.n_class - 1].occ != occ(wk) || L.cls[L.n_class - 1].bw != wk.bw ||
+            L.cls[L.n_class - 1].resident != (wk.resident ? 1u : 0u)) {
             if (L.n_class == kMaxBatchClasses) return PDF_ENOTSUP;
             BatchClass &k2 = L.cls[L.n_class++];
-            k2.bw = p.bw;
-            k2.occ = p.occ;
+            k2.bw = wk.bw;
+            k2.occ = occ(wk);
+            k2.resident = wk.resident ? 1u : 0u;
             k2.blk0 = bp[i];
         }
         BatchClass &cl = L.cls[L.n_class - 1];
-        cl.threads = std::max(cl.threads, p.threads);
-        cl.smem = std::max(cl.smem, p.fwd_smem);
+        cl.threads = std::max(cl.threads, wk.resident ? wk.rs.threads : p.threads);
+        cl.smem = std::max(cl.smem, smem);
         b->gate_evals += (uint64_t)c->info.n_gates * n;
         b->circuits.push_back(c);
         b->states.push_back(s);
@@ -1963,6 +2059,6 @@ extern "C" pdf_status pdf_state_reserve(pdf_state *s, uint64_t n_pairs) {
     if (!dg.ok) return PDF_ECUDA;
     std::lock_guard<std::mutex> lk(s->mu);
     const uint64_t W = (n_pairs + 31) / 32;
-    const pdf_status st = ensure_ws(s->c, s->c->lean(), s->ws, W, true);
-    return st == PDF_OK ? ensure_ws(s->c, s->c->full, s->ws, W, true) : st;
+    const pdf_status st = ensure_ws(s->c, s->c->lean_walk(W), s->ws, W, true);
+    return st == PDF_OK ? ensure_ws(s->c, s->c->full_walk(), s->ws, W, true) : st;
 }

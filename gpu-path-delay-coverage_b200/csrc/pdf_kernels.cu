@@ -15,14 +15,13 @@
 //               (every other pair credits nothing), over only the nets those
 //               pairs mark, in exact 128-bit integers.
 #include "pdf_kernels.cuh"
+#include "pdf_ptx.cuh"
 
 #include <algorithm>
 #include <map>
 #include <mutex>
 
 namespace {
-
-constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 
 __device__ __forceinline__ GateRec load_rec(const GateRec *p) {
     const uint4 *q = reinterpret_cast<const uint4 *>(p);
@@ -49,72 +48,7 @@ __device__ __forceinline__ void bitmap_set_aggregated(uint32_t *bm, uint32_t g) 
     if ((threadIdx.x & 31) == (uint32_t)(__ffs(grp) - 1)) atomicOr(bm + word, bits);
 }
 
-// The caller's id of gate g of a (possibly reduced) netlist, kEmpty for a
-// constant: the index of its first-detect ids.
-__device__ __forceinline__ uint32_t net_id(const DevCircuit &c, uint32_t g) { return c.orig ? __ldg(c.orig + g) : g; }
-
 __device__ __forceinline__ bool bit_test(const uint32_t *bm, uint32_t g) { return (bm[g >> 5] >> (g & 31)) & 1u; }
-
-// ---- TMA bulk copies and mbarriers (inline PTX, sm_90+ / sm_100a) ----
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t *m, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(m)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void fence_mbar_init() {
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void fence_proxy_async() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *m, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(m)), "r"(bytes)
-                 : "memory");
-}
-// One untiled bulk copy global -> shared; both addresses 16-byte aligned,
-// bytes a multiple of 16.
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *m) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(m))
-        : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *m, uint32_t phase) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(smem_u32(m)), "r"(phase)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_test_wait(uint64_t *m, uint32_t phase) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(smem_u32(m)), "r"(phase)
-        : "memory");
-    return ok != 0;
-}
-// Every wait is bounded: on expiry the caller reports PDF_ETIMEOUT.  polls =
-// 0: up to kSpinLimit blocking polls (try_wait may suspend the thread until
-// the phase completes); polls > 0: that many non-blocking polls, a bound
-// small enough to run out (tests of the timeout path).
-constexpr uint32_t kSpinLimit = 1u << 24;
-__device__ __forceinline__ bool mbar_wait(uint64_t *m, uint32_t phase, uint32_t polls = 0) {
-    if (polls) {
-        for (uint32_t i = 0; i < polls; i++)
-            if (mbar_test_wait(m, phase)) return true;
-        return false;
-    }
-    for (uint32_t i = 0; i < kSpinLimit; i++)
-        if (mbar_try_wait(m, phase)) return true;
-    return false;
-}
 
 // Asynchronous global -> shared copy of BW words (cp.async, completed by
 // cp.async.wait_all in the issuing thread).
@@ -1913,16 +1847,6 @@ __global__ void __launch_bounds__(kCoverThreads) k_cover_spill(const CoverArgs a
 // advances every circuit's pair_base by its pair count, so the next replay
 // grades the next vector pairs of each circuit.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t prefix_find(const uint32_t *pref, uint32_t n, uint32_t x) {
-    uint32_t lo = 0, hi = n;  // last i with pref[i] <= x
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(pref + mid) <= x) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
 // One launch per class of circuits (equal CTAs per SM): this launch's CTAs
 // are the batch's CTAs blk0 .. blk0 + gridDim.x - 1.
 template <int BW, int SEM>
@@ -1935,15 +1859,7 @@ __global__ void __launch_bounds__(BW >= 8 ? 512 : 1024)
         const uint32_t ci = prefix_find(bpref, n, gb);
         s_a = args[ci];
         s_blk = gb - __ldg(bpref + ci);
-        if (gb == 0) {
-            ctl->n_items = 0;
-            ctl->done = 0;
-            ctl->err = 0;
-            ctl->n_over = 0;
-            ctl->done_over = 0;
-            ctl->n_mid = 0;
-            ctl->done_mid = 0;
-        }
+        if (gb == 0) batch_begin(ctl);
     }
     __syncthreads();
     forward_cta<BW, SEM, FWD_FUSED>(s_a, s_blk);
@@ -1960,15 +1876,7 @@ __global__ void __launch_bounds__(lane_threads(32 * LW), 1)
         const uint32_t ci = prefix_find(bpref, n, gb);
         s_a = args[ci];
         s_blk = gb - __ldg(bpref + ci);
-        if (gb == 0) {
-            ctl->n_items = 0;
-            ctl->done = 0;
-            ctl->err = 0;
-            ctl->n_over = 0;
-            ctl->done_over = 0;
-            ctl->n_mid = 0;
-            ctl->done_mid = 0;
-        }
+        if (gb == 0) batch_begin(ctl);
     }
     __syncthreads();
     forward_lanes_cta<SEM, FWD_FUSED, LaneU<SEM, FWD_FUSED, LW>::value, LW>(s_a, s_blk);
@@ -2130,10 +2038,31 @@ __global__ void k_batch_begin(DevAcc *acc) {
     acc->done_over = 0;
 }
 
+}  // namespace
+
+// The dynamic shared-memory limit of a kernel on the current device, raised only
+// when a launch asks for more than any earlier one did (only this function
+// sets the limits, so a limit never falls below a request).
+cudaError_t raise_smem_limit(const void *fn, size_t smem) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, size_t> have;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    size_t &h = have[{dev, fn}];
+    if (smem <= h) return cudaSuccess;
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) h = smem;
+    return e;
+}
+
+namespace {
+
 template <int BW, int SEM, int MODE>
 cudaError_t launch_fwd_t(const FwdArgs &a, uint32_t threads, size_t smem, cudaStream_t st) {
     auto kern = k_forward<BW, SEM, MODE>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
     if (e != cudaSuccess) return e;
     const uint32_t blocks = (a.W + BW - 1) / BW;
     if (blocks == 0 || a.n_pieces == 0) return cudaErrorInvalidValue;
@@ -2144,7 +2073,7 @@ cudaError_t launch_fwd_t(const FwdArgs &a, uint32_t threads, size_t smem, cudaSt
 template <int SEM, int MODE, int LW>
 cudaError_t launch_lanes_t(const FwdArgs &a, uint32_t threads, size_t smem, cudaStream_t st) {
     auto kern = k_forward_lanes<SEM, MODE, LW>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
     if (e != cudaSuccess) return e;
     const uint32_t blocks = (a.W + 32 * LW - 1) / (32 * LW);
     if (blocks == 0 || threads % 32 || threads > lane_threads(32 * LW)) return cudaErrorInvalidValue;
@@ -2305,7 +2234,7 @@ cudaError_t launch_cover(const CoverArgs &a, uint32_t grid, uint32_t threads, bo
     }
     if (threads != kCoverThreads) return cudaErrorInvalidValue;
     const size_t smem = cover_smem_bytes(a.hash_cap);
-    cudaError_t e = cudaFuncSetAttribute(k_cover, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(k_cover), smem);
     if (e != cudaSuccess) return e;
     k_cover<<<grid, threads, smem, st>>>(a);
     if (a.spill_slots) {
@@ -2316,23 +2245,6 @@ cudaError_t launch_cover(const CoverArgs &a, uint32_t grid, uint32_t threads, bo
 }
 
 namespace {
-// The dynamic shared-memory limit of a batch kernel on the current device,
-// raised only when a batch asks for more than any earlier one did: a
-// serving loop rebinds its batch every step, and only these calls set the
-// batch kernels' limits, so the limit never falls below a request.
-cudaError_t raise_smem_limit(const void *fn, size_t smem) {
-    static std::mutex mu;
-    static std::map<std::pair<int, const void *>, size_t> have;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lk(mu);
-    size_t &h = have[{dev, fn}];
-    if (smem <= h) return cudaSuccess;
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) h = smem;
-    return e;
-}
 template <typename F>
 cudaError_t raise_smem(F *fn, size_t smem) {
     return raise_smem_limit(reinterpret_cast<const void *>(fn), smem);
@@ -2394,11 +2306,8 @@ cudaError_t launch_class(const BatchLaunch &b, const BatchClass &c, cudaStream_t
 
 cudaError_t prepare_batch(const BatchLaunch &b) {
     for (uint32_t k = 0; k < b.n_class; k++) {
-        // every class of one tile width shares its kernel: the largest request wins
-        size_t smem = 0;
-        for (uint32_t j = 0; j < b.n_class; j++)
-            if (b.cls[j].bw == b.cls[k].bw) smem = std::max(smem, b.cls[j].smem);
-        const cudaError_t e = prepare_class(b.sem, b.cls[k].bw, smem);
+        const BatchClass &c = b.cls[k];
+        const cudaError_t e = c.resident ? prepare_resident_class(b.sem, c.bw, c.smem) : prepare_class(b.sem, c.bw, c.smem);
         if (e != cudaSuccess) return e;
     }
     const cudaError_t e = raise_smem(k_batch_cover<0>, cover_small_smem_bytes(b.small_cap));
@@ -2427,7 +2336,7 @@ cudaError_t launch_batch(const BatchLaunch &b, cudaStream_t st) {
             s = b.side[k - 1];
             if ((e = cudaStreamWaitEvent(s, b.fork, 0)) != cudaSuccess) return e;
         }
-        if ((e = launch_class(b, c, s)) != cudaSuccess) return e;
+        if ((e = c.resident ? launch_resident_class(b, c, s) : launch_class(b, c, s)) != cudaSuccess) return e;
         if (s != st) {
             if ((e = cudaEventRecord(b.join[k - 1], s)) != cudaSuccess) return e;
             if ((e = cudaStreamWaitEvent(st, b.join[k - 1], 0)) != cudaSuccess) return e;

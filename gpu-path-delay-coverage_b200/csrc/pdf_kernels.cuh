@@ -73,6 +73,11 @@ struct FwdArgs {
     uint32_t pair_base;
     uint32_t ring_gates;          // forward ring slots R (power of two, >= cap)
     uint32_t ring2_gates;         // reverse ring slots (power of two, or 0)
+    // resident kernel: the netlist's image in device memory, column blocks per
+    // CTA and in all (off_edge, off_fid, off_ring, off_rec: its edges, level
+    // table, V / T words and marks)
+    const void *image;
+    uint32_t image_bytes, per, n_blocks;
     // shared-memory byte offsets
     uint32_t off_ring;            // forward: ring [3][R][BW]; reverse: ring2 [R2][BW]
     uint32_t off_rec;             // [2][cap] staged gate records
@@ -161,8 +166,9 @@ constexpr uint32_t lane_threads(uint32_t bw) {
 // block, an eighth of a 64-word one, ...).
 constexpr uint32_t kLaneCoverWords = 8;
 // Forward launches of a batch at most: (tile width, CTAs per SM) classes of
-// the thread-per-gate kernel and the two lane tiles.
-constexpr uint32_t kMaxBatchClasses = 20;
+// the thread-per-gate kernel, the lane tiles, and (tile width, CTAs per SM)
+// classes of the resident kernel.
+constexpr uint32_t kMaxBatchClasses = 40;
 
 // Batched grading (k_batch_forward, k_batch_active, k_batch_cover).
 struct BatchCtl {
@@ -175,9 +181,9 @@ struct BatchCtl {
     unsigned int done_mid;
     unsigned int pad[1];
 };
-// One forward launch of a batch: jobs of equal tile width and CTAs per SM.
+// One forward launch of a batch: jobs of one kernel, tile width and CTAs per SM.
 struct BatchClass {
-    uint32_t bw, occ, blk0, blocks, threads;
+    uint32_t bw, occ, resident, blk0, blocks, threads;
     size_t smem;
 };
 struct BatchLaunch {
@@ -212,6 +218,16 @@ struct BatchLaunch {
 int forward_kernel_regs(int bw, int sem);
 cudaError_t prepare_batch(const BatchLaunch &b);  // kernel attributes; call before launching or capturing
 cudaError_t launch_batch(const BatchLaunch &b, cudaStream_t st);
+
+// The resident forward kernel (pdf_resident.cu): threads per CTA at most, and
+// its launches.
+constexpr uint32_t kResidentThreads = 512;
+cudaError_t launch_resident(const FwdArgs &a, int sem, uint32_t bw, uint32_t ctas, uint32_t threads, size_t smem,
+                            cudaStream_t st);
+cudaError_t prepare_resident_class(uint32_t sem, uint32_t bw, size_t smem);
+cudaError_t launch_resident_class(const BatchLaunch &b, const BatchClass &c, cudaStream_t st);
+// Raises a kernel's dynamic shared-memory limit on the current device.
+cudaError_t raise_smem_limit(const void *fn, size_t smem);
 
 // Host-side launchers (pdf_kernels.cu).  All return cudaError_t of the launch.
 cudaError_t launch_forward(const FwdArgs &a, int mode, int sem, uint32_t bw, uint32_t threads,

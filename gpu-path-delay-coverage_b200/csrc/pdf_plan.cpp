@@ -5,13 +5,11 @@
 
 #include "pdf_kernels.cuh"
 
-pdf_status build_plan(const NetPlan &n, const PlanOpts &o, LaunchPlan &pl) {
-    const uint32_t G = n.n_gates(), L = n.n_levels();
-    uint32_t widest_level = 0;
-    for (uint32_t l = 0; l < L; l++) widest_level = std::max(widest_level, n.level_off[l + 1] - n.level_off[l]);
+void build_records(const NetPlan &n, LaunchPlan &pl) {
+    const uint32_t G = n.n_gates();
     pl.n_gates = G;
-    pl.n_levels = L;
-    pl.bw = o.bw;
+    pl.n_levels = n.n_levels();
+    pl.nfo_mask = 0xFFFFFFFFu;
     pl.recs.assign(G, GateRec{});
     for (uint32_t g = 0; g < G; g++) {
         GateRec &r = pl.recs[g];
@@ -21,6 +19,105 @@ pdf_status build_plan(const NetPlan &n, const PlanOpts &o, LaunchPlan &pl) {
         // fan-in 0; of an input, its row in the pair planes
         r.w[7] = n.nfi[g] ? n.edges[n.eoff[g]] : (n.hdr[g] & RF_INPT ? (n.orig.empty() ? g : n.orig[g]) : 0u);
     }
+}
+
+ResidentImage build_resident(const NetPlan &n, size_t smem) {
+    ResidentImage im;
+    const uint32_t G = n.n_gates(), L = n.n_levels();
+    if (G > 0xFFFFu || L > 0xFFFFu || (size_t)G * 28 > smem) return im;
+    uint64_t n_edge = 0;
+    for (uint32_t g = 0; g < G; g++) n_edge += n.nfo[g] + (n.nfi[g] > kInlineFanins ? n.nfi[g] : 0);
+    if (n_edge > 0xFFFFu) return im;
+    const auto a16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
+    const size_t o_edge = 16 * ((size_t)G + 1), o_lvl = o_edge + a16(2 * n_edge), total = o_lvl + a16(8 * ((size_t)L + 1));
+    if (total + (size_t)G * 12 + a16((G + 31) / 32 * 4) + 64 > smem) return im;  // one word per block at least
+    // how far each gate's mark reaches: the last level of the gates it carries to
+    std::vector<uint16_t> reach(G, 0);
+    for (uint32_t l = 0; l < L; l++)
+        for (uint32_t g = n.level_off[l]; g < n.level_off[l + 1]; g++) {
+            const uint32_t *fin = n.edges.data() + n.eoff[g];
+            if (n.hdr[g] & RF_MANY)
+                for (uint32_t q = 0; q < n.nfi[g]; q++) reach[fin[q]] = (uint16_t)l;
+            else if ((n.hdr[g] & RF_MARKF0) && n.nfi[g])
+                reach[fin[0]] = (uint16_t)l;
+        }
+    im.bytes.assign(total, 0);
+    im.off_edge = (uint32_t)o_edge;
+    im.off_lvl = (uint32_t)o_lvl;
+    uint32_t *rec = reinterpret_cast<uint32_t *>(im.bytes.data());
+    uint16_t *edge = reinterpret_cast<uint16_t *>(im.bytes.data() + o_edge);
+    uint32_t *lvl = reinterpret_cast<uint32_t *>(im.bytes.data() + o_lvl), at = 0;
+    for (uint32_t g = 0; g < G; g++) {
+        const uint32_t *e = n.edges.data() + n.eoff[g], nfi = n.nfi[g];
+        uint32_t *r = rec + 4 * (size_t)g, f[4] = {0, 0, 0, 0};
+        for (uint32_t q = 0; q < nfi && q < 4; q++) f[q] = e[q];
+        r[0] = n.hdr[g];
+        r[1] = f[0] | f[1] << 16;
+        r[2] = f[2] | f[3] << 16;
+        if (n.hdr[g] & RF_INPT) r[1] = n.orig.empty() ? g : n.orig[g];
+        r[3] = at | (uint32_t)reach[g] << 16;
+        for (uint32_t q = nfi > kInlineFanins ? 0 : nfi; q < nfi + n.nfo[g]; q++) edge[at++] = (uint16_t)e[q];
+    }
+    rec[4 * (size_t)G + 3] = at;
+    for (uint32_t l = 0; l <= L; l++) {
+        lvl[2 * l] = n.level_off[l];
+        // gates up to the last that marks (a reduced netlist lists those first)
+        if (l < L)
+            for (uint32_t g = n.level_off[l]; g < n.level_off[l + 1]; g++)
+                if (n.hdr[g] & (RF_MARKF0 | RF_MANY)) lvl[2 * l + 1] = g + 1 - n.level_off[l];
+    }
+    return im;
+}
+
+// Column block and CTAs of a resident walk over W words: the block width with
+// the least modelled time.  A block costs its level chain (forward and prune,
+// about 0.3 us a level, of as many blocks at once as CTAs fit an SM) or its
+// instructions (about 0.42 ns per gate and word of an SM), whichever is more;
+// a CTA the copy of the image first, shared by the blocks it takes in turn.
+ResidentShape resident_shape(const ResidentSizes &z, uint64_t W) {
+    const auto al = [](size_t x) { return (x + 15) & ~(size_t)15; };
+    ResidentShape best;
+    double best_t = 0;
+    for (uint32_t bw = 1; bw <= 8; bw *= 2) {
+        ResidentShape s;
+        s.bw = bw;
+        size_t off = al(z.image_bytes);
+        s.off_vt = (uint32_t)off;
+        off += 8 * (size_t)bw * z.n_gates;
+        s.off_m = (uint32_t)off;
+        off = al(off + 4 * (size_t)bw * z.n_gates);
+        s.off_bm = (uint32_t)off;
+        off = al(off + ((size_t)z.n_gates + 31) / 32 * 4);
+        s.off_mbar = (uint32_t)off;
+        s.smem = off + 16;
+        if (s.smem + 1024 > z.smem_block) break;  // (and the kernels' static variables)
+        const uint32_t by_smem = (uint32_t)std::max<size_t>(1, z.smem_sm / (s.smem + 2048));
+        s.threads = by_smem >= 2 ? 256 : 512;
+        s.occ = std::min({by_smem, 2048 / s.threads, 65536 / (s.threads * std::max(z.regs, 32u)), 8u});
+        while (s.occ & (s.occ - 1)) s.occ &= s.occ - 1;  // 1, 2, 4 or 8: few classes in a batch
+        s.blocks = (uint32_t)((W + bw - 1) / bw);
+        const uint32_t slots = z.sms * s.occ;
+        s.per = (s.blocks + slots - 1) / slots;
+        s.ctas = (s.blocks + s.per - 1) / s.per;
+        const double load = 2.0 + z.image_bytes / 95e3, chain = 1.0 + 0.3 * z.n_levels;
+        const uint32_t together = std::min(s.occ, (s.ctas + z.sms - 1) / z.sms);
+        const double issue = 0.42e-3 * z.n_gates * bw;
+        s.block_us = std::max(chain / s.occ, issue);
+        const double t = load + s.per * std::max(chain, together * issue);
+        if (!best.bw || t < best_t * 0.97) {
+            best = s;
+            best_t = t;
+        }
+    }
+    return best;
+}
+
+pdf_status build_plan(const NetPlan &n, const PlanOpts &o, LaunchPlan &pl) {
+    const uint32_t G = n.n_gates(), L = n.n_levels();
+    uint32_t widest_level = 0;
+    for (uint32_t l = 0; l < L; l++) widest_level = std::max(widest_level, n.level_off[l + 1] - n.level_off[l]);
+    build_records(n, pl);
+    pl.bw = o.bw;
     const bool lanes = lane_tile(pl.bw);
     if (lanes) {
         // The lane kernel reads every fan-in from its plane row: source words

@@ -31,12 +31,41 @@ struct PlanShape {
     uint64_t chain = 0;  // length of one CTA's walk (pieces, or gates for the lane kernel)
 };
 
+// The image of a netlist that the resident kernel keeps in shared memory: 16
+// bytes per gate (header; fan-ins 0..3 as 16-bit ids, of an input its row in
+// the pair planes; edge offset | last level its mark reaches << 16) and one
+// more for the end of the edges, 16-bit edges (fan-ins of gates with more
+// than four, then fan-outs), and per level its first gate and how many of its
+// gates may hold a mark after the prune.
+struct ResidentImage {
+    std::vector<unsigned char> bytes;  // empty: the netlist does not fit
+    uint32_t off_edge = 0, off_lvl = 0;
+};
+// `smem`: dynamic shared memory a CTA may have.
+ResidentImage build_resident(const NetPlan &n, size_t smem);
+
+// Shared memory and column blocks of one resident walk.
+struct ResidentShape {
+    uint32_t bw = 0, threads = 0, per = 0, ctas = 0, occ = 0, blocks = 0;
+    uint32_t off_vt = 0, off_m = 0, off_bm = 0, off_mbar = 0;
+    size_t smem = 0;
+    double block_us = 0;  // modelled time of one column block
+};
+struct ResidentSizes {
+    uint32_t n_gates = 0, n_levels = 0, image_bytes = 0;
+    uint32_t sms = 0, regs = 0;
+    size_t smem_block = 0, smem_sm = 0;
+};
+ResidentShape resident_shape(const ResidentSizes &z, uint64_t W);
+
 struct LaunchPlan : PlanShape {
     std::vector<GateRec> recs;
     std::vector<Piece> pieces;
     std::vector<uint32_t> far_ids;
 };
 
+// Records only (what the cover reads), for a netlist that the resident kernel walks.
+void build_records(const NetPlan &n, LaunchPlan &pl);
 pdf_status build_plan(const NetPlan &n, const PlanOpts &o, LaunchPlan &pl);
 
 #endif

@@ -1,0 +1,316 @@
+// pdf_resident.cu -- the resident forward kernel: sim, forward mark, prune
+// and merge of a netlist that fits on chip.
+//
+// What bounds such a walk is its chain of levels, not bytes: the staged
+// kernel (forward_cta) pays a piece descriptor, a TMA copy and a barrier of a
+// whole CTA for every level, about 1 us each, on levels of a few dozen gates.
+// Here a CTA brings the whole netlist into shared memory with one bulk copy
+// (16-byte records and 16-bit edges, the image that build_resident lays out),
+// keeps every gate's V, T and M words there, and then takes a level in one
+// shared-memory round trip and one barrier.  A thread is one (gate, word) of
+// the block of BW words: narrow levels still give BW times their gates in
+// threads.  Only the surviving marks (for the cover) and the first-detecting
+// pairs leave the SM.  A CTA grades `per` column blocks one after another, so
+// the image is read once per CTA.
+//
+// Measured (B200, whole call with cover and reset, us): a 20,000-gate
+// circuit's 523 needed gates at 32,768 pairs 121 -> MEDIUM_NOW; 2,000 gates at
+// 1,024 pairs 67 -> SMALL_NOW.
+#include "pdf_kernels.cuh"
+#include "pdf_ptx.cuh"
+
+#include <algorithm>
+
+namespace {
+
+template <int BW, int SEM>
+__device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t cta) {
+    constexpr bool FIX = SEM >= 2;
+    constexpr uint32_t kGroup = BW == 32 ? 0xFFFFFFFFu : (1u << BW) - 1u;
+    extern __shared__ __align__(128) unsigned char smraw[];
+    const uint4 *rec = reinterpret_cast<const uint4 *>(smraw);
+    const uint16_t *edge = reinterpret_cast<const uint16_t *>(smraw + a.off_edge);
+    const uint2 *lvl = reinterpret_cast<const uint2 *>(smraw + a.off_fid);  // first gate, observable gates
+    uint2 *vt = reinterpret_cast<uint2 *>(smraw + a.off_ring);              // [gate][BW] V, T
+    uint32_t *ms = reinterpret_cast<uint32_t *>(smraw + a.off_rec);         // [gate][BW] marks
+    uint32_t *bm = reinterpret_cast<uint32_t *>(smraw + a.off_bm);
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(smraw + a.off_mbar);
+    __shared__ uint32_t s_reach, s_top, s_max;
+    const uint32_t tid = threadIdx.x, NT = blockDim.x, lane = tid & 31;
+    const uint32_t L = a.c.n_levels;
+    const uint32_t b0 = cta * a.per, b1 = min(a.n_blocks, b0 + a.per);
+    if (tid == 0) {
+        mbar_init(mbar, 1);
+        fence_mbar_init();
+        mbar_expect_tx(mbar, a.image_bytes);
+        bulk_g2s(smraw, a.image, a.image_bytes, mbar);
+    }
+    // the batch's cover state (the cover kernels run after this one)
+    if (a.active) {
+        for (uint32_t w = b0 * BW + tid; w < min(a.W, b1 * BW); w += NT) a.active[w] = 0;
+        if (b1 == a.n_blocks && tid == 0) a.active[a.W] = 0;
+    }
+    if (a.acc && cta == 0 && tid == 0) {
+        a.acc->batch_lo = 0;
+        a.acc->batch_hi = 0;
+        a.acc->batch_flags = 0;
+        a.acc->done = 0;
+        a.acc->n_over = 0;
+        a.acc->done_over = 0;
+    }
+    __syncthreads();
+    if (__syncthreads_or(!mbar_wait(mbar, 0, a.wait_polls))) {
+        // no CTA leaves with a copy in flight; its blocks are published empty
+        (void)mbar_wait(mbar, 0);
+        for (uint32_t blk = b0; blk < b1; blk++) {
+            for (uint32_t q = tid; q < a.bm_words; q += NT) a.nzb[(size_t)blk * a.bm_words + q] = 0;
+            if (tid == 0) a.blk_maxlvl[blk] = 0;
+        }
+        if (tid == 0) atomicOr(a.err, kErrTimeout);
+        return;
+    }
+    const uint32_t j = tid & (BW - 1);         // this thread's word of the block (NT is a multiple of BW)
+    const uint32_t step = NT / BW;             // gates per pass
+    for (uint32_t blk = b0; blk < b1; blk++) {
+        const uint32_t w = blk * BW + j;
+        const uint32_t wm = w + 1 < a.W ? 0xFFFFFFFFu
+                                        : (w + 1 == a.W ? ((a.n_pairs & 31) ? (1u << (a.n_pairs & 31)) - 1u : 0xFFFFFFFFu)
+                                                        : 0u);
+        for (uint32_t q = tid; q < a.bm_words; q += NT) bm[q] = 0;
+        if (tid == 0) {
+            s_reach = 0;
+            s_top = 0;
+            s_max = 0;
+        }
+        // ---- level 0: inputs (simkernel.cuh:112-125) and the constants; four
+        // input words in flight per thread
+        uint32_t my_reach = 0;
+        bool any = false;
+        const uint32_t n0 = lvl[1].x;
+        __syncthreads();
+        for (uint32_t g0 = tid / BW; g0 < n0; g0 += 4 * step) {
+            uint32_t h[4], v[4], t[4], rw[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint32_t g = g0 + u * step;
+                h[u] = v[u] = t[u] = 0;
+                if (g >= n0) continue;
+                const uint4 r = rec[g];
+                h[u] = r.x;
+                rw[u] = r.w;
+                if ((r.x & RF_INPT) && wm) {
+                    v[u] = __ldg(a.pi_v + (size_t)r.y * a.pi_ld + w);
+                    t[u] = __ldg(a.pi_t + (size_t)r.y * a.pi_ld + w);
+                } else if (r.x & RF_OINV) {
+                    v[u] = 0xFFFFFFFFu;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint32_t g = g0 + u * step;
+                if (g >= n0) continue;
+                const uint32_t T = t[u] & wm, M = T & flagmask(h[u], RF_MARKF0);
+                vt[g * BW + j] = make_uint2(v[u] & wm, T);
+                ms[g * BW + j] = M;
+                if (M) {
+                    any = true;
+                    my_reach = max(my_reach, rw[u] >> 16);
+                }
+            }
+        }
+        // ---- the levels above (simkernel.cuh:126-149, markkernel.cuh:226-267),
+        // until no marked gate carries further
+        for (uint32_t l = 0;; l++) {
+            if (l) {
+                any = false;
+                const uint32_t g1 = lvl[l + 1].x;
+                for (uint32_t g = lvl[l].x + tid / BW; g < g1; g += step) {
+                    const uint4 r = rec[g];
+                    const uint32_t h = r.x, nfi = (h >> 8) & 0xFFu, nfold = hdr_nfold(h), eo = r.w & 0xFFFFu;
+                    const auto fan = [&](uint32_t q) -> uint32_t {
+                        return q < 4 ? ((q < 2 ? r.y : r.z) >> (16 * (q & 1))) & 0xFFFFu : edge[eo + q];
+                    };
+                    uint2 f[kInlineFanins];  // fan-ins 0..3
+#pragma unroll
+                    for (int q = 0; q < kInlineFanins; q++)
+                        if ((uint32_t)q < nfi) f[q] = vt[fan(q) * BW + j];
+                    uint32_t V, T, v1, M = 0;
+                    eval_first(h, f[0].x, f[0].y, V, v1);
+#pragma unroll
+                    for (int q = 1; q < kInlineFanins; q++)
+                        if ((uint32_t)q <= nfold) eval_fold<FIX>(h, V, v1, f[q].x, f[q].y);
+                    for (uint32_t q = kInlineFanins; q <= nfold; q++) {
+                        const uint2 x = vt[fan(q) * BW + j];
+                        eval_fold<FIX>(h, V, v1, x.x, x.y);
+                    }
+                    eval_finish<FIX>(h, V, v1, T);
+                    V &= wm;
+                    T &= wm;
+                    if ((h & RF_MARKF0) && T) {
+                        M = T & ms[fan(0) * BW + j];
+                        if ((h & RF_SENS) && M) {
+                            SensAcc s;
+                            sens_init(s);
+                            const bool or_like = (h & RF_IM) != 0;
+#pragma unroll
+                            for (int q = 0; q < kInlineFanins; q++)
+                                if ((uint32_t)q < nfi) sens_step<SEM & 1>(s, or_like, f[q].x, f[q].y);
+                            for (uint32_t q = kInlineFanins; q < nfi; q++) {
+                                const uint2 x = vt[fan(q) * BW + j];
+                                sens_step<SEM & 1>(s, or_like, x.x, x.y);
+                            }
+                            M &= sens_result<SEM & 1>(s);
+                        }
+                    } else if (FIX && (h & RF_MANY) && T) {
+                        const uint32_t mor = flagmask(h, RF_IM), mxor = flagmask(h, RF_XOR), mand = ~(mor | mxor);
+                        SensAcc s;
+                        sens_init(s);
+#pragma unroll
+                        for (int q = 0; q < kInlineFanins; q++)
+                            if ((uint32_t)q < nfi)
+                                sens_step_fixed<SEM == PDF_MARK_FIXED_NONROBUST>(s, mand, mor, mxor, f[q].x, f[q].y,
+                                                                                 ms[fan(q) * BW + j]);
+                        for (uint32_t q = kInlineFanins; q < nfi; q++) {
+                            const uint2 x = vt[fan(q) * BW + j];
+                            sens_step_fixed<SEM == PDF_MARK_FIXED_NONROBUST>(s, mand, mor, mxor, x.x, x.y,
+                                                                             ms[fan(q) * BW + j]);
+                        }
+                        M = T & sens_result<SEM == PDF_MARK_FIXED_NONROBUST>(s);
+                    }
+                    vt[g * BW + j] = make_uint2(V, T);
+                    ms[g * BW + j] = M;
+                    if (M) {
+                        any = true;
+                        my_reach = max(my_reach, r.w >> 16);
+                    }
+                }
+            }
+            if (__any_sync(0xFFFFFFFFu, any)) {
+                const uint32_t wr = __reduce_max_sync(0xFFFFFFFFu, my_reach);
+                if (lane == 0) {
+                    s_top = l + 1;  // every warp that stores in level l stores this
+                    if (wr > l) atomicMax(&s_reach, wr);
+                }
+            }
+            __syncthreads();
+            // s_reach grows past l only in threads that go on, so all decide alike
+            if (l + 1 >= L || s_reach <= l) break;
+        }
+        // ---- prune (markkernel.cuh:271-293) and merge (mergekernel.cuh:116-198),
+        // levels descending: a gate's mark is final once its fan-outs' are.
+        // Gates from level s_top on hold no mark, and past the last level walked
+        // their words are not this block's.
+        const uint32_t g_top = lvl[s_top].x;
+        for (int l = (int)s_top - 1; l >= 0; l--) {
+            const uint2 lv = lvl[l];
+            for (uint32_t k0 = 0; k0 < lv.y; k0 += step) {
+                const uint32_t k = k0 + tid / BW, g = lv.x + k;
+                uint32_t nm = 0;
+                if (k < lv.y) {
+                    const uint32_t m = ms[g * BW + j];
+                    if (m) {
+                        const uint4 r = rec[g];
+                        uint32_t keep = (r.x & (1u << 4)) ? 0xFFFFFFFFu : 0u;
+                        if (!keep) {
+                            const uint32_t nfi = (r.x >> 8) & 0xFFu, e1 = rec[g + 1].w & 0xFFFFu;
+                            for (uint32_t e = (r.w & 0xFFFFu) + (nfi > kInlineFanins ? nfi : 0); e < e1; e++)
+                                if (edge[e] < g_top) keep |= ms[(uint32_t)edge[e] * BW + j];
+                        }
+                        nm = m & keep;
+                        if (nm != m) ms[g * BW + j] = nm;
+                    }
+                }
+                const uint32_t z = __ballot_sync(0xFFFFFFFFu, nm != 0);
+                if (!z) continue;  // the same on every lane
+                const uint32_t sh = lane & ~(uint32_t)(BW - 1), below = (1u << j) - 1u;
+                const uint32_t V = nm ? vt[g * BW + j].x : 0u, x = nm & ~V, y = nm & V;
+                const uint32_t bx = (__ballot_sync(0xFFFFFFFFu, x != 0) >> sh) & kGroup;
+                const uint32_t by = (__ballot_sync(0xFFFFFFFFu, y != 0) >> sh) & kGroup;
+                if ((z >> sh) & kGroup) {  // the gate keeps a mark in the block
+                    a.M[(size_t)g * a.ld + w] = nm;  // (rows hold whole blocks)
+                    if (j == 0) atomicOr(bm + (g >> 5), 1u << (g & 31));
+                    // the lowest word of each direction holds its first pair
+                    if (x && !(bx & below)) atomicMin(a.first_x + net_id(a.c, g), a.pair_base + w * 32 + (__ffs(x) - 1));
+                    if (y && !(by & below)) atomicMin(a.first_y + net_id(a.c, g), a.pair_base + w * 32 + (__ffs(y) - 1));
+                }
+                if (lane == 0) atomicMax(&s_max, (uint32_t)l + 1);
+            }
+            __syncthreads();
+        }
+        // the bitmap of surviving marks, for the cover kernels
+        for (uint32_t q = tid; q < a.bm_words; q += NT) a.nzb[(size_t)blk * a.bm_words + q] = bm[q];
+        if (tid == 0) a.blk_maxlvl[blk] = s_max;
+        __syncthreads();
+    }
+}
+
+template <int BW, int SEM>
+__global__ void __launch_bounds__(kResidentThreads) k_resident(const FwdArgs a) {
+    resident_cta<BW, SEM>(a, blockIdx.x);
+}
+
+// The circuits of a batch whose netlists fit on chip.
+template <int BW, int SEM>
+__global__ void __launch_bounds__(kResidentThreads)
+    k_batch_resident(const FwdArgs *args, const uint32_t *bpref, uint32_t n, BatchCtl *ctl, uint32_t blk0) {
+    __shared__ FwdArgs s_a;
+    __shared__ uint32_t s_blk;
+    if (threadIdx.x == 0) {
+        const uint32_t gb = blk0 + blockIdx.x;
+        const uint32_t ci = prefix_find(bpref, n, gb);
+        s_a = args[ci];
+        s_blk = gb - __ldg(bpref + ci);
+        if (gb == 0) batch_begin(ctl);
+    }
+    __syncthreads();
+    resident_cta<BW, SEM>(s_a, s_blk);
+}
+
+template <int BW, int SEM>
+cudaError_t launch_t(const FwdArgs &a, uint32_t ctas, uint32_t threads, size_t smem, cudaStream_t st) {
+    const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(k_resident<BW, SEM>), smem);
+    if (e != cudaSuccess) return e;
+    if (!ctas || threads % 32 || threads > kResidentThreads) return cudaErrorInvalidValue;
+    k_resident<BW, SEM><<<ctas, threads, smem, st>>>(a);
+    return cudaGetLastError();
+}
+template <int BW, int SEM>
+cudaError_t launch_batch_t(const BatchLaunch &b, const BatchClass &c, cudaStream_t st) {
+    k_batch_resident<BW, SEM><<<c.blocks, c.threads, c.smem, st>>>(b.fargs, b.bpref, b.n, b.ctl, c.blk0);
+    return cudaGetLastError();
+}
+
+// f<BW, SEM>() for run-time values.
+#define PDF_RES_SEM(BW, F, ...)                      \
+    switch (sem) {                                   \
+        case 0: return F<BW, 0>(__VA_ARGS__);        \
+        case 1: return F<BW, 1>(__VA_ARGS__);        \
+        case 2: return F<BW, 2>(__VA_ARGS__);        \
+        case 3: return F<BW, 3>(__VA_ARGS__);        \
+        default: return cudaErrorInvalidValue;       \
+    }
+#define PDF_RES(F, ...)                              \
+    switch (bw) {                                    \
+        case 1: PDF_RES_SEM(1, F, __VA_ARGS__)       \
+        case 2: PDF_RES_SEM(2, F, __VA_ARGS__)       \
+        case 4: PDF_RES_SEM(4, F, __VA_ARGS__)       \
+        case 8: PDF_RES_SEM(8, F, __VA_ARGS__)       \
+        default: return cudaErrorInvalidValue;       \
+    }
+
+template <int BW, int SEM>
+cudaError_t raise_batch_t(size_t smem) {
+    return raise_smem_limit(reinterpret_cast<const void *>(k_batch_resident<BW, SEM>), smem);
+}
+
+}  // namespace
+
+cudaError_t launch_resident(const FwdArgs &a, int sem, uint32_t bw, uint32_t ctas, uint32_t threads, size_t smem,
+                            cudaStream_t st) {
+    PDF_RES(launch_t, a, ctas, threads, smem, st)
+}
+cudaError_t prepare_resident_class(uint32_t sem, uint32_t bw, size_t smem) { PDF_RES(raise_batch_t, smem) }
+cudaError_t launch_resident_class(const BatchLaunch &b, const BatchClass &c, cudaStream_t st) {
+    const uint32_t sem = b.sem, bw = c.bw;
+    PDF_RES(launch_batch_t, b, c, st)
+}

@@ -137,6 +137,7 @@ struct DeviceGuard {
 struct Workspace {
     DevBuf nzb, maxlvl, active, active_list;
     DevBuf over_list, spill;  // pairs for the spill cover and its per-net (h, c) slots
+    DevBuf flags, sync;       // wide kernel: mark flags per (segment, gate), barrier counters
     DevBuf nzb_fine, maxlvl_fine;  // lane circuits: the cover's bitmaps per quarter column block
     DevBuf pi_counts;         // pdf_cover_counts: paths per (primary input, pair)
     DevBuf seg_first;  // (net, pair) hash set of the cover with segments
@@ -150,6 +151,8 @@ struct Workspace {
         active_list.release();
         over_list.release();
         spill.release();
+        flags.release();
+        sync.release();
         nzb_fine.release();
         maxlvl_fine.release();
         pi_counts.release();
@@ -167,6 +170,8 @@ struct Plan : PlanShape {
     DevCircuit dc{};
     const Piece *pieces = nullptr;
     const uint32_t *far_ids = nullptr;
+    bool wide = false;  // its staged walk is the wide kernel's (a lane plan)
+    uint32_t mean_width = 0;
     // the resident kernel's image of the netlist (null: it does not fit)
     const void *image = nullptr;
     uint32_t off_edge_im = 0, off_lvl_im = 0;
@@ -181,6 +186,10 @@ struct Walk {
     const Plan *p = nullptr;
     uint32_t bw = 0;
     bool resident = false;
+    // wide kernel: words per lane (0: not it), its chunks per segment and segments
+    uint32_t wide = 0, cps = 0, nseg = 0, chunks = 0;
+    // the cover's bitmaps are per kLaneCoverWords words
+    bool fine() const { return wide || (!resident && lane_tile(bw)); }
     ResidentShape rs;
 };
 
@@ -265,12 +274,41 @@ struct pdf_circuit {
     Plan full, red;   // every gate; the reduced netlist (n_gates 0: none)
     // the plan of grading calls that ask for no plane
     const Plan &lean() const { return red.n_gates ? red : full; }
-    Walk full_walk() const { return Walk{&full, full.bw, false, {}}; }
+    // The wide kernel's shape with lw words per lane: the segment length with
+    // the fewest rounds of chunks (and about 1.5 chunks' worth per gate).
+    void wide_shape(Walk &k, uint64_t W, uint32_t lw) const {
+        k.wide = lw;
+        k.chunks = (uint32_t)((W + 32 * lw - 1) / (32 * lw));
+        const uint64_t warps = (uint64_t)k.p->res.sms * kWideCtas * (kWideThreads / 32);
+        double best = 0;
+        for (uint32_t cps = 1; cps <= 8; cps *= 2) {
+            const uint64_t items = (uint64_t)k.p->mean_width * ((k.chunks + cps - 1) / cps);
+            const double t = (double)((items + warps - 1) / warps) * (cps + 1.5);
+            if (!k.cps || t < best) {
+                k.cps = cps;
+                best = t;
+            }
+        }
+        k.nseg = (k.chunks + k.cps - 1) / k.cps;
+    }
+    // the staged kernels' walk of plan p over W words
+    Walk staged_walk(const Plan &p, uint64_t W) const {
+        Walk k;
+        k.p = &p;
+        k.bw = p.bw;
+        if (p.wide) wide_shape(k, W, 2);
+        return k;
+    }
+    Walk full_walk(uint64_t W) const { return staged_walk(full, W); }
     Walk lean_walk(uint64_t W) const {
         const Plan &p = lean();
-        if (!p.image) return Walk{&p, p.bw, false, {}};
-        const ResidentShape r = resident_shape(p.res, W);
-        return Walk{&p, r.bw, true, r};
+        if (!p.image) return staged_walk(p, W);
+        Walk k;
+        k.p = &p;
+        k.resident = true;
+        k.rs = resident_shape(p.res, W);
+        k.bw = k.rs.bw;
+        return k;
     }
     uint32_t hash_cap = 4096, cover_threads = 256, cover_grid = 0;
     uint32_t wait_polls = 0;  // bound of the forward kernels' waits (0 = the default)
@@ -528,6 +566,13 @@ pdf_status build_segments(pdf_circuit *c, const pdf_netlist *nl, uint32_t N) {
 
 namespace {
 
+// Levels wide enough for the wide kernel: its rounds then outweigh its grid
+// barriers (about 2 us a level).  Kernel times (us) at the thread-per-gate
+// kernel and at this one: 3,550 gates a level and 32,768 pairs with planes
+// 4,032 and 1,200; 1,500 a level and 65,536 pairs without 1,733 and 895; 308
+// a level and 32,768 pairs with planes 277 and 445.
+constexpr uint64_t kWideLevel = 1024;
+
 // Column block of the reduced walk of a circuit whose tile is bw words, by
 // the mean width of its levels above the inputs.  Narrow levels leave most
 // warps of the lane kernel without a gate.
@@ -629,7 +674,12 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     }
     const bool fixed = o.mark_mode >= PDF_MARK_FIXED_ROBUST;
     PlanOpts po;
-    po.bw = c->bw;
+    // a caller that asks for a tile gets its kernel for the whole walk (the
+    // reduced one takes the wide kernel unless a thread per gate was asked for)
+    const bool wide_full = !o.tile_words && mean_width >= kWideLevel;
+    bool wide_red = false;
+    const uint32_t wide_bw = lane_tile(c->bw) ? c->bw : kLaneWords;  // (a batch's lane kernel)
+    po.bw = wide_full ? wide_bw : c->bw;
     po.threads = o.threads;
     po.regs = forward_kernel_regs((int)po.bw, o.mark_mode);
     po.smem_block = prop.sharedMemPerBlockOptin;
@@ -659,13 +709,16 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         const NetFacts facts = net_facts(net, fixed);
         const bool reduced = facts.n_needed <= (uint64_t)G * 9 / 10;
         if (reduced) rnet = reduce_net(net, facts);
-        image = build_resident(reduced ? rnet : net, res_smem);
+        image = build_resident(reduced ? rnet : net, res_smem - 1024);
         if (reduced && !image.bytes.empty()) {
             build_records(rnet, red);
         } else if (reduced) {
             const uint32_t rl = rnet.n_levels();
             PlanOpts ro = po;
-            ro.bw = reduced_tile(c->bw, rl > 1 ? (rnet.n_gates() - rnet.level_off[1]) / (rl - 1) : 0);
+            const uint64_t rw = rl > 1 ? (rnet.n_gates() - rnet.level_off[1]) / (rl - 1) : 0;
+            wide_red = (!o.tile_words || lane_tile(o.tile_words)) && rw >= kWideLevel;
+            ro.bw = wide_red ? wide_bw : reduced_tile(c->bw, rw);
+            ro.threads = wide_red ? 0 : o.threads;
             if (ro.bw != po.bw) ro.regs = forward_kernel_regs((int)ro.bw, o.mark_mode);
             pst = build_plan(rnet, ro, red);
         }
@@ -710,6 +763,10 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         c->err = c->mem.as<uint32_t>();
         c->full.bind(full, net, reduced ? none : image, c->mem.as<unsigned char>(), fo);
         if (reduced) c->red.bind(red, rnet, image, c->mem.as<unsigned char>(), ro);
+        c->full.wide = wide_full;
+        c->red.wide = wide_red;
+        c->full.mean_width = (uint32_t)mean_width;
+        c->red.mean_width = red.n_levels > 1 ? (red.n_gates - rnet.level_off[1]) / (red.n_levels - 1) : 0;
         for (Plan *p : {&c->full, &c->red}) {
             p->res.sms = (uint32_t)prop.multiProcessorCount;
             p->res.regs = 64;  // its launch bound's
@@ -952,12 +1009,21 @@ pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, b
     const Plan &p = *k.p;
     const uint64_t n_blocks = k.resident ? W : (W + k.bw - 1) / k.bw;
     const uint64_t bm_words = (p.n_gates + 31) / 32;
-    PDF_CUDA(ws.nzb.ensure(n_blocks * bm_words * 4));
-    PDF_CUDA(ws.maxlvl.ensure(n_blocks * 4));
-    if (lane_tile(k.bw)) {  // the cover's bitmaps per kLaneCoverWords words of a column block
-        const uint64_t nf = k.bw / kLaneCoverWords;
-        PDF_CUDA(ws.nzb_fine.ensure(nf * n_blocks * bm_words * 4));
-        PDF_CUDA(ws.maxlvl_fine.ensure(nf * n_blocks * 4));
+    if (k.wide) {
+        // (segments of one chunk are the most there can be, for either width)
+        PDF_CUDA(ws.flags.ensure((uint64_t)p.n_gates * ((W + 31) / 32)));
+        if (!ws.sync.p) {
+            PDF_CUDA(ws.sync.ensure(sizeof(WideSync)));
+            PDF_CUDA(cudaMemset(ws.sync.p, 0, sizeof(WideSync)));
+        }
+    } else {
+        PDF_CUDA(ws.nzb.ensure(n_blocks * bm_words * 4));
+        PDF_CUDA(ws.maxlvl.ensure(n_blocks * 4));
+    }
+    if (k.fine()) {  // the cover's bitmaps per kLaneCoverWords words of a column block
+        const uint64_t nf = n_blocks * (k.bw / kLaneCoverWords);
+        PDF_CUDA(ws.nzb_fine.ensure(nf * bm_words * 4));
+        PDF_CUDA(ws.maxlvl_fine.ensure(nf * 4));
     }
     // active bitmap [W], then the count; the list holds <= 2 pairs per gate
     PDF_CUDA(ws.active.ensure(W * 4 + 16));
@@ -1043,6 +1109,32 @@ FwdArgs base_fwd(pdf_circuit *c, const Walk &k, uint64_t n_pairs) {
     return a;
 }
 
+cudaError_t launch_walk(const pdf_circuit *c, const Walk &k0, Workspace &ws, const FwdArgs &a, int mode,
+                        cudaStream_t cs) {
+    Walk k = k0;
+    const Plan &p = *k.p;
+    if (k.wide) {
+        // two words per lane need rows and inputs that start on 8 bytes
+        const auto even = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 7) == 0; };
+        const bool two = a.ld % 2 == 0 && even(a.V) && even(a.T) && even(a.M) &&
+                         (mode == FWD_MARK || (a.pi_ld % 2 == 0 && even(a.pi_v) && even(a.pi_t)));
+        if (!two) {
+            k.cps = 0;
+            c->wide_shape(k, a.W, 1);
+        }
+        WideArgs wa{};
+        wa.flags = ws.flags.as<uint8_t>();
+        wa.sync = ws.sync.as<WideSync>();
+        wa.cps = k.cps;
+        wa.nseg = k.nseg;
+        wa.chunks = k.chunks;
+        return launch_wide(a, wa, mode, c->mark_mode, k.wide, p.res.sms, cs);
+    }
+    if (k.resident) return launch_resident(a, c->mark_mode, k.bw, k.rs.ctas, k.rs.threads, k.rs.smem, cs);
+    if (lane_tile(k.bw)) return launch_lanes(a, mode, c->mark_mode, k.bw, p.threads, p.fwd_smem, cs);
+    return launch_forward(a, mode, c->mark_mode, k.bw, p.threads, p.fwd_smem, cs);
+}
+
 // The device error word of the circuit's stage calls (pdf_sim, pdf_mark):
 // read after the call's work is done, then cleared, so that an expired wait
 // is reported by the call that met it and by no later one.
@@ -1066,7 +1158,7 @@ CoverArgs base_cover(pdf_circuit *c, const Walk &k, Workspace &ws, const uint32_
     a.ld = ld;
     // a lane walk's cover reads bitmaps per 8 words of its column blocks
     // (fewer candidate nets per pair than the whole block's)
-    const bool fine = lane_tile(k.bw);
+    const bool fine = k.fine();
     a.nzb = fine ? ws.nzb_fine.as<uint32_t>() : ws.nzb.as<uint32_t>();
     a.blk_maxlvl = fine ? ws.maxlvl_fine.as<uint32_t>() : ws.maxlvl.as<uint32_t>();
     a.bm_words = (p.n_gates + 31) / 32;
@@ -1105,6 +1197,16 @@ bool planes_fit(const pdf_circuit *c, uint64_t W, uint64_t ld, std::initializer_
     return true;
 }
 
+// The same for output and stage planes on walk k: the wide kernel takes any
+// pitch and word-aligned rows.
+bool planes_fit(const pdf_circuit *c, const Walk &k, uint64_t W, uint64_t ld, std::initializer_list<const void *> ptrs) {
+    if (!k.wide) return planes_fit(c, W, ld, ptrs);
+    if (ld < W || ld >= (1ull << 30)) return false;
+    for (const void *p : ptrs)
+        if (!p || (reinterpret_cast<uintptr_t>(p) & 3)) return false;
+    return true;
+}
+
 // Device pointers of the pairs, staging them through the workspace when
 // they are host memory or not in the kernels' layout.
 // A resident walk reads them word by word, at any pitch.
@@ -1112,7 +1214,7 @@ pdf_status stage_pairs(pdf_circuit *c, const Walk &k, Workspace &ws, const pdf_p
                        const uint32_t **t, uint64_t *ld, cudaStream_t st) {
     const uint64_t W = (pr->n_pairs + 31) / 32, npi = c->info.n_pi;
     const bool words = ((reinterpret_cast<uintptr_t>(pr->v) | reinterpret_cast<uintptr_t>(pr->t)) & 3) == 0;
-    if (pr->on_device && (k.resident ? words : planes_fit(c, W, pr->ld, {pr->v, pr->t}))) {
+    if (pr->on_device && pr->ld < (1ull << 30) && (k.resident || k.wide ? words : planes_fit(c, W, pr->ld, {pr->v, pr->t}))) {
         *v = pr->v;
         *t = pr->t;
         *ld = pr->ld;
@@ -1156,9 +1258,9 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     // with no plane asked for, only what the marks depend on is evaluated,
     // and only the rows read back are written
     const bool planes = out && (out->sim_v || out->sim_t || out->mark);
-    const Walk k = planes ? c->full_walk() : c->lean_walk(W);
+    const Walk k = planes ? c->full_walk(W) : c->lean_walk(W);
     const Plan &p = *k.p;
-    const bool direct = out && out->on_device && planes_fit(c, W, out->ld, {out->sim_v, out->sim_t, out->mark});
+    const bool direct = out && out->on_device && planes_fit(c, k, W, out->ld, {out->sim_v, out->sim_t, out->mark});
     pdf_status st = ensure_ws(c, k, s->ws, W, !direct);
     if (st != PDF_OK) return st;
     const uint32_t *pv, *pt;
@@ -1206,24 +1308,21 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     // the forward kernel also clears the batch count and the cover's active pairs
     a.acc = acc;
     a.active = s->ws.active.as<uint32_t>();
-    if (k.resident)
-        PDF_CUDA(launch_resident(a, c->mark_mode, k.bw, k.rs.ctas, k.rs.threads, k.rs.smem, cs));
-    else
-        PDF_CUDA(launch_forward(a, FWD_FUSED, c->mark_mode, p.bw, p.threads, p.fwd_smem, cs));
+    PDF_CUDA(launch_walk(c, k, s->ws, a, FWD_FUSED, cs));
     if (c->seg_len > 1) {
         SegMergeArgs sm{};
         sm.seg = c->seg_args();
         sm.V = a.V;
         sm.M = a.M;
         sm.ld = a.ld;
-        sm.nzb = a.nzb;
+        sm.nzb = k.fine() ? a.nzb_fine : a.nzb;
         sm.bm_words = a.bm_words;
-        sm.bw = p.bw;
+        sm.bw = k.fine() ? kLaneCoverWords : p.bw;
         sm.W = (uint32_t)W;
         sm.pair_base = (uint32_t)pair_base;
         sm.first_x = s->first_x.as<uint32_t>();
         sm.first_y = s->first_y.as<uint32_t>();
-        PDF_CUDA(launch_seg_merge(sm, (uint32_t)((W + p.bw - 1) / p.bw), cs));
+        PDF_CUDA(launch_seg_merge(sm, (uint32_t)((W + sm.bw - 1) / sm.bw), cs));
     }
     if (s->pe) PDF_CUDA(cudaEventRecord(s->pe->ev[1], cs));
     if (out && !direct) {
@@ -1341,14 +1440,14 @@ extern "C" pdf_status pdf_sim(pdf_circuit *c, const pdf_pairs *pr, uint32_t *sim
     DeviceGuard dg(c->device);
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     std::lock_guard<std::mutex> lk(c->mu);
-    const bool direct = planes_fit(c, W, ld, {sim_v, sim_t});
-    st = ensure_ws(c, c->full_walk(), c->stage, W, !direct);
+    const bool direct = planes_fit(c, c->full_walk(W), W, ld, {sim_v, sim_t});
+    st = ensure_ws(c, c->full_walk(W), c->stage, W, !direct);
     if (st != PDF_OK) return st;
     const uint32_t *pv, *pt;
     uint64_t pld;
-    st = stage_pairs(c, c->full_walk(), c->stage, pr, &pv, &pt, &pld, cs);
+    st = stage_pairs(c, c->full_walk(W), c->stage, pr, &pv, &pt, &pld, cs);
     if (st != PDF_OK) return st;
-    FwdArgs a = base_fwd(c, c->full_walk(), pr->n_pairs);
+    FwdArgs a = base_fwd(c, c->full_walk(W), pr->n_pairs);
     a.pi_v = pv;
     a.pi_t = pt;
     a.pi_ld = pld;
@@ -1357,9 +1456,9 @@ extern "C" pdf_status pdf_sim(pdf_circuit *c, const pdf_pairs *pr, uint32_t *sim
         a.T = sim_t;
         a.ld = ld;
     } else {
-        use_ws_planes(a, c->full_walk(), c->stage, W);
+        use_ws_planes(a, c->full_walk(W), c->stage, W);
     }
-    PDF_CUDA(launch_forward(a, FWD_SIM, c->mark_mode, c->bw, c->full.threads, c->full.fwd_smem, cs));
+    PDF_CUDA(launch_walk(c, c->full_walk(W), c->stage, a, FWD_SIM, cs));
     if (!direct) {
         PDF_CUDA(cudaMemcpy2DAsync(sim_v, ld * 4, a.V, a.ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
         PDF_CUDA(cudaMemcpy2DAsync(sim_t, ld * 4, a.T, a.ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
@@ -1377,24 +1476,24 @@ pdf_status mark_planes(pdf_circuit *c, const uint32_t *sim_v, const uint32_t *si
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     std::lock_guard<std::mutex> lk(c->mu);
     const uint64_t W = (n_pairs + 31) / 32, G = c->info.n_gates;
-    const bool direct = planes_fit(c, W, ld, {sim_v, sim_t, mark});
-    pdf_status st = ensure_ws(c, c->full_walk(), c->stage, W, !direct);
+    const bool direct = planes_fit(c, c->full_walk(W), W, ld, {sim_v, sim_t, mark});
+    pdf_status st = ensure_ws(c, c->full_walk(W), c->stage, W, !direct);
     if (st != PDF_OK) return st;
-    FwdArgs a = base_fwd(c, c->full_walk(), n_pairs);
+    FwdArgs a = base_fwd(c, c->full_walk(W), n_pairs);
     if (direct) {
         a.V = const_cast<uint32_t *>(sim_v);
         a.T = const_cast<uint32_t *>(sim_t);
         a.M = mark;
         a.ld = ld;
     } else {
-        use_ws_planes(a, c->full_walk(), c->stage, W);
+        use_ws_planes(a, c->full_walk(W), c->stage, W);
         PDF_CUDA(cudaMemcpy2DAsync(a.V, a.ld * 4, sim_v, ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
         PDF_CUDA(cudaMemcpy2DAsync(a.T, a.ld * 4, sim_t, ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
     }
     a.nzb = c->stage.nzb.as<uint32_t>();
     a.blk_maxlvl = c->stage.maxlvl.as<uint32_t>();
     a.no_prune = prune ? 0u : 1u;
-    PDF_CUDA(launch_forward(a, FWD_MARK, c->mark_mode, c->bw, c->full.threads, c->full.fwd_smem, cs));
+    PDF_CUDA(launch_walk(c, c->full_walk(W), c->stage, a, FWD_MARK, cs));
     if (!direct)
         PDF_CUDA(cudaMemcpy2DAsync(mark, ld * 4, a.M, a.ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
     PDF_CUDA(cudaStreamSynchronize(cs));
@@ -1437,7 +1536,7 @@ pdf_status cover_chunk(pdf_circuit *c, pdf_state *s, const uint32_t *mark, uint6
                        uint64_t pair_base, uint64_t *counts, pdf_totals *chunk, cudaStream_t cs) {
     std::lock_guard<std::mutex> lk(s->mu);
     const uint64_t W = (n_pairs + 31) / 32;
-    pdf_status st = ensure_ws(c, c->full_walk(), s->ws, W, false);
+    pdf_status st = ensure_ws(c, c->full_walk(W), s->ws, W, false);
     if (st != PDF_OK) return st;
     const size_t count_bytes = (size_t)c->info.n_pi * n_pairs * 16;
     if (counts) {
@@ -1446,7 +1545,7 @@ pdf_status cover_chunk(pdf_circuit *c, pdf_state *s, const uint32_t *mark, uint6
     }
     DevAcc *acc = s->acc.as<DevAcc>();
     PDF_CUDA(launch_batch_begin(acc, cs));
-    CoverArgs ca = base_cover(c, c->full_walk(), s->ws, mark, ld, n_pairs, (uint32_t)pair_base, s->first_x.as<uint32_t>(),
+    CoverArgs ca = base_cover(c, c->full_walk(W), s->ws, mark, ld, n_pairs, (uint32_t)pair_base, s->first_x.as<uint32_t>(),
                               s->first_y.as<uint32_t>(), acc);
     // the bitmaps the cover reads, at its granularity, from the given marks
     PDF_CUDA(launch_bitmap_from_marks(c->full.dc, mark, ld, n_pairs, ca.bw, const_cast<uint32_t *>(ca.nzb),
@@ -1653,6 +1752,7 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
     uint64_t res_ctas = 0;
     for (uint32_t i = 0; i < n_jobs; i++) {
         Walk &k = walks[i] = jobs[i].circuit->lean_walk((jobs[i].pairs.n_pairs + 31) / 32);
+        k.wide = 0;  // a batch's circuits share the GPU: a wide plan takes the lane kernel
         if (!k.resident) continue;
         // a CTA takes blocks worth about twice its copy of the image
         const double load = 2.0 + k.p->res.image_bytes / 95e3;
@@ -2060,5 +2160,5 @@ extern "C" pdf_status pdf_state_reserve(pdf_state *s, uint64_t n_pairs) {
     std::lock_guard<std::mutex> lk(s->mu);
     const uint64_t W = (n_pairs + 31) / 32;
     const pdf_status st = ensure_ws(s->c, s->c->lean_walk(W), s->ws, W, true);
-    return st == PDF_OK ? ensure_ws(s->c, s->c->full_walk(), s->ws, W, true) : st;
+    return st == PDF_OK ? ensure_ws(s->c, s->c->full_walk(W), s->ws, W, true) : st;
 }

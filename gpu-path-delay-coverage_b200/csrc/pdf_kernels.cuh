@@ -226,6 +226,27 @@ cudaError_t launch_resident(const FwdArgs &a, int sem, uint32_t bw, uint32_t cta
                             cudaStream_t st);
 cudaError_t prepare_resident_class(uint32_t sem, uint32_t bw, size_t smem);
 cudaError_t launch_resident_class(const BatchLaunch &b, const BatchClass &c, cudaStream_t st);
+// The wide forward kernel (pdf_wide.cu): a cooperative grid of kWideCtas CTAs
+// per SM on one level at a time.
+constexpr uint32_t kWideThreads = 512;
+constexpr uint32_t kWideCtas = 2;
+struct WideSync {            // zero between launches
+    uint32_t arrived, left;  // barrier arrivals, CTAs done
+    uint32_t reach, top;     // last level that can still hold a mark; levels below top hold one
+};
+struct WideArgs {
+    uint8_t *flags;          // [nseg][n_gates]: bit k = a mark in the segment's chunk k
+    WideSync *sync;
+    uint32_t cps, nseg, chunks;  // chunks (32 LW words) per segment, segments, chunks of a row
+};
+cudaError_t launch_wide(const FwdArgs &a, const WideArgs &wa, int mode, int sem, uint32_t lw, uint32_t sms,
+                        cudaStream_t st);
+// The lane forward kernel (pdf_lanes.cu).
+int lane_kernel_regs(int bw, int sem);
+cudaError_t launch_lanes(const FwdArgs &a, int mode, int sem, uint32_t bw, uint32_t threads, size_t smem,
+                         cudaStream_t st);
+cudaError_t prepare_lanes_class(uint32_t sem, uint32_t bw, size_t smem);
+cudaError_t launch_lanes_class(const BatchLaunch &b, const BatchClass &c, cudaStream_t st);
 // Raises a kernel's dynamic shared-memory limit on the current device.
 cudaError_t raise_smem_limit(const void *fn, size_t smem);
 

@@ -30,7 +30,7 @@ ResidentImage build_resident(const NetPlan &n, size_t smem) {
     if (n_edge > 0xFFFFu) return im;
     const auto a16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
     const size_t o_edge = 16 * ((size_t)G + 1), o_lvl = o_edge + a16(2 * n_edge), total = o_lvl + a16(8 * ((size_t)L + 1));
-    if (total + (size_t)G * 12 + a16((G + 31) / 32 * 4) + 64 > smem) return im;  // one word per block at least
+    if (total + (size_t)G * 12 + a16((G + 31) / 32 * 4) + 128 > smem) return im;  // one word per block at least
     // how far each gate's mark reaches: the last level of the gates it carries to
     std::vector<uint16_t> reach(G, 0);
     for (uint32_t l = 0; l < L; l++)
@@ -327,22 +327,23 @@ pdf_status build_plan(const NetPlan &n, const PlanOpts &o, LaunchPlan &pl) {
         pl.fwd_smem = off + ring_bytes(ring);
         pl.chain = pl.n_pieces;
     }
-    // How far a gate's mark can reach: the last piece that holds a gate whose
-    // mark this one can carry.  Kept above the fan-out count in w[1] where
+    // How far a gate's mark can reach: the last piece (of a lane plan, level)
+    // that holds a gate whose mark this one can carry.  Kept above the fan-out count in w[1] where
     // both fit 16 bits; else the walk never ends early.
     pl.nfo_mask = 0xFFFFFFFFu;
     const uint32_t max_nfo = n.nfo.empty() ? 0 : *std::max_element(n.nfo.begin(), n.nfo.end());
-    if (max_nfo <= 0xFFFFu && pl.n_pieces <= 0xFFFFu) {
+    if (max_nfo <= 0xFFFFu && pl.n_pieces <= 0xFFFFu && L <= 0xFFFFu) {
         pl.nfo_mask = 0xFFFFu;
         while (pl.in_pieces < pl.n_pieces && pl.pieces[pl.in_pieces].level == 0) pl.in_pieces++;
         std::vector<uint16_t> reach(G, 0);
+        const auto at = [&](uint32_t i) { return (uint16_t)(lanes ? pl.pieces[i].level : i); };
         for (uint32_t i = 0; i < pl.n_pieces; i++)  // ascending: the last reader's piece stays
             for (uint32_t g = pl.pieces[i].a; g < pl.pieces[i].b; g++) {
                 const uint32_t *fin = n.edges.data() + n.eoff[g];
                 if (n.hdr[g] & RF_MANY)
-                    for (uint32_t q = 0; q < n.nfi[g]; q++) reach[fin[q]] = (uint16_t)i;
+                    for (uint32_t q = 0; q < n.nfi[g]; q++) reach[fin[q]] = at(i);
                 else if ((n.hdr[g] & RF_MARKF0) && n.nfi[g])
-                    reach[fin[0]] = (uint16_t)i;
+                    reach[fin[0]] = at(i);
             }
         for (uint32_t g = 0; g < G; g++) pl.recs[g].w[1] |= (uint32_t)reach[g] << 16;
     }

@@ -12,6 +12,23 @@ constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 // constant: the index of its first-detect ids.
 __device__ __forceinline__ uint32_t net_id(const DevCircuit &c, uint32_t g) { return c.orig ? __ldg(c.orig + g) : g; }
 
+__device__ __forceinline__ GateRec load_rec(const GateRec *p) {
+    const uint4 *q = reinterpret_cast<const uint4 *>(p);
+    const uint4 a = __ldg(q), b = __ldg(q + 1);
+    GateRec r;
+    r.w[0] = a.x;
+    r.w[1] = a.y;
+    r.w[2] = a.z;
+    r.w[3] = a.w;
+    r.w[4] = b.x;
+    r.w[5] = b.y;
+    r.w[6] = b.z;
+    r.w[7] = b.w;
+    return r;
+}
+
+__device__ __forceinline__ bool bit_test(const uint32_t *bm, uint32_t g) { return (bm[g >> 5] >> (g & 31)) & 1u; }
+
 // ---- TMA bulk copies and mbarriers (inline PTX, sm_90+ / sm_100a) ----
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -72,6 +89,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *m, uint32_t phase, uint32_t 
         if (mbar_try_wait(m, phase)) return true;
     return false;
 }
+
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Last i with pref[i] <= x.
 __device__ __forceinline__ uint32_t prefix_find(const uint32_t *pref, uint32_t n, uint32_t x) {

@@ -136,6 +136,7 @@ struct DeviceGuard {
 // stage calls).
 struct Workspace {
     DevBuf nzb, maxlvl, active, active_list;
+    DevBuf mid_list;          // pairs for the cover's large table
     DevBuf over_list, spill;  // pairs for the spill cover and its per-net (h, c) slots
     DevBuf flags, sync;       // wide kernel: mark flags per (segment, gate), barrier counters
     DevBuf nzb_fine, maxlvl_fine;  // lane circuits: the cover's bitmaps per quarter column block
@@ -149,6 +150,7 @@ struct Workspace {
         maxlvl.release();
         active.release();
         active_list.release();
+        mid_list.release();
         over_list.release();
         spill.release();
         flags.release();
@@ -174,7 +176,7 @@ struct Plan : PlanShape {
     uint32_t mean_width = 0;
     // the resident kernel's image of the netlist (null: it does not fit)
     const void *image = nullptr;
-    uint32_t off_edge_im = 0, off_lvl_im = 0;
+    uint32_t off_edge_im = 0, off_lvl_im = 0, image_ids = 0;
     ResidentSizes res;
     void bind(const LaunchPlan &l, const NetPlan &n, const ResidentImage &im, const unsigned char *base,
               const struct PlanOffsets &o);
@@ -213,6 +215,7 @@ void Plan::bind(const LaunchPlan &l, const NetPlan &n, const ResidentImage &im, 
     image = base + o.image;
     off_edge_im = im.off_edge;
     off_lvl_im = im.off_lvl;
+    image_ids = im.ids ? 1u : 0u;
     res.n_gates = n_gates;
     res.n_levels = n_levels;
     res.image_bytes = (uint32_t)im.bytes.size();
@@ -311,6 +314,7 @@ struct pdf_circuit {
         return k;
     }
     uint32_t hash_cap = 4096, cover_threads = 256, cover_grid = 0;
+    uint32_t small_cap = 0;  // nets per pair of the cover's small-table pass
     uint32_t wait_polls = 0;  // bound of the forward kernels' waits (0 = the default)
     Workspace stage;  // scratch of the stage calls
     std::mutex mu;    // serialises the stage scratch
@@ -340,8 +344,11 @@ struct pdf_state {
     pdf_circuit *c = nullptr;
     int device = 0;  // the circuit's device (destroy does not need the circuit)
     DevBuf first_x, first_y, acc;
-    DevAcc *host_acc = nullptr;  // host copy of the accumulators (pinned: read back by DMA, after a
-                                 // stream sync, without the driver's staging of pageable copies)
+    // two host copies of the accumulators (pinned and mapped): [0] read back by
+    // DMA after a stream sync (snapshots), [1] written by the cover kernel that
+    // closes a batch
+    DevAcc *host_acc = nullptr;
+    DevAcc *mirror = nullptr;  // device address of host_acc[1]
     Workspace ws;
     std::mutex mu;
     bool profiling = false;
@@ -734,6 +741,11 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     // nets one pair may mark in the cover: as many as its shared memory holds
     c->hash_cap = 4096;
     while (c->hash_cap > 256 && cover_smem_bytes(c->hash_cap) > (size_t)prop.sharedMemPerBlockOptin) c->hash_cap -= 256;
+    c->small_cap = std::min(cover_small_cap(o.device, nullptr), c->hash_cap);
+    if (c->small_cap < 256) {  // (the level table comes out of it)
+        delete c;
+        return PDF_ECUDA;
+    }
     c->cover_threads = 256;
     c->cover_grid = (uint32_t)prop.multiProcessorCount;
 
@@ -832,13 +844,13 @@ extern "C" pdf_status pdf_state_create(pdf_circuit *c, pdf_state **out) {
     const size_t G = c->n_first();  // first-detect entries: nets, or segments
     if (s->first_x.ensure(4 * G) != cudaSuccess || s->first_y.ensure(4 * G) != cudaSuccess ||
         s->acc.ensure(sizeof(DevAcc)) != cudaSuccess ||
-        cudaHostAlloc(reinterpret_cast<void **>(&s->host_acc), sizeof(DevAcc), cudaHostAllocDefault) != cudaSuccess) {
-        s->host_acc = nullptr;
+        cudaHostAlloc(reinterpret_cast<void **>(&s->host_acc), 2 * sizeof(DevAcc), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(reinterpret_cast<void **>(&s->mirror), s->host_acc + 1, 0) != cudaSuccess) {
         (void)cudaGetLastError();
         pdf_state_destroy(s);
         return PDF_ENOMEM;
     }
-    std::memset(s->host_acc, 0, sizeof(DevAcc));
+    std::memset(s->host_acc, 0, 2 * sizeof(DevAcc));
     // cleared on a stream of its own: a device-wide sync here would wait for
     // every other circuit's work in flight (a server creates states while it
     // grades)
@@ -1029,6 +1041,7 @@ pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, b
     PDF_CUDA(ws.active.ensure(W * 4 + 16));
     const uint64_t list = std::min<uint64_t>(W * 32, 2 * std::max<uint64_t>(c->n_first(), c->info.n_gates));
     PDF_CUDA(ws.active_list.ensure(list * 4));
+    PDF_CUDA(ws.mid_list.ensure(list * 4));
     // A pair can mark more nets than the cover's table holds only when the
     // walk has more gates than that; its count then goes through the spill
     // cover.
@@ -1097,6 +1110,7 @@ FwdArgs base_fwd(pdf_circuit *c, const Walk &k, uint64_t n_pairs) {
     if (k.resident) {
         a.image = p.image;
         a.image_bytes = p.res.image_bytes;
+        a.image_ids = p.image_ids;
         a.per = k.rs.per;
         a.n_blocks = k.rs.blocks;
         a.off_edge = p.off_edge_im;
@@ -1172,6 +1186,8 @@ CoverArgs base_cover(pdf_circuit *c, const Walk &k, Workspace &ws, const uint32_
     a.active_list = ws.active_list.as<uint32_t>();
     a.acc = acc;
     a.hash_cap = c->hash_cap;
+    a.mid_list = ws.mid_list.as<uint32_t>();
+    a.small_cap = c->small_cap;
     a.over_list = ws.over_list.as<uint32_t>();
     a.spill = ws.spill.as<unsigned char>();
     uint64_t slot;
@@ -1349,6 +1365,7 @@ pdf_status grade_cover_locked(pdf_circuit *c, pdf_state *s, cudaStream_t cs) {
     const uint32_t base = (uint32_t)s->pend_base;
     CoverArgs ca = base_cover(c, s->pend_walk, s->ws, s->pend_M, s->pend_ld, s->pend_n, base, s->first_x.as<uint32_t>(),
                               s->first_y.as<uint32_t>(), acc);
+    ca.mirror = s->mirror;
     if (s->pe) PDF_CUDA(cudaEventRecord(s->pe->ev[2], cs));  // cover starts (after any exchange)
     PDF_CUDA(launch_cover(ca, c->cover_grid, c->cover_threads, false, cs));  // closes the batch
     if (s->pe) {
@@ -1415,9 +1432,8 @@ extern "C" pdf_status pdf_grade(pdf_circuit *c, pdf_state *s, const pdf_pairs *p
     if (st != PDF_OK) return st;
     DeviceGuard dg(c->device);
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
-    PDF_CUDA(cudaMemcpyAsync(s->host_acc, s->acc.p, sizeof(DevAcc), cudaMemcpyDeviceToHost, cs));
     PDF_CUDA(cudaStreamSynchronize(cs));
-    const DevAcc &h = *s->host_acc;
+    const DevAcc h = s->host_acc[1];  // left there by the cover
     if (batch) {
         batch->lo = h.batch_lo;
         batch->hi = h.batch_hi;
@@ -1550,12 +1566,12 @@ pdf_status cover_chunk(pdf_circuit *c, pdf_state *s, const uint32_t *mark, uint6
     // the bitmaps the cover reads, at its granularity, from the given marks
     PDF_CUDA(launch_bitmap_from_marks(c->full.dc, mark, ld, n_pairs, ca.bw, const_cast<uint32_t *>(ca.nzb),
                                       const_cast<uint32_t *>(ca.blk_maxlvl), ca.bm_words, cs));
+    ca.mirror = s->mirror;
     if (counts) ca.pi_counts = s->ws.pi_counts.as<unsigned long long>();
     PDF_CUDA(launch_cover(ca, c->cover_grid, c->cover_threads, true, cs));  // closes the batch
-    PDF_CUDA(cudaMemcpyAsync(s->host_acc, s->acc.p, sizeof(DevAcc), cudaMemcpyDeviceToHost, cs));
     if (counts) PDF_CUDA(cudaMemcpyAsync(counts, s->ws.pi_counts.p, count_bytes, cudaMemcpyDeviceToHost, cs));
     PDF_CUDA(cudaStreamSynchronize(cs));
-    const DevAcc &h = *s->host_acc;
+    const DevAcc h = s->host_acc[1];  // left there by the cover
     if (chunk) {
         chunk->lo = h.batch_lo;
         chunk->hi = h.batch_hi;

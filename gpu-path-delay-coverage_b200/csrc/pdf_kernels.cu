@@ -940,12 +940,12 @@ constexpr uint32_t kNetPo = 1u << 31, kNetInpt = 1u << 30, kNetFirst = 1u << 29,
 __host__ __device__ constexpr size_t cover_smem_tables(uint32_t cap, uint32_t cand) {
     return (size_t)cap * (2 * sizeof(pdf_u128) + 4 * 4 + 4 * 4) + (size_t)cand * 4;
 }
-// Byte offset of the level table in k_cover's shared memory (after the tables).
-__host__ __device__ constexpr size_t cover_smem_lvt(uint32_t cap) { return cover_smem_tables(cap, kCoverCand); }
-
 // Each thread of the candidate test below takes up to CAND / blockDim
 // candidates in registers: the cover kernels run 256 threads.
 constexpr uint32_t kCoverThreads = 256;
+constexpr uint32_t kCoverSmallCtas = 4;     // CTAs per SM of the small-table passes
+constexpr uint32_t kCoverLeanGates = 1536;  // k_cover_lean: nets and words of pairs at most
+constexpr uint32_t kCoverLeanWords = 4096;
 static_assert(kCoverCand / kCoverThreads <= 16, "cover_pair keeps 16 candidate mark words per thread");
 static_assert(kCoverCandSmall % kCoverThreads == 0 && kCoverCandSmall <= kCoverCand, "small window");
 
@@ -957,14 +957,23 @@ __device__ __forceinline__ void put_pi_count(const CoverArgs &a, uint32_t g, uin
     d[1] = (unsigned long long)(c >> 64);
 }
 
+// Whether a pair first-detects net g, from the state's ids.
+__device__ __forceinline__ bool net_first(const CoverArgs &a, uint32_t g, uint32_t pid) {
+    if (a.seg.N > 1)
+        return first_set_find(a.seg_first, a.seg_first_mask, ((unsigned long long)g << 32) | (pid - a.pair_base));
+    const uint32_t id = net_id(a.c, g), fx = a.first_x[id], fy = a.first_y[id];
+    return fx == pid || fy == pid;
+}
+
 // The cover of pair p (index within the batch) of the circuit in `a`;
 // lo_tab is its level table (shared or global memory); cap: nets the table
-// holds; CAND: candidates per window.  Returns true (the same in every
+// holds; CAND: candidates per window; is_first(g, pair id): whether the pair
+// first-detects net g.  Returns true (the same in every
 // thread) when the pair marks more nets than the table holds: then nothing
 // is counted.
-template <uint32_t CAND>
+template <uint32_t CAND, class First>
 __device__ __forceinline__ bool cover_pair(const CoverArgs &a, const uint32_t p, const uint32_t *lo_tab,
-                                           const uint32_t cap) {
+                                           const uint32_t cap, First is_first) {
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr uint32_t kPer = CAND / kCoverThreads;  // candidates per thread and window
     const uint32_t acap = 4 * cap;
@@ -1060,13 +1069,7 @@ __device__ __forceinline__ bool cover_pair(const CoverArgs &a, const uint32_t p,
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
         const uint32_t g = lid[i];
         const GateRec r = load_rec(a.c.rec + g);
-        bool first;
-        if (a.seg.N > 1) {
-            first = first_set_find(a.seg_first, a.seg_first_mask, ((unsigned long long)g << 32) | p);
-        } else {
-            const uint32_t id = net_id(a.c, g), fx = a.first_x[id], fy = a.first_y[id];
-            first = fx == pid || fy == pid;
-        }
+        const bool first = is_first(g, pid);
         const uint32_t nfo = r.w[1] & a.c.nfo_mask, eb = r.w[2] + rec_nfi(r);
         uint32_t k = 0;
         for (uint32_t j = 0; j < nfo; j += 4) {  // four fan-out loads in flight
@@ -1246,30 +1249,118 @@ __device__ __forceinline__ pdf_u128 *spill_slot(const CoverArgs &a, uint32_t k) 
     return reinterpret_cast<pdf_u128 *>(a.spill) + (size_t)k * 2 * a.c.n_gates;
 }
 
-__global__ void __launch_bounds__(kCoverThreads) k_cover(const CoverArgs a) {
+// The last CTA to finish closes the batch, and leaves the accumulators where
+// the host reads them.
+__device__ __forceinline__ void close_and_tell(const CoverArgs &a) {
+    batch_close(a.acc, a.n_pairs);
+    if (a.mirror) *a.mirror = *a.acc;
+}
+
+// The cover in two passes over the same pairs (as k_batch_cover): TIER 0 with
+// a small table, several CTAs per SM, queues the pairs that mark more nets
+// for TIER 1, whose table takes an SM; what does not fit there either is
+// queued for the spill cover.
+template <int TIER>
+__global__ void __launch_bounds__(kCoverThreads) k_cover(const CoverArgs a, uint32_t cap) {
     extern __shared__ __align__(128) unsigned char smraw[];
-    uint32_t *lvt = reinterpret_cast<uint32_t *>(smraw + cover_smem_lvt(a.hash_cap));  // [kCoverLevels] level_off
+    constexpr uint32_t CAND = TIER == 0 ? kCoverCandSmall : kCoverCand;
+    const bool direct = TIER == 0 || !a.mid_list;  // without a queue the large table takes every pair
+    const uint32_t n_items = direct ? *a.active_count : a.acc->n_mid;
+    if (!direct && !n_items) return;  // the small-table pass closed the batch
+    uint32_t *lvt = reinterpret_cast<uint32_t *>(smraw + cover_smem_tables(cap, CAND));  // [kCoverLevels] level_off
     const uint32_t L = a.c.n_levels;
     const bool lv_shared = L + 1 <= kCoverLevels;
-    if (lv_shared)
+    if (lv_shared && blockIdx.x < n_items)
         for (uint32_t i = threadIdx.x; i <= L; i += blockDim.x) lvt[i] = a.c.level_off[i];
     const uint32_t *lo_tab = lv_shared ? lvt : a.c.level_off;
     __syncthreads();
-    const uint32_t n_active = *a.active_count;
-    for (uint32_t ai = blockIdx.x; ai < n_active; ai += gridDim.x) {
-        const uint32_t p = a.active_list[ai];
-        if (cover_pair<kCoverCand>(a, p, lo_tab, a.hash_cap) && threadIdx.x == 0) {
-            if (a.spill_slots) a.over_list[atomicAdd(&a.acc->n_over, 1u)] = p;  // for k_cover_spill
+    const uint32_t *in = direct ? a.active_list : a.mid_list;
+    for (uint32_t ai = blockIdx.x; ai < n_items; ai += gridDim.x) {
+        const uint32_t p = in[ai];
+        const bool over = cover_pair<CAND>(a, p, lo_tab, cap, [&](uint32_t g, uint32_t pid) { return net_first(a, g, pid); });
+        if (over && threadIdx.x == 0) {
+            if (TIER == 0) a.mid_list[atomicAdd(&a.acc->n_mid, 1u)] = p;
+            else if (a.spill_slots) a.over_list[atomicAdd(&a.acc->n_over, 1u)] = p;  // for k_cover_spill
             else atomicOr(&a.acc->err, kErrHashFull);
         }
     }
-    // the last CTA to finish closes the batch, unless pairs wait for the spill cover
+    // the last CTA closes the batch, unless pairs wait for the next pass
+    if (threadIdx.x == 0) {
+        __threadfence();
+        unsigned int *done = TIER == 0 ? &a.acc->done : &a.acc->done_mid;
+        if (atomicAdd(done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            *done = 0;
+            const unsigned int waiting = TIER == 0 ? a.acc->n_mid : a.acc->n_over;
+            if (TIER == 1) a.acc->n_mid = 0;
+            if (!waiting) close_and_tell(a);
+        }
+    }
+}
+
+// The cover of a small netlist in one launch: every CTA reads the first ids of
+// all its nets, finds the first-detecting pairs itself (a bitmap in shared
+// memory, ranked by a scan) and takes every gridDim-th of them, with a table
+// that holds every net.  No pair list, no second pass.
+__global__ void __launch_bounds__(kCoverThreads) k_cover_lean(const CoverArgs a) {
+    extern __shared__ __align__(128) unsigned char smraw[];
+    __shared__ uint32_t s_scan[32], s_pairs[8];
+    const uint32_t N = a.c.n_gates, L = a.c.n_levels, W = (uint32_t)((a.n_pairs + 31) / 32);
+    uint32_t *lvt = reinterpret_cast<uint32_t *>(smraw + cover_smem_tables(N, kCoverCandSmall));  // [L + 1]
+    uint2 *first = reinterpret_cast<uint2 *>(lvt + ((L + 2) & ~1u));                              // [N]
+    uint32_t *bits = reinterpret_cast<uint32_t *>(first + N);                                     // [W]
+    for (uint32_t w = threadIdx.x; w < W; w += blockDim.x) bits[w] = 0;
+    for (uint32_t i = threadIdx.x; i <= L; i += blockDim.x) lvt[i] = a.c.level_off[i];
+    __syncthreads();
+    // every thread's nets at once: two loads deep, whatever their number
+    constexpr int kPer = kCoverLeanGates / kCoverThreads;
+    uint32_t id[kPer];
+    uint2 f[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; u++) {
+        const uint32_t g = threadIdx.x + u * kCoverThreads;
+        id[u] = g < N ? net_id(a.c, g) : kEmpty;
+    }
+#pragma unroll
+    for (int u = 0; u < kPer; u++)
+        f[u] = id[u] == kEmpty ? make_uint2(kEmpty, kEmpty) : make_uint2(a.first_x[id[u]], a.first_y[id[u]]);
+#pragma unroll
+    for (int u = 0; u < kPer; u++) {
+        const uint32_t g = threadIdx.x + u * kCoverThreads;
+        if (g >= N) continue;
+        first[g] = f[u];
+        const uint32_t x = f[u].x - a.pair_base, y = f[u].y - a.pair_base;
+        if (f[u].x != kEmpty && x < a.n_pairs) atomicOr(bits + (x >> 5), 1u << (x & 31));
+        if (f[u].y != kEmpty && y < a.n_pairs) atomicOr(bits + (y >> 5), 1u << (y & 31));
+    }
+    __syncthreads();
+    const uint32_t per = (W + blockDim.x - 1) / blockDim.x;
+    const uint32_t w_lo = min(W, threadIdx.x * per), w_hi = min(W, w_lo + per);
+    uint32_t mine = 0, total;
+    for (uint32_t w = w_lo; w < w_hi; w++) mine += __popc(bits[w]);
+    const uint32_t rank0 = block_scan_excl(mine, s_scan, &total);
+    for (uint32_t k = blockIdx.x; k < total; k += 8 * gridDim.x) {  // up to 8 pairs of this CTA at a time
+        // pair u of them has rank k + u * gridDim: its thread finds the bit
+        uint32_t r = rank0, u = rank0 <= k ? 0u : (rank0 - k + gridDim.x - 1) / gridDim.x;
+        for (uint32_t w = w_lo; w < w_hi && u < 8; w++) {
+            const uint32_t b = bits[w], n = __popc(b);
+            for (; u < 8 && k + u * gridDim.x < r + n; u++)
+                s_pairs[u] = w * 32 + __fns(b, 0, (int)(k + u * gridDim.x - r) + 1);
+            r += n;
+        }
+        __syncthreads();
+        for (uint32_t u = 0; u < 8 && k + u * gridDim.x < total; u++)
+            (void)cover_pair<kCoverCandSmall>(a, s_pairs[u], lvt, N, [&](uint32_t g, uint32_t pid) {
+                return first[g].x == pid || first[g].y == pid;
+            });
+        __syncthreads();
+    }
     if (threadIdx.x == 0) {
         __threadfence();
         if (atomicAdd(&a.acc->done, 1u) == gridDim.x - 1) {
             __threadfence();
-            if (!a.acc->n_over) batch_close(a.acc, a.n_pairs);
             a.acc->done = 0;
+            close_and_tell(a);
         }
     }
 }
@@ -1284,9 +1375,9 @@ __global__ void __launch_bounds__(kCoverThreads) k_cover_spill(const CoverArgs a
         __threadfence();
         if (atomicAdd(&a.acc->done_over, 1u) == gridDim.x - 1) {
             __threadfence();
-            batch_close(a.acc, a.n_pairs);
             a.acc->n_over = 0;
             a.acc->done_over = 0;
+            close_and_tell(a);
         }
     }
 }
@@ -1365,8 +1456,8 @@ __global__ void __launch_bounds__(kCoverThreads) k_batch_cover(CoverArgs *args, 
         const uint2 it = in_items[ai];
         if (threadIdx.x == 0) s_a = args[it.x];
         __syncthreads();
-        const bool over = TIER == 0 ? cover_pair<kCoverCandSmall>(s_a, it.y, s_a.c.level_off, cap)
-                                    : cover_pair<kCoverCand>(s_a, it.y, s_a.c.level_off, cap);  // end with a barrier
+        const bool over = cover_pair<TIER == 0 ? kCoverCandSmall : kCoverCand>(  // ends with a barrier
+            s_a, it.y, s_a.c.level_off, cap, [&](uint32_t g, uint32_t pid) { return net_first(s_a, g, pid); });
         if (over && threadIdx.x == 0) {
             if (TIER == 0) out_items[atomicAdd(&ctl->n_mid, 1u)] = it;             // for the large table
             else if (s_a.spill_slots) out_items[atomicAdd(&ctl->n_over, 1u)] = it;  // for k_batch_cover_spill
@@ -1574,7 +1665,7 @@ cudaError_t launch_forward(const FwdArgs &a, int mode, int sem, uint32_t bw, uin
     }
 }
 
-size_t cover_smem_bytes(uint32_t net_cap) { return cover_smem_lvt(net_cap) + (size_t)kCoverLevels * 4; }
+size_t cover_smem_bytes(uint32_t net_cap) { return cover_smem_tables(net_cap, kCoverCand) + (size_t)kCoverLevels * 4; }
 size_t cover_small_smem_bytes(uint32_t cap) { return cover_smem_tables(cap, kCoverCandSmall); }
 
 // CTAs per SM of the batch's small-table cover, and the nets per pair its
@@ -1582,7 +1673,7 @@ size_t cover_small_smem_bytes(uint32_t cap) { return cover_smem_tables(cap, kCov
 // system keeps per CTA and the kernel's static variables.  Four CTAs of 256
 // threads: the kernel's registers allow five.
 uint32_t cover_small_cap(int device, uint32_t *ctas_per_sm) {
-    constexpr uint32_t kCtas = 4;
+    constexpr uint32_t kCtas = kCoverSmallCtas;
     int per_sm = 0, reserved = 0, optin = 0;
     cudaFuncAttributes fa{};
     if (cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device) != cudaSuccess ||
@@ -1600,6 +1691,17 @@ uint32_t cover_small_cap(int device, uint32_t *ctas_per_sm) {
 
 cudaError_t launch_cover(const CoverArgs &a, uint32_t grid, uint32_t threads, bool zero_active, cudaStream_t st) {
     const uint32_t W = (uint32_t)((a.n_pairs + 31) / 32);
+    // one launch for a netlist of a few thousand nets (every CTA reads all
+    // their first ids) whose pairs' bitmap and table fit beside them
+    if (a.seg.N <= 1 && !a.pi_counts && a.c.n_gates <= kCoverLeanGates && W <= kCoverLeanWords &&
+        a.c.n_levels + 1 <= kCoverLevels) {
+        const size_t smem = cover_smem_tables(a.c.n_gates, kCoverCandSmall) + ((size_t)a.c.n_levels + 4) * 4 +
+                            8 * (size_t)a.c.n_gates + 4 * (size_t)W;
+        const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(k_cover_lean), smem);
+        if (e != cudaSuccess) return e;
+        k_cover_lean<<<std::min(2 * grid, std::max(8u, a.c.n_gates / 3)), threads, smem, st>>>(a);
+        return cudaGetLastError();
+    }
     if (zero_active) {
         cudaError_t e = cudaMemsetAsync(a.active, 0, (size_t)(W + 1) * sizeof(uint32_t), st);
         if (e != cudaSuccess) return e;
@@ -1612,11 +1714,24 @@ cudaError_t launch_cover(const CoverArgs &a, uint32_t grid, uint32_t threads, bo
     } else {
         k_active<<<(a.c.n_gates + 255) / 256, 256, 0, st>>>(a);
     }
-    if (threads != kCoverThreads) return cudaErrorInvalidValue;
-    const size_t smem = cover_smem_bytes(a.hash_cap);
-    cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(k_cover), smem);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_cover<<<grid, threads, smem, st>>>(a);
+    if (threads != kCoverThreads) return cudaErrorInvalidValue;
+    if (a.mid_list) {
+        // the small table, beside the level table in its share of the SM, and
+        // for no more nets than there are
+        const size_t lv = a.c.n_levels + 1 <= kCoverLevels ? ((size_t)a.c.n_levels + 1) * 4 : 0;
+        const uint32_t per_net = (uint32_t)cover_smem_tables(1, 0);
+        const uint32_t cap0 = std::min(a.small_cap - (uint32_t)((lv + per_net - 1) / per_net), a.c.n_gates);
+        const size_t smem0 = cover_smem_tables(cap0, kCoverCandSmall) + lv;
+        if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_cover<0>), smem0)) != cudaSuccess) return e;
+        k_cover<0><<<grid * kCoverSmallCtas, threads, smem0, st>>>(a, cap0);
+        if (a.c.n_gates <= cap0) return cudaGetLastError();  // no pair can mark more
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    const size_t smem = cover_smem_bytes(a.hash_cap);
+    if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_cover<1>), smem)) != cudaSuccess) return e;
+    k_cover<1><<<grid, threads, smem, st>>>(a, a.hash_cap);
     if (a.spill_slots) {
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         k_cover_spill<<<a.spill_slots, kCoverThreads, 0, st>>>(a);

@@ -35,6 +35,8 @@ struct DevAcc {
     unsigned int done;                      // cover CTAs finished (the last one closes the batch)
     unsigned int n_over;                    // pairs queued for the spill cover (more nets than the table)
     unsigned int done_over;                 // spill-cover CTAs finished
+    unsigned int n_mid;                     // pairs queued for the large-table cover
+    unsigned int done_mid;                  // its CTAs finished
 };
 
 struct FwdArgs {
@@ -77,7 +79,7 @@ struct FwdArgs {
     // CTA and in all (off_edge, off_fid, off_ring, off_rec: its edges, level
     // table, V / T words and marks)
     const void *image;
-    uint32_t image_bytes, per, n_blocks;
+    uint32_t image_bytes, image_ids, per, n_blocks;
     // shared-memory byte offsets
     uint32_t off_ring;            // forward: ring [3][R][BW]; reverse: ring2 [R2][BW]
     uint32_t off_rec;             // [2][cap] staged gate records
@@ -120,6 +122,11 @@ struct CoverArgs {
     // memory, slot k ([2][n_gates] u128) for its CTA k; spill_slots = 0: no
     // spill scratch (such a pair reports kErrHashFull)
     uint32_t *over_list;          // [min(n_pairs, 2 * n_gates)]
+    // pairs that mark more than small_cap nets (the small-table pass's table):
+    // queued here (count in acc->n_mid) for the large-table pass
+    uint32_t *mid_list;           // [min(n_pairs, 2 * n_gates)]
+    uint32_t small_cap;
+    DevAcc *mirror;               // host memory that gets the accumulators once the batch is closed, or null
     unsigned char *spill;
     uint32_t spill_slots;
     // optional: the paths each primary input credits to each pair,

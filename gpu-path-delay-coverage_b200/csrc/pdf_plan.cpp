@@ -29,8 +29,12 @@ ResidentImage build_resident(const NetPlan &n, size_t smem) {
     for (uint32_t g = 0; g < G; g++) n_edge += n.nfo[g] + (n.nfi[g] > kInlineFanins ? n.nfi[g] : 0);
     if (n_edge > 0xFFFFu) return im;
     const auto a16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
-    const size_t o_edge = 16 * ((size_t)G + 1), o_lvl = o_edge + a16(2 * n_edge), total = o_lvl + a16(8 * ((size_t)L + 1));
-    if (total + (size_t)G * 12 + a16((G + 31) / 32 * 4) + 128 > smem) return im;  // one word per block at least
+    const size_t o_edge = 16 * ((size_t)G + 1), o_lvl = o_edge + a16(2 * n_edge), o_ids = o_lvl + 8 * ((size_t)L + 1);
+    // one word per block at least, and the ids where there is room for them
+    const size_t words = (size_t)G * 12 + a16((G + 31) / 32 * 4) + 128;
+    if (a16(o_ids) + words > smem) return im;
+    im.ids = a16(o_ids + 4 * (size_t)G) + words <= smem;
+    const size_t total = a16(o_ids + (im.ids ? 4 * (size_t)G : 0));
     // how far each gate's mark reaches: the last level of the gates it carries to
     std::vector<uint16_t> reach(G, 0);
     for (uint32_t l = 0; l < L; l++)
@@ -59,6 +63,7 @@ ResidentImage build_resident(const NetPlan &n, size_t smem) {
         for (uint32_t q = nfi > kInlineFanins ? 0 : nfi; q < nfi + n.nfo[g]; q++) edge[at++] = (uint16_t)e[q];
     }
     rec[4 * (size_t)G + 3] = at;
+    for (uint32_t g = 0; im.ids && g < G; g++) lvl[2 * ((size_t)L + 1) + g] = n.orig.empty() ? g : n.orig[g];
     for (uint32_t l = 0; l <= L; l++) {
         lvl[2 * l] = n.level_off[l];
         // gates up to the last that marks (a reduced netlist lists those first)

@@ -35,11 +35,12 @@ struct PlanShape {
 // bytes per gate (header; fan-ins 0..3 as 16-bit ids, of an input its row in
 // the pair planes; edge offset | last level its mark reaches << 16) and one
 // more for the end of the edges, 16-bit edges (fan-ins of gates with more
-// than four, then fan-outs), and per level its first gate and how many of its
-// gates may hold a mark after the prune.
+// than four, then fan-outs), per level its first gate and how many of its
+// gates may hold a mark after the prune, and, where they fit, the caller's ids.
 struct ResidentImage {
     std::vector<unsigned char> bytes;  // empty: the netlist does not fit
     uint32_t off_edge = 0, off_lvl = 0;
+    bool ids = false;  // holds the caller's ids (else read from device memory)
 };
 // `smem`: dynamic shared memory a CTA may have.
 ResidentImage build_resident(const NetPlan &n, size_t smem);

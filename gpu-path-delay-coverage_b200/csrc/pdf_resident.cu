@@ -31,6 +31,9 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
     const uint4 *rec = reinterpret_cast<const uint4 *>(smraw);
     const uint16_t *edge = reinterpret_cast<const uint16_t *>(smraw + a.off_edge);
     const uint2 *lvl = reinterpret_cast<const uint2 *>(smraw + a.off_fid);  // first gate, observable gates
+    // the caller's gate ids (in the image where they fit)
+    const uint32_t *ids = a.image_ids ? reinterpret_cast<const uint32_t *>(lvl + a.c.n_levels + 1) : nullptr;
+    const auto net = [&](uint32_t g) { return ids ? ids[g] : net_id(a.c, g); };
     uint2 *vt = reinterpret_cast<uint2 *>(smraw + a.off_ring);              // [gate][BW] V, T
     uint32_t *ms = reinterpret_cast<uint32_t *>(smraw + a.off_rec);         // [gate][BW] marks
     uint32_t *bm = reinterpret_cast<uint32_t *>(smraw + a.off_bm);
@@ -230,8 +233,8 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
                     a.M[(size_t)g * a.ld + w] = nm;  // (rows hold whole blocks)
                     if (j == 0) atomicOr(bm + (g >> 5), 1u << (g & 31));
                     // the lowest word of each direction holds its first pair
-                    if (x && !(bx & below)) atomicMin(a.first_x + net_id(a.c, g), a.pair_base + w * 32 + (__ffs(x) - 1));
-                    if (y && !(by & below)) atomicMin(a.first_y + net_id(a.c, g), a.pair_base + w * 32 + (__ffs(y) - 1));
+                    if (x && !(bx & below)) atomicMin(a.first_x + net(g), a.pair_base + w * 32 + (__ffs(x) - 1));
+                    if (y && !(by & below)) atomicMin(a.first_y + net(g), a.pair_base + w * 32 + (__ffs(y) - 1));
                 }
                 if (lane == 0) atomicMax(&s_max, (uint32_t)l + 1);
             }

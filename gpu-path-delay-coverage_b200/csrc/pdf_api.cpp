@@ -343,10 +343,15 @@ struct ProfEvents {
 struct pdf_state {
     pdf_circuit *c = nullptr;
     int device = 0;  // the circuit's device (destroy does not need the circuit)
-    DevBuf first_x, first_y, acc;
+    DevBuf mem;  // first-detect ids, falling then rising, and the accumulators
+    struct Ref {
+        void *p = nullptr;
+        template <class T>
+        T *as() const { return static_cast<T *>(p); }
+    } first_x, first_y, acc;
     // two host copies of the accumulators (pinned and mapped): [0] read back by
-    // DMA after a stream sync (snapshots), [1] written by the cover kernel that
-    // closes a batch
+    // DMA after a stream sync, [1] the mirror, which whatever changes the totals
+    // writes too: the cover kernel that closes a batch, a reset, a restore
     DevAcc *host_acc = nullptr;
     DevAcc *mirror = nullptr;  // device address of host_acc[1]
     Workspace ws;
@@ -842,8 +847,8 @@ extern "C" pdf_status pdf_state_create(pdf_circuit *c, pdf_state **out) {
     s->c = c;
     s->device = c->device;
     const size_t G = c->n_first();  // first-detect entries: nets, or segments
-    if (s->first_x.ensure(4 * G) != cudaSuccess || s->first_y.ensure(4 * G) != cudaSuccess ||
-        s->acc.ensure(sizeof(DevAcc)) != cudaSuccess ||
+    const size_t acc_off = (8 * G + 255) & ~(size_t)255;
+    if (s->mem.ensure(acc_off + sizeof(DevAcc)) != cudaSuccess ||
         cudaHostAlloc(reinterpret_cast<void **>(&s->host_acc), 2 * sizeof(DevAcc), cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer(reinterpret_cast<void **>(&s->mirror), s->host_acc + 1, 0) != cudaSuccess) {
         (void)cudaGetLastError();
@@ -851,14 +856,16 @@ extern "C" pdf_status pdf_state_create(pdf_circuit *c, pdf_state **out) {
         return PDF_ENOMEM;
     }
     std::memset(s->host_acc, 0, 2 * sizeof(DevAcc));
+    s->first_x.p = s->mem.p;
+    s->first_y.p = s->mem.as<uint32_t>() + G;
+    s->acc.p = s->mem.as<unsigned char>() + acc_off;
     // cleared on a stream of its own: a device-wide sync here would wait for
     // every other circuit's work in flight (a server creates states while it
     // grades)
     cudaStream_t cs = nullptr;
     const bool ok = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) == cudaSuccess &&
-                    cudaMemsetAsync(s->first_x.p, 0xFF, 4 * G, cs) == cudaSuccess &&
-                    cudaMemsetAsync(s->first_y.p, 0xFF, 4 * G, cs) == cudaSuccess &&
-                    cudaMemsetAsync(s->acc.p, 0, sizeof(DevAcc), cs) == cudaSuccess &&
+                    launch_state_reset(s->first_x.as<uint32_t>(), 2 * G, s->acc.as<DevAcc>(), s->mirror, cs) ==
+                        cudaSuccess &&
                     cudaStreamSynchronize(cs) == cudaSuccess;
     if (cs) cudaStreamDestroy(cs);
     if (!ok) {
@@ -876,9 +883,7 @@ extern "C" void pdf_state_destroy(pdf_state *s) {
     prof_release(s->prof);
     prof_release(s->pool);
     s->ws.release();
-    s->first_x.release();
-    s->first_y.release();
-    s->acc.release();
+    s->mem.release();
     if (s->host_acc && cudaFreeHost(s->host_acc) != cudaSuccess) (void)cudaGetLastError();
     delete s;
 }
@@ -888,9 +893,7 @@ extern "C" pdf_status pdf_state_reset(pdf_state *s) {
     DeviceGuard dg(s->c->device);
     const size_t G = s->c->n_first();
     PDF_CUDA(cudaDeviceSynchronize());
-    PDF_CUDA(cudaMemset(s->first_x.p, 0xFF, 4 * G));
-    PDF_CUDA(cudaMemset(s->first_y.p, 0xFF, 4 * G));
-    PDF_CUDA(cudaMemset(s->acc.p, 0, sizeof(DevAcc)));
+    PDF_CUDA(launch_state_reset(s->first_x.as<uint32_t>(), 2 * G, s->acc.as<DevAcc>(), s->mirror, nullptr));
     PDF_CUDA(cudaDeviceSynchronize());
     return PDF_OK;
 }
@@ -900,9 +903,7 @@ extern "C" pdf_status pdf_state_reset_async(pdf_state *s, void *stream) {
     DeviceGuard dg(s->c->device);
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     const size_t G = s->c->n_first();
-    PDF_CUDA(cudaMemsetAsync(s->first_x.p, 0xFF, 4 * G, cs));
-    PDF_CUDA(cudaMemsetAsync(s->first_y.p, 0xFF, 4 * G, cs));
-    PDF_CUDA(cudaMemsetAsync(s->acc.p, 0, sizeof(DevAcc), cs));
+    PDF_CUDA(launch_state_reset(s->first_x.as<uint32_t>(), 2 * G, s->acc.as<DevAcc>(), s->mirror, cs));
     return PDF_OK;
 }
 
@@ -964,9 +965,12 @@ extern "C" pdf_status pdf_state_snapshot_on(pdf_state *s, uint32_t *first_x, uin
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     if (first_x) PDF_CUDA(cudaMemcpyAsync(first_x, s->first_x.p, 4 * G, cudaMemcpyDeviceToHost, cs));
     if (first_y) PDF_CUDA(cudaMemcpyAsync(first_y, s->first_y.p, 4 * G, cudaMemcpyDeviceToHost, cs));
-    PDF_CUDA(cudaMemcpyAsync(s->host_acc, s->acc.p, sizeof(DevAcc), cudaMemcpyDeviceToHost, cs));
+    // the mirror holds the accumulators, unless a batch is marked and not yet
+    // counted (its marking may have left an error there)
+    const bool fetch = s->pending;
+    if (fetch) PDF_CUDA(cudaMemcpyAsync(s->host_acc, s->acc.p, sizeof(DevAcc), cudaMemcpyDeviceToHost, cs));
     PDF_CUDA(cudaStreamSynchronize(cs));
-    const DevAcc &h = *s->host_acc;
+    const DevAcc h = s->host_acc[fetch ? 0 : 1];
     if (tot) {
         tot->lo = h.total_lo;
         tot->hi = h.total_hi;
@@ -992,6 +996,7 @@ extern "C" pdf_status pdf_state_restore(pdf_state *s, const uint32_t *first_x,
     h.flags = tot->flags;
     PDF_CUDA(cudaMemcpy(s->acc.p, &h, sizeof h, cudaMemcpyHostToDevice));
     PDF_CUDA(cudaDeviceSynchronize());
+    s->host_acc[1] = h;
     return PDF_OK;
 }
 
@@ -1416,12 +1421,19 @@ extern "C" pdf_status pdf_state_first_copy(pdf_state *s, uint32_t *first_x, uint
     DeviceGuard dg(s->c->device);
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     const size_t bytes = 4 * (size_t)s->c->n_first();
-    if (to_state) {
-        PDF_CUDA(cudaMemcpyAsync(s->first_x.p, first_x, bytes, cudaMemcpyDeviceToDevice, cs));
-        PDF_CUDA(cudaMemcpyAsync(s->first_y.p, first_y, bytes, cudaMemcpyDeviceToDevice, cs));
+    uint32_t *sx = s->first_x.as<uint32_t>(), *sy = s->first_y.as<uint32_t>();
+    // the state's two arrays are rows of one block, and so are the caller's
+    // when the second lies past the first: one copy of two rows
+    const uintptr_t x = reinterpret_cast<uintptr_t>(first_x), y = reinterpret_cast<uintptr_t>(first_y);
+    if (y >= x + bytes && y - x < (1ull << 31)) {
+        if (to_state) PDF_CUDA(cudaMemcpy2DAsync(sx, bytes, first_x, y - x, bytes, 2, cudaMemcpyDeviceToDevice, cs));
+        else PDF_CUDA(cudaMemcpy2DAsync(first_x, y - x, sx, bytes, bytes, 2, cudaMemcpyDeviceToDevice, cs));
+    } else if (to_state) {
+        PDF_CUDA(cudaMemcpyAsync(sx, first_x, bytes, cudaMemcpyDeviceToDevice, cs));
+        PDF_CUDA(cudaMemcpyAsync(sy, first_y, bytes, cudaMemcpyDeviceToDevice, cs));
     } else {
-        PDF_CUDA(cudaMemcpyAsync(first_x, s->first_x.p, bytes, cudaMemcpyDeviceToDevice, cs));
-        PDF_CUDA(cudaMemcpyAsync(first_y, s->first_y.p, bytes, cudaMemcpyDeviceToDevice, cs));
+        PDF_CUDA(cudaMemcpyAsync(first_x, sx, bytes, cudaMemcpyDeviceToDevice, cs));
+        PDF_CUDA(cudaMemcpyAsync(first_y, sy, bytes, cudaMemcpyDeviceToDevice, cs));
     }
     return PDF_OK;
 }
@@ -1686,6 +1698,8 @@ struct pdf_batch {
     cudaStream_t side[kMaxBatchClasses - 1] = {};
     cudaEvent_t fork = nullptr, join[kMaxBatchClasses - 1] = {};
     cudaStream_t up = nullptr;  // uploads of the control block
+    cudaEvent_t uploaded = nullptr;
+    bool wait_upload = false;   // the next run's stream still has to wait for it
     unsigned char *host_ctl = nullptr;  // mapped pinned staging of the control block
     size_t host_bytes = 0;
     cudaEvent_t prof[3] = {};  // pdf_batch_profile: pass start, forward joined, pass end
@@ -1708,6 +1722,8 @@ struct pdf_batch {
         if (cap_stream) cudaStreamDestroy(cap_stream);
         if (up) cudaStreamDestroy(up);
         up = nullptr;
+        if (uploaded) cudaEventDestroy(uploaded);
+        uploaded = nullptr;
         for (auto &x : side)
             if (x) cudaStreamDestroy(x);
         for (auto &x : join)
@@ -1780,6 +1796,20 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
     for (Walk &k : walks)
         if (k.resident && res_ctas < 2 * sms)
             k.rs.per = std::max<uint32_t>(1, (uint32_t)(k.rs.per * res_ctas / (2 * sms)));
+    // Jobs of one block width whose CTAs all fit the GPU at the lowest occupancy
+    // among them share one launch.
+    for (uint32_t bw = 1; bw <= 8; bw *= 2) {
+        uint64_t ctas = 0;
+        uint32_t low = ~0u;
+        for (const Walk &k : walks)
+            if (k.resident && k.bw == bw) {
+                ctas += (k.rs.blocks + k.rs.per - 1) / k.rs.per;
+                low = std::min(low, k.rs.occ);
+            }
+        if (ctas && ctas <= sms * low)
+            for (Walk &k : walks)
+                if (k.resident && k.bw == bw) k.rs.occ = low;
+    }
     const auto occ = [](const Walk &k) { return k.resident ? k.rs.occ : k.p->occ; };
     std::vector<uint32_t> order(n_jobs);
     for (uint32_t i = 0; i < n_jobs; i++) order[i] = i;
@@ -1820,6 +1850,7 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
         a.active = s->ws.active.as<uint32_t>();
         fa[i] = a;
         ca[i] = base_cover(c, wk, s->ws, a.M, a.ld, n, (uint32_t)j.pair_base, a.first_x, a.first_y, acc);
+        ca[i].mirror = s->mirror;
         const uint64_t blocks = wk.resident ? (wk.rs.blocks + wk.rs.per - 1) / wk.rs.per : (W + p.bw - 1) / p.bw;
         if (bp[i] + blocks > 0x7FFFFFFFull || gp[i] + G > 0xFFFFFFFFull) return PDF_ENOTSUP;
         bp[i + 1] = bp[i] + (uint32_t)blocks;
@@ -1892,6 +1923,7 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
     // transfer would queue behind other host threads' bulk uploads (a
     // server's arriving jobs), which held passes up for hundreds of ms.
     if (b->host_bytes < o_i) {
+        if (b->uploaded) PDF_CUDA(cudaEventSynchronize(b->uploaded));
         const size_t want = std::max<size_t>({o_i, 2 * b->host_bytes, (size_t)256 << 10});
         if (b->host_ctl) cudaFreeHost(b->host_ctl);
         b->host_ctl = nullptr;
@@ -1900,6 +1932,8 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
             return PDF_ENOMEM;
         b->host_bytes = want;
     }
+    // (the upload before this one may not have been run, or waited for, yet)
+    if (b->uploaded) PDF_CUDA(cudaEventSynchronize(b->uploaded));
     unsigned char *hbuf = b->host_ctl;
     std::memset(hbuf, 0, o_i);
     std::memcpy(hbuf + o_f, fa.data(), sizeof(FwdArgs) * n_jobs);
@@ -1911,13 +1945,16 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
         return PDF_ENOMEM;
     void *src = nullptr;
     if (!up && !b->up) PDF_CUDA(cudaStreamCreateWithFlags(&b->up, cudaStreamNonBlocking));
+    if (!up && !b->uploaded) PDF_CUDA(cudaEventCreateWithFlags(&b->uploaded, cudaEventDisableTiming));
     PDF_CUDA(cudaHostGetDevicePointer(&src, hbuf, 0));
+    L.host_ctl = static_cast<BatchCtl *>(src);
     // the launch below is checked with cudaGetLastError, which would also
     // report an unchecked failure left on this thread by an earlier call
     // (this library's or the caller's); start from a clean slate
     (void)cudaGetLastError();
     PDF_CUDA(launch_copy_from_host(b->ctl.p, src, o_i / 16, up ? up : b->up));
-    if (!up) PDF_CUDA(cudaStreamSynchronize(b->up));
+    b->wait_upload = !up;
+    if (!up) PDF_CUDA(cudaEventRecord(b->uploaded, b->up));
     unsigned char *base = b->ctl.as<unsigned char>();
     L.ctl = reinterpret_cast<BatchCtl *>(base);
     L.fargs = reinterpret_cast<FwdArgs *>(base + o_f);
@@ -1991,6 +2028,15 @@ extern "C" pdf_status pdf_batch_run_async(pdf_batch *b, void *stream) {
     DeviceGuard dg(b->device);
     if (!dg.ok) return PDF_ECUDA;
     (void)cudaGetLastError();  // an unchecked failure of an earlier call is not this run's
+    if (b->wait_upload) {
+        // in stream order; a stream that the caller captures cannot wait for
+        // work outside its graph, so there the host does
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        PDF_CUDA(cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &cap));
+        if (cap != cudaStreamCaptureStatusNone) PDF_CUDA(cudaEventSynchronize(b->uploaded));
+        else PDF_CUDA(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), b->uploaded, 0));
+        b->wait_upload = false;
+    }
     if (!b->use_graph) {
         PDF_CUDA(launch_batch(b->L, static_cast<cudaStream_t>(stream)));
         return PDF_OK;
@@ -2049,11 +2095,7 @@ pdf_status batch_rebind_on(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_j
 }
 
 pdf_status batch_pass_async(pdf_batch *b, cudaStream_t stream) {
-    pdf_status st = pdf_batch_run_async(b, stream);
-    if (st != PDF_OK) return st;
-    DeviceGuard dg(b->device);
-    PDF_CUDA(cudaMemcpyAsync(b->host_ctl, b->ctl.p, sizeof(BatchCtl), cudaMemcpyDeviceToHost, stream));
-    return PDF_OK;
+    return pdf_batch_run_async(b, stream);
 }
 
 pdf_status batch_pass_status(const pdf_batch *b) {
@@ -2065,12 +2107,8 @@ extern "C" pdf_status pdf_batch_run(pdf_batch *b, void *stream) {
     if (st != PDF_OK) return st;
     DeviceGuard dg(b->device);
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
-    // read back into the pinned staging of the control block (its image is
-    // rewritten at the next rebind): a DMA, not a staged pageable copy
-    BatchCtl *h = reinterpret_cast<BatchCtl *>(b->host_ctl);
-    PDF_CUDA(cudaMemcpyAsync(h, b->ctl.p, sizeof(BatchCtl), cudaMemcpyDeviceToHost, cs));
     PDF_CUDA(cudaStreamSynchronize(cs));
-    return err_status(h->err);
+    return batch_pass_status(b);  // the control word, left there by the kernel that closed the pass
 }
 
 // Autotuner of the batch tile width: times the whole batch at each candidate.

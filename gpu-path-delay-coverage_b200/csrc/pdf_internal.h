@@ -22,8 +22,8 @@ struct pdf_netbuf {
 //                     enqueued on `stream` (in order before the next pass on
 //                     it) instead of waited for; the batch must not be
 //                     rebound again before that pass is done
-//   batch_pass_async  one pass on `stream`, its control word read back into
-//                     the batch's pinned staging after it
+//   batch_pass_async  one pass on `stream`; the kernel that closes it leaves
+//                     its error word in the batch's pinned staging
 //   batch_pass_status the status of that pass, once the stream has passed it
 typedef struct CUstream_st *cudaStream_t;
 pdf_status batch_rebind_on(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs, uint32_t flags,

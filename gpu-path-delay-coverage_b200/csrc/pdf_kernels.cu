@@ -1421,19 +1421,29 @@ __global__ void k_batch_active(const CoverArgs *args, const uint32_t *gpref, uin
 }
 
 // Close every circuit's batch (by the last CTA of a batch's cover).
-__device__ void batch_close_all(CoverArgs *args, FwdArgs *fargs, uint32_t n, BatchCtl *ctl, uint32_t append) {
+__device__ void batch_close_all(CoverArgs *args, FwdArgs *fargs, uint32_t n, BatchCtl *ctl, uint32_t append,
+                                BatchCtl *host_ctl) {
+    __shared__ unsigned int s_err;
+    if (threadIdx.x == 0) s_err = 0;
+    __syncthreads();
     unsigned int err = 0;
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
         const uint64_t np = args[i].n_pairs;
         err |= args[i].acc->err;
         batch_close(args[i].acc, np);
+        if (args[i].mirror) *args[i].mirror = *args[i].acc;
         if (append) {
             args[i].pair_base += (uint32_t)np;
             fargs[i].pair_base += (uint32_t)np;
         }
     }
     err = __reduce_or_sync(0xFFFFFFFFu, err);
-    if ((threadIdx.x & 31) == 0 && err) atomicOr(&ctl->err, err);
+    if ((threadIdx.x & 31) == 0 && err) atomicOr(&s_err, err);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        ctl->err = s_err;
+        host_ctl->err = s_err;  // the host reads it there
+    }
 }
 
 // The batch's cover in two passes of the same code.  TIER 0 lists at most
@@ -1447,7 +1457,7 @@ __device__ void batch_close_all(CoverArgs *args, FwdArgs *fargs, uint32_t n, Bat
 template <int TIER>
 __global__ void __launch_bounds__(kCoverThreads) k_batch_cover(CoverArgs *args, FwdArgs *fargs, uint32_t n,
                                                                const uint2 *in_items, uint2 *out_items, BatchCtl *ctl,
-                                                               uint32_t append, uint32_t cap) {
+                                                               uint32_t append, uint32_t cap, BatchCtl *host_ctl) {
     __shared__ CoverArgs s_a;
     __shared__ uint32_t s_last;
     const uint32_t n_items = TIER == 0 ? ctl->n_items : ctl->n_mid;
@@ -1475,7 +1485,7 @@ __global__ void __launch_bounds__(kCoverThreads) k_batch_cover(CoverArgs *args, 
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    if (!(TIER == 0 ? ctl->n_mid : ctl->n_over)) batch_close_all(args, fargs, n, ctl, append);
+    if (!(TIER == 0 ? ctl->n_mid : ctl->n_over)) batch_close_all(args, fargs, n, ctl, append, host_ctl);
     if (threadIdx.x == 0) *done = 0;
 }
 
@@ -1483,7 +1493,7 @@ __global__ void __launch_bounds__(kCoverThreads) k_batch_cover(CoverArgs *args, 
 // item's circuit; every spilling circuit has at least gridDim slots).
 __global__ void __launch_bounds__(kCoverThreads) k_batch_cover_spill(CoverArgs *args, FwdArgs *fargs, uint32_t n,
                                                                      const uint2 *over_items, BatchCtl *ctl,
-                                                                     uint32_t append) {
+                                                                     uint32_t append, BatchCtl *host_ctl) {
     __shared__ CoverArgs s_a;
     __shared__ uint32_t s_last;
     const uint32_t n_over = ctl->n_over;
@@ -1501,7 +1511,7 @@ __global__ void __launch_bounds__(kCoverThreads) k_batch_cover_spill(CoverArgs *
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    batch_close_all(args, fargs, n, ctl, append);
+    batch_close_all(args, fargs, n, ctl, append, host_ctl);
     if (threadIdx.x == 0) {
         ctl->n_over = 0;
         ctl->done_over = 0;
@@ -1834,14 +1844,14 @@ cudaError_t launch_batch(const BatchLaunch &b, cudaStream_t st) {
     k_batch_active<<<(b.total_gates + 255) / 256, 256, 0, st>>>(b.cargs, b.gpref, b.n, b.items, b.ctl);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     k_batch_cover<0><<<b.small_grid, kCoverThreads, cover_small_smem_bytes(b.small_cap), st>>>(
-        b.cargs, b.fargs, b.n, b.items, b.mid_items, b.ctl, b.append, b.small_cap);
+        b.cargs, b.fargs, b.n, b.items, b.mid_items, b.ctl, b.append, b.small_cap, b.host_ctl);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     k_batch_cover<1><<<b.cover_grid, kCoverThreads, cover_smem_tables(b.hash_cap, kCoverCand), st>>>(
-        b.cargs, b.fargs, b.n, b.mid_items, b.over_items, b.ctl, b.append, b.hash_cap);
+        b.cargs, b.fargs, b.n, b.mid_items, b.over_items, b.ctl, b.append, b.hash_cap, b.host_ctl);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (b.spill_grid) {
         k_batch_cover_spill<<<b.spill_grid, kCoverThreads, 0, st>>>(b.cargs, b.fargs, b.n, b.over_items, b.ctl,
-                                                                    b.append);
+                                                                    b.append, b.host_ctl);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if (b.prof[2] && (e = cudaEventRecordWithFlags(b.prof[2], st, pflag)) != cudaSuccess) return e;
@@ -1900,6 +1910,23 @@ cudaError_t launch_copy_from_host(void *dst, const void *src_mapped, size_t n16,
     const unsigned blocks = (unsigned)std::min<size_t>((n16 + 255) / 256, 64);
     k_copy_from_host<<<blocks, 256, 0, st>>>(static_cast<uint4 *>(dst), static_cast<const uint4 *>(src_mapped),
                                              n16);
+    return cudaGetLastError();
+}
+
+// A state as new: no first-detecting pair, zero totals (also where the host
+// reads them).
+__global__ void k_state_reset(uint32_t *first, size_t n, DevAcc *acc, DevAcc *mirror) {
+    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x, T = (size_t)gridDim.x * blockDim.x;
+    uint4 *f4 = reinterpret_cast<uint4 *>(first);
+    for (size_t i = t; i < n / 4; i += T) f4[i] = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
+    if (t < n % 4) first[n - 1 - t] = kEmpty;
+    if (t == 0) {
+        *acc = DevAcc{};
+        *mirror = DevAcc{};
+    }
+}
+cudaError_t launch_state_reset(uint32_t *first, size_t n, DevAcc *acc, DevAcc *mirror, cudaStream_t st) {
+    k_state_reset<<<(unsigned)std::min<size_t>(n / 1024 + 1, 592), 256, 0, st>>>(first, n, acc, mirror);
     return cudaGetLastError();
 }
 

@@ -203,6 +203,7 @@ struct BatchLaunch {
     uint2 *over_items;     // [same]: items whose pair marks more nets than the cover's table
     uint32_t spill_grid;   // CTAs of the batch's spill cover (<= every spilling circuit's slots)
     BatchCtl *ctl;
+    BatchCtl *host_ctl;    // mapped host memory: the pass's error word
     uint32_t n, total_blocks, total_gates;
     uint32_t sem, threads, cover_grid, hash_cap, append;  // sem: PDF_MARK_*
     uint32_t tile;         // the widest circuit tile
@@ -283,6 +284,8 @@ cudaError_t launch_bitmap_from_marks(const DevCircuit &c, const uint32_t *M, uin
 constexpr size_t kNoAllocScratchBytes = (size_t)8 << 20;
 cudaError_t noalloc_scratch(int device, unsigned char **out);
 
+// first: n words (16-byte aligned), set to "none"; acc and its host mirror zeroed.
+cudaError_t launch_state_reset(uint32_t *first, size_t n, DevAcc *acc, DevAcc *mirror, cudaStream_t st);
 cudaError_t launch_batch_begin(DevAcc *acc, cudaStream_t st);
 // Copies n16 16-byte words from mapped pinned host memory to device memory
 // with SM loads, so the copy does not queue behind other host threads'

@@ -1694,6 +1694,7 @@ struct pdf_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     bool use_graph = true;
+    bool ran = false;  // since it was built: the first run launches directly, the second captures
     // side streams and fork/join events of the forward launches per class
     cudaStream_t side[kMaxBatchClasses - 1] = {};
     cudaEvent_t fork = nullptr, join[kMaxBatchClasses - 1] = {};
@@ -1763,6 +1764,7 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
             return PDF_EINVAL;
     }
     b->drop_graph();
+    b->ran = false;
     b->device = c0->device;
     b->circuits.clear();
     b->states.clear();
@@ -2037,11 +2039,17 @@ extern "C" pdf_status pdf_batch_run_async(pdf_batch *b, void *stream) {
         else PDF_CUDA(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), b->uploaded, 0));
         b->wait_upload = false;
     }
-    if (!b->use_graph) {
-        PDF_CUDA(launch_batch(b->L, static_cast<cudaStream_t>(stream)));
+    // A graph pays from its second replay on (capturing, instantiating and
+    // destroying one takes over 200 us, more than a small pass): a batch that is
+    // bound anew for every pass launches directly.
+    if (!b->use_graph || (!b->exec && !b->ran)) {
+        BatchLaunch L = b->L;
+        L.prof_external = 0;
+        PDF_CUDA(launch_batch(L, static_cast<cudaStream_t>(stream)));
+        b->ran = true;
         return PDF_OK;
     }
-    if (!b->exec) {  // capture the three launches once
+    if (!b->exec) {  // capture the launches once
         PDF_CUDA(cudaStreamBeginCapture(b->cap_stream, cudaStreamCaptureModeThreadLocal));
         const cudaError_t le = launch_batch(b->L, b->cap_stream);
         cudaGraph_t g = nullptr;

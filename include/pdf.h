@@ -383,8 +383,8 @@ pdf_status pdf_cover_noalloc(pdf_circuit *c, const uint32_t *mark, uint64_t n_pa
 
 /*
  * A batch grades the vector pairs of many (circuit, state) jobs in one pass of
- * a few kernel launches, captured once as a CUDA graph and replayed by each
- * pdf_batch_run.  Each job's result is the same as pdf_grade of that job alone
+ * a few kernel launches, captured as a CUDA graph at the second pdf_batch_run
+ * after it was built and replayed by each run from then on.  Each job's result is the same as pdf_grade of that job alone
  * (its state's first-detect ids and totals).  No reference counterpart: the
  * reference grades one circuit per process (main.cu:129-235).
  *
@@ -406,7 +406,7 @@ typedef struct pdf_batch_job {
 } pdf_batch_job;
 enum {
     PDF_BATCH_APPEND = 1,   /* each run advances every job's pair_base by its pair count */
-    PDF_BATCH_NO_GRAPH = 2  /* launch the kernels directly instead of replaying a captured graph
+    PDF_BATCH_NO_GRAPH = 2  /* always launch the kernels directly instead of replaying a captured graph
                                (for batches rebuilt often, or when other host threads make
                                device-synchronising CUDA calls while a run might capture) */
 };
@@ -428,7 +428,7 @@ void pdf_batch_destroy(pdf_batch *b);
  * run until a rebind succeeds. */
 pdf_status pdf_batch_rebind(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs, uint32_t flags);
 pdf_status pdf_batch_query(const pdf_batch *b, pdf_batch_info *info);
-/* One pass over every job, stream-ordered (the first call captures the graph). */
+/* One pass over every job, stream-ordered (the second call captures the graph). */
 pdf_status pdf_batch_run_async(pdf_batch *b, void *stream);
 /* pdf_batch_run_async, then wait; reports a device-side error of any job. */
 pdf_status pdf_batch_run(pdf_batch *b, void *stream);

@@ -271,8 +271,10 @@ struct pdf_circuit {
     int device = 0;
     int mark_mode = PDF_MARK_DEFAULT;
     pdf_circuit_info info{};
-    DevBuf mem;  // the error word and both plans' arrays
-    uint32_t *err = nullptr;
+    DevBuf mem;  // both plans' arrays
+    // the stage calls' error word: mapped host memory, from the first such call
+    // on (read after the call's sync, without a copy)
+    uint32_t *host_err = nullptr, *err = nullptr;
     uint32_t bw = 4;  // the tile: column block of the full walk, divisor of the device planes' pitch
     Plan full, red;   // every gate; the reduced netlist (n_gates 0: none)
     // the plan of grading calls that ask for no plane
@@ -761,10 +763,9 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         delete c;
         return st2;
     };
-    // One device block: the error word, then both plans' arrays.
+    // One device block: both plans' arrays.
     {
         PlanUpload up;
-        up.add(nullptr, 16);
         const ResidentImage none;
         const bool reduced = rnet.n_gates() != 0;
         const PlanOffsets fo = up.add_plan(net, full, reduced ? none : image);
@@ -777,7 +778,6 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
             (void)cudaGetLastError();
             return fail(PDF_ECUDA);
         }
-        c->err = c->mem.as<uint32_t>();
         c->full.bind(full, net, reduced ? none : image, c->mem.as<unsigned char>(), fo);
         if (reduced) c->red.bind(red, rnet, image, c->mem.as<unsigned char>(), ro);
         c->full.wide = wide_full;
@@ -823,6 +823,7 @@ extern "C" void pdf_circuit_destroy(pdf_circuit *c) {
     if (!c) return;
     DeviceGuard dg(c->device);
     c->stage.release();
+    if (c->host_err && cudaFreeHost(c->host_err) != cudaSuccess) (void)cudaGetLastError();
     c->mem.release();
     c->segs.release();
     c->seg_off.release();
@@ -1154,17 +1155,25 @@ cudaError_t launch_walk(const pdf_circuit *c, const Walk &k0, Workspace &ws, con
     return launch_forward(a, mode, c->mark_mode, k.bw, p.threads, p.fwd_smem, cs);
 }
 
-// The device error word of the circuit's stage calls (pdf_sim, pdf_mark):
-// read after the call's work is done, then cleared, so that an expired wait
-// is reported by the call that met it and by no later one.
-pdf_status take_circuit_err(pdf_circuit *c, cudaStream_t cs) {
-    unsigned int e = 0;
-    PDF_CUDA(cudaMemcpyAsync(&e, c->err, sizeof e, cudaMemcpyDeviceToHost, cs));
-    PDF_CUDA(cudaStreamSynchronize(cs));
-    if (e) {
-        PDF_CUDA(cudaMemsetAsync(c->err, 0, sizeof e, cs));
-        PDF_CUDA(cudaStreamSynchronize(cs));
+// The error word of the circuit's stage calls (pdf_sim, pdf_mark): read after
+// the call's work is done, then cleared, so that an expired wait is reported by
+// the call that met it and by no later one.
+pdf_status open_circuit_err(pdf_circuit *c) {
+    if (c->host_err) return PDF_OK;
+    PDF_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&c->host_err), 64, cudaHostAllocMapped));
+    *c->host_err = 0;
+    const cudaError_t e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&c->err), c->host_err, 0);
+    if (e != cudaSuccess) {
+        cudaFreeHost(c->host_err);
+        c->host_err = nullptr;
     }
+    PDF_CUDA(e);
+    return PDF_OK;
+}
+pdf_status take_circuit_err(pdf_circuit *c, cudaStream_t cs) {
+    PDF_CUDA(cudaStreamSynchronize(cs));
+    const unsigned int e = *reinterpret_cast<volatile uint32_t *>(c->host_err);
+    *c->host_err = 0;
     return err_status(e);
 }
 
@@ -1468,6 +1477,7 @@ extern "C" pdf_status pdf_sim(pdf_circuit *c, const pdf_pairs *pr, uint32_t *sim
     DeviceGuard dg(c->device);
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     std::lock_guard<std::mutex> lk(c->mu);
+    if ((st = open_circuit_err(c)) != PDF_OK) return st;
     const bool direct = planes_fit(c, c->full_walk(W), W, ld, {sim_v, sim_t});
     st = ensure_ws(c, c->full_walk(W), c->stage, W, !direct);
     if (st != PDF_OK) return st;
@@ -1491,8 +1501,7 @@ extern "C" pdf_status pdf_sim(pdf_circuit *c, const pdf_pairs *pr, uint32_t *sim
         PDF_CUDA(cudaMemcpy2DAsync(sim_v, ld * 4, a.V, a.ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
         PDF_CUDA(cudaMemcpy2DAsync(sim_t, ld * 4, a.T, a.ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
     }
-    PDF_CUDA(cudaStreamSynchronize(cs));  // the stage scratch is reused by the next stage call
-    return take_circuit_err(c, cs);
+    return take_circuit_err(c, cs);  // waits: the stage scratch is reused by the next stage call
 }
 
 namespace {
@@ -1505,7 +1514,8 @@ pdf_status mark_planes(pdf_circuit *c, const uint32_t *sim_v, const uint32_t *si
     std::lock_guard<std::mutex> lk(c->mu);
     const uint64_t W = (n_pairs + 31) / 32, G = c->info.n_gates;
     const bool direct = planes_fit(c, c->full_walk(W), W, ld, {sim_v, sim_t, mark});
-    pdf_status st = ensure_ws(c, c->full_walk(W), c->stage, W, !direct);
+    pdf_status st = open_circuit_err(c);
+    if (st == PDF_OK) st = ensure_ws(c, c->full_walk(W), c->stage, W, !direct);
     if (st != PDF_OK) return st;
     FwdArgs a = base_fwd(c, c->full_walk(W), n_pairs);
     if (direct) {
@@ -1524,7 +1534,6 @@ pdf_status mark_planes(pdf_circuit *c, const uint32_t *sim_v, const uint32_t *si
     PDF_CUDA(launch_walk(c, c->full_walk(W), c->stage, a, FWD_MARK, cs));
     if (!direct)
         PDF_CUDA(cudaMemcpy2DAsync(mark, ld * 4, a.M, a.ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
-    PDF_CUDA(cudaStreamSynchronize(cs));
     return take_circuit_err(c, cs);
 }
 

@@ -1518,27 +1518,55 @@ __global__ void __launch_bounds__(kCoverThreads) k_batch_cover_spill(CoverArgs *
     }
 }
 
-// Dense first-detect merge over given planes (stage call pdf_merge): one warp
-// per (gate, 32-word chunk), warp minimum, one atomicMin per warp.
+// Dense passes over a mark plane (stage calls): a warp takes a gate and up to
+// kDenseWords words of its row, four 32-word loads in flight.  What bounds
+// them is the plane read once; a warp per 32 words (one load each) ran at a
+// sixth of the copy rate (20,000 gates x 16,384 pairs, 41 MB: merge 36, bitmap
+// 40 us).
+constexpr uint32_t kDenseWords = 512;
+
+// Calls f(k, m): k words past the part's first, m[u] = the lane's valid mark
+// bits in words k + 32 u + lane, until f returns false (in every lane).
+template <class F>
+__device__ __forceinline__ void dense_row(const uint32_t *row, uint32_t w0, uint32_t w1, uint32_t W, uint64_t n_pairs,
+                                          F f) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t last = (n_pairs & 31) ? (1u << (n_pairs & 31)) - 1u : 0xFFFFFFFFu;
+    for (uint32_t w = w0; w < w1; w += 128) {
+        uint32_t m[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t x = w + 32 * u + lane;
+            m[u] = x < w1 ? row[x] : 0u;
+            if (x == W - 1) m[u] &= last;
+        }
+        if (!f(w, m)) break;
+    }
+}
+
+// First-detect merge over given planes (pdf_merge).
 __global__ void k_merge_dense(const DevCircuit c, const uint32_t *V, const uint32_t *M, uint64_t ld,
                               uint64_t n_pairs, uint32_t W, uint32_t pair_base, uint32_t *first_x,
                               uint32_t *first_y) {
-    const uint32_t chunks = (W + 31) / 32;
+    const uint32_t parts = (W + kDenseWords - 1) / kDenseWords;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31;
-    if (warp >= (uint64_t)c.n_gates * chunks) return;
-    const uint32_t g = (uint32_t)(warp / chunks), w = (uint32_t)(warp % chunks) * 32 + lane;
+    if (warp >= (uint64_t)c.n_gates * parts) return;
+    const uint32_t g = (uint32_t)(warp / parts), w0 = (uint32_t)(warp % parts) * kDenseWords;
     uint32_t cx = kEmpty, cy = kEmpty;
-    if (w < W) {
-        uint32_t m = M[(size_t)g * ld + w];
-        if (w == W - 1 && (n_pairs & 31)) m &= (1u << (n_pairs & 31)) - 1u;
-        if (m) {
-            const uint32_t v = V[(size_t)g * ld + w];
-            const uint32_t x = m & ~v, y = m & v;
-            if (x) cx = w * 32 + (__ffs(x) - 1);
-            if (y) cy = w * 32 + (__ffs(y) - 1);
+    dense_row(M + (size_t)g * ld, w0, min(W, w0 + kDenseWords), W, n_pairs, [&](uint32_t w, const uint32_t (&m)[4]) {
+        if (!__any_sync(0xFFFFFFFFu, m[0] | m[1] | m[2] | m[3])) return true;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (!m[u]) continue;
+            const uint32_t x = w + 32 * u + lane, v = V[(size_t)g * ld + x];
+            const uint32_t fx = m[u] & ~v, fy = m[u] & v;
+            if (fx) cx = min(cx, x * 32 + (__ffs(fx) - 1));
+            if (fy) cy = min(cy, x * 32 + (__ffs(fy) - 1));
         }
-    }
+        // later words hold later pairs
+        return !(__any_sync(0xFFFFFFFFu, cx != kEmpty) && __any_sync(0xFFFFFFFFu, cy != kEmpty));
+    });
     cx = __reduce_min_sync(0xFFFFFFFFu, cx);
     cy = __reduce_min_sync(0xFFFFFFFFu, cy);
     if (lane == 0) {
@@ -1549,22 +1577,26 @@ __global__ void k_merge_dense(const DevCircuit c, const uint32_t *V, const uint3
 
 // Column-block bitmaps of nets with a nonzero mark, from a mark plane (stage
 // call pdf_cover).
+// (bw: a power of two, up to 128; the bitmaps are zero before).
 __global__ void k_bitmap_from_marks(const DevCircuit c, const uint32_t *M, uint64_t ld,
                                     uint64_t n_pairs, uint32_t W, uint32_t bw, uint32_t n_blocks,
                                     uint32_t *nzb, uint32_t *blk_maxlvl, uint32_t bm_words) {
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n_blocks) blk_maxlvl[t] = c.n_levels;
-    if (t >= (uint64_t)c.n_gates * n_blocks) return;
-    const uint32_t g = (uint32_t)(t % c.n_gates), blk = (uint32_t)(t / c.n_gates);
-    uint32_t any = 0;
-    for (uint32_t j = 0; j < bw; j++) {
-        const uint32_t w = blk * bw + j;
-        if (w >= W) break;
-        uint32_t m = M[(size_t)g * ld + w];
-        if (w == W - 1 && (n_pairs & 31)) m &= (1u << (n_pairs & 31)) - 1u;
-        any |= m;
-    }
-    if (any) atomicOr(nzb + (size_t)blk * bm_words + (g >> 5), 1u << (g & 31));
+    const uint32_t parts = (W + kDenseWords - 1) / kDenseWords, lane = threadIdx.x & 31;
+    if (t >> 5 >= (uint64_t)c.n_gates * parts) return;
+    const uint32_t g = (uint32_t)((t >> 5) / parts), w0 = (uint32_t)((t >> 5) % parts) * kDenseWords;
+    const uint32_t span = min(bw, 32u), per = 32 / span;  // words of a block within 32, blocks in 32 words
+    dense_row(M + (size_t)g * ld, w0, min(W, w0 + kDenseWords), W, n_pairs, [&](uint32_t w, const uint32_t (&m)[4]) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t z = __ballot_sync(0xFFFFFFFFu, m[u] != 0);
+            const uint32_t part = span == 32 ? z : (z >> (span * lane)) & ((1u << span) - 1u);
+            if (lane < per && part)
+                atomicOr(nzb + (size_t)((w + 32 * u + span * lane) / bw) * bm_words + (g >> 5), 1u << (g & 31));
+        }
+        return true;
+    });
 }
 
 __global__ void k_batch_begin(DevAcc *acc) {
@@ -1880,9 +1912,10 @@ cudaError_t launch_merge_dense(const DevCircuit &c, const uint32_t *V, const uin
                                uint64_t n_pairs, uint32_t pair_base, uint32_t *first_x,
                                uint32_t *first_y, cudaStream_t st) {
     const uint32_t W = (uint32_t)((n_pairs + 31) / 32);
-    const uint64_t warps = (uint64_t)c.n_gates * ((W + 31) / 32);
+    const uint64_t warps = (uint64_t)c.n_gates * ((W + kDenseWords - 1) / kDenseWords);
     const uint64_t blocks = (warps * 32 + 255) / 256;
     if (blocks == 0) return cudaSuccess;
+    if (blocks > 0x7FFFFFFFull) return cudaErrorInvalidValue;
     k_merge_dense<<<(unsigned)blocks, 256, 0, st>>>(c, V, M, ld, n_pairs, W, pair_base, first_x, first_y);
     return cudaGetLastError();
 }
@@ -1894,7 +1927,8 @@ cudaError_t launch_bitmap_from_marks(const DevCircuit &c, const uint32_t *M, uin
     const uint32_t n_blocks = (W + bw - 1) / bw;
     cudaError_t e = cudaMemsetAsync(nzb, 0, (size_t)n_blocks * bm_words * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
-    const uint64_t n = std::max<uint64_t>((uint64_t)c.n_gates * n_blocks, n_blocks);
+    const uint64_t n = std::max<uint64_t>((uint64_t)c.n_gates * ((W + kDenseWords - 1) / kDenseWords) * 32, n_blocks);
+    if ((n + 255) / 256 > 0x7FFFFFFFull) return cudaErrorInvalidValue;
     k_bitmap_from_marks<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(c, M, ld, n_pairs, W, bw, n_blocks,
                                                                      nzb, blk_maxlvl, bm_words);
     return cudaGetLastError();

@@ -1531,6 +1531,7 @@ pdf_status mark_planes(pdf_circuit *c, const uint32_t *sim_v, const uint32_t *si
     a.nzb = c->stage.nzb.as<uint32_t>();
     a.blk_maxlvl = c->stage.maxlvl.as<uint32_t>();
     a.no_prune = prune ? 0u : 1u;
+    a.in_pieces = c->full.in_pieces;
     PDF_CUDA(launch_walk(c, c->full_walk(W), c->stage, a, FWD_MARK, cs));
     if (!direct)
         PDF_CUDA(cudaMemcpy2DAsync(mark, ld * 4, a.M, a.ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));

@@ -455,7 +455,7 @@ __device__ __forceinline__ void forward_cta(const FwdArgs &a, const uint32_t blk
     // the last piece that can still hold a marked gate: the inputs' last, then
     // as far as a marked gate reaches
     __shared__ uint32_t s_fail, s_reach;
-    const bool early = MODE == FWD_FUSED && a.in_pieces;
+    const bool early = MODE != FWD_SIM && a.in_pieces;
     uint32_t my_reach = 0;
     if (threadIdx.x == 0) {
         s_fail = 0;
@@ -656,6 +656,11 @@ __device__ __forceinline__ void forward_cta(const FwdArgs &a, const uint32_t blk
                 empty_block(a, blk, gbm);
                 if (threadIdx.x == 0) atomicOr(a.err, kErrTimeout);
                 return;
+            }
+            if (MODE == FWD_MARK) {  // the rows that the walk leaves out hold no mark
+                const Vec<BW> none{};
+                for (uint32_t g = P.b + threadIdx.x; g < a.c.n_gates; g += blockDim.x)
+                    vst<BW>(a.M + (size_t)g * a.ld + w0, none);
             }
             break;
         }

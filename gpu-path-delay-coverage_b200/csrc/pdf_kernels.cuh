@@ -43,8 +43,8 @@ struct FwdArgs {
     DevCircuit c;
     const Piece *pieces;          // level-ordered runs of gates (the unit of staging and of sync)
     uint32_t n_pieces;
-    uint32_t in_pieces;           // pieces of level 0 when the walk may end before the last piece that
-                                  // can hold a mark (no plane asked for); 0: it never does
+    uint32_t in_pieces;           // pieces of level 0 when the walk may end at the last piece that can hold
+                                  // a mark (FWD_FUSED without planes, FWD_MARK); 0: it never does
     uint32_t cap, ecap;           // gates / edge words per staging buffer
     const uint32_t *far_ids;      // per piece, the far fan-ins it reads (Piece::far_off / far_n),
                                   // each list padded to a multiple of 4 entries

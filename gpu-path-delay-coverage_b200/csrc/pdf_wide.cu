@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(kWideThreads, kWideCtas) k_wide(const FwdArgs 
         }
     };
     // ------------------------------------------------------------- forward
-    const bool early = MODE == FWD_FUSED && !a.store_all && a.in_pieces;
+    const bool early = MODE != FWD_SIM && a.in_pieces;
     const uint32_t cps = wa.cps, nseg = wa.nseg;
     bool ok = true;
     for (uint32_t l = 0; l < L && ok; l++) {
@@ -473,7 +473,13 @@ __global__ void __launch_bounds__(kWideThreads, kWideCtas) k_wide(const FwdArgs 
         }
         if (l + 1 == L && MODE == FWD_SIM) break;
         ok = level_done();
-        if (early && s_seen <= l) break;  // no gate above can be marked
+        if (early && s_seen <= l) {  // no gate above can be marked
+            if (MODE == FWD_MARK) {   // the rows left out hold no mark
+                for (uint32_t g = ga + n + blockIdx.x; g < G; g += gridDim.x)
+                    for (uint32_t x = tid; x < a.W; x += blockDim.x) __stcs(a.M + (size_t)g * a.ld + x, 0u);
+            }
+            break;
+        }
     }
     if (MODE == FWD_SIM || !ok || (MODE == FWD_MARK && a.no_prune)) {
         finish(ok);

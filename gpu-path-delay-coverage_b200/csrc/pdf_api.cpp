@@ -3,6 +3,7 @@
 // Every call returns a status and never exits: the reference's HANDLE_ERROR
 // exit(EXIT_FAILURE) (simkernel.cuh:32-39, markkernel.cuh:13-20,
 // mergekernel.cuh:17-24, coverkernel.cuh:15-25) becomes PDF_ECUDA / PDF_EINVAL.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -138,7 +139,8 @@ struct Workspace {
     DevBuf nzb, maxlvl, active, active_list;
     DevBuf mid_list;          // pairs for the cover's large table
     DevBuf over_list, spill;  // pairs for the spill cover and its per-net (h, c) slots
-    DevBuf flags, sync;       // wide kernel: mark flags per (segment, gate), barrier counters
+    DevBuf flags;             // wide kernel: mark flags per (segment, gate)
+    WideSync *sync = nullptr;  // and its barrier counters, zero between launches (in the owner's block)
     DevBuf nzb_fine, maxlvl_fine;  // lane circuits: the cover's bitmaps per quarter column block
     DevBuf pi_counts;         // pdf_cover_counts: paths per (primary input, pair)
     DevBuf seg_first;  // (net, pair) hash set of the cover with segments
@@ -154,7 +156,6 @@ struct Workspace {
         over_list.release();
         spill.release();
         flags.release();
-        sync.release();
         nzb_fine.release();
         maxlvl_fine.release();
         pi_counts.release();
@@ -248,7 +249,10 @@ struct PlanUpload {
         o.image = add(im.bytes.data(), im.bytes.size());
         return o;
     }
-    bool copy(unsigned char *dst) const {
+    // Done when it returns: work on streams that do not wait for the legacy
+    // stream may follow at once.
+    bool copy(unsigned char *dst) const { return put(dst) && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess; }
+    bool put(unsigned char *dst) const {
         if (bytes <= (1u << 20)) {
             std::vector<unsigned char> img(bytes, 0);
             for (const Part &p : parts)
@@ -271,7 +275,7 @@ struct pdf_circuit {
     int device = 0;
     int mark_mode = PDF_MARK_DEFAULT;
     pdf_circuit_info info{};
-    DevBuf mem;  // both plans' arrays
+    DevBuf mem;  // both plans' arrays and stage.sync
     // the stage calls' error word: mapped host memory, from the first such call
     // on (read after the call's sync, without a copy)
     uint32_t *host_err = nullptr, *err = nullptr;
@@ -345,7 +349,7 @@ struct ProfEvents {
 struct pdf_state {
     pdf_circuit *c = nullptr;
     int device = 0;  // the circuit's device (destroy does not need the circuit)
-    DevBuf mem;  // first-detect ids, falling then rising, and the accumulators
+    DevBuf mem;  // first-detect ids, falling then rising, the accumulators, ws.sync
     struct Ref {
         void *p = nullptr;
         template <class T>
@@ -770,6 +774,8 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         const bool reduced = rnet.n_gates() != 0;
         const PlanOffsets fo = up.add_plan(net, full, reduced ? none : image);
         const PlanOffsets ro = reduced ? up.add_plan(rnet, red, image) : PlanOffsets{};
+        const WideSync rest{};
+        const size_t so = up.add(&rest, sizeof rest);
         if (c->mem.ensure(up.bytes) != cudaSuccess) {
             (void)cudaGetLastError();
             return fail(PDF_ENOMEM);
@@ -778,6 +784,7 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
             (void)cudaGetLastError();
             return fail(PDF_ECUDA);
         }
+        c->stage.sync = reinterpret_cast<WideSync *>(c->mem.as<unsigned char>() + so);
         c->full.bind(full, net, reduced ? none : image, c->mem.as<unsigned char>(), fo);
         if (reduced) c->red.bind(red, rnet, image, c->mem.as<unsigned char>(), ro);
         c->full.wide = wide_full;
@@ -849,7 +856,8 @@ extern "C" pdf_status pdf_state_create(pdf_circuit *c, pdf_state **out) {
     s->device = c->device;
     const size_t G = c->n_first();  // first-detect entries: nets, or segments
     const size_t acc_off = (8 * G + 255) & ~(size_t)255;
-    if (s->mem.ensure(acc_off + sizeof(DevAcc)) != cudaSuccess ||
+    const size_t sync_off = acc_off + ((sizeof(DevAcc) + 255) & ~(size_t)255);
+    if (s->mem.ensure(sync_off + sizeof(WideSync)) != cudaSuccess ||
         cudaHostAlloc(reinterpret_cast<void **>(&s->host_acc), 2 * sizeof(DevAcc), cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer(reinterpret_cast<void **>(&s->mirror), s->host_acc + 1, 0) != cudaSuccess) {
         (void)cudaGetLastError();
@@ -860,11 +868,13 @@ extern "C" pdf_status pdf_state_create(pdf_circuit *c, pdf_state **out) {
     s->first_x.p = s->mem.p;
     s->first_y.p = s->mem.as<uint32_t>() + G;
     s->acc.p = s->mem.as<unsigned char>() + acc_off;
+    s->ws.sync = reinterpret_cast<WideSync *>(s->mem.as<unsigned char>() + sync_off);
     // cleared on a stream of its own: a device-wide sync here would wait for
     // every other circuit's work in flight (a server creates states while it
     // grades)
     cudaStream_t cs = nullptr;
     const bool ok = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) == cudaSuccess &&
+                    cudaMemsetAsync(s->ws.sync, 0, sizeof(WideSync), cs) == cudaSuccess &&
                     launch_state_reset(s->first_x.as<uint32_t>(), 2 * G, s->acc.as<DevAcc>(), s->mirror, cs) ==
                         cudaSuccess &&
                     cudaStreamSynchronize(cs) == cudaSuccess;
@@ -1030,10 +1040,6 @@ pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, b
     if (k.wide) {
         // (segments of one chunk are the most there can be, for either width)
         PDF_CUDA(ws.flags.ensure((uint64_t)p.n_gates * ((W + 31) / 32)));
-        if (!ws.sync.p) {
-            PDF_CUDA(ws.sync.ensure(sizeof(WideSync)));
-            PDF_CUDA(cudaMemset(ws.sync.p, 0, sizeof(WideSync)));
-        }
     } else {
         PDF_CUDA(ws.nzb.ensure(n_blocks * bm_words * 4));
         PDF_CUDA(ws.maxlvl.ensure(n_blocks * 4));
@@ -1144,7 +1150,7 @@ cudaError_t launch_walk(const pdf_circuit *c, const Walk &k0, Workspace &ws, con
         }
         WideArgs wa{};
         wa.flags = ws.flags.as<uint8_t>();
-        wa.sync = ws.sync.as<WideSync>();
+        wa.sync = ws.sync;
         wa.cps = k.cps;
         wa.nseg = k.nseg;
         wa.chunks = k.chunks;
@@ -1424,6 +1430,24 @@ extern "C" pdf_status pdf_grade_async(pdf_circuit *c, pdf_state *s, const pdf_pa
     return grade_cover_locked(c, s, cs);
 }
 
+// Whether [x, end) lies in one device allocation (0.2 us; a second copy takes 3).
+static bool one_allocation(uintptr_t x, uintptr_t end) {
+    using Range = CUresult (*)(CUdeviceptr *, size_t *, CUdeviceptr);
+    static const Range range = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            (void)cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Range>(f);
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    return range && range(&base, &size, x) == CUDA_SUCCESS && end <= base + size;
+}
+
 extern "C" pdf_status pdf_state_first_copy(pdf_state *s, uint32_t *first_x, uint32_t *first_y, int to_state,
                                            void *stream) {
     if (!s || !first_x || !first_y) return PDF_EINVAL;
@@ -1432,9 +1456,9 @@ extern "C" pdf_status pdf_state_first_copy(pdf_state *s, uint32_t *first_x, uint
     const size_t bytes = 4 * (size_t)s->c->n_first();
     uint32_t *sx = s->first_x.as<uint32_t>(), *sy = s->first_y.as<uint32_t>();
     // the state's two arrays are rows of one block, and so are the caller's
-    // when the second lies past the first: one copy of two rows
+    // when the second lies past the first in one allocation: one copy of two rows
     const uintptr_t x = reinterpret_cast<uintptr_t>(first_x), y = reinterpret_cast<uintptr_t>(first_y);
-    if (y >= x + bytes && y - x < (1ull << 31)) {
+    if (y >= x + bytes && y - x < (1ull << 31) && one_allocation(x, y + bytes)) {
         if (to_state) PDF_CUDA(cudaMemcpy2DAsync(sx, bytes, first_x, y - x, bytes, 2, cudaMemcpyDeviceToDevice, cs));
         else PDF_CUDA(cudaMemcpy2DAsync(first_x, y - x, sx, bytes, bytes, 2, cudaMemcpyDeviceToDevice, cs));
     } else if (to_state) {
@@ -2186,7 +2210,7 @@ extern "C" pdf_status pdf_batch_autotune(const pdf_netlist *const *netlists, con
             jobs[i] = pdf_batch_job{cs[i], ss[i], pdf_pairs{dv, dt, np, ld, 1}, 0};
         }
         if (st == PDF_OK) st = pdf_batch_create(jobs.data(), n, 0, &b);
-        if (st == PDF_OK) st = pdf_batch_run(b, nullptr);  // warm-up (captures the graph)
+        for (int r = 0; r < 2 && st == PDF_OK; r++) st = pdf_batch_run(b, nullptr);  // warm-up; the second captures the graph
         float ms = 0.0f;
         if (st == PDF_OK) {
             if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess ||

@@ -14,6 +14,7 @@
 #include <mutex>
 #include <new>
 #include <system_error>
+#include <type_traits>
 #include <vector>
 
 #include "pdf.h"
@@ -90,14 +91,25 @@ void set_msg(char *msg, size_t len, const char *fmt, unsigned long long a = 0,
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
+    bool held = false;  // a batch or a captured graph has the address
     void release() {
         if (p && cudaFree(p) != cudaSuccess) (void)cudaGetLastError();
         p = nullptr;
         bytes = 0;
+        held = false;
     }
-    // Grow to at least `need` bytes (contents are not kept).
-    cudaError_t ensure(size_t need) {
+    // Grow to at least `need` bytes (contents are not kept).  A held block goes
+    // to `kept` instead of being freed.
+    cudaError_t ensure(size_t need, std::vector<void *> *kept = nullptr) {
         if (bytes >= need) return cudaSuccess;
+        if (held && kept) {
+            try {
+                kept->push_back(p);
+            } catch (const std::bad_alloc &) {
+                return cudaErrorMemoryAllocation;
+            }
+            p = nullptr;
+        }
         release();
         cudaError_t e = dev_alloc(&p, need ? need : 16);
         if (e == cudaSuccess) bytes = need;
@@ -136,33 +148,27 @@ struct DeviceGuard {
 // Per-batch device workspace (owned by a state, or by a circuit for the
 // stage calls).
 struct Workspace {
-    DevBuf nzb, maxlvl, active, active_list;
-    DevBuf mid_list;          // pairs for the cover's large table
-    DevBuf over_list, spill;  // pairs for the spill cover and its per-net (h, c) slots
-    DevBuf flags;             // wide kernel: mark flags per (segment, gate)
-    WideSync *sync = nullptr;  // and its barrier counters, zero between launches (in the owner's block)
-    DevBuf nzb_fine, maxlvl_fine;  // lane circuits: the cover's bitmaps per quarter column block
-    DevBuf pi_counts;         // pdf_cover_counts: paths per (primary input, pair)
-    DevBuf seg_first;  // (net, pair) hash set of the cover with segments
+    DevBuf scratch;            // one block, laid out by scratch_of
+    WideSync *sync = nullptr;  // wide kernel: its barrier counters, zero between launches (in the owner's block)
+    DevBuf pi_counts;          // pdf_cover_counts: paths per (primary input, pair)
+    DevBuf seg_first;          // (net, pair) hash set of the cover with segments
     uint64_t seg_first_mask = 0;
-    DevBuf planes;   // internal V, T, M planes when the caller gives none
-    DevBuf pi;       // staged host pairs
+    DevBuf planes;  // internal V, T, M planes when the caller gives none
+    DevBuf pi;      // staged host pairs
+    // blocks that were outgrown while held: calls of one walk (with planes, say)
+    // grow a state's workspace past what a batch of the other was bound to
+    std::vector<void *> kept;
+    void hold() { scratch.held = seg_first.held = planes.held = pi.held = true; }
     void release() {
-        nzb.release();
-        maxlvl.release();
-        active.release();
-        active_list.release();
-        mid_list.release();
-        over_list.release();
-        spill.release();
-        flags.release();
-        nzb_fine.release();
-        maxlvl_fine.release();
+        scratch.release();
         pi_counts.release();
         seg_first.release();
         seg_first_mask = 0;
         planes.release();
         pi.release();
+        for (void *q : kept)
+            if (cudaFree(q) != cudaSuccess) (void)cudaGetLastError();
+        kept.clear();
     }
 };
 
@@ -1031,38 +1037,63 @@ uint32_t spill_slots(uint64_t n, uint64_t *slot) {
     return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(16, (16ull << 20) / *slot));
 }
 
-// Sizes the workspace for a walk over W words of pairs.  A resident walk's
+// A walk's part of the workspace, W words of pairs: one block, since each
+// allocation costs a new state's first call 20 to 300 us.  A resident walk's
 // column block depends on W, so its share is sized for every smaller W too.
-pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, bool need_planes) {
+struct Scratch {
+    uint32_t *nzb = nullptr, *maxlvl = nullptr;
+    uint32_t *nzb_fine = nullptr, *maxlvl_fine = nullptr;  // the cover's bitmaps per kLaneCoverWords words
+    uint32_t *active = nullptr, *active_list = nullptr;    // bitmap [W], then the count; <= 2 pairs per gate
+    uint32_t *mid_list = nullptr;                          // pairs for the cover's large table
+    uint32_t *over_list = nullptr;                         // pairs for the spill cover
+    unsigned char *spill = nullptr;                        // and its per-net (h, c) slots
+    uint8_t *flags = nullptr;                              // wide kernel: mark flags per (segment, gate)
+    size_t bytes = 0;
+};
+Scratch scratch_of(const pdf_circuit *c, const Walk &k, uint64_t W, unsigned char *base) {
     const Plan &p = *k.p;
     const uint64_t n_blocks = k.resident ? W : (W + k.bw - 1) / k.bw;
-    const uint64_t bm_words = (p.n_gates + 31) / 32;
+    const uint64_t bm_bytes = (uint64_t)(p.n_gates + 31) / 32 * 4;
+    Scratch x;
+    const auto take = [&](auto *&q, uint64_t n) {
+        q = reinterpret_cast<std::remove_reference_t<decltype(q)>>(base + x.bytes);
+        x.bytes += (n + 255) & ~(uint64_t)255;
+    };
     if (k.wide) {
         // (segments of one chunk are the most there can be, for either width)
-        PDF_CUDA(ws.flags.ensure((uint64_t)p.n_gates * ((W + 31) / 32)));
+        take(x.flags, (uint64_t)p.n_gates * ((W + 31) / 32));
     } else {
-        PDF_CUDA(ws.nzb.ensure(n_blocks * bm_words * 4));
-        PDF_CUDA(ws.maxlvl.ensure(n_blocks * 4));
+        take(x.nzb, n_blocks * bm_bytes);
+        take(x.maxlvl, n_blocks * 4);
     }
-    if (k.fine()) {  // the cover's bitmaps per kLaneCoverWords words of a column block
+    if (k.fine()) {
         const uint64_t nf = n_blocks * (k.bw / kLaneCoverWords);
-        PDF_CUDA(ws.nzb_fine.ensure(nf * bm_words * 4));
-        PDF_CUDA(ws.maxlvl_fine.ensure(nf * 4));
+        take(x.nzb_fine, nf * bm_bytes);
+        take(x.maxlvl_fine, nf * 4);
     }
-    // active bitmap [W], then the count; the list holds <= 2 pairs per gate
-    PDF_CUDA(ws.active.ensure(W * 4 + 16));
-    const uint64_t list = std::min<uint64_t>(W * 32, 2 * std::max<uint64_t>(c->n_first(), c->info.n_gates));
-    PDF_CUDA(ws.active_list.ensure(list * 4));
-    PDF_CUDA(ws.mid_list.ensure(list * 4));
+    take(x.active, W * 4 + 16);
+    const uint64_t list = std::min<uint64_t>(W * 32, 2 * std::max<uint64_t>(c->n_first(), c->info.n_gates)) * 4;
+    take(x.active_list, list);
+    take(x.mid_list, list);
     // A pair can mark more nets than the cover's table holds only when the
     // walk has more gates than that; its count then goes through the spill
     // cover.
     if (p.n_gates > c->hash_cap) {
         uint64_t slot;
         const uint32_t slots = spill_slots(p.n_gates, &slot);
-        PDF_CUDA(ws.over_list.ensure(list * 4));
-        PDF_CUDA(ws.spill.ensure(slots * slot));
+        take(x.over_list, list);
+        take(x.spill, slots * slot);
     }
+    return x;
+}
+
+// Sizes the workspace for a walk over W words of pairs.  `keep`: held blocks
+// that are too small stay (not so for a batch that is bound to more pairs than
+// one before it: the older batch is then not run any more).
+pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, bool need_planes, bool keep = true) {
+    const Plan &p = *k.p;
+    std::vector<void *> *kept = keep ? &ws.kept : nullptr;
+    PDF_CUDA(ws.scratch.ensure(scratch_of(c, k, W, nullptr).bytes, kept));
     if (c->seg_len > 1) {
         // (net, pair) entries: at most N per first pair of a segment, two per
         // segment, and one per (net, pair); a table at least twice that
@@ -1070,15 +1101,25 @@ pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, b
         uint64_t cap = 1024;
         while (cap < 2 * most && cap < (1ull << 27)) cap <<= 1;
         if (ws.seg_first_mask + 1 < cap) {
-            PDF_CUDA(ws.seg_first.ensure(cap * 8));
+            PDF_CUDA(ws.seg_first.ensure(cap * 8, kept));
             ws.seg_first_mask = cap - 1;
         }
     }
     // a resident walk keeps V and T on chip: marks only
     if (need_planes)
         PDF_CUDA(ws.planes.ensure((k.resident ? 1 : 3) * (uint64_t)p.n_gates *
-                                  (k.resident ? (W + 7) / 8 * 8 : n_blocks * k.bw) * 4));
+                                      (k.resident ? (W + 7) / 8 * 8 : (W + k.bw - 1) / k.bw * k.bw) * 4,
+                                  kept));
     return PDF_OK;
+}
+Scratch ws_scratch(const pdf_circuit *c, const Walk &k, const Workspace &ws, uint64_t W) {
+    return scratch_of(c, k, W, ws.scratch.as<unsigned char>());
+}
+void use_scratch(FwdArgs &a, const Scratch &x) {
+    a.nzb = x.nzb;
+    a.blk_maxlvl = x.maxlvl;
+    a.nzb_fine = x.nzb_fine;
+    a.maxlvl_fine = x.maxlvl_fine;
 }
 
 // The workspace's planes for a walk over W words (after ensure_ws).
@@ -1149,7 +1190,7 @@ cudaError_t launch_walk(const pdf_circuit *c, const Walk &k0, Workspace &ws, con
             c->wide_shape(k, a.W, 1);
         }
         WideArgs wa{};
-        wa.flags = ws.flags.as<uint8_t>();
+        wa.flags = ws_scratch(c, k0, ws, a.W).flags;
         wa.sync = ws.sync;
         wa.cps = k.cps;
         wa.nseg = k.nseg;
@@ -1193,23 +1234,24 @@ CoverArgs base_cover(pdf_circuit *c, const Walk &k, Workspace &ws, const uint32_
     // a lane walk's cover reads bitmaps per 8 words of its column blocks
     // (fewer candidate nets per pair than the whole block's)
     const bool fine = k.fine();
-    a.nzb = fine ? ws.nzb_fine.as<uint32_t>() : ws.nzb.as<uint32_t>();
-    a.blk_maxlvl = fine ? ws.maxlvl_fine.as<uint32_t>() : ws.maxlvl.as<uint32_t>();
+    const Scratch x = ws_scratch(c, k, ws, (n_pairs + 31) / 32);
+    a.nzb = fine ? x.nzb_fine : x.nzb;
+    a.blk_maxlvl = fine ? x.maxlvl_fine : x.maxlvl;
     a.bm_words = (p.n_gates + 31) / 32;
     a.bw = fine ? kLaneCoverWords : k.bw;
     a.first_x = fx;
     a.first_y = fy;
     a.n_pairs = n_pairs;
     a.pair_base = pair_base;
-    a.active = ws.active.as<uint32_t>();
+    a.active = x.active;
     a.active_count = a.active + (n_pairs + 31) / 32;
-    a.active_list = ws.active_list.as<uint32_t>();
+    a.active_list = x.active_list;
     a.acc = acc;
     a.hash_cap = c->hash_cap;
-    a.mid_list = ws.mid_list.as<uint32_t>();
+    a.mid_list = x.mid_list;
     a.small_cap = c->small_cap;
-    a.over_list = ws.over_list.as<uint32_t>();
-    a.spill = ws.spill.as<unsigned char>();
+    a.over_list = x.over_list;
+    a.spill = x.spill;
     uint64_t slot;
     a.spill_slots = p.n_gates > c->hash_cap ? spill_slots(p.n_gates, &slot) : 0;
     a.seg = c->seg_args();
@@ -1257,7 +1299,7 @@ pdf_status stage_pairs(pdf_circuit *c, const Walk &k, Workspace &ws, const pdf_p
         return PDF_OK;
     }
     const uint64_t Wp = k.resident ? W : (W + c->bw - 1) / c->bw * c->bw;
-    PDF_CUDA(ws.pi.ensure(2 * npi * ((W + c->bw - 1) / c->bw * c->bw) * 4));
+    PDF_CUDA(ws.pi.ensure(2 * npi * ((W + c->bw - 1) / c->bw * c->bw) * 4, &ws.kept));
     uint32_t *dv = ws.pi.as<uint32_t>(), *dt = dv + npi * Wp;
     const cudaMemcpyKind kind = pr->on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     if (pr->ld == Wp) {  // rows already at the device pitch: one contiguous copy per plane
@@ -1295,6 +1337,8 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     // and only the rows read back are written
     const bool planes = out && (out->sim_v || out->sim_t || out->mark);
     const Walk k = planes ? c->full_walk(W) : c->lean_walk(W);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    PDF_CUDA(cudaStreamIsCapturing(cs, &cap));
     const Plan &p = *k.p;
     const bool direct = out && out->on_device && planes_fit(c, k, W, out->ld, {out->sim_v, out->sim_t, out->mark});
     pdf_status st = ensure_ws(c, k, s->ws, W, !direct);
@@ -1303,6 +1347,7 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     uint64_t pld;
     st = stage_pairs(c, k, s->ws, pr, &pv, &pt, &pld, cs);
     if (st != PDF_OK) return st;
+    if (cap != cudaStreamCaptureStatusNone) s->ws.hold();  // the caller's graph will have its addresses
 
     FwdArgs a = base_fwd(c, k, n);
     a.pi_v = pv;
@@ -1318,10 +1363,8 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     } else {
         use_ws_planes(a, k, s->ws, W);
     }
-    a.nzb = s->ws.nzb.as<uint32_t>();
-    a.blk_maxlvl = s->ws.maxlvl.as<uint32_t>();
-    a.nzb_fine = s->ws.nzb_fine.as<uint32_t>();
-    a.maxlvl_fine = s->ws.maxlvl_fine.as<uint32_t>();
+    const Scratch x = ws_scratch(c, k, s->ws, W);
+    use_scratch(a, x);
     // with segments the state holds per-segment ids, merged after the kernel
     a.first_x = c->seg_len > 1 ? nullptr : s->first_x.as<uint32_t>();
     a.first_y = c->seg_len > 1 ? nullptr : s->first_y.as<uint32_t>();
@@ -1343,7 +1386,7 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     }
     // the forward kernel also clears the batch count and the cover's active pairs
     a.acc = acc;
-    a.active = s->ws.active.as<uint32_t>();
+    a.active = x.active;
     PDF_CUDA(launch_walk(c, k, s->ws, a, FWD_FUSED, cs));
     if (c->seg_len > 1) {
         SegMergeArgs sm{};
@@ -1552,8 +1595,7 @@ pdf_status mark_planes(pdf_circuit *c, const uint32_t *sim_v, const uint32_t *si
         PDF_CUDA(cudaMemcpy2DAsync(a.V, a.ld * 4, sim_v, ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
         PDF_CUDA(cudaMemcpy2DAsync(a.T, a.ld * 4, sim_t, ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
     }
-    a.nzb = c->stage.nzb.as<uint32_t>();
-    a.blk_maxlvl = c->stage.maxlvl.as<uint32_t>();
+    use_scratch(a, ws_scratch(c, c->full_walk(W), c->stage, W));
     a.no_prune = prune ? 0u : 1u;
     a.in_pieces = c->full.in_pieces;
     PDF_CUDA(launch_walk(c, c->full_walk(W), c->stage, a, FWD_MARK, cs));
@@ -1865,7 +1907,8 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
         const Walk &wk = walks[order[k]];
         const Plan &p = *wk.p;
         const uint64_t n = j.pairs.n_pairs, W = (n + 31) / 32, G = p.n_gates;
-        if (ensure_ws(c, wk, s->ws, W, true) != PDF_OK) return PDF_ENOMEM;
+        if (ensure_ws(c, wk, s->ws, W, true, false) != PDF_OK) return PDF_ENOMEM;
+        s->ws.hold();  // the batch's arguments hold its addresses
         FwdArgs a = base_fwd(c, wk, n);
         a.pi_v = j.pairs.v;
         a.pi_t = j.pairs.t;
@@ -1873,17 +1916,15 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
         a.store_all = 0;
         a.in_pieces = p.in_pieces;
         use_ws_planes(a, wk, s->ws, W);
-        a.nzb = s->ws.nzb.as<uint32_t>();
-        a.blk_maxlvl = s->ws.maxlvl.as<uint32_t>();
-        a.nzb_fine = s->ws.nzb_fine.as<uint32_t>();
-        a.maxlvl_fine = s->ws.maxlvl_fine.as<uint32_t>();
+        const Scratch x = ws_scratch(c, wk, s->ws, W);
+        use_scratch(a, x);
         a.first_x = s->first_x.as<uint32_t>();
         a.first_y = s->first_y.as<uint32_t>();
         a.pair_base = (uint32_t)j.pair_base;
         DevAcc *acc = s->acc.as<DevAcc>();
         a.err = &acc->err;
         a.acc = acc;
-        a.active = s->ws.active.as<uint32_t>();
+        a.active = x.active;
         fa[i] = a;
         ca[i] = base_cover(c, wk, s->ws, a.M, a.ld, n, (uint32_t)j.pair_base, a.first_x, a.first_y, acc);
         ca[i].mirror = s->mirror;

@@ -195,6 +195,7 @@ struct Walk {
     const Plan *p = nullptr;
     uint32_t bw = 0;
     bool resident = false;
+    int out = RES_LEAN;  // resident: the planes it writes
     // wide kernel: words per lane (0: not it), its chunks per segment and segments
     uint32_t wide = 0, cps = 0, nseg = 0, chunks = 0;
     // the cover's bitmaps are per kLaneCoverWords words
@@ -289,6 +290,11 @@ struct pdf_circuit {
     Plan full, red;   // every gate; the reduced netlist (n_gates 0: none)
     // the plan of grading calls that ask for no plane
     const Plan &lean() const { return red.n_gates ? red : full; }
+    // Planes from the resident kernel: every gate whose value is not constant,
+    // where they fit on chip (the constant rows are filled in), else null.
+    Plan live;
+    const Plan *out_plan = nullptr;
+    const int8_t *value = nullptr;  // [n_gates] the constant value, or -1
     // The wide kernel's shape with lw words per lane: the segment length with
     // the fewest rounds of chunks (and about 1.5 chunks' worth per gate).
     void wide_shape(Walk &k, uint64_t W, uint32_t lw) const {
@@ -318,12 +324,20 @@ struct pdf_circuit {
     Walk lean_walk(uint64_t W) const {
         const Plan &p = lean();
         if (!p.image) return staged_walk(p, W);
+        return resident_walk(p, W, RES_LEAN);
+    }
+    static Walk resident_walk(const Plan &p, uint64_t W, int out) {
         Walk k;
         k.p = &p;
         k.resident = true;
+        k.out = out;
         k.rs = resident_shape(p.res, W);
         k.bw = k.rs.bw;
         return k;
+    }
+    // the walk of calls that ask for planes: all three, or the codes alone (out = RES_SIM)
+    Walk planes_walk(uint64_t W, int out = RES_PLANES) const {
+        return out_plan ? resident_walk(*out_plan, W, out) : full_walk(W);
     }
     uint32_t hash_cap = 4096, cover_threads = 256, cover_grid = 0;
     uint32_t small_cap = 0;  // nets per pair of the cover's small-table pass
@@ -726,11 +740,14 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     if (!other.valid()) pst = build_plan(net, po, full);
     // The reduced netlist (single nets; segments are listed over every net),
     // and the resident kernel's image of what a lean call walks.
-    NetPlan rnet;
-    ResidentImage image;
+    NetPlan rnet, lnet;
+    ResidentImage image, limage;
+    LaunchPlan live;
+    std::vector<int8_t> value;
+    enum { kNoOut, kOutFull, kOutRed, kOutLive } out_of = kNoOut;  // whose image writes planes
     const size_t res_smem = (size_t)prop.sharedMemPerBlockOptin - 1024;
     if (pst == PDF_OK && o.seg_len <= 1) {
-        const NetFacts facts = net_facts(net, fixed);
+        NetFacts facts = net_facts(net, fixed);
         const bool reduced = facts.n_needed <= (uint64_t)G * 9 / 10;
         if (reduced) rnet = reduce_net(net, facts);
         image = build_resident(reduced ? rnet : net, res_smem - 1024);
@@ -746,6 +763,25 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
             if (ro.bw != po.bw) ro.regs = forward_kernel_regs((int)ro.bw, o.mark_mode);
             pst = build_plan(rnet, ro, red);
         }
+        // planes: what the lean image holds if that is all that is not
+        // constant, else an image of its own
+        uint64_t n_live = 0;
+        for (uint32_t g = 0; g < G; g++) n_live += facts.value[g] < 0;
+        if (!image.bytes.empty() && !reduced) {
+            out_of = kOutFull;
+        } else if (!image.bytes.empty() && n_live == facts.n_needed) {
+            out_of = kOutRed;
+        } else if (n_live * 28 <= res_smem) {
+            for (uint32_t g = 0; g < G; g++) facts.needed[g] = facts.value[g] < 0;
+            facts.n_needed = n_live;
+            lnet = reduce_net(net, facts);
+            limage = build_resident(lnet, res_smem - 1024);
+            if (!limage.bytes.empty()) {
+                build_records(lnet, live);
+                out_of = kOutLive;
+            }
+        }
+        if (out_of != kNoOut) value.swap(facts.value);
     }
     if (other.valid()) {
         const pdf_status fst = other.get();
@@ -780,6 +816,8 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         const bool reduced = rnet.n_gates() != 0;
         const PlanOffsets fo = up.add_plan(net, full, reduced ? none : image);
         const PlanOffsets ro = reduced ? up.add_plan(rnet, red, image) : PlanOffsets{};
+        const PlanOffsets lo = out_of == kOutLive ? up.add_plan(lnet, live, limage) : PlanOffsets{};
+        const size_t vo = up.add(value.data(), value.size());
         const WideSync rest{};
         const size_t so = up.add(&rest, sizeof rest);
         if (c->mem.ensure(up.bytes) != cudaSuccess) {
@@ -793,11 +831,14 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         c->stage.sync = reinterpret_cast<WideSync *>(c->mem.as<unsigned char>() + so);
         c->full.bind(full, net, reduced ? none : image, c->mem.as<unsigned char>(), fo);
         if (reduced) c->red.bind(red, rnet, image, c->mem.as<unsigned char>(), ro);
+        if (out_of == kOutLive) c->live.bind(live, lnet, limage, c->mem.as<unsigned char>(), lo);
+        c->out_plan = out_of == kOutLive ? &c->live : out_of == kOutRed ? &c->red : out_of == kOutFull ? &c->full : nullptr;
+        c->value = reinterpret_cast<const int8_t *>(c->mem.as<unsigned char>() + vo);
         c->full.wide = wide_full;
         c->red.wide = wide_red;
         c->full.mean_width = (uint32_t)mean_width;
         c->red.mean_width = red.n_levels > 1 ? (red.n_gates - rnet.level_off[1]) / (red.n_levels - 1) : 0;
-        for (Plan *p : {&c->full, &c->red}) {
+        for (Plan *p : {&c->full, &c->red, &c->live}) {
             p->res.sms = (uint32_t)prop.multiProcessorCount;
             p->res.regs = 64;  // its launch bound's
             p->res.smem_block = res_smem;
@@ -1055,6 +1096,7 @@ Scratch scratch_of(const pdf_circuit *c, const Walk &k, uint64_t W, unsigned cha
     const uint64_t n_blocks = k.resident ? W : (W + k.bw - 1) / k.bw;
     const uint64_t bm_bytes = (uint64_t)(p.n_gates + 31) / 32 * 4;
     Scratch x;
+    if (k.out == RES_SIM) return x;
     const auto take = [&](auto *&q, uint64_t n) {
         q = reinterpret_cast<std::remove_reference_t<decltype(q)>>(base + x.bytes);
         x.bytes += (n + 255) & ~(uint64_t)255;
@@ -1087,11 +1129,21 @@ Scratch scratch_of(const pdf_circuit *c, const Walk &k, uint64_t W, unsigned cha
     return x;
 }
 
+// A resident walk keeps V and T on chip: marks only in the workspace, of its own gates.
+uint64_t resident_mark_words(const Walk &k, uint64_t W) {
+    return k.out == RES_SIM ? 0 : (uint64_t)k.p->n_gates * ((W + 7) / 8 * 8);
+}
+uint64_t out_pitch(uint64_t W) { return (W + 3) / 4 * 4; }  // of planes that it writes into the workspace
+// Words of the workspace's planes; `need`: the caller gives none that the walk can write.
+uint64_t ws_plane_words(const pdf_circuit *c, const Walk &k, uint64_t W, bool need) {
+    if (!k.resident) return need ? 3 * (uint64_t)k.p->n_gates * ((W + k.bw - 1) / k.bw * k.bw) : 0;
+    return resident_mark_words(k, W) + (k.out != RES_LEAN && need ? 3 * (uint64_t)c->info.n_gates * out_pitch(W) : 0);
+}
+
 // Sizes the workspace for a walk over W words of pairs.  `keep`: held blocks
 // that are too small stay (not so for a batch that is bound to more pairs than
 // one before it: the older batch is then not run any more).
 pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, bool need_planes, bool keep = true) {
-    const Plan &p = *k.p;
     std::vector<void *> *kept = keep ? &ws.kept : nullptr;
     PDF_CUDA(ws.scratch.ensure(scratch_of(c, k, W, nullptr).bytes, kept));
     if (c->seg_len > 1) {
@@ -1105,11 +1157,7 @@ pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, b
             ws.seg_first_mask = cap - 1;
         }
     }
-    // a resident walk keeps V and T on chip: marks only
-    if (need_planes)
-        PDF_CUDA(ws.planes.ensure((k.resident ? 1 : 3) * (uint64_t)p.n_gates *
-                                      (k.resident ? (W + 7) / 8 * 8 : (W + k.bw - 1) / k.bw * k.bw) * 4,
-                                  kept));
+    PDF_CUDA(ws.planes.ensure(ws_plane_words(c, k, W, need_planes) * 4, kept));
     return PDF_OK;
 }
 Scratch ws_scratch(const pdf_circuit *c, const Walk &k, const Workspace &ws, uint64_t W) {
@@ -1132,6 +1180,21 @@ void use_ws_planes(FwdArgs &a, const Walk &k, const Workspace &ws, uint64_t W) {
     a.V = ws.planes.as<uint32_t>();
     a.T = a.V + k.p->n_gates * a.ld;
     a.M = a.T + k.p->n_gates * a.ld;
+}
+
+// The planes that a resident walk writes: the caller's (direct), or the workspace's.
+void use_out_planes(FwdArgs &a, const pdf_circuit *c, const Walk &k, const Workspace &ws, uint64_t W, bool direct,
+                    uint32_t *v, uint32_t *t, uint32_t *m, uint64_t ld) {
+    if (!direct) {
+        ld = out_pitch(W);
+        v = ws.planes.as<uint32_t>() + resident_mark_words(k, W);
+        t = v + c->info.n_gates * ld;
+        m = k.out == RES_SIM ? nullptr : t + c->info.n_gates * ld;
+    }
+    a.out_v = v;
+    a.out_t = t;
+    a.out_m = m;
+    a.out_ld = ld;
 }
 
 FwdArgs base_fwd(pdf_circuit *c, const Walk &k, uint64_t n_pairs) {
@@ -1197,7 +1260,12 @@ cudaError_t launch_walk(const pdf_circuit *c, const Walk &k0, Workspace &ws, con
         wa.chunks = k.chunks;
         return launch_wide(a, wa, mode, c->mark_mode, k.wide, p.res.sms, cs);
     }
-    if (k.resident) return launch_resident(a, c->mark_mode, k.bw, k.rs.ctas, k.rs.threads, k.rs.smem, cs);
+    if (k.resident && k.out != RES_LEAN) {
+        const cudaError_t e = launch_fill_planes(c->value, c->info.n_gates, a.n_pairs, a.out_v, a.out_t, a.out_m,
+                                                 a.out_ld, p.res.sms, cs);
+        if (e != cudaSuccess) return e;
+    }
+    if (k.resident) return launch_resident(a, c->mark_mode, k.out, k.bw, k.rs.ctas, k.rs.threads, k.rs.smem, cs);
     if (lane_tile(k.bw)) return launch_lanes(a, mode, c->mark_mode, k.bw, p.threads, p.fwd_smem, cs);
     return launch_forward(a, mode, c->mark_mode, k.bw, p.threads, p.fwd_smem, cs);
 }
@@ -1275,10 +1343,10 @@ bool planes_fit(const pdf_circuit *c, uint64_t W, uint64_t ld, std::initializer_
     return true;
 }
 
-// The same for output and stage planes on walk k: the wide kernel takes any
-// pitch and word-aligned rows.
+// The same for output and stage planes on walk k: the wide and the resident
+// kernel take any pitch and word-aligned rows.
 bool planes_fit(const pdf_circuit *c, const Walk &k, uint64_t W, uint64_t ld, std::initializer_list<const void *> ptrs) {
-    if (!k.wide) return planes_fit(c, W, ld, ptrs);
+    if (!k.wide && !k.resident) return planes_fit(c, W, ld, ptrs);
     if (ld < W || ld >= (1ull << 30)) return false;
     for (const void *p : ptrs)
         if (!p || (reinterpret_cast<uintptr_t>(p) & 3)) return false;
@@ -1336,7 +1404,7 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     // with no plane asked for, only what the marks depend on is evaluated,
     // and only the rows read back are written
     const bool planes = out && (out->sim_v || out->sim_t || out->mark);
-    const Walk k = planes ? c->full_walk(W) : c->lean_walk(W);
+    const Walk k = planes ? c->planes_walk(W) : c->lean_walk(W);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     PDF_CUDA(cudaStreamIsCapturing(cs, &cap));
     const Plan &p = *k.p;
@@ -1355,13 +1423,14 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     a.pi_ld = pld;
     a.store_all = planes ? 1u : 0u;
     a.in_pieces = planes ? 0u : p.in_pieces;
-    if (direct) {
+    if (k.resident || !direct) use_ws_planes(a, k, s->ws, W);
+    if (k.out == RES_PLANES) {
+        use_out_planes(a, c, k, s->ws, W, direct, out->sim_v, out->sim_t, out->mark, out->ld);
+    } else if (direct) {
         a.V = out->sim_v;
         a.T = out->sim_t;
         a.M = out->mark;
         a.ld = out->ld;
-    } else {
-        use_ws_planes(a, k, s->ws, W);
     }
     const Scratch x = ws_scratch(c, k, s->ws, W);
     use_scratch(a, x);
@@ -1405,9 +1474,11 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     }
     if (s->pe) PDF_CUDA(cudaEventRecord(s->pe->ev[1], cs));
     if (out && !direct) {
-        st = copy_plane_out(out->sim_v, out->ld, out->on_device, a.V, a.ld, W, G, cs);
-        if (st == PDF_OK) st = copy_plane_out(out->sim_t, out->ld, out->on_device, a.T, a.ld, W, G, cs);
-        if (st == PDF_OK) st = copy_plane_out(out->mark, out->ld, out->on_device, a.M, a.ld, W, G, cs);
+        const bool o = k.out == RES_PLANES;
+        const uint64_t ld = o ? a.out_ld : a.ld;
+        st = copy_plane_out(out->sim_v, out->ld, out->on_device, o ? a.out_v : a.V, ld, W, G, cs);
+        if (st == PDF_OK) st = copy_plane_out(out->sim_t, out->ld, out->on_device, o ? a.out_t : a.T, ld, W, G, cs);
+        if (st == PDF_OK) st = copy_plane_out(out->mark, out->ld, out->on_device, o ? a.out_m : a.M, ld, W, G, cs);
         if (st != PDF_OK) return st;
     }
     s->pend_walk = k;
@@ -1545,28 +1616,33 @@ extern "C" pdf_status pdf_sim(pdf_circuit *c, const pdf_pairs *pr, uint32_t *sim
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     std::lock_guard<std::mutex> lk(c->mu);
     if ((st = open_circuit_err(c)) != PDF_OK) return st;
-    const bool direct = planes_fit(c, c->full_walk(W), W, ld, {sim_v, sim_t});
-    st = ensure_ws(c, c->full_walk(W), c->stage, W, !direct);
+    const Walk k = c->planes_walk(W, RES_SIM);
+    const bool direct = planes_fit(c, k, W, ld, {sim_v, sim_t});
+    st = ensure_ws(c, k, c->stage, W, !direct);
     if (st != PDF_OK) return st;
     const uint32_t *pv, *pt;
     uint64_t pld;
-    st = stage_pairs(c, c->full_walk(W), c->stage, pr, &pv, &pt, &pld, cs);
+    st = stage_pairs(c, k, c->stage, pr, &pv, &pt, &pld, cs);
     if (st != PDF_OK) return st;
-    FwdArgs a = base_fwd(c, c->full_walk(W), pr->n_pairs);
+    FwdArgs a = base_fwd(c, k, pr->n_pairs);
     a.pi_v = pv;
     a.pi_t = pt;
     a.pi_ld = pld;
-    if (direct) {
+    if (k.resident) {
+        use_out_planes(a, c, k, c->stage, W, direct, sim_v, sim_t, nullptr, ld);
+    } else if (direct) {
         a.V = sim_v;
         a.T = sim_t;
         a.ld = ld;
     } else {
-        use_ws_planes(a, c->full_walk(W), c->stage, W);
+        use_ws_planes(a, k, c->stage, W);
     }
-    PDF_CUDA(launch_walk(c, c->full_walk(W), c->stage, a, FWD_SIM, cs));
+    PDF_CUDA(launch_walk(c, k, c->stage, a, FWD_SIM, cs));
     if (!direct) {
-        PDF_CUDA(cudaMemcpy2DAsync(sim_v, ld * 4, a.V, a.ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
-        PDF_CUDA(cudaMemcpy2DAsync(sim_t, ld * 4, a.T, a.ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
+        const uint32_t *v = k.resident ? a.out_v : a.V, *t = k.resident ? a.out_t : a.T;
+        const uint64_t from = (k.resident ? a.out_ld : a.ld) * 4;
+        PDF_CUDA(cudaMemcpy2DAsync(sim_v, ld * 4, v, from, W * 4, G, cudaMemcpyDeviceToDevice, cs));
+        PDF_CUDA(cudaMemcpy2DAsync(sim_t, ld * 4, t, from, W * 4, G, cudaMemcpyDeviceToDevice, cs));
     }
     return take_circuit_err(c, cs);  // waits: the stage scratch is reused by the next stage call
 }
@@ -2296,6 +2372,7 @@ extern "C" pdf_status pdf_state_reserve(pdf_state *s, uint64_t n_pairs) {
     if (!dg.ok) return PDF_ECUDA;
     std::lock_guard<std::mutex> lk(s->mu);
     const uint64_t W = (n_pairs + 31) / 32;
-    const pdf_status st = ensure_ws(s->c, s->c->lean_walk(W), s->ws, W, true);
-    return st == PDF_OK ? ensure_ws(s->c, s->c->full_walk(W), s->ws, W, true) : st;
+    pdf_status st = ensure_ws(s->c, s->c->lean_walk(W), s->ws, W, true);
+    if (st == PDF_OK) st = ensure_ws(s->c, s->c->planes_walk(W), s->ws, W, true);
+    return st == PDF_OK ? ensure_ws(s->c, s->c->full_walk(W), s->ws, W, !s->c->out_plan) : st;
 }

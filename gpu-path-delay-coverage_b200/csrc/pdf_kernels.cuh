@@ -80,6 +80,10 @@ struct FwdArgs {
     // table, V / T words and marks)
     const void *image;
     uint32_t image_bytes, image_ids, per, n_blocks;
+    // and, where planes are asked for (RES_PLANES; RES_SIM: V and T), the
+    // planes of the caller's gates [n_gates][out_ld]
+    uint32_t *out_v, *out_t, *out_m;
+    uint64_t out_ld;
     // shared-memory byte offsets
     uint32_t off_ring;            // forward: ring [3][R][BW]; reverse: ring2 [R2][BW]
     uint32_t off_rec;             // [2][cap] staged gate records
@@ -230,8 +234,13 @@ cudaError_t launch_batch(const BatchLaunch &b, cudaStream_t st);
 // The resident forward kernel (pdf_resident.cu): threads per CTA at most, and
 // its launches.
 constexpr uint32_t kResidentThreads = 512;
-cudaError_t launch_resident(const FwdArgs &a, int sem, uint32_t bw, uint32_t ctas, uint32_t threads, size_t smem,
-                            cudaStream_t st);
+enum ResidentOut : int { RES_LEAN = 0, RES_PLANES = 1, RES_SIM = 2 };  // no planes; all three; V and T only
+cudaError_t launch_resident(const FwdArgs &a, int sem, int out, uint32_t bw, uint32_t ctas, uint32_t threads,
+                            size_t smem, cudaStream_t st);
+// What such a walk leaves out of the planes: V and T rows of gates of constant
+// value (value[g] 0 or 1), and every gate's M row as zeros (m may be null).
+cudaError_t launch_fill_planes(const int8_t *value, uint32_t n_gates, uint64_t n_pairs, uint32_t *v, uint32_t *t,
+                               uint32_t *m, uint64_t ld, uint32_t sms, cudaStream_t st);
 cudaError_t prepare_resident_class(uint32_t sem, uint32_t bw, size_t smem);
 cudaError_t launch_resident_class(const BatchLaunch &b, const BatchClass &c, cudaStream_t st);
 // The wide forward kernel (pdf_wide.cu): a cooperative grid of kWideCtas CTAs

@@ -23,7 +23,7 @@
 
 namespace {
 
-template <int BW, int SEM>
+template <int BW, int SEM, int OUT>
 __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t cta) {
     constexpr bool FIX = SEM >= 2;
     constexpr uint32_t kGroup = BW == 32 ? 0xFFFFFFFFu : (1u << BW) - 1u;
@@ -38,6 +38,14 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
     uint32_t *ms = reinterpret_cast<uint32_t *>(smraw + a.off_rec);         // [gate][BW] marks
     uint32_t *bm = reinterpret_cast<uint32_t *>(smraw + a.off_bm);
     uint64_t *mbar = reinterpret_cast<uint64_t *>(smraw + a.off_mbar);
+    // a gate's words of the caller's planes (what is asked for in full is
+    // written as it is found; stores do not hold the level chain up)
+    const auto put = [&](uint32_t g, uint32_t w, uint32_t V, uint32_t T) {
+        const uint32_t id = net(g);
+        if (id == kEmpty) return;  // a constant that stands for the fan-ins left out
+        a.out_v[(size_t)id * a.out_ld + w] = V;
+        a.out_t[(size_t)id * a.out_ld + w] = T;
+    };
     __shared__ uint32_t s_reach, s_top, s_max;
     const uint32_t tid = threadIdx.x, NT = blockDim.x, lane = tid & 31;
     const uint32_t L = a.c.n_levels;
@@ -65,7 +73,7 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
     if (__syncthreads_or(!mbar_wait(mbar, 0, a.wait_polls))) {
         // no CTA leaves with a copy in flight; its blocks are published empty
         (void)mbar_wait(mbar, 0);
-        for (uint32_t blk = b0; blk < b1; blk++) {
+        for (uint32_t blk = b0; OUT != RES_SIM && blk < b1; blk++) {
             for (uint32_t q = tid; q < a.bm_words; q += NT) a.nzb[(size_t)blk * a.bm_words + q] = 0;
             if (tid == 0) a.blk_maxlvl[blk] = 0;
         }
@@ -112,8 +120,10 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
             for (int u = 0; u < 4; u++) {
                 const uint32_t g = g0 + u * step;
                 if (g >= n0) continue;
-                const uint32_t T = t[u] & wm, M = T & flagmask(h[u], RF_MARKF0);
+                const uint32_t T = t[u] & wm, M = OUT == RES_SIM ? 0u : T & flagmask(h[u], RF_MARKF0);
                 vt[g * BW + j] = make_uint2(v[u] & wm, T);
+                if (OUT != RES_LEAN && wm) put(g, w, v[u] & wm, T);
+                if (OUT == RES_SIM) continue;
                 ms[g * BW + j] = M;
                 if (M) {
                     any = true;
@@ -149,6 +159,9 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
                     eval_finish<FIX>(h, V, v1, T);
                     V &= wm;
                     T &= wm;
+                    vt[g * BW + j] = make_uint2(V, T);
+                    if (OUT != RES_LEAN && wm) put(g, w, V, T);
+                    if (OUT == RES_SIM) continue;
                     if ((h & RF_MARKF0) && T) {
                         M = T & ms[fan(0) * BW + j];
                         if ((h & RF_SENS) && M) {
@@ -180,7 +193,6 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
                         }
                         M = T & sens_result<SEM == PDF_MARK_FIXED_NONROBUST>(s);
                     }
-                    vt[g * BW + j] = make_uint2(V, T);
                     ms[g * BW + j] = M;
                     if (M) {
                         any = true;
@@ -197,8 +209,9 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
             }
             __syncthreads();
             // s_reach grows past l only in threads that go on, so all decide alike
-            if (l + 1 >= L || s_reach <= l) break;
+            if (l + 1 >= L || (OUT == RES_LEAN && s_reach <= l)) break;
         }
+        if (OUT == RES_SIM) continue;
         // ---- prune (markkernel.cuh:271-293) and merge (mergekernel.cuh:116-198),
         // levels descending: a gate's mark is final once its fan-outs' are.
         // Gates from level s_top on hold no mark, and past the last level walked
@@ -231,6 +244,7 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
                 const uint32_t by = (__ballot_sync(0xFFFFFFFFu, y != 0) >> sh) & kGroup;
                 if ((z >> sh) & kGroup) {  // the gate keeps a mark in the block
                     a.M[(size_t)g * a.ld + w] = nm;  // (rows hold whole blocks)
+                    if (OUT == RES_PLANES && nm) a.out_m[(size_t)net(g) * a.out_ld + w] = nm;
                     if (j == 0) atomicOr(bm + (g >> 5), 1u << (g & 31));
                     // the lowest word of each direction holds its first pair
                     if (x && !(bx & below)) atomicMin(a.first_x + net(g), a.pair_base + w * 32 + (__ffs(x) - 1));
@@ -247,9 +261,31 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
     }
 }
 
-template <int BW, int SEM>
+template <int BW, int SEM, int OUT>
 __global__ void __launch_bounds__(kResidentThreads) k_resident(const FwdArgs a) {
-    resident_cta<BW, SEM>(a, blockIdx.x);
+    resident_cta<BW, SEM, OUT>(a, blockIdx.x);
+}
+
+// Rows that a resident walk with planes leaves out, a warp per row: bound by
+// the stores (20,000 gates, of which 3,400 are not constant, x 32,768 pairs:
+// 220 MB).  VEC: rows start on 16 bytes.
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_fill_planes(const int8_t *value, uint32_t G, uint32_t W, uint32_t last,
+                                                     uint32_t *v, uint32_t *t, uint32_t *m, uint64_t ld) {
+    const uint32_t lane = threadIdx.x & 31;
+    const auto fill = [&](uint32_t *p, uint32_t x) {
+        const uint32_t n4 = VEC ? (W - 1) / 4 : 0;  // the last word, which may hold fewer pairs, is not among them
+        if constexpr (VEC)
+            for (uint32_t q = lane; q < n4; q += 32) __stcs(reinterpret_cast<uint4 *>(p) + q, make_uint4(x, x, x, x));
+        for (uint32_t w = 4 * n4 + lane; w < W; w += 32) __stcs(p + w, w + 1 == W ? x & last : x);
+    };
+    for (uint32_t g = blockIdx.x * 8 + threadIdx.x / 32; g < G; g += gridDim.x * 8) {
+        const int c = value[g];
+        if (m) fill(m + (size_t)g * ld, 0u);
+        if (c < 0) continue;
+        fill(v + (size_t)g * ld, c ? 0xFFFFFFFFu : 0u);
+        fill(t + (size_t)g * ld, 0u);
+    }
 }
 
 // The circuits of a batch whose netlists fit on chip.
@@ -266,16 +302,25 @@ __global__ void __launch_bounds__(kResidentThreads)
         if (gb == 0) batch_begin(ctl);
     }
     __syncthreads();
-    resident_cta<BW, SEM>(s_a, s_blk);
+    resident_cta<BW, SEM, RES_LEAN>(s_a, s_blk);
 }
 
-template <int BW, int SEM>
-cudaError_t launch_t(const FwdArgs &a, uint32_t ctas, uint32_t threads, size_t smem, cudaStream_t st) {
-    const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(k_resident<BW, SEM>), smem);
+template <int BW, int SEM, int OUT>
+cudaError_t launch_out(const FwdArgs &a, uint32_t ctas, uint32_t threads, size_t smem, cudaStream_t st) {
+    const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(k_resident<BW, SEM, OUT>), smem);
     if (e != cudaSuccess) return e;
     if (!ctas || threads % 32 || threads > kResidentThreads) return cudaErrorInvalidValue;
-    k_resident<BW, SEM><<<ctas, threads, smem, st>>>(a);
+    k_resident<BW, SEM, OUT><<<ctas, threads, smem, st>>>(a);
     return cudaGetLastError();
+}
+template <int BW, int SEM>
+cudaError_t launch_t(const FwdArgs &a, int out, uint32_t ctas, uint32_t threads, size_t smem, cudaStream_t st) {
+    switch (out) {
+        case RES_LEAN: return launch_out<BW, SEM, RES_LEAN>(a, ctas, threads, smem, st);
+        case RES_PLANES: return launch_out<BW, SEM, RES_PLANES>(a, ctas, threads, smem, st);
+        // the values depend on the marks' table only through n-input XOR
+        default: return launch_out<BW, SEM & 2, RES_SIM>(a, ctas, threads, smem, st);
+    }
 }
 template <int BW, int SEM>
 cudaError_t launch_batch_t(const BatchLaunch &b, const BatchClass &c, cudaStream_t st) {
@@ -308,9 +353,18 @@ cudaError_t raise_batch_t(size_t smem) {
 
 }  // namespace
 
-cudaError_t launch_resident(const FwdArgs &a, int sem, uint32_t bw, uint32_t ctas, uint32_t threads, size_t smem,
-                            cudaStream_t st) {
-    PDF_RES(launch_t, a, ctas, threads, smem, st)
+cudaError_t launch_resident(const FwdArgs &a, int sem, int out, uint32_t bw, uint32_t ctas, uint32_t threads,
+                            size_t smem, cudaStream_t st) {
+    PDF_RES(launch_t, a, out, ctas, threads, smem, st)
+}
+cudaError_t launch_fill_planes(const int8_t *value, uint32_t n_gates, uint64_t n_pairs, uint32_t *v, uint32_t *t,
+                               uint32_t *m, uint64_t ld, uint32_t sms, cudaStream_t st) {
+    const uint32_t W = (uint32_t)((n_pairs + 31) / 32), last = n_pairs & 31 ? (1u << (n_pairs & 31)) - 1u : 0xFFFFFFFFu;
+    const uint32_t grid = std::min((n_gates + 7) / 8, sms * 8);
+    const auto at16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    if (ld % 4 == 0 && at16(v) && at16(t) && at16(m)) k_fill_planes<true><<<grid, 256, 0, st>>>(value, n_gates, W, last, v, t, m, ld);
+    else k_fill_planes<false><<<grid, 256, 0, st>>>(value, n_gates, W, last, v, t, m, ld);
+    return cudaGetLastError();
 }
 cudaError_t prepare_resident_class(uint32_t sem, uint32_t bw, size_t smem) { PDF_RES(raise_batch_t, smem) }
 cudaError_t launch_resident_class(const BatchLaunch &b, const BatchClass &c, cudaStream_t st) {

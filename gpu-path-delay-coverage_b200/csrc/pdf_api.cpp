@@ -781,7 +781,8 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
                 out_of = kOutLive;
             }
         }
-        if (out_of != kNoOut) value.swap(facts.value);
+        if (out_of == kOutFull) value.assign(G, -1);  // its walk writes every row
+        else if (out_of != kNoOut) value.swap(facts.value);
     }
     if (other.valid()) {
         const pdf_status fst = other.get();

@@ -699,6 +699,8 @@ __device__ __forceinline__ void active_gate(const CoverArgs &a, uint32_t g, Emit
     }
 }
 __global__ void k_active(const CoverArgs a) {
+    grid_trigger();
+    grid_wait();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= a.c.n_gates) return;
     active_gate(a, g, [&](uint32_t d) { a.active_list[atomicAdd(a.active_count, 1u)] = d; });
@@ -1269,6 +1271,8 @@ template <int TIER>
 __global__ void __launch_bounds__(kCoverThreads) k_cover(const CoverArgs a, uint32_t cap) {
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr uint32_t CAND = TIER == 0 ? kCoverCandSmall : kCoverCand;
+    grid_trigger();
+    grid_wait();
     const bool direct = TIER == 0 || !a.mid_list;  // without a queue the large table takes every pair
     const uint32_t n_items = direct ? *a.active_count : a.acc->n_mid;
     if (!direct && !n_items) return;  // the small-table pass closed the batch
@@ -1310,6 +1314,7 @@ __global__ void __launch_bounds__(kCoverThreads) k_cover(const CoverArgs a, uint
 __global__ void __launch_bounds__(kCoverThreads) k_cover_lean(const CoverArgs a) {
     extern __shared__ __align__(128) unsigned char smraw[];
     __shared__ uint32_t s_scan[32], s_pairs[8];
+    grid_trigger();
     const uint32_t N = a.c.n_gates, L = a.c.n_levels, W = (uint32_t)((a.n_pairs + 31) / 32);
     uint32_t *lvt = reinterpret_cast<uint32_t *>(smraw + cover_smem_tables(N, kCoverCandSmall));  // [L + 1]
     uint2 *first = reinterpret_cast<uint2 *>(lvt + ((L + 2) & ~1u));                              // [N]
@@ -1326,6 +1331,7 @@ __global__ void __launch_bounds__(kCoverThreads) k_cover_lean(const CoverArgs a)
         const uint32_t g = threadIdx.x + u * kCoverThreads;
         id[u] = g < N ? net_id(a.c, g) : kEmpty;
     }
+    grid_wait();  // (all above is the circuit's own)
 #pragma unroll
     for (int u = 0; u < kPer; u++)
         f[u] = id[u] == kEmpty ? make_uint2(kEmpty, kEmpty) : make_uint2(a.first_x[id[u]], a.first_y[id[u]]);
@@ -1373,6 +1379,7 @@ __global__ void __launch_bounds__(kCoverThreads) k_cover_lean(const CoverArgs a)
 // After k_cover: the pairs it queued, one per CTA at a time (CTA k uses
 // spill slot k); the last CTA closes the batch.
 __global__ void __launch_bounds__(kCoverThreads) k_cover_spill(const CoverArgs a) {
+    grid_wait();
     const uint32_t n_over = a.acc->n_over;
     if (!n_over) return;  // k_cover closed the batch
     for (uint32_t j = blockIdx.x; j < n_over; j += gridDim.x) spill_pair(a, a.over_list[j], spill_slot(a, blockIdx.x));
@@ -1746,8 +1753,7 @@ cudaError_t launch_cover(const CoverArgs &a, uint32_t grid, uint32_t threads, bo
                             8 * (size_t)a.c.n_gates + 4 * (size_t)W;
         const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(k_cover_lean), smem);
         if (e != cudaSuccess) return e;
-        k_cover_lean<<<std::min(2 * grid, std::max(8u, a.c.n_gates / 3)), threads, smem, st>>>(a);
-        return cudaGetLastError();
+        return launch_next(k_cover_lean, std::min(2 * grid, std::max(8u, a.c.n_gates / 3)), threads, smem, st, a);
     }
     if (zero_active) {
         cudaError_t e = cudaMemsetAsync(a.active, 0, (size_t)(W + 1) * sizeof(uint32_t), st);
@@ -1758,10 +1764,8 @@ cudaError_t launch_cover(const CoverArgs &a, uint32_t grid, uint32_t threads, bo
         if (e != cudaSuccess) return e;
         const uint32_t blocks = (uint32_t)std::min<uint64_t>(((uint64_t)a.seg.S + 255) / 256, 148u * 16u);
         k_seg_first<<<std::max(1u, blocks), 256, 0, st>>>(a);
-    } else {
-        k_active<<<(a.c.n_gates + 255) / 256, 256, 0, st>>>(a);
     }
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = a.seg.N > 1 ? cudaGetLastError() : launch_next(k_active, (a.c.n_gates + 255) / 256, 256, 0, st, a);
     if (e != cudaSuccess) return e;
     if (threads != kCoverThreads) return cudaErrorInvalidValue;
     if (a.mid_list) {
@@ -1772,18 +1776,14 @@ cudaError_t launch_cover(const CoverArgs &a, uint32_t grid, uint32_t threads, bo
         const uint32_t cap0 = std::min(a.small_cap - (uint32_t)((lv + per_net - 1) / per_net), a.c.n_gates);
         const size_t smem0 = cover_smem_tables(cap0, kCoverCandSmall) + lv;
         if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_cover<0>), smem0)) != cudaSuccess) return e;
-        k_cover<0><<<grid * kCoverSmallCtas, threads, smem0, st>>>(a, cap0);
-        if (a.c.n_gates <= cap0) return cudaGetLastError();  // no pair can mark more
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        e = launch_next(k_cover<0>, grid * kCoverSmallCtas, threads, smem0, st, a, cap0);
+        if (e != cudaSuccess || a.c.n_gates <= cap0) return e;  // (no pair can mark more)
     }
     const size_t smem = cover_smem_bytes(a.hash_cap);
     if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_cover<1>), smem)) != cudaSuccess) return e;
-    k_cover<1><<<grid, threads, smem, st>>>(a, a.hash_cap);
-    if (a.spill_slots) {
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        k_cover_spill<<<a.spill_slots, kCoverThreads, 0, st>>>(a);
-    }
-    return cudaGetLastError();
+    e = launch_next(k_cover<1>, grid, threads, smem, st, a, a.hash_cap);
+    if (e != cudaSuccess || !a.spill_slots) return e;
+    return launch_next(k_cover_spill, a.spill_slots, kCoverThreads, 0, st, a);
 }
 
 namespace {

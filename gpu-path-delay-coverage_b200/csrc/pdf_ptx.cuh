@@ -92,6 +92,28 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *m, uint32_t phase, uint32_t 
 
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// Launches of one call follow each other without the gap between grids (about
+// 1.5 us each): the next one is started once every CTA of this one has passed
+// grid_trigger, and waits in grid_wait until this one is complete and visible.
+// Each kernel launched by launch_next waits before it ends, so that whatever
+// follows it in the stream follows all before it too.
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+cudaError_t launch_next(void (*kernel)(P...), uint32_t grid, uint32_t threads, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchConfig_t c{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // Last i with pref[i] <= x.
 __device__ __forceinline__ uint32_t prefix_find(const uint32_t *pref, uint32_t n, uint32_t x) {
     uint32_t lo = 0, hi = n;

@@ -56,6 +56,11 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
         mbar_expect_tx(mbar, a.image_bytes);
         bulk_g2s(smraw, a.image, a.image_bytes, mbar);
     }
+    // The image is the circuit's own; the rest follows what is before this
+    // launch in the stream.  With planes that is k_fill_planes, which itself
+    // followed everything else and writes other rows of V and T: only the marks
+    // wait for it.
+    if (OUT == RES_LEAN) grid_wait();
     // the batch's cover state (the cover kernels run after this one)
     if (a.active) {
         for (uint32_t w = b0 * BW + tid; w < min(a.W, b1 * BW); w += NT) a.active[w] = 0;
@@ -78,6 +83,7 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
             if (tid == 0) a.blk_maxlvl[blk] = 0;
         }
         if (tid == 0) atomicOr(a.err, kErrTimeout);
+        grid_wait();
         return;
     }
     const uint32_t j = tid & (BW - 1);         // this thread's word of the block (NT is a multiple of BW)
@@ -212,6 +218,7 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
             if (l + 1 >= L || (OUT == RES_LEAN && s_reach <= l)) break;
         }
         if (OUT == RES_SIM) continue;
+        if (OUT == RES_PLANES) grid_wait();
         // ---- prune (markkernel.cuh:271-293) and merge (mergekernel.cuh:116-198),
         // levels descending: a gate's mark is final once its fan-outs' are.
         // Gates from level s_top on hold no mark, and past the last level walked
@@ -263,15 +270,20 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
 
 template <int BW, int SEM, int OUT>
 __global__ void __launch_bounds__(kResidentThreads) k_resident(const FwdArgs a) {
+    grid_trigger();
     resident_cta<BW, SEM, OUT>(a, blockIdx.x);
+    grid_wait();
 }
 
 // Rows that a resident walk with planes leaves out, a warp per row: bound by
 // the stores (20,000 gates, of which 3,400 are not constant, x 32,768 pairs:
-// 220 MB).  VEC: rows start on 16 bytes.
+// 220 MB in 42 us).  VEC: rows start on 16 bytes.  A CTA per SM, so that the
+// resident walk's fit beside them.
+constexpr uint32_t kFillThreads = 512;
 template <bool VEC>
-__global__ void __launch_bounds__(256) k_fill_planes(const int8_t *value, uint32_t G, uint32_t W, uint32_t last,
+__global__ void __launch_bounds__(kFillThreads) k_fill_planes(const int8_t *value, uint32_t G, uint32_t W, uint32_t last,
                                                      uint32_t *v, uint32_t *t, uint32_t *m, uint64_t ld) {
+    grid_trigger();  // k_resident computes beside the stores
     const uint32_t lane = threadIdx.x & 31;
     const auto fill = [&](uint32_t *p, uint32_t x) {
         const uint32_t n4 = VEC ? (W - 1) / 4 : 0;  // the last word, which may hold fewer pairs, is not among them
@@ -279,7 +291,8 @@ __global__ void __launch_bounds__(256) k_fill_planes(const int8_t *value, uint32
             for (uint32_t q = lane; q < n4; q += 32) __stcs(reinterpret_cast<uint4 *>(p) + q, make_uint4(x, x, x, x));
         for (uint32_t w = 4 * n4 + lane; w < W; w += 32) __stcs(p + w, w + 1 == W ? x & last : x);
     };
-    for (uint32_t g = blockIdx.x * 8 + threadIdx.x / 32; g < G; g += gridDim.x * 8) {
+    constexpr uint32_t kWarps = kFillThreads / 32;
+    for (uint32_t g = blockIdx.x * kWarps + threadIdx.x / 32; g < G; g += gridDim.x * kWarps) {
         const int c = value[g];
         if (m) fill(m + (size_t)g * ld, 0u);
         if (c < 0) continue;
@@ -310,8 +323,7 @@ cudaError_t launch_out(const FwdArgs &a, uint32_t ctas, uint32_t threads, size_t
     const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(k_resident<BW, SEM, OUT>), smem);
     if (e != cudaSuccess) return e;
     if (!ctas || threads % 32 || threads > kResidentThreads) return cudaErrorInvalidValue;
-    k_resident<BW, SEM, OUT><<<ctas, threads, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_next(k_resident<BW, SEM, OUT>, ctas, threads, smem, st, a);
 }
 template <int BW, int SEM>
 cudaError_t launch_t(const FwdArgs &a, int out, uint32_t ctas, uint32_t threads, size_t smem, cudaStream_t st) {
@@ -360,10 +372,10 @@ cudaError_t launch_resident(const FwdArgs &a, int sem, int out, uint32_t bw, uin
 cudaError_t launch_fill_planes(const int8_t *value, uint32_t n_gates, uint64_t n_pairs, uint32_t *v, uint32_t *t,
                                uint32_t *m, uint64_t ld, uint32_t sms, cudaStream_t st) {
     const uint32_t W = (uint32_t)((n_pairs + 31) / 32), last = n_pairs & 31 ? (1u << (n_pairs & 31)) - 1u : 0xFFFFFFFFu;
-    const uint32_t grid = std::min((n_gates + 7) / 8, sms * 8);
+    const uint32_t grid = std::min((n_gates + kFillThreads / 32 - 1) / (kFillThreads / 32), sms);
     const auto at16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    if (ld % 4 == 0 && at16(v) && at16(t) && at16(m)) k_fill_planes<true><<<grid, 256, 0, st>>>(value, n_gates, W, last, v, t, m, ld);
-    else k_fill_planes<false><<<grid, 256, 0, st>>>(value, n_gates, W, last, v, t, m, ld);
+    if (ld % 4 == 0 && at16(v) && at16(t) && at16(m)) k_fill_planes<true><<<grid, kFillThreads, 0, st>>>(value, n_gates, W, last, v, t, m, ld);
+    else k_fill_planes<false><<<grid, kFillThreads, 0, st>>>(value, n_gates, W, last, v, t, m, ld);
     return cudaGetLastError();
 }
 cudaError_t prepare_resident_class(uint32_t sem, uint32_t bw, size_t smem) { PDF_RES(raise_batch_t, smem) }

@@ -290,6 +290,9 @@ struct pdf_circuit {
     Plan full, red;   // every gate; the reduced netlist (n_gates 0: none)
     // the plan of grading calls that ask for no plane
     const Plan &lean() const { return red.n_gates ? red : full; }
+    // Where single calls walk narrower column blocks than the tile (single_tile):
+    // the lean plan at the tile, for batches, whose circuits fill the GPU together.
+    Plan batch;
     // Planes from the resident kernel: every gate whose value is not constant,
     // where they fit on chip (the constant rows are filled in), else null.
     Plan live;
@@ -321,8 +324,8 @@ struct pdf_circuit {
         return k;
     }
     Walk full_walk(uint64_t W) const { return staged_walk(full, W); }
-    Walk lean_walk(uint64_t W) const {
-        const Plan &p = lean();
+    Walk lean_walk(uint64_t W, bool in_batch = false) const {
+        const Plan &p = in_batch && batch.n_gates ? batch : lean();
         if (!p.image) return staged_walk(p, W);
         return resident_walk(p, W, RES_LEAN);
     }
@@ -611,6 +614,18 @@ namespace {
 // a level and 32,768 pairs with planes 277 and 445.
 constexpr uint64_t kWideLevel = 1024;
 
+// Column block of single calls over at most `words` words when the caller asked
+// for no tile: the widest of 1, 2 and 4 words that still gives every SM a CTA.
+// A walk is a chain of levels, whose steps are shorter with fewer words.
+// Measured (us; blocks of 1, 2, 4 words), four stage calls over 20,000 gates
+// without XOR: 96 words 329, 349, 388; 256 words 398, 348, 387; 384 words 660,
+// 432, 403; 45,000 gates FIXED: 96 words 2,101, 2,270, 2,429; 256 words 3,239,
+// 2,994, 3,195; 384 words 3,811, 3,649, 3,363.
+uint32_t single_tile(uint32_t bw, uint64_t words, uint64_t sms) {
+    if (bw != 4 || words > 2 * sms) return bw;
+    return words > sms ? 2 : 1;
+}
+
 // Column block of the reduced walk of a circuit whose tile is bw words, by
 // the mean width of its levels above the inputs.  Narrow levels leave most
 // warps of the lane kernel without a gate.
@@ -717,7 +732,8 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     const bool wide_full = !o.tile_words && mean_width >= kWideLevel;
     bool wide_red = false;
     const uint32_t wide_bw = lane_tile(c->bw) ? c->bw : kLaneWords;  // (a batch's lane kernel)
-    po.bw = wide_full ? wide_bw : c->bw;
+    const uint32_t single_bw = o.tile_words || wide_full ? c->bw : single_tile(c->bw, max_words, sms);
+    po.bw = wide_full ? wide_bw : single_bw;
     po.threads = o.threads;
     po.regs = forward_kernel_regs((int)po.bw, o.mark_mode);
     po.smem_block = prop.sharedMemPerBlockOptin;
@@ -742,7 +758,8 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     // and the resident kernel's image of what a lean call walks.
     NetPlan rnet, lnet;
     ResidentImage image, limage;
-    LaunchPlan live;
+    LaunchPlan live, batch;
+    std::future<pdf_status> third;  // the batch's plan, beside the single calls'
     std::vector<int8_t> value;
     enum { kNoOut, kOutFull, kOutRed, kOutLive } out_of = kNoOut;  // whose image writes planes
     const size_t res_smem = (size_t)prop.sharedMemPerBlockOptin - 1024;
@@ -758,10 +775,28 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
             PlanOpts ro = po;
             const uint64_t rw = rl > 1 ? (rnet.n_gates() - rnet.level_off[1]) / (rl - 1) : 0;
             wide_red = (!o.tile_words || lane_tile(o.tile_words)) && rw >= kWideLevel;
-            ro.bw = wide_red ? wide_bw : reduced_tile(c->bw, rw);
+            const uint32_t tile = wide_red ? wide_bw : reduced_tile(c->bw, rw);
+            ro.bw = !wide_red && single_bw != c->bw ? single_bw : tile;
             ro.threads = wide_red ? 0 : o.threads;
             if (ro.bw != po.bw) ro.regs = forward_kernel_regs((int)ro.bw, o.mark_mode);
-            pst = build_plan(rnet, ro, red);
+            if (ro.bw != tile) {
+                PlanOpts bo = ro;
+                bo.bw = tile;
+                bo.regs = forward_kernel_regs((int)tile, o.mark_mode);
+                if (G >= 16384) {
+                    try {
+                        third = std::async(std::launch::async, [&rnet, bo, &batch] { return build_plan(rnet, bo, batch); });
+                    } catch (const std::system_error &) {
+                    }
+                }
+                if (!third.valid()) pst = build_plan(rnet, bo, batch);
+            }
+            if (pst == PDF_OK) pst = build_plan(rnet, ro, red);
+        } else if (image.bytes.empty() && single_bw != c->bw) {
+            PlanOpts bo = po;
+            bo.bw = c->bw;
+            bo.regs = forward_kernel_regs((int)c->bw, o.mark_mode);
+            pst = build_plan(net, bo, batch);
         }
         // planes: what the lean image holds if that is all that is not
         // constant, else an image of its own
@@ -784,10 +819,11 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         if (out_of == kOutFull) value.assign(G, -1);  // its walk writes every row
         else if (out_of != kNoOut) value.swap(facts.value);
     }
-    if (other.valid()) {
-        const pdf_status fst = other.get();
-        if (fst != PDF_OK) pst = fst;
-    }
+    for (auto *f : {&other, &third})
+        if (f->valid()) {
+            const pdf_status fst = f->get();
+            if (fst != PDF_OK) pst = fst;
+        }
     if (pst != PDF_OK) {
         delete c;
         return pst;
@@ -818,6 +854,8 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         const PlanOffsets fo = up.add_plan(net, full, reduced ? none : image);
         const PlanOffsets ro = reduced ? up.add_plan(rnet, red, image) : PlanOffsets{};
         const PlanOffsets lo = out_of == kOutLive ? up.add_plan(lnet, live, limage) : PlanOffsets{};
+        const NetPlan &bnet = reduced ? rnet : net;
+        const PlanOffsets bo = batch.n_gates ? up.add_plan(bnet, batch, none) : PlanOffsets{};
         const size_t vo = up.add(value.data(), value.size());
         const WideSync rest{};
         const size_t so = up.add(&rest, sizeof rest);
@@ -832,6 +870,7 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         c->stage.sync = reinterpret_cast<WideSync *>(c->mem.as<unsigned char>() + so);
         c->full.bind(full, net, reduced ? none : image, c->mem.as<unsigned char>(), fo);
         if (reduced) c->red.bind(red, rnet, image, c->mem.as<unsigned char>(), ro);
+        if (batch.n_gates) c->batch.bind(batch, bnet, none, c->mem.as<unsigned char>(), bo);
         if (out_of == kOutLive) c->live.bind(live, lnet, limage, c->mem.as<unsigned char>(), lo);
         c->out_plan = out_of == kOutLive ? &c->live : out_of == kOutRed ? &c->red : out_of == kOutFull ? &c->full : nullptr;
         c->value = reinterpret_cast<const int8_t *>(c->mem.as<unsigned char>() + vo);
@@ -839,7 +878,7 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         c->red.wide = wide_red;
         c->full.mean_width = (uint32_t)mean_width;
         c->red.mean_width = red.n_levels > 1 ? (red.n_gates - rnet.level_off[1]) / (red.n_levels - 1) : 0;
-        for (Plan *p : {&c->full, &c->red, &c->live}) {
+        for (Plan *p : {&c->full, &c->red, &c->live, &c->batch}) {
             p->res.sms = (uint32_t)prop.multiProcessorCount;
             p->res.regs = 64;  // its launch bound's
             p->res.smem_block = res_smem;
@@ -1938,7 +1977,7 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
     std::vector<Walk> walks(n_jobs);
     uint64_t res_ctas = 0;
     for (uint32_t i = 0; i < n_jobs; i++) {
-        Walk &k = walks[i] = jobs[i].circuit->lean_walk((jobs[i].pairs.n_pairs + 31) / 32);
+        Walk &k = walks[i] = jobs[i].circuit->lean_walk((jobs[i].pairs.n_pairs + 31) / 32, true);
         k.wide = 0;  // a batch's circuits share the GPU: a wide plan takes the lane kernel
         if (!k.resident) continue;
         // a CTA takes blocks worth about twice its copy of the image

@@ -11,6 +11,7 @@
 #include <cstring>
 #include <future>
 #include <initializer_list>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <system_error>
@@ -88,23 +89,43 @@ void set_msg(char *msg, size_t len, const char *fmt, unsigned long long a = 0,
     if (msg && len) std::snprintf(msg, len, fmt, a, b);
 }
 
+// Who else has a device block's address: batches bound to it (each binding has
+// a token, dropped when the batch is bound anew or destroyed) and graphs that
+// the caller captured (until the block's owner is destroyed).
+struct Holders {
+    std::vector<std::weak_ptr<const void>> batches;
+    bool graph = false;
+    bool any() const {
+        for (const auto &b : batches)
+            if (!b.expired()) return true;
+        return graph;
+    }
+    void add(const std::weak_ptr<const void> &batch) {
+        batches.erase(std::remove_if(batches.begin(), batches.end(), [](const auto &b) { return b.expired(); }),
+                      batches.end());
+        batches.push_back(batch);
+    }
+};
+
+using KeptBlocks = std::vector<std::pair<void *, Holders>>;
+
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
-    bool held = false;  // a batch or a captured graph has the address
+    Holders holders;
     void release() {
         if (p && cudaFree(p) != cudaSuccess) (void)cudaGetLastError();
         p = nullptr;
         bytes = 0;
-        held = false;
+        holders = Holders{};
     }
-    // Grow to at least `need` bytes (contents are not kept).  A held block goes
-    // to `kept` instead of being freed.
-    cudaError_t ensure(size_t need, std::vector<void *> *kept = nullptr) {
+    // Grow to at least `need` bytes (contents are not kept).  A block that a
+    // batch or a graph holds goes to `kept` instead of being freed.
+    cudaError_t ensure(size_t need, KeptBlocks *kept = nullptr) {
         if (bytes >= need) return cudaSuccess;
-        if (held && kept) {
+        if (kept && p && holders.any()) {
             try {
-                kept->push_back(p);
+                kept->emplace_back(p, holders);
             } catch (const std::bad_alloc &) {
                 return cudaErrorMemoryAllocation;
             }
@@ -157,8 +178,27 @@ struct Workspace {
     DevBuf pi;      // staged host pairs
     // blocks that were outgrown while held: calls of one walk (with planes, say)
     // grow a state's workspace past what a batch of the other was bound to
-    std::vector<void *> kept;
-    void hold() { scratch.held = seg_first.held = planes.held = pi.held = true; }
+    KeptBlocks kept;
+    // From here on the current blocks belong to a graph that the caller
+    // captures, or also to the binding of a batch; false: out of host memory.
+    void hold_for_graph() { scratch.holders.graph = seg_first.holders.graph = planes.holders.graph = pi.holders.graph = true; }
+    bool hold_for(const std::weak_ptr<const void> &batch) {
+        try {
+            for (DevBuf *b : {&scratch, &seg_first, &planes, &pi}) b->holders.add(batch);
+        } catch (const std::bad_alloc &) {
+            return false;
+        }
+        return true;
+    }
+    // frees the kept blocks that nobody holds any more
+    void sweep() {
+        const auto gone = std::remove_if(kept.begin(), kept.end(), [](const auto &k) {
+            if (k.second.any()) return false;
+            if (cudaFree(k.first) != cudaSuccess) (void)cudaGetLastError();
+            return true;
+        });
+        kept.erase(gone, kept.end());
+    }
     void release() {
         scratch.release();
         pi_counts.release();
@@ -166,8 +206,8 @@ struct Workspace {
         seg_first_mask = 0;
         planes.release();
         pi.release();
-        for (void *q : kept)
-            if (cudaFree(q) != cudaSuccess) (void)cudaGetLastError();
+        for (const auto &k : kept)
+            if (cudaFree(k.first) != cudaSuccess) (void)cudaGetLastError();
         kept.clear();
     }
 };
@@ -1180,12 +1220,13 @@ uint64_t ws_plane_words(const pdf_circuit *c, const Walk &k, uint64_t W, bool ne
     return resident_mark_words(k, W) + (k.out != RES_LEAN && need ? 3 * (uint64_t)c->info.n_gates * out_pitch(W) : 0);
 }
 
-// Sizes the workspace for a walk over W words of pairs.  `keep`: held blocks
-// that are too small stay (not so for a batch that is bound to more pairs than
-// one before it: the older batch is then not run any more).
-pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, bool need_planes, bool keep = true) {
-    std::vector<void *> *kept = keep ? &ws.kept : nullptr;
-    PDF_CUDA(ws.scratch.ensure(scratch_of(c, k, W, nullptr).bytes, kept));
+// Sizes the workspace for a walk over W words of pairs.  A block that is too
+// small and held stays allocated until nobody holds it.
+pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, bool need_planes) {
+    KeptBlocks *kept = &ws.kept;
+    const uint64_t scratch = scratch_of(c, k, W, nullptr).bytes, planes = ws_plane_words(c, k, W, need_planes) * 4;
+    if (ws.scratch.bytes < scratch || ws.planes.bytes < planes) ws.sweep();  // (this call allocates anyway)
+    PDF_CUDA(ws.scratch.ensure(scratch, kept));
     if (c->seg_len > 1) {
         // (net, pair) entries: at most N per first pair of a segment, two per
         // segment, and one per (net, pair); a table at least twice that
@@ -1197,7 +1238,7 @@ pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, b
             ws.seg_first_mask = cap - 1;
         }
     }
-    PDF_CUDA(ws.planes.ensure(ws_plane_words(c, k, W, need_planes) * 4, kept));
+    PDF_CUDA(ws.planes.ensure(planes, kept));
     return PDF_OK;
 }
 Scratch ws_scratch(const pdf_circuit *c, const Walk &k, const Workspace &ws, uint64_t W) {
@@ -1455,7 +1496,7 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     uint64_t pld;
     st = stage_pairs(c, k, s->ws, pr, &pv, &pt, &pld, cs);
     if (st != PDF_OK) return st;
-    if (cap != cudaStreamCaptureStatusNone) s->ws.hold();  // the caller's graph will have its addresses
+    if (cap != cudaStreamCaptureStatusNone) s->ws.hold_for_graph();  // it will have its addresses
 
     FwdArgs a = base_fwd(c, k, n);
     a.pi_v = pv;
@@ -1881,6 +1922,7 @@ struct pdf_batch {
     std::vector<pdf_state *> states;
     BatchLaunch L{};
     DevBuf ctl;  // control word, arguments, prefixes and items in one block
+    std::shared_ptr<const void> bound;  // token of this binding, in the blocks of its states' workspaces
     uint64_t gate_evals = 0, bytes = 0;
     cudaStream_t cap_stream = nullptr;
     cudaGraph_t graph = nullptr;
@@ -1957,6 +1999,8 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
     }
     b->drop_graph();
     b->ran = false;
+    // blocks that only the binding before this one held may be freed from here on
+    b->bound = std::make_shared<char>();
     b->device = c0->device;
     b->circuits.clear();
     b->states.clear();
@@ -2023,8 +2067,8 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
         const Walk &wk = walks[order[k]];
         const Plan &p = *wk.p;
         const uint64_t n = j.pairs.n_pairs, W = (n + 31) / 32, G = p.n_gates;
-        if (ensure_ws(c, wk, s->ws, W, true, false) != PDF_OK) return PDF_ENOMEM;
-        s->ws.hold();  // the batch's arguments hold its addresses
+        if (ensure_ws(c, wk, s->ws, W, true) != PDF_OK) return PDF_ENOMEM;
+        if (!s->ws.hold_for(b->bound)) return PDF_ENOMEM;  // the batch's arguments hold its addresses
         FwdArgs a = base_fwd(c, wk, n);
         a.pi_v = j.pairs.v;
         a.pi_t = j.pairs.t;

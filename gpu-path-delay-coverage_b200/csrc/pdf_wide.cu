@@ -345,11 +345,11 @@ __device__ __forceinline__ uint32_t wide_gate(const FwdArgs &a, const WideArgs &
 }
 
 // All CTAs of the (cooperative) grid; what each wrote before is visible after.
-// Bounded: false when the others did not come.
-__device__ __forceinline__ bool grid_sync(WideSync *s, uint32_t target) {
+// Bounded: false when the others did not come within `polls` (0: 2^22, seconds).
+__device__ __forceinline__ bool grid_sync(WideSync *s, uint32_t target, uint32_t polls) {
     __threadfence();
     atomicAdd(&s->arrived, 1u);
-    for (uint32_t i = 0; i < (1u << 22); i++) {
+    for (uint32_t i = 0, n = polls ? polls : 1u << 22; i < n; i++) {
         uint32_t v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&s->arrived) : "memory");
         if (v >= target) return true;
@@ -373,6 +373,8 @@ __global__ void __launch_bounds__(kWideThreads, kWideCtas) k_wide(const FwdArgs 
     }
     if (MODE == FWD_FUSED) {  // the batch's cover state (the cover kernels run after this one)
         for (size_t i = gt; i < (size_t)nf * a.bm_words; i += GT) a.nzb_fine[i] = 0;
+        // no marked level, should this CTA leave before the prune
+        for (uint32_t b = gt; b < nf; b += GT) a.maxlvl_fine[b] = 0;
         if (a.active)
             for (uint32_t w = gt; w <= a.W; w += GT) a.active[w] = 0;
         if (a.acc && gt == 0) {
@@ -403,7 +405,7 @@ __global__ void __launch_bounds__(kWideThreads, kWideCtas) k_wide(const FwdArgs 
                 atomicMax(&wa.sync->reach, s_reach);
                 atomicMax(&wa.sync->top, s_top);
             }
-            if (!grid_sync(wa.sync, ++phase * gridDim.x)) s_fail = 1;
+            if (!grid_sync(wa.sync, ++phase * gridDim.x, a.wait_polls)) s_fail = 1;
             s_seen = MODE != FWD_SIM ? __ldcg(&wa.sync->reach) : 0u;
             s_next = 0;
         }

@@ -177,8 +177,9 @@ typedef struct pdf_circuit_opts {
                             tiles then hold at most threads - 64 gates */
     uint32_t seg_len;    /* path segments of this many nets, 0 or 1 = single nets; up to 8
                             (fcount --segs N, main.cu:76-81,185-223) */
-    uint32_t wait_polls; /* bound on each device-side wait of the forward kernels for its staged
-                            copy: 0 = 2^24 blocking polls (the default); n > 0 = n non-blocking
+    uint32_t wait_polls; /* bound on each device-side wait of the forward kernels, for a staged
+                            copy or (wide kernel) for the grid: 0 = 2^24 blocking polls, 2^22
+                            polls of the grid barrier (the default); n > 0 = n non-blocking
                             polls, after which the call reports PDF_ETIMEOUT (small values
                             exist to test that path).  The lane kernel (tile_words 32, 64,
                             128) waits for nothing. */

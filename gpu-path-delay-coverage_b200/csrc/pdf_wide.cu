@@ -25,6 +25,8 @@
 #include "pdf_kernels.cuh"
 #include "pdf_ptx.cuh"
 
+#include <cuda.h>
+
 #include <algorithm>
 #include <type_traits>
 
@@ -654,10 +656,36 @@ cudaError_t launch_sem(const FwdArgs &a, const WideArgs &wa, int mode, int sem, 
     }
 }
 
+// SMs that a kernel on `st` can take, at most `sms`: a stream of a green context
+// has a part of the device's, and a cooperative grid has to fit it.
+uint32_t stream_sms(cudaStream_t st, uint32_t sms) {
+    using GetCtx = CUresult (*)(CUstream, CUcontext *, CUgreenCtx *);
+    using GetRes = CUresult (*)(CUgreenCtx, CUdevResource *, CUdevResourceType);
+    static const auto entry = [](const char *name) -> void * {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion(name, &f, 12050, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            return f;
+        (void)cudaGetLastError();
+        return nullptr;
+    };
+    static const GetCtx get_ctx = reinterpret_cast<GetCtx>(entry("cuStreamGetCtx"));
+    static const GetRes get_res = reinterpret_cast<GetRes>(entry("cuGreenCtxGetDevResource"));
+    CUcontext ctx = nullptr;
+    CUgreenCtx green = nullptr;
+    CUdevResource res{};
+    if (!get_ctx || !get_res || get_ctx(st, &ctx, &green) != CUDA_SUCCESS || !green ||
+        get_res(green, &res, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS || !res.sm.smCount)
+        return sms;
+    return std::min(sms, res.sm.smCount);
+}
+
 }  // namespace
 
 cudaError_t launch_wide(const FwdArgs &a, const WideArgs &wa, int mode, int sem, uint32_t lw, uint32_t sms,
                         cudaStream_t st) {
     if (!wa.chunks || !wa.cps || wa.cps > 8) return cudaErrorInvalidValue;
+    sms = stream_sms(st, sms);
     return lw == 2 ? launch_sem<2>(a, wa, mode, sem, sms, st) : launch_sem<1>(a, wa, mode, sem, sms, st);
 }

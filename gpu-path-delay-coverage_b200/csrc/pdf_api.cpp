@@ -832,6 +832,19 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
                 if (!third.valid()) pst = build_plan(rnet, bo, batch);
             }
             if (pst == PDF_OK) pst = build_plan(rnet, ro, red);
+            if (third.valid()) {
+                const pdf_status tst = third.get();
+                if (pst == PDF_OK) pst = tst;
+            }
+            // no plan of the reduced netlist (the thread-per-gate kernel takes
+            // 65,536 pieces at most, the lane kernel any number): lean calls
+            // walk all of it
+            if (pst == PDF_ENOTSUP) {
+                rnet = NetPlan{};
+                red = batch = LaunchPlan{};
+                wide_red = false;
+                pst = PDF_OK;
+            }
         } else if (image.bytes.empty() && single_bw != c->bw) {
             PlanOpts bo = po;
             bo.bw = c->bw;

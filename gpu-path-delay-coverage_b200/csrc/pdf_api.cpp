@@ -970,10 +970,11 @@ extern "C" void pdf_circuit_destroy(pdf_circuit *c) {
     if (!c) return;
     DeviceGuard dg(c->device);
     c->stage.release();
-    if (c->host_err && cudaFreeHost(c->host_err) != cudaSuccess) (void)cudaGetLastError();
     c->mem.release();
     c->segs.release();
     c->seg_off.release();
+    // after a cudaFree, which waits for what may still write there
+    if (c->host_err && cudaFreeHost(c->host_err) != cudaSuccess) (void)cudaGetLastError();
     delete c;
 }
 
@@ -1962,6 +1963,11 @@ struct pdf_batch {
         for (auto &x : prof)
             if (x) cudaEventDestroy(x);
         for (auto &x : prof) x = nullptr;
+        // the upload may not have been run, or a run that leaves its error word
+        // there not have ended: the staging goes after the wait for the one and
+        // the device block, whose cudaFree waits for the other
+        if (uploaded && cudaEventSynchronize(uploaded) != cudaSuccess) (void)cudaGetLastError();
+        ctl.release();
         if (host_ctl) cudaFreeHost(host_ctl);
         host_ctl = nullptr;
         host_bytes = 0;
@@ -1983,7 +1989,6 @@ struct pdf_batch {
         for (auto &x : side) x = nullptr;
         for (auto &x : join) x = nullptr;
         fork = nullptr;
-        ctl.release();
     }
 };
 

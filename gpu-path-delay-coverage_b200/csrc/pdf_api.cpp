@@ -1240,18 +1240,18 @@ pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, b
     KeptBlocks *kept = &ws.kept;
     const uint64_t scratch = scratch_of(c, k, W, nullptr).bytes, planes = ws_plane_words(c, k, W, need_planes) * 4;
     if (ws.scratch.bytes < scratch || ws.planes.bytes < planes) ws.sweep();  // (this call allocates anyway)
-    PDF_CUDA(ws.scratch.ensure(scratch, kept));
     if (c->seg_len > 1) {
         // (net, pair) entries: at most N per first pair of a segment, two per
         // segment, and one per (net, pair); a table at least twice that
         const uint64_t most = std::min<uint64_t>(2 * c->n_segs * c->seg_len, (uint64_t)c->info.n_gates * W * 32);
         uint64_t cap = 1024;
         while (cap < 2 * most && cap < (1ull << 27)) cap <<= 1;
-        if (ws.seg_first_mask + 1 < cap) {
+        if (ws.seg_first.bytes < cap * 8) {  // (the block itself: a growth that failed has left none)
             PDF_CUDA(ws.seg_first.ensure(cap * 8, kept));
             ws.seg_first_mask = cap - 1;
         }
     }
+    PDF_CUDA(ws.scratch.ensure(scratch, kept));
     PDF_CUDA(ws.planes.ensure(planes, kept));
     return PDF_OK;
 }

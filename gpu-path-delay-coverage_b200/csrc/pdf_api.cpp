@@ -1234,12 +1234,21 @@ uint64_t ws_plane_words(const pdf_circuit *c, const Walk &k, uint64_t W, bool ne
     return resident_mark_words(k, W) + (k.out != RES_LEAN && need ? 3 * (uint64_t)c->info.n_gates * out_pitch(W) : 0);
 }
 
-// Sizes the workspace for a walk over W words of pairs.  A block that is too
-// small and held stays allocated until nobody holds it.
-pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, bool need_planes) {
+// What walks over W words of pairs take of a workspace.
+struct WsNeed {
+    uint64_t scratch = 0, planes = 0;  // bytes
+    WsNeed &with(const pdf_circuit *c, const Walk &k, uint64_t W, bool need_planes) {
+        scratch = std::max<uint64_t>(scratch, scratch_of(c, k, W, nullptr).bytes);
+        planes = std::max(planes, ws_plane_words(c, k, W, need_planes) * 4);
+        return *this;
+    }
+};
+
+// Sizes the workspace.  A block that is too small and held stays allocated
+// until nobody holds it.
+pdf_status ensure_ws(pdf_circuit *c, const WsNeed &need, Workspace &ws, uint64_t W) {
     KeptBlocks *kept = &ws.kept;
-    const uint64_t scratch = scratch_of(c, k, W, nullptr).bytes, planes = ws_plane_words(c, k, W, need_planes) * 4;
-    if (ws.scratch.bytes < scratch || ws.planes.bytes < planes) ws.sweep();  // (this call allocates anyway)
+    if (ws.scratch.bytes < need.scratch || ws.planes.bytes < need.planes) ws.sweep();  // (this call allocates anyway)
     if (c->seg_len > 1) {
         // (net, pair) entries: at most N per first pair of a segment, two per
         // segment, and one per (net, pair); a table at least twice that
@@ -1251,9 +1260,12 @@ pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, b
             ws.seg_first_mask = cap - 1;
         }
     }
-    PDF_CUDA(ws.scratch.ensure(scratch, kept));
-    PDF_CUDA(ws.planes.ensure(planes, kept));
+    PDF_CUDA(ws.scratch.ensure(need.scratch, kept));
+    PDF_CUDA(ws.planes.ensure(need.planes, kept));
     return PDF_OK;
+}
+pdf_status ensure_ws(pdf_circuit *c, const Walk &k, Workspace &ws, uint64_t W, bool need_planes) {
+    return ensure_ws(c, WsNeed{}.with(c, k, W, need_planes), ws, W);
 }
 Scratch ws_scratch(const pdf_circuit *c, const Walk &k, const Workspace &ws, uint64_t W) {
     return scratch_of(c, k, W, ws.scratch.as<unsigned char>());
@@ -1994,6 +2006,14 @@ struct pdf_batch {
 
 namespace {
 
+// A batch's walk of one of its circuits: they share the GPU, so a wide plan
+// takes the lane kernel.
+Walk batch_walk(const pdf_circuit *c, uint64_t W) {
+    Walk k = c->lean_walk(W, true);
+    k.wide = 0;
+    return k;
+}
+
 // (Re)build batch b for these jobs: per-circuit arguments and prefixes in
 // one device block, which is reused when it is large enough.
 // up: the stream that uploads the control block, in order before the next
@@ -2039,8 +2059,7 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
     std::vector<Walk> walks(n_jobs);
     uint64_t res_ctas = 0;
     for (uint32_t i = 0; i < n_jobs; i++) {
-        Walk &k = walks[i] = jobs[i].circuit->lean_walk((jobs[i].pairs.n_pairs + 31) / 32, true);
-        k.wide = 0;  // a batch's circuits share the GPU: a wide plan takes the lane kernel
+        Walk &k = walks[i] = batch_walk(jobs[i].circuit, (jobs[i].pairs.n_pairs + 31) / 32);
         if (!k.resident) continue;
         // a CTA takes blocks worth about twice its copy of the image
         const double load = 2.0 + k.p->res.image_bytes / 95e3;
@@ -2468,13 +2487,27 @@ extern "C" pdf_status pdf_batch_autotune(const pdf_netlist *const *netlists, con
     return PDF_OK;
 }
 
+// One sizing for all the walks: growing a block step by step would free each
+// step's, and cudaFree waits for the whole device.
 extern "C" pdf_status pdf_state_reserve(pdf_state *s, uint64_t n_pairs) {
     if (!s || !n_pairs) return PDF_EINVAL;
     DeviceGuard dg(s->c->device);
     if (!dg.ok) return PDF_ECUDA;
     std::lock_guard<std::mutex> lk(s->mu);
     const uint64_t W = (n_pairs + 31) / 32;
-    pdf_status st = ensure_ws(s->c, s->c->lean_walk(W), s->ws, W, true);
-    if (st == PDF_OK) st = ensure_ws(s->c, s->c->planes_walk(W), s->ws, W, true);
-    return st == PDF_OK ? ensure_ws(s->c, s->c->full_walk(W), s->ws, W, !s->c->out_plan) : st;
+    pdf_circuit *c = s->c;
+    WsNeed need;
+    need.with(c, c->lean_walk(W), W, true);
+    if (c->seg_len <= 1) need.with(c, batch_walk(c, W), W, true);
+    need.with(c, c->planes_walk(W), W, true).with(c, c->full_walk(W), W, !c->out_plan);
+    return ensure_ws(c, need, s->ws, W);
+}
+
+// The workspace of a state that only batches grade.
+pdf_status state_reserve_batch(pdf_state *s, uint64_t n_pairs) {
+    DeviceGuard dg(s->c->device);
+    if (!dg.ok) return PDF_ECUDA;
+    std::lock_guard<std::mutex> lk(s->mu);
+    const uint64_t W = (n_pairs + 31) / 32;
+    return ensure_ws(s->c, batch_walk(s->c, W), s->ws, W, true);
 }

@@ -31,4 +31,7 @@ pdf_status batch_rebind_on(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_j
 pdf_status batch_pass_async(pdf_batch *b, cudaStream_t stream);
 pdf_status batch_pass_status(const pdf_batch *b);
 
+// pdf_state_reserve for a state that only batches grade.
+pdf_status state_reserve_batch(pdf_state *s, uint64_t n_pairs);
+
 #endif

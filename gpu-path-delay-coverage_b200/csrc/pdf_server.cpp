@@ -169,7 +169,7 @@ void prepare(const pdf_server_opts &o, Job *j, cudaStream_t up, Stage &sg) {
     const size_t hb = (size_t)npi * j->hld * 4;
     pdf_status st = pdf_circuit_create(&j->view, &co, &j->c);
     if (st == PDF_OK) st = pdf_state_create(j->c, &j->s);
-    if (st == PDF_OK) st = pdf_state_reserve(j->s, o.batch_pairs);
+    if (st == PDF_OK) st = state_reserve_batch(j->s, o.batch_pairs);
     if (st == PDF_OK && (cudaMalloc(&j->dv, 2 * npi * j->ld * 4) != cudaSuccess ||
                          cudaMalloc(&j->dall, pairs_bytes(j->view, j->hld)) != cudaSuccess))
         st = PDF_ENOMEM;

@@ -102,17 +102,23 @@ struct pdf_server {
 
 namespace {
 
-// Device bytes of an active job: netlist, plan, state, workspace and pair
+// Device bytes of an active job: netlist, plans, state, workspace and pair
 // buffer (an upper estimate from the netlist and the batch size).
 uint64_t footprint(const pdf_netlist &nl, uint64_t batch_pairs, uint32_t bw) {
     const uint64_t G = nl.n_gates, W = (batch_pairs + 31) / 32, ld = (W + bw - 1) / bw * bw;
     const uint64_t npi = nl.level_offsets[1];
-    return 64 * G + 24 * nl.n_edges       // records, edges, fan-out lists, far lists
+    // bitmaps: one per column block (a netlist on chip, of at most 8,400 gates,
+    // may walk blocks of one word), a lane tile's also one per 8 words
+    const uint64_t on_chip = std::min<uint64_t>(G, 8400);
+    const uint64_t bitmaps =
+        std::max(W * ((on_chip + 31) / 32), (ld / bw + (bw >= 32 ? ld / 8 : 0)) * ((G + 31) / 32)) * 4;
+    return 70 * G + 24 * nl.n_edges       // records of the whole and the reduced netlist, edges, fan-out and far lists
            + 8 * G                        // first-detect ids
            + 12 * G * ld                  // V, T, M planes of one batch
-           + (ld / bw) * ((G + 31) / 32) * 4 + 8 * ld * 32 + 4 * ld  // bitmaps, active pairs
+           + bitmaps + 4 * 4 * std::min<uint64_t>(32 * ld, 2 * G) + 8 * ld  // active pairs and the cover's queues
+           + std::max<uint64_t>(32 * G, std::min<uint64_t>(512 * G, 16u << 20))  // the spill cover's slots, 1 to 16
            + 8 * npi * ld                 // pair buffer
-           + (1u << 20);
+           + (2u << 20);
 }
 
 // The job's pairs, uploaded once at admission.

@@ -330,9 +330,21 @@ struct pdf_circuit {
     Plan full, red;   // every gate; the reduced netlist (n_gates 0: none)
     // the plan of grading calls that ask for no plane
     const Plan &lean() const { return red.n_gates ? red : full; }
-    // Where single calls walk narrower column blocks than the tile (single_tile):
-    // the lean plan at the tile, for batches, whose circuits fill the GPU together.
-    Plan batch;
+    // Plans at the tile of circuits whose single calls take another column block
+    // (narrower ones, single_tile; the wide kernel's), built when first asked
+    // for: of the reduced netlist, and of all gates.
+    struct TilePlan {
+        bool wanted = false;
+        PlanOpts opts;
+        NetPlan net;
+        DevBuf mem;
+        Plan plan;
+        std::mutex mu;
+    };
+    mutable TilePlan tile_red, tile_full;
+    uint64_t narrow_words = ~0ull;  // single calls over more words than this take them
+    const Plan &at_tile(TilePlan &t, const Plan &otherwise) const;
+    const Plan &lean_at_tile() const { return red.n_gates ? at_tile(tile_red, red) : at_tile(tile_full, full); }
     // Planes from the resident kernel: every gate whose value is not constant,
     // where they fit on chip (the constant rows are filled in), else null.
     Plan live;
@@ -363,11 +375,19 @@ struct pdf_circuit {
         if (p.wide) wide_shape(k, W, 2);
         return k;
     }
-    Walk full_walk(uint64_t W) const { return staged_walk(full, W); }
-    Walk lean_walk(uint64_t W, bool in_batch = false) const {
-        const Plan &p = in_batch && batch.n_gates ? batch : lean();
-        if (!p.image) return staged_walk(p, W);
-        return resident_walk(p, W, RES_LEAN);
+    Walk full_walk(uint64_t W) const { return staged_walk(W > narrow_words ? at_tile(tile_full, full) : full, W); }
+    Walk lean_walk(uint64_t W) const {
+        if (lean().image) return resident_walk(lean(), W, RES_LEAN);
+        return staged_walk(W > narrow_words ? lean_at_tile() : lean(), W);
+    }
+    // A batch's: its circuits share the GPU, so a wide plan takes the lane kernel
+    // (lanes) or the plan at the tile.
+    Walk batch_walk(uint64_t W, bool lanes) const {
+        if (lean().image) return resident_walk(lean(), W, RES_LEAN);
+        Walk k;
+        k.p = lean().wide && lanes ? &lean() : &lean_at_tile();
+        k.bw = k.p->bw;
+        return k;
     }
     static Walk resident_walk(const Plan &p, uint64_t W, int out) {
         Walk k;
@@ -676,6 +696,31 @@ uint32_t reduced_tile(uint32_t bw, uint64_t mean_width) {
 
 }  // namespace
 
+// Where it cannot be built (out of memory, too many pieces) the call walks the
+// plan there is, and the next one tries again.
+const Plan &pdf_circuit::at_tile(TilePlan &t, const Plan &otherwise) const {
+    if (!t.wanted) return otherwise;
+    std::lock_guard<std::mutex> lk(t.mu);
+    if (t.plan.n_gates) return t.plan;
+    try {
+        PlanOpts po = t.opts;
+        po.regs = forward_kernel_regs((int)po.bw, mark_mode);
+        LaunchPlan l;
+        if (build_plan(t.net, po, l) != PDF_OK) return otherwise;
+        PlanUpload up;
+        const PlanOffsets at = up.add_plan(t.net, l, ResidentImage{});
+        if (t.mem.ensure(up.bytes) != cudaSuccess || !up.copy(t.mem.as<unsigned char>())) {
+            (void)cudaGetLastError();
+            return otherwise;
+        }
+        t.plan.bind(l, t.net, ResidentImage{}, t.mem.as<unsigned char>(), at);
+        t.net = NetPlan{};
+    } catch (const std::bad_alloc &) {
+        return otherwise;
+    }
+    return t.plan;
+}
+
 extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circuit_opts *opts,
                                          pdf_circuit **out) {
     if (!out) return PDF_EINVAL;
@@ -773,6 +818,7 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     bool wide_red = false;
     const uint32_t wide_bw = lane_tile(c->bw) ? c->bw : kLaneWords;  // (a batch's lane kernel)
     const uint32_t single_bw = o.tile_words || wide_full ? c->bw : single_tile(c->bw, max_words, sms);
+    if (single_bw != c->bw) c->narrow_words = single_bw * sms;
     po.bw = wide_full ? wide_bw : single_bw;
     po.threads = o.threads;
     po.regs = forward_kernel_regs((int)po.bw, o.mark_mode);
@@ -781,7 +827,7 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     // Canonical edge array: each gate's fan-ins then fan-outs, gates in id
     // order, so that a run of gates owns one contiguous slice (staged into
     // shared memory by a bulk copy).
-    const NetPlan net = net_plan(nl, fixed);
+    NetPlan net = net_plan(nl, fixed);
     LaunchPlan full, red;
     // The plan of the whole netlist is built on a second thread where there
     // is enough of it, beside the reduced netlist and its plan here.
@@ -798,8 +844,7 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     // and the resident kernel's image of what a lean call walks.
     NetPlan rnet, lnet;
     ResidentImage image, limage;
-    LaunchPlan live, batch;
-    std::future<pdf_status> third;  // the batch's plan, beside the single calls'
+    LaunchPlan live;
     std::vector<int8_t> value;
     enum { kNoOut, kOutFull, kOutRed, kOutLive } out_of = kNoOut;  // whose image writes planes
     const size_t res_smem = (size_t)prop.sharedMemPerBlockOptin - 1024;
@@ -815,41 +860,22 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
             PlanOpts ro = po;
             const uint64_t rw = rl > 1 ? (rnet.n_gates() - rnet.level_off[1]) / (rl - 1) : 0;
             wide_red = (!o.tile_words || lane_tile(o.tile_words)) && rw >= kWideLevel;
-            const uint32_t tile = wide_red ? wide_bw : reduced_tile(c->bw, rw);
-            ro.bw = !wide_red && single_bw != c->bw ? single_bw : tile;
+            const uint32_t tile = reduced_tile(c->bw, rw);
+            ro.bw = wide_red ? wide_bw : single_bw != c->bw ? single_bw : tile;
             ro.threads = wide_red ? 0 : o.threads;
             if (ro.bw != po.bw) ro.regs = forward_kernel_regs((int)ro.bw, o.mark_mode);
-            if (ro.bw != tile) {
-                PlanOpts bo = ro;
-                bo.bw = tile;
-                bo.regs = forward_kernel_regs((int)tile, o.mark_mode);
-                if (G >= 16384) {
-                    try {
-                        third = std::async(std::launch::async, [&rnet, bo, &batch] { return build_plan(rnet, bo, batch); });
-                    } catch (const std::system_error &) {
-                    }
-                }
-                if (!third.valid()) pst = build_plan(rnet, bo, batch);
-            }
-            if (pst == PDF_OK) pst = build_plan(rnet, ro, red);
-            if (third.valid()) {
-                const pdf_status tst = third.get();
-                if (pst == PDF_OK) pst = tst;
-            }
+            pst = build_plan(rnet, ro, red);
+            c->tile_red.wanted = ro.bw != tile;
+            c->tile_red.opts.bw = tile;
             // no plan of the reduced netlist (the thread-per-gate kernel takes
             // 65,536 pieces at most, the lane kernel any number): lean calls
             // walk all of it
             if (pst == PDF_ENOTSUP) {
                 rnet = NetPlan{};
-                red = batch = LaunchPlan{};
-                wide_red = false;
+                red = LaunchPlan{};
+                wide_red = c->tile_red.wanted = false;
                 pst = PDF_OK;
             }
-        } else if (image.bytes.empty() && single_bw != c->bw) {
-            PlanOpts bo = po;
-            bo.bw = c->bw;
-            bo.regs = forward_kernel_regs((int)c->bw, o.mark_mode);
-            pst = build_plan(net, bo, batch);
         }
         // planes: what the lean image holds if that is all that is not
         // constant, else an image of its own
@@ -872,11 +898,14 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         if (out_of == kOutFull) value.assign(G, -1);  // its walk writes every row
         else if (out_of != kNoOut) value.swap(facts.value);
     }
-    for (auto *f : {&other, &third})
-        if (f->valid()) {
-            const pdf_status fst = f->get();
-            if (fst != PDF_OK) pst = fst;
-        }
+    if (other.valid()) {
+        const pdf_status fst = other.get();
+        if (fst != PDF_OK) pst = fst;
+    }
+    // (a wide plan of all gates is walked by batches only where it is the lean one)
+    c->tile_full.wanted =
+        po.bw != c->bw && (!wide_full || (o.seg_len <= 1 && image.bytes.empty() && !rnet.n_gates()));
+    c->tile_full.opts.bw = c->bw;
     if (pst != PDF_OK) {
         delete c;
         return pst;
@@ -907,8 +936,6 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         const PlanOffsets fo = up.add_plan(net, full, reduced ? none : image);
         const PlanOffsets ro = reduced ? up.add_plan(rnet, red, image) : PlanOffsets{};
         const PlanOffsets lo = out_of == kOutLive ? up.add_plan(lnet, live, limage) : PlanOffsets{};
-        const NetPlan &bnet = reduced ? rnet : net;
-        const PlanOffsets bo = batch.n_gates ? up.add_plan(bnet, batch, none) : PlanOffsets{};
         const size_t vo = up.add(value.data(), value.size());
         const WideSync rest{};
         const size_t so = up.add(&rest, sizeof rest);
@@ -923,7 +950,6 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         c->stage.sync = reinterpret_cast<WideSync *>(c->mem.as<unsigned char>() + so);
         c->full.bind(full, net, reduced ? none : image, c->mem.as<unsigned char>(), fo);
         if (reduced) c->red.bind(red, rnet, image, c->mem.as<unsigned char>(), ro);
-        if (batch.n_gates) c->batch.bind(batch, bnet, none, c->mem.as<unsigned char>(), bo);
         if (out_of == kOutLive) c->live.bind(live, lnet, limage, c->mem.as<unsigned char>(), lo);
         c->out_plan = out_of == kOutLive ? &c->live : out_of == kOutRed ? &c->red : out_of == kOutFull ? &c->full : nullptr;
         c->value = reinterpret_cast<const int8_t *>(c->mem.as<unsigned char>() + vo);
@@ -931,12 +957,19 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         c->red.wide = wide_red;
         c->full.mean_width = (uint32_t)mean_width;
         c->red.mean_width = red.n_levels > 1 ? (red.n_gates - rnet.level_off[1]) / (red.n_levels - 1) : 0;
-        for (Plan *p : {&c->full, &c->red, &c->live, &c->batch}) {
+        for (Plan *p : {&c->full, &c->red, &c->live, &c->tile_full.plan, &c->tile_red.plan}) {
             p->res.sms = (uint32_t)prop.multiProcessorCount;
             p->res.regs = 64;  // its launch bound's
             p->res.smem_block = res_smem;
             p->res.smem_sm = (size_t)prop.sharedMemPerMultiprocessor;
         }
+        for (auto *t : {&c->tile_full, &c->tile_red})
+            if (t->wanted) {
+                const uint32_t bw = t->opts.bw;
+                t->opts = po;
+                t->opts.bw = bw;
+                t->net = std::move(t == &c->tile_full ? net : rnet);
+            }
     }
     inf.tile_words = c->bw;
     inf.threads = c->full.threads;
@@ -971,6 +1004,8 @@ extern "C" void pdf_circuit_destroy(pdf_circuit *c) {
     DeviceGuard dg(c->device);
     c->stage.release();
     c->mem.release();
+    c->tile_full.mem.release();
+    c->tile_red.mem.release();
     c->segs.release();
     c->seg_off.release();
     // after a cudaFree, which waits for what may still write there
@@ -1763,25 +1798,26 @@ pdf_status mark_planes(pdf_circuit *c, const uint32_t *sim_v, const uint32_t *si
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     std::lock_guard<std::mutex> lk(c->mu);
     const uint64_t W = (n_pairs + 31) / 32, G = c->info.n_gates;
-    const bool direct = planes_fit(c, c->full_walk(W), W, ld, {sim_v, sim_t, mark});
+    const Walk k = c->full_walk(W);
+    const bool direct = planes_fit(c, k, W, ld, {sim_v, sim_t, mark});
     pdf_status st = open_circuit_err(c);
-    if (st == PDF_OK) st = ensure_ws(c, c->full_walk(W), c->stage, W, !direct);
+    if (st == PDF_OK) st = ensure_ws(c, k, c->stage, W, !direct);
     if (st != PDF_OK) return st;
-    FwdArgs a = base_fwd(c, c->full_walk(W), n_pairs);
+    FwdArgs a = base_fwd(c, k, n_pairs);
     if (direct) {
         a.V = const_cast<uint32_t *>(sim_v);
         a.T = const_cast<uint32_t *>(sim_t);
         a.M = mark;
         a.ld = ld;
     } else {
-        use_ws_planes(a, c->full_walk(W), c->stage, W);
+        use_ws_planes(a, k, c->stage, W);
         PDF_CUDA(cudaMemcpy2DAsync(a.V, a.ld * 4, sim_v, ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
         PDF_CUDA(cudaMemcpy2DAsync(a.T, a.ld * 4, sim_t, ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
     }
-    use_scratch(a, ws_scratch(c, c->full_walk(W), c->stage, W));
+    use_scratch(a, ws_scratch(c, k, c->stage, W));
     a.no_prune = prune ? 0u : 1u;
-    a.in_pieces = c->full.in_pieces;
-    PDF_CUDA(launch_walk(c, c->full_walk(W), c->stage, a, FWD_MARK, cs));
+    a.in_pieces = k.p->in_pieces;
+    PDF_CUDA(launch_walk(c, k, c->stage, a, FWD_MARK, cs));
     if (!direct)
         PDF_CUDA(cudaMemcpy2DAsync(mark, ld * 4, a.M, a.ld * 4, W * 4, G, cudaMemcpyDeviceToDevice, cs));
     return take_circuit_err(c, cs);
@@ -1823,7 +1859,8 @@ pdf_status cover_chunk(pdf_circuit *c, pdf_state *s, const uint32_t *mark, uint6
                        uint64_t pair_base, uint64_t *counts, pdf_totals *chunk, cudaStream_t cs) {
     std::lock_guard<std::mutex> lk(s->mu);
     const uint64_t W = (n_pairs + 31) / 32;
-    pdf_status st = ensure_ws(c, c->full_walk(W), s->ws, W, false);
+    const Walk k = c->full_walk(W);
+    pdf_status st = ensure_ws(c, k, s->ws, W, false);
     if (st != PDF_OK) return st;
     const size_t count_bytes = (size_t)c->info.n_pi * n_pairs * 16;
     if (counts) {
@@ -1832,7 +1869,7 @@ pdf_status cover_chunk(pdf_circuit *c, pdf_state *s, const uint32_t *mark, uint6
     }
     DevAcc *acc = s->acc.as<DevAcc>();
     PDF_CUDA(launch_batch_begin(acc, cs));
-    CoverArgs ca = base_cover(c, c->full_walk(W), s->ws, mark, ld, n_pairs, (uint32_t)pair_base, s->first_x.as<uint32_t>(),
+    CoverArgs ca = base_cover(c, k, s->ws, mark, ld, n_pairs, (uint32_t)pair_base, s->first_x.as<uint32_t>(),
                               s->first_y.as<uint32_t>(), acc);
     // the bitmaps the cover reads, at its granularity, from the given marks
     PDF_CUDA(launch_bitmap_from_marks(c->full.dc, mark, ld, n_pairs, ca.bw, const_cast<uint32_t *>(ca.nzb),
@@ -2006,14 +2043,6 @@ struct pdf_batch {
 
 namespace {
 
-// A batch's walk of one of its circuits: they share the GPU, so a wide plan
-// takes the lane kernel.
-Walk batch_walk(const pdf_circuit *c, uint64_t W) {
-    Walk k = c->lean_walk(W, true);
-    k.wide = 0;
-    return k;
-}
-
 // (Re)build batch b for these jobs: per-circuit arguments and prefixes in
 // one device block, which is reused when it is large enough.
 // up: the stream that uploads the control block, in order before the next
@@ -2059,7 +2088,7 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
     std::vector<Walk> walks(n_jobs);
     uint64_t res_ctas = 0;
     for (uint32_t i = 0; i < n_jobs; i++) {
-        Walk &k = walks[i] = batch_walk(jobs[i].circuit, (jobs[i].pairs.n_pairs + 31) / 32);
+        Walk &k = walks[i] = jobs[i].circuit->batch_walk((jobs[i].pairs.n_pairs + 31) / 32, true);
         if (!k.resident) continue;
         // a CTA takes blocks worth about twice its copy of the image
         const double load = 2.0 + k.p->res.image_bytes / 95e3;
@@ -2498,7 +2527,7 @@ extern "C" pdf_status pdf_state_reserve(pdf_state *s, uint64_t n_pairs) {
     pdf_circuit *c = s->c;
     WsNeed need;
     need.with(c, c->lean_walk(W), W, true);
-    if (c->seg_len <= 1) need.with(c, batch_walk(c, W), W, true);
+    if (c->seg_len <= 1) need.with(c, c->batch_walk(W, false), W, true).with(c, c->batch_walk(W, true), W, true);
     need.with(c, c->planes_walk(W), W, true).with(c, c->full_walk(W), W, !c->out_plan);
     return ensure_ws(c, need, s->ws, W);
 }
@@ -2509,5 +2538,6 @@ pdf_status state_reserve_batch(pdf_state *s, uint64_t n_pairs) {
     if (!dg.ok) return PDF_ECUDA;
     std::lock_guard<std::mutex> lk(s->mu);
     const uint64_t W = (n_pairs + 31) / 32;
-    return ensure_ws(s->c, batch_walk(s->c, W), s->ws, W, true);
+    return ensure_ws(s->c, WsNeed{}.with(s->c, s->c->batch_walk(W, false), W, true).with(s->c, s->c->batch_walk(W, true), W, true),
+                     s->ws, W);
 }

@@ -694,6 +694,17 @@ uint32_t reduced_tile(uint32_t bw, uint64_t mean_width) {
     return bw;
 }
 
+// A batch's circuits with wide levels take the lane kernel from this many of
+// its CTAs on, else the thread-per-gate kernel at the tile: a lane CTA takes a
+// level's gates 32 at a time, so few of them leave the GPU waiting for one
+// another's chains.  Measured (us a pass, robust table, no XOR; lane kernel at
+// 32 words and thread per gate at 4): 150,000 gates, 40 levels: 4 lane CTAs
+// 3,157 and 1,060, 48: 5,525 and 4,266, 64: 5,234 and 4,776, 96: 6,030 and
+// 6,975, 192: 9,293 and 11,455; 60,000 gates, 30 levels: 4: 1,510 and 464, 64:
+// 2,299 and 1,935, 96: 2,616 and 2,819; FIXED 4: 3,272 and 1,571, 64: 11,100 and
+// 10,619, 96: 14,994 and 15,349.
+uint64_t batch_lanes_from(uint64_t sms) { return sms * 9 / 16; }
+
 }  // namespace
 
 // Where it cannot be built (out of memory, too many pieces) the call walks the
@@ -2086,9 +2097,14 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
     // instead of holding the shared memory of the widest member; within a
     // class the longest CTA walks go first.
     std::vector<Walk> walks(n_jobs);
-    uint64_t res_ctas = 0;
+    uint64_t res_ctas = 0, lane_ctas = 0;
     for (uint32_t i = 0; i < n_jobs; i++) {
-        Walk &k = walks[i] = jobs[i].circuit->batch_walk((jobs[i].pairs.n_pairs + 31) / 32, true);
+        const Plan &p = jobs[i].circuit->lean();
+        if (p.wide && !p.image) lane_ctas += ((jobs[i].pairs.n_pairs + 31) / 32 + p.bw - 1) / p.bw;
+    }
+    const bool lanes = lane_ctas >= batch_lanes_from(c0->full.res.sms);
+    for (uint32_t i = 0; i < n_jobs; i++) {
+        Walk &k = walks[i] = jobs[i].circuit->batch_walk((jobs[i].pairs.n_pairs + 31) / 32, lanes);
         if (!k.resident) continue;
         // a CTA takes blocks worth about twice its copy of the image
         const double load = 2.0 + k.p->res.image_bytes / 95e3;

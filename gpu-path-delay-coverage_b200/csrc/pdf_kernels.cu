@@ -1556,7 +1556,50 @@ __device__ __forceinline__ void dense_row(const uint32_t *row, uint32_t w0, uint
     }
 }
 
+// Rows of at most 32 words: S lanes a row (the power of two that holds W), 128 / S
+// rows a warp, so that few pairs do not cost a warp a gate (1,000,000 gates x 32
+// pairs, a warp per row: bitmap 191, merge 131 us).  Calls f(g, x, m) in every
+// lane for each of its four rows: m = the valid mark bits of gate g's word x (0
+// where there is none).
+template <class F>
+__device__ __forceinline__ void dense_rows(const uint32_t *M, uint32_t G, uint64_t ld, uint32_t W, uint64_t n_pairs,
+                                           uint32_t S, F f) {
+    const uint32_t lane = threadIdx.x & 31, x = lane & (S - 1), per = 32 / S;
+    const uint64_t g0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4 * per + lane / S;
+    const uint32_t valid = x + 1 < W || !(n_pairs & 31) ? 0xFFFFFFFFu : (1u << (n_pairs & 31)) - 1u;
+    uint32_t m[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const uint64_t g = g0 + u * per;
+        m[u] = g < G && x < W ? M[g * ld + x] & valid : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) f((uint32_t)(g0 + u * per), x, m[u]);
+}
+constexpr uint32_t kShortRow = 32;
+uint32_t short_row_lanes(uint32_t W) {
+    uint32_t s = 1;
+    while (s < W) s *= 2;
+    return s;
+}
+
 // First-detect merge over given planes (pdf_merge).
+__global__ void k_merge_short(const DevCircuit c, const uint32_t *V, const uint32_t *M, uint64_t ld,
+                              uint64_t n_pairs, uint32_t W, uint32_t S, uint32_t pair_base, uint32_t *first_x,
+                              uint32_t *first_y) {
+    dense_rows(M, c.n_gates, ld, W, n_pairs, S, [&](uint32_t g, uint32_t x, uint32_t m) {
+        if (!__any_sync(0xFFFFFFFFu, m)) return;
+        const uint32_t v = m ? V[(size_t)g * ld + x] : 0u, fx = m & ~v, fy = m & v;
+        uint32_t cx = fx ? x * 32 + (__ffs(fx) - 1) : kEmpty, cy = fy ? x * 32 + (__ffs(fy) - 1) : kEmpty;
+        for (uint32_t d = S / 2; d; d /= 2) {  // within the row's lanes
+            cx = min(cx, __shfl_xor_sync(0xFFFFFFFFu, cx, d));
+            cy = min(cy, __shfl_xor_sync(0xFFFFFFFFu, cy, d));
+        }
+        if (x) return;
+        if (cx != kEmpty) atomicMin(first_x + g, pair_base + cx);
+        if (cy != kEmpty) atomicMin(first_y + g, pair_base + cy);
+    });
+}
 __global__ void k_merge_dense(const DevCircuit c, const uint32_t *V, const uint32_t *M, uint64_t ld,
                               uint64_t n_pairs, uint32_t W, uint32_t pair_base, uint32_t *first_x,
                               uint32_t *first_y) {
@@ -1590,6 +1633,19 @@ __global__ void k_merge_dense(const DevCircuit c, const uint32_t *V, const uint3
 // Column-block bitmaps of nets with a nonzero mark, from a mark plane (stage
 // call pdf_cover).
 // (bw: a power of two, up to 128; the bitmaps are zero before).
+__global__ void k_bitmap_short(const DevCircuit c, const uint32_t *M, uint64_t ld, uint64_t n_pairs, uint32_t W,
+                               uint32_t S, uint32_t bw, uint32_t n_blocks, uint32_t *nzb, uint32_t *blk_maxlvl,
+                               uint32_t bm_words) {
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n_blocks) blk_maxlvl[t] = c.n_levels;
+    const uint32_t span = min(bw, S), lane = threadIdx.x & 31;  // lanes of a block's words
+    dense_rows(M, c.n_gates, ld, W, n_pairs, S, [&](uint32_t g, uint32_t x, uint32_t m) {
+        const uint32_t z = __ballot_sync(0xFFFFFFFFu, m != 0);
+        if (x & (span - 1)) return;
+        const uint32_t part = span == 32 ? z : (z >> lane) & ((1u << span) - 1u);
+        if (part) atomicOr(nzb + (size_t)(x / bw) * bm_words + (g >> 5), 1u << (g & 31));
+    });
+}
 __global__ void k_bitmap_from_marks(const DevCircuit c, const uint32_t *M, uint64_t ld,
                                     uint64_t n_pairs, uint32_t W, uint32_t bw, uint32_t n_blocks,
                                     uint32_t *nzb, uint32_t *blk_maxlvl, uint32_t bm_words) {
@@ -1913,10 +1969,23 @@ cudaError_t launch_seg_merge_dense(const SegArgs &seg, const uint32_t *V, const 
     return cudaGetLastError();
 }
 
+namespace {
+unsigned short_row_blocks(uint32_t G, uint32_t S) {  // of 8 warps, 128 / S rows each
+    const uint64_t rows = 8 * (128 / S);
+    return (unsigned)((G + rows - 1) / rows);
+}
+}  // namespace
+
 cudaError_t launch_merge_dense(const DevCircuit &c, const uint32_t *V, const uint32_t *M, uint64_t ld,
                                uint64_t n_pairs, uint32_t pair_base, uint32_t *first_x,
                                uint32_t *first_y, cudaStream_t st) {
     const uint32_t W = (uint32_t)((n_pairs + 31) / 32);
+    if (W <= kShortRow) {
+        const uint32_t S = short_row_lanes(W);
+        k_merge_short<<<short_row_blocks(c.n_gates, S), 256, 0, st>>>(c, V, M, ld, n_pairs, W, S, pair_base, first_x,
+                                                                      first_y);
+        return cudaGetLastError();
+    }
     const uint64_t warps = (uint64_t)c.n_gates * ((W + kDenseWords - 1) / kDenseWords);
     const uint64_t blocks = (warps * 32 + 255) / 256;
     if (blocks == 0) return cudaSuccess;
@@ -1932,6 +2001,12 @@ cudaError_t launch_bitmap_from_marks(const DevCircuit &c, const uint32_t *M, uin
     const uint32_t n_blocks = (W + bw - 1) / bw;
     cudaError_t e = cudaMemsetAsync(nzb, 0, (size_t)n_blocks * bm_words * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
+    if (W <= kShortRow) {
+        const uint32_t S = short_row_lanes(W);  // (at least as many threads as column blocks)
+        k_bitmap_short<<<short_row_blocks(c.n_gates, S), 256, 0, st>>>(c, M, ld, n_pairs, W, S, bw, n_blocks, nzb,
+                                                                       blk_maxlvl, bm_words);
+        return cudaGetLastError();
+    }
     const uint64_t n = std::max<uint64_t>((uint64_t)c.n_gates * ((W + kDenseWords - 1) / kDenseWords) * 32, n_blocks);
     if ((n + 255) / 256 > 0x7FFFFFFFull) return cudaErrorInvalidValue;
     k_bitmap_from_marks<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(c, M, ld, n_pairs, W, bw, n_blocks,

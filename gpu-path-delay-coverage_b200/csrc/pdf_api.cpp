@@ -1445,6 +1445,21 @@ pdf_status take_circuit_err(pdf_circuit *c, cudaStream_t cs) {
     return err_status(e);
 }
 
+// How many first-detecting pairs skip the cover's small table.  Up to one per
+// SM, the large table takes them side by side too, and those that would not fit
+// the small one are not walked twice; up to two where pairs mostly do not fit
+// (the FIXED non-robust table, netlists of 2^18 gates or more).  Measured (cover
+// kernels, us; through both tables and at once): 20,000 gates, 100 pairs 30 and
+// 29; 200,000 gates, 100 pairs 90 and 79; 1,000,000 gates, 32 pairs 459 and 211,
+// 256 pairs 591 and 485; FIXED non-robust, 20,000 gates, 32 pairs 211 and 139, 247
+// pairs 364 and 330, 477 pairs 565 and 585 (one table).  Where they fit, more
+// pairs than SMs are faster through the small one: FIXED robust, 60,000 gates,
+// 238 pairs 103 and 160.
+uint32_t cover_few(const pdf_circuit *c, const Plan &p) {
+    const bool large = c->mark_mode == PDF_MARK_FIXED_NONROBUST || p.n_gates >= 1u << 18;
+    return (large ? 2 : 1) * c->cover_grid;
+}
+
 CoverArgs base_cover(pdf_circuit *c, const Walk &k, Workspace &ws, const uint32_t *M, uint64_t ld, uint64_t n_pairs,
                      uint32_t pair_base, const uint32_t *fx, const uint32_t *fy, DevAcc *acc) {
     const Plan &p = *k.p;
@@ -1471,6 +1486,7 @@ CoverArgs base_cover(pdf_circuit *c, const Walk &k, Workspace &ws, const uint32_
     a.hash_cap = c->hash_cap;
     a.mid_list = x.mid_list;
     a.small_cap = c->small_cap;
+    a.few = cover_few(c, p);
     a.over_list = x.over_list;
     a.spill = x.spill;
     uint64_t slot;

@@ -1266,9 +1266,9 @@ __device__ __forceinline__ void close_and_tell(const CoverArgs &a) {
 // The cover in two passes over the same pairs (as k_batch_cover): TIER 0 with
 // a small table, several CTAs per SM, queues the pairs that mark more nets
 // for TIER 1, whose table takes an SM; what does not fit there either is
-// queued for the spill cover.
+// queued for the spill cover.  Up to `few` pairs skip the small table.
 template <int TIER>
-__global__ void __launch_bounds__(kCoverThreads) k_cover(const CoverArgs a, uint32_t cap) {
+__global__ void __launch_bounds__(kCoverThreads) k_cover(const CoverArgs a, uint32_t cap, uint32_t few) {
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr uint32_t CAND = TIER == 0 ? kCoverCandSmall : kCoverCand;
     grid_trigger();
@@ -1276,6 +1276,14 @@ __global__ void __launch_bounds__(kCoverThreads) k_cover(const CoverArgs a, uint
     const bool direct = TIER == 0 || !a.mid_list;  // without a queue the large table takes every pair
     const uint32_t n_items = direct ? *a.active_count : a.acc->n_mid;
     if (!direct && !n_items) return;  // the small-table pass closed the batch
+    // few pairs that will mostly not fit: all for the large table at once, instead
+    // of one pass after the other
+    const bool pass_on = TIER == 0 && n_items <= few;
+    if (pass_on && blockIdx.x == 0) {
+        for (uint32_t i = threadIdx.x; i < n_items; i += blockDim.x) a.mid_list[i] = a.active_list[i];
+        if (threadIdx.x == 0) a.acc->n_mid = n_items;
+        __syncthreads();  // (before this CTA counts itself done)
+    }
     uint32_t *lvt = reinterpret_cast<uint32_t *>(smraw + cover_smem_tables(cap, CAND));  // [kCoverLevels] level_off
     const uint32_t L = a.c.n_levels;
     const bool lv_shared = L + 1 <= kCoverLevels;
@@ -1284,7 +1292,7 @@ __global__ void __launch_bounds__(kCoverThreads) k_cover(const CoverArgs a, uint
     const uint32_t *lo_tab = lv_shared ? lvt : a.c.level_off;
     __syncthreads();
     const uint32_t *in = direct ? a.active_list : a.mid_list;
-    for (uint32_t ai = blockIdx.x; ai < n_items; ai += gridDim.x) {
+    for (uint32_t ai = blockIdx.x; ai < n_items && !pass_on; ai += gridDim.x) {
         const uint32_t p = in[ai];
         const bool over = cover_pair<CAND>(a, p, lo_tab, cap, [&](uint32_t g, uint32_t pid) { return net_first(a, g, pid); });
         if (over && threadIdx.x == 0) {
@@ -1832,12 +1840,13 @@ cudaError_t launch_cover(const CoverArgs &a, uint32_t grid, uint32_t threads, bo
         const uint32_t cap0 = std::min(a.small_cap - (uint32_t)((lv + per_net - 1) / per_net), a.c.n_gates);
         const size_t smem0 = cover_smem_tables(cap0, kCoverCandSmall) + lv;
         if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_cover<0>), smem0)) != cudaSuccess) return e;
-        e = launch_next(k_cover<0>, grid * kCoverSmallCtas, threads, smem0, st, a, cap0);
-        if (e != cudaSuccess || a.c.n_gates <= cap0) return e;  // (no pair can mark more)
+        const bool all_fit = a.c.n_gates <= cap0;  // no pair can mark more
+        e = launch_next(k_cover<0>, grid * kCoverSmallCtas, threads, smem0, st, a, cap0, all_fit ? 0u : a.few);
+        if (e != cudaSuccess || all_fit) return e;
     }
     const size_t smem = cover_smem_bytes(a.hash_cap);
     if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_cover<1>), smem)) != cudaSuccess) return e;
-    e = launch_next(k_cover<1>, grid, threads, smem, st, a, a.hash_cap);
+    e = launch_next(k_cover<1>, grid, threads, smem, st, a, a.hash_cap, 0u);
     if (e != cudaSuccess || !a.spill_slots) return e;
     return launch_next(k_cover_spill, a.spill_slots, kCoverThreads, 0, st, a);
 }

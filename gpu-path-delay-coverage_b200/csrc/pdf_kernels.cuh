@@ -131,6 +131,7 @@ struct CoverArgs {
     // queued here (count in acc->n_mid) for the large-table pass
     uint32_t *mid_list;           // [min(n_pairs, 2 * n_gates)]
     uint32_t small_cap;
+    uint32_t few;                 // up to this many pairs go to the large table at once (cover_few)
     DevAcc *mirror;               // host memory that gets the accumulators once the batch is closed, or null
     unsigned char *spill;
     uint32_t spill_slots;

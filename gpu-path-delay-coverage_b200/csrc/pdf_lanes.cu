@@ -179,11 +179,14 @@ __device__ __forceinline__ void lane_load(const FwdArgs &a, const LanePlanes &P,
 }
 
 // Evaluate, mark and store one gate; returns whether it holds a mark in the
-// block (warp-uniform).  wm: the lane's word masks (pairs present).
+// block (warp-uniform).  wm: the lane's word masks (pairs present); reach (in
+// shared memory) grows to the last level that a marked gate carries to: kept by
+// the caller in registers it spilled the forward pass (64-word tile, 183,874
+// gates, planes: 6.6 -> 7.7 ms).
 template <int SEM, int MODE, int LW>
 __device__ __forceinline__ bool lane_gate(const FwdArgs &a, const LanePlanes &P, uint32_t *bm, const GateRec *rp,
                                           uint32_t g, bool live, uint32_t nw, const uint32_t (&wm)[LW],
-                                          const LaneIn<LW> &x) {
+                                          uint32_t *reach, const LaneIn<LW> &x) {
     constexpr bool FIX = SEM >= 2;
     const uint32_t h = x.h, nfi = (h >> 8) & 0xFFu;
     // fan-in q > 3 of the gate (its id from the edge array), read from its rows
@@ -249,11 +252,13 @@ __device__ __forceinline__ bool lane_gate(const FwdArgs &a, const LanePlanes &P,
         }
     }
     if (MODE != FWD_SIM) {  // markkernel.cuh:226-267
+        const bool anyT = __any_sync(0xFFFFFFFFu, lany<LW>(T));
         if (h & RF_INPT) {
-            const uint32_t on = flagmask(h, RF_MARKF0);
+            // (the whole netlist's inputs always)
+            const uint32_t on = MODE == FWD_MARK ? 0xFFFFFFFFu : flagmask(h, RF_MARKF0);
 #pragma unroll
             for (int j = 0; j < LW; j++) M[j] = T[j] & on;
-        } else if ((h & RF_MARKF0) && x.bit0) {
+        } else if ((h & RF_MARKF0) && x.bit0 && anyT) {
             // fan-in 0 (gate w[7]) holds a mark: its bitmap bit is set
 #pragma unroll
             for (int j = 0; j < LW; j++) M[j] = T[j] & x.m0[j];
@@ -278,7 +283,7 @@ __device__ __forceinline__ bool lane_gate(const FwdArgs &a, const LanePlanes &P,
 #pragma unroll
                 for (int j = 0; j < LW; j++) M[j] &= sens_result<SEM & 1>(s[j]);
             }
-        } else if (FIX && (h & RF_MANY) && __any_sync(0xFFFFFFFFu, lany<LW>(T))) {
+        } else if (FIX && (h & RF_MANY) && anyT) {
             // any fan-in may carry the path: its own mark enters the side test
             const uint32_t mor = flagmask(h, RF_IM), mxor = flagmask(h, RF_XOR), mand = ~(mor | mxor);
             SensAcc s[LW];
@@ -312,7 +317,10 @@ __device__ __forceinline__ bool lane_gate(const FwdArgs &a, const LanePlanes &P,
         }
         if (MODE != FWD_SIM && (a.store_all || marked)) lstore<LW>(lrow(P.M, g, P.ld4), M, nw);
     }
-    if (marked && (threadIdx.x & 31) == 0) atomicOr(bm + (g >> 5), 1u << (g & 31));
+    if (marked && (threadIdx.x & 31) == 0) {
+        atomicOr(bm + (g >> 5), 1u << (g & 31));
+        if (MODE == FWD_FUSED) atomicMax(reach, rp->w[1] >> 16);
+    }
     return marked;
 }
 
@@ -361,15 +369,10 @@ __device__ __forceinline__ void forward_lanes_cta(const FwdArgs &a, const uint32
             a.acc->done_over = 0;
         }
     }
-    // the last level that can still hold a marked gate (a lane plan's reach);
-    // levels below s_top may hold a forward mark, below s_max one that stays
-    __shared__ uint32_t s_reach, s_top, s_max;
+    // the last level that can still hold a marked gate (a lane plan's reach)
+    __shared__ uint32_t s_reach;
     const bool early = MODE == FWD_FUSED && a.in_pieces;
-    if (threadIdx.x == 0) {
-        s_reach = 0;
-        s_top = 0;
-        s_max = 0;
-    }
+    if (threadIdx.x == 0) s_reach = 0;
     __syncthreads();
 
     // ------------------------------------------------------------- forward
@@ -385,6 +388,7 @@ __device__ __forceinline__ void forward_lanes_cta(const FwdArgs &a, const uint32
     };
     // gates [pa, pb) of level pl: the next piece to evaluate; (na, nb, nlv):
     // the one after it, loaded a piece ahead
+    uint32_t top = 0;  // levels below `top` may hold a forward mark
     uint32_t pa = a.pieces[0].a, pb = a.pieces[0].b, pl = a.pieces[0].level, na = 0, nb = 0, nlv = 0;
     if (a.n_pieces > 1) {
         na = a.pieces[1].a;
@@ -392,14 +396,18 @@ __device__ __forceinline__ void forward_lanes_cta(const FwdArgs &a, const uint32
         nlv = a.pieces[1].level;
     }
     stage(pa, pb, 0);
+    bool any = false;
+    uint32_t prev_level = 0;
     for (uint32_t i = 0; i < a.n_pieces; i++) {
         cp_async_wait_all();  // this thread's copies of piece i's records
-        __syncthreads();
+        if (__syncthreads_or(any) && i) top = max(top, prev_level + 1);
+        any = false;
         // nothing from this level on can be marked (decided where every mark of
         // the levels below is known; s_reach grows only in CTAs that went on)
         if (early && s_reach < pl) break;
         if (i + 1 < a.n_pieces) stage(na, nb, (i + 1) & 1);  // into the buffer of piece i - 1, which every warp has left
-        const uint32_t ga = pa, gb = pb, level = pl;
+        const uint32_t ga = pa, gb = pb;
+        prev_level = pl;
         pa = na;
         pb = nb;
         pl = nlv;
@@ -409,8 +417,6 @@ __device__ __forceinline__ void forward_lanes_cta(const FwdArgs &a, const uint32
             nlv = __ldg(&a.pieces[i + 2].level);
         }
         const GateRec *rb = recs + (size_t)(i & 1) * a.cap;
-        bool any = false;
-        uint32_t reach = 0;
         for (uint32_t g = ga + warp; g < gb; g += U * NW) {
             LaneIn<LW> x[U];
 #pragma unroll
@@ -421,18 +427,11 @@ __device__ __forceinline__ void forward_lanes_cta(const FwdArgs &a, const uint32
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 const uint32_t gu = g + u * NW;
-                if (gu < gb && lane_gate<SEM, MODE, LW>(a, P, bm, rb + (gu - ga), gu, live, nw, wm, x[u])) {
-                    any = true;
-                    if (early) reach = max(reach, rb[gu - ga].w[1] >> 16);
-                }
+                if (gu < gb) any |= lane_gate<SEM, MODE, LW>(a, P, bm, rb + (gu - ga), gu, live, nw, wm, &s_reach, x[u]);
             }
         }
-        if (MODE != FWD_SIM && any && lane == 0) {  // (the same on every lane)
-            atomicMax(&s_top, level + 1);
-            if (reach > level) atomicMax(&s_reach, reach);
-        }
     }
-    __syncthreads();
+    if (__syncthreads_or(any)) top = max(top, prev_level + 1);
     if constexpr (MODE == FWD_SIM) {
         return;
     } else {
@@ -441,7 +440,8 @@ __device__ __forceinline__ void forward_lanes_cta(const FwdArgs &a, const uint32
         // (markkernel.cuh:271-293, mergekernel.cuh:116-198) levels descending;
         // a warp takes 32-gate words of the bitmap and visits their marked
         // gates; a gate's pruned mark is final once its fan-outs' are.
-        for (int l = (int)s_top - 1; l >= 0; l--) {
+        uint32_t maxlvl = 0;
+        for (int l = (int)top - 1; l >= 0; l--) {
             const uint32_t ga = __ldg(lo + l), gb = __ldg(lo + l + 1);
             bool any = false;
             for (uint32_t q = (ga >> 5) + warp; q < (gb + 31) >> 5; q += NW) {
@@ -512,14 +512,13 @@ __device__ __forceinline__ void forward_lanes_cta(const FwdArgs &a, const uint32
                     any |= nz;
                 }
             }
-            if (any && lane == 0) atomicMax(&s_max, (uint32_t)l + 1);
-            __syncthreads();
+            if (__syncthreads_or(any) && !maxlvl) maxlvl = (uint32_t)l + 1;
         }
         // publish the bitmap of surviving marks for the cover kernels
         if (a.bm_shared && gbm)
             for (uint32_t q = threadIdx.x; q < a.bm_words; q += blockDim.x) gbm[q] = bm[q];
-        if (threadIdx.x == 0) a.blk_maxlvl[blk] = s_max;
-        if (fine && threadIdx.x < NF) a.maxlvl_fine[blk * NF + threadIdx.x] = s_max;
+        if (threadIdx.x == 0) a.blk_maxlvl[blk] = maxlvl;
+        if (fine && threadIdx.x < NF) a.maxlvl_fine[blk * NF + threadIdx.x] = maxlvl;
     }
 }
 

@@ -1387,7 +1387,6 @@ __global__ void __launch_bounds__(kCoverThreads) k_cover_lean(const CoverArgs a)
 // After k_cover: the pairs it queued, one per CTA at a time (CTA k uses
 // spill slot k); the last CTA closes the batch.
 __global__ void __launch_bounds__(kCoverThreads) k_cover_spill(const CoverArgs a) {
-    grid_wait();
     const uint32_t n_over = a.acc->n_over;
     if (!n_over) return;  // k_cover closed the batch
     for (uint32_t j = blockIdx.x; j < n_over; j += gridDim.x) spill_pair(a, a.over_list[j], spill_slot(a, blockIdx.x));
@@ -1848,7 +1847,11 @@ cudaError_t launch_cover(const CoverArgs &a, uint32_t grid, uint32_t threads, bo
     if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_cover<1>), smem)) != cudaSuccess) return e;
     e = launch_next(k_cover<1>, grid, threads, smem, st, a, a.hash_cap, 0u);
     if (e != cudaSuccess || !a.spill_slots) return e;
-    return launch_next(k_cover_spill, a.spill_slots, kCoverThreads, 0, st, a);
+    // A plain launch: started early it runs on SMs split for k_cover's tables, with
+    // next to no L1, which its walks over the netlist live on (335 pairs of 214,501
+    // gates 302 ms, 266 so; 666 pairs of 111,483 gates 99 and 71).
+    k_cover_spill<<<a.spill_slots, kCoverThreads, 0, st>>>(a);
+    return cudaGetLastError();
 }
 
 namespace {

@@ -330,9 +330,10 @@ struct pdf_circuit {
     Plan full, red;   // every gate; the reduced netlist (n_gates 0: none)
     // the plan of grading calls that ask for no plane
     const Plan &lean() const { return red.n_gates ? red : full; }
-    // Plans at the tile of circuits whose single calls take another column block
-    // (narrower ones, single_tile; the wide kernel's), built when first asked
-    // for: of the reduced netlist, and of all gates.
+    // Plans at the tile for the staged kernels, of the reduced netlist and of all
+    // gates, built when first asked for: of circuits whose single calls take
+    // another column block (narrower ones, single_tile; the wide kernel's) or
+    // walk a reduced netlist on chip.
     struct TilePlan {
         bool wanted = false;
         PlanOpts opts;
@@ -344,7 +345,12 @@ struct pdf_circuit {
     mutable TilePlan tile_red, tile_full;
     uint64_t narrow_words = ~0ull;  // single calls over more words than this take them
     const Plan &at_tile(TilePlan &t, const Plan &otherwise) const;
-    const Plan &lean_at_tile() const { return red.n_gates ? at_tile(tile_red, red) : at_tile(tile_full, full); }
+    // The lean calls' plan for the staged kernels, at the tile; of a reduced
+    // netlist that fits on chip, null where it could not be built.
+    const Plan *lean_at_tile() const {
+        const Plan &p = red.n_gates ? at_tile(tile_red, red) : at_tile(tile_full, full);
+        return &p == &red && red.image ? nullptr : &p;
+    }
     // Planes from the resident kernel: every gate whose value is not constant,
     // where they fit on chip (the constant rows are filled in), else null.
     Plan live;
@@ -377,15 +383,22 @@ struct pdf_circuit {
     }
     Walk full_walk(uint64_t W) const { return staged_walk(W > narrow_words ? at_tile(tile_full, full) : full, W); }
     Walk lean_walk(uint64_t W) const {
-        if (lean().image) return resident_walk(lean(), W, RES_LEAN);
-        return staged_walk(W > narrow_words ? lean_at_tile() : lean(), W);
+        if (lean().image) {
+            const Walk k = resident_walk(lean(), W, RES_LEAN);
+            if (resident_pays(k.rs, W, lean().res.sms)) return k;
+            const Plan *p = red.n_gates || W > narrow_words ? lean_at_tile() : &full;
+            return p ? staged_walk(*p, W) : k;
+        }
+        return staged_walk(W > narrow_words ? *lean_at_tile() : lean(), W);
     }
     // A batch's: its circuits share the GPU, so a wide plan takes the lane kernel
-    // (lanes) or the plan at the tile.
-    Walk batch_walk(uint64_t W, bool lanes) const {
-        if (lean().image) return resident_walk(lean(), W, RES_LEAN);
+    // (lanes) or the plan at the tile, and a netlist that fits on chip may be
+    // walked there (chip) or not.
+    Walk batch_walk(uint64_t W, bool lanes, bool chip) const {
         Walk k;
-        k.p = lean().wide && lanes ? &lean() : &lean_at_tile();
+        const bool on_chip = lean().image && chip;
+        if (!on_chip) k.p = lean().wide && lanes ? &lean() : lean_at_tile();
+        if (!k.p) return resident_walk(lean(), W, RES_LEAN);
         k.bw = k.p->bw;
         return k;
     }
@@ -394,13 +407,17 @@ struct pdf_circuit {
         k.p = &p;
         k.resident = true;
         k.out = out;
-        k.rs = resident_shape(p.res, W);
+        k.rs = resident_shape(p.res, W, out == RES_LEAN ? 0 : out == RES_SIM ? 2 : 3);
         k.bw = k.rs.bw;
         return k;
     }
     // the walk of calls that ask for planes: all three, or the codes alone (out = RES_SIM)
     Walk planes_walk(uint64_t W, int out = RES_PLANES) const {
-        return out_plan ? resident_walk(*out_plan, W, out) : full_walk(W);
+        if (out_plan) {
+            const Walk k = resident_walk(*out_plan, W, out);
+            if (resident_planes_pay(k.rs, W, out == RES_SIM ? 2 : 3, info.n_gates, full.n_pieces)) return k;
+        }
+        return full_walk(W);
     }
     uint32_t hash_cap = 4096, cover_threads = 256, cover_grid = 0;
     uint32_t small_cap = 0;  // nets per pair of the cover's small-table pass
@@ -686,6 +703,11 @@ uint32_t single_tile(uint32_t bw, uint64_t words, uint64_t sms) {
     return words > sms ? 2 : 1;
 }
 
+// Mean width of the levels above the inputs.
+uint64_t mean_level(const NetPlan &n) {
+    return n.n_levels() > 1 ? (n.n_gates() - n.level_off[1]) / (n.n_levels() - 1) : 0;
+}
+
 // Column block of the reduced walk of a circuit whose tile is bw words, by
 // the mean width of its levels above the inputs.  Narrow levels leave most
 // warps of the lane kernel without a gate.
@@ -866,10 +888,11 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         image = build_resident(reduced ? rnet : net, res_smem - 1024);
         if (reduced && !image.bytes.empty()) {
             build_records(rnet, red);
+            c->tile_red.wanted = true;
+            c->tile_red.opts.bw = reduced_tile(c->bw, mean_level(rnet));
         } else if (reduced) {
-            const uint32_t rl = rnet.n_levels();
             PlanOpts ro = po;
-            const uint64_t rw = rl > 1 ? (rnet.n_gates() - rnet.level_off[1]) / (rl - 1) : 0;
+            const uint64_t rw = mean_level(rnet);
             wide_red = (!o.tile_words || lane_tile(o.tile_words)) && rw >= kWideLevel;
             const uint32_t tile = reduced_tile(c->bw, rw);
             ro.bw = wide_red ? wide_bw : single_bw != c->bw ? single_bw : tile;
@@ -915,7 +938,7 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     }
     // (a wide plan of all gates is walked by batches only where it is the lean one)
     c->tile_full.wanted =
-        po.bw != c->bw && (!wide_full || (o.seg_len <= 1 && image.bytes.empty() && !rnet.n_gates()));
+        po.bw != c->bw && (!wide_full || (o.seg_len <= 1 && !rnet.n_gates()));
     c->tile_full.opts.bw = c->bw;
     if (pst != PDF_OK) {
         delete c;
@@ -967,7 +990,7 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         c->full.wide = wide_full;
         c->red.wide = wide_red;
         c->full.mean_width = (uint32_t)mean_width;
-        c->red.mean_width = red.n_levels > 1 ? (red.n_gates - rnet.level_off[1]) / (red.n_levels - 1) : 0;
+        if (reduced) c->red.mean_width = (uint32_t)mean_level(rnet);
         for (Plan *p : {&c->full, &c->red, &c->live, &c->tile_full.plan, &c->tile_red.plan}) {
             p->res.sms = (uint32_t)prop.multiProcessorCount;
             p->res.regs = 64;  // its launch bound's
@@ -1288,6 +1311,24 @@ struct WsNeed {
         planes = std::max(planes, ws_plane_words(c, k, W, need_planes) * 4);
         return *this;
     }
+    // ... and what the resident walk takes that calls over fewer words may have
+    // instead (calls within a workspace allocate nothing)
+    WsNeed &lean(const pdf_circuit *c, const Walk &k, uint64_t W) {
+        if (!k.resident && c->lean().image) {
+            const Plan &p = c->lean();
+            const uint64_t w = std::min<uint64_t>(W, resident_words(pdf_circuit::resident_walk(p, W, RES_LEAN).rs, p.res.sms));
+            with(c, pdf_circuit::resident_walk(p, w, RES_LEAN), w, true);
+        }
+        return with(c, k, W, true);
+    }
+    WsNeed &out(const pdf_circuit *c, const Walk &k, uint64_t W, int out, bool need_planes) {
+        if (!k.resident && c->out_plan) with(c, pdf_circuit::resident_walk(*c->out_plan, W, out), W, need_planes);
+        return with(c, k, W, need_planes);
+    }
+    WsNeed &batch(const pdf_circuit *c, uint64_t W) {
+        for (int i = 0; i < 4; i++) with(c, c->batch_walk(W, i & 1, i & 2), W, true);
+        return *this;
+    }
 };
 
 // Sizes the workspace.  A block that is too small and held stays allocated
@@ -1578,7 +1619,10 @@ pdf_status grade_mark_locked(pdf_circuit *c, pdf_state *s, const pdf_pairs *pr, 
     PDF_CUDA(cudaStreamIsCapturing(cs, &cap));
     const Plan &p = *k.p;
     const bool direct = out && out->on_device && planes_fit(c, k, W, out->ld, {out->sim_v, out->sim_t, out->mark});
-    pdf_status st = ensure_ws(c, k, s->ws, W, !direct);
+    WsNeed need;
+    if (planes) need.out(c, k, W, RES_PLANES, !direct);
+    else need.lean(c, k, W);
+    pdf_status st = ensure_ws(c, need, s->ws, W);
     if (st != PDF_OK) return st;
     const uint32_t *pv, *pt;
     uint64_t pld;
@@ -1787,7 +1831,7 @@ extern "C" pdf_status pdf_sim(pdf_circuit *c, const pdf_pairs *pr, uint32_t *sim
     if ((st = open_circuit_err(c)) != PDF_OK) return st;
     const Walk k = c->planes_walk(W, RES_SIM);
     const bool direct = planes_fit(c, k, W, ld, {sim_v, sim_t});
-    st = ensure_ws(c, k, c->stage, W, !direct);
+    st = ensure_ws(c, WsNeed{}.out(c, k, W, RES_SIM, !direct), c->stage, W);
     if (st != PDF_OK) return st;
     const uint32_t *pv, *pt;
     uint64_t pld;
@@ -2113,14 +2157,28 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
     // instead of holding the shared memory of the widest member; within a
     // class the longest CTA walks go first.
     std::vector<Walk> walks(n_jobs);
-    uint64_t res_ctas = 0, lane_ctas = 0;
+    uint64_t res_ctas = 0, lane_ctas = 0, all_words = 0;
+    double rounds = 0;  // of blocks of the netlists that fit on chip only just
     for (uint32_t i = 0; i < n_jobs; i++) {
         const Plan &p = jobs[i].circuit->lean();
-        if (p.wide && !p.image) lane_ctas += ((jobs[i].pairs.n_pairs + 31) / 32 + p.bw - 1) / p.bw;
+        const uint64_t W = (jobs[i].pairs.n_pairs + 31) / 32;
+        all_words += W;
+        if (p.image) {
+            const uint32_t at_once = resident_shape(p.res, W).words;
+            if (at_once < kResidentWords) rounds += (double)W / (at_once * p.res.sms);
+        } else if (p.wide) {
+            lane_ctas += (W + p.bw - 1) / p.bw;
+        }
     }
-    const bool lanes = lane_ctas >= batch_lanes_from(c0->full.res.sms);
+    const uint64_t sms = c0->full.res.sms;
+    const bool lanes = lane_ctas >= batch_lanes_from(sms);
+    // (as resident_pays, over all the jobs)
+    const bool chip = rounds <= 2.5 * std::max(1.0, (double)all_words / (10.0 * sms));
     for (uint32_t i = 0; i < n_jobs; i++) {
-        Walk &k = walks[i] = jobs[i].circuit->batch_walk((jobs[i].pairs.n_pairs + 31) / 32, lanes);
+        const uint64_t W = (jobs[i].pairs.n_pairs + 31) / 32;
+        const Plan &p = jobs[i].circuit->lean();
+        Walk &k = walks[i] = jobs[i].circuit->batch_walk(
+            W, lanes, chip || (p.image && resident_shape(p.res, W).words >= kResidentWords));
         if (!k.resident) continue;
         // a CTA takes blocks worth about twice its copy of the image
         const double load = 2.0 + k.p->res.image_bytes / 95e3;
@@ -2128,7 +2186,6 @@ pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs,
         res_ctas += (k.rs.blocks + k.rs.per - 1) / k.rs.per;
     }
     // ... or fewer while that leaves SMs without a CTA
-    const uint64_t sms = c0->full.res.sms;
     for (Walk &k : walks)
         if (k.resident && res_ctas < 2 * sms)
             k.rs.per = std::max<uint32_t>(1, (uint32_t)(k.rs.per * res_ctas / (2 * sms)));
@@ -2558,9 +2615,9 @@ extern "C" pdf_status pdf_state_reserve(pdf_state *s, uint64_t n_pairs) {
     const uint64_t W = (n_pairs + 31) / 32;
     pdf_circuit *c = s->c;
     WsNeed need;
-    need.with(c, c->lean_walk(W), W, true);
-    if (c->seg_len <= 1) need.with(c, c->batch_walk(W, false), W, true).with(c, c->batch_walk(W, true), W, true);
-    need.with(c, c->planes_walk(W), W, true).with(c, c->full_walk(W), W, !c->out_plan);
+    need.lean(c, c->lean_walk(W), W);
+    if (c->seg_len <= 1) need.batch(c, W);
+    need.out(c, c->planes_walk(W), W, RES_PLANES, true).with(c, c->full_walk(W), W, !c->out_plan);
     return ensure_ws(c, need, s->ws, W);
 }
 
@@ -2570,6 +2627,5 @@ pdf_status state_reserve_batch(pdf_state *s, uint64_t n_pairs) {
     if (!dg.ok) return PDF_ECUDA;
     std::lock_guard<std::mutex> lk(s->mu);
     const uint64_t W = (n_pairs + 31) / 32;
-    return ensure_ws(s->c, WsNeed{}.with(s->c, s->c->batch_walk(W, false), W, true).with(s->c, s->c->batch_walk(W, true), W, true),
-                     s->ws, W);
+    return ensure_ws(s->c, WsNeed{}.batch(s->c, W), s->ws, W);
 }

@@ -79,10 +79,12 @@ ResidentImage build_resident(const NetPlan &n, size_t smem) {
 // about 0.3 us a level, of as many blocks at once as CTAs fit an SM) or its
 // instructions (about 0.42 ns per gate and word of an SM), whichever is more;
 // a CTA the copy of the image first, shared by the blocks it takes in turn.
-ResidentShape resident_shape(const ResidentSizes &z, uint64_t W) {
+// With plane rows every gate also stores a piece of each, a sector whatever the
+// block's width: 5.5 ns a gate for three, 3.2 for two, and all levels are walked.
+ResidentShape resident_shape(const ResidentSizes &z, uint64_t W, uint32_t rows) {
     const auto al = [](size_t x) { return (x + 15) & ~(size_t)15; };
     ResidentShape best;
-    double best_t = 0;
+    uint32_t words = 0;
     for (uint32_t bw = 1; bw <= 8; bw *= 2) {
         ResidentShape s;
         s.bw = bw;
@@ -100,21 +102,58 @@ ResidentShape resident_shape(const ResidentSizes &z, uint64_t W) {
         s.threads = by_smem >= 2 ? 256 : 512;
         s.occ = std::min({by_smem, 2048 / s.threads, 65536 / (s.threads * std::max(z.regs, 32u)), 8u});
         while (s.occ & (s.occ - 1)) s.occ &= s.occ - 1;  // 1, 2, 4 or 8: few classes in a batch
+        words = std::max(words, s.occ * bw);
         s.blocks = (uint32_t)((W + bw - 1) / bw);
         const uint32_t slots = z.sms * s.occ;
         s.per = (s.blocks + slots - 1) / slots;
         s.ctas = (s.blocks + s.per - 1) / s.per;
-        const double load = 2.0 + z.image_bytes / 95e3, chain = 1.0 + 0.3 * z.n_levels;
+        const double load = 2.0 + z.image_bytes / 95e3;
         const uint32_t together = std::min(s.occ, (s.ctas + z.sms - 1) / z.sms);
         const double issue = 0.42e-3 * z.n_gates * bw;
-        s.block_us = std::max(chain / s.occ, issue);
-        const double t = load + s.per * std::max(chain, together * issue);
-        if (!best.bw || t < best_t * 0.97) {
-            best = s;
-            best_t = t;
+        if (rows) {
+            const double chain = rows == 3 ? 4.0 + 0.25 * z.n_levels : 3.0 + 0.2 * z.n_levels;
+            const double stores = (rows == 3 ? 5.5e-3 : 3.2e-3) * z.n_gates;
+            s.us = load + s.per * (chain + together * (stores + issue));
+        } else {
+            const double chain = 1.0 + 0.3 * z.n_levels;
+            s.block_us = std::max(chain / s.occ, issue);
+            s.us = load + s.per * std::max(chain, together * issue);
         }
+        if (!best.bw || s.us < best.us * 0.97) best = s;
     }
+    best.words = words;
     return best;
+}
+
+// A round of blocks costs about 0.4 of the staged kernel's walk, whose CTAs take
+// about 10 words an SM at a time: where an SM has room for fewer, two rounds pay.
+// Measured (kernels, us, resident and staged; 7,182 gates, 1 word an SM): 256 words
+// 56 and 74, 512 words 108 and 81, 2,048 words 339 and 111, 32,768 words 4,988 and
+// 1,433; 4,191 gates, 2 words: 512 words 48 and 81, 2,048 words 159 and 103 (FIXED
+// 384 and 239); 3,159 gates, 4 words: 512 words 20 and 68, 2,048 words 71 and 68,
+// 8,192 words 236 and 160; 1,554 gates, 8 words: 8,192 words 112 and 154, 32,768
+// words 418 and 492.
+uint64_t resident_words(const ResidentShape &s, uint32_t sms) {
+    return s.words >= kResidentWords ? ~0ull : 2ull * s.words * sms;
+}
+bool resident_pays(const ResidentShape &s, uint64_t W, uint32_t sms) { return W <= resident_words(s, sms); }
+
+// The staged kernel walks all gates: about 1 us a piece and 11 ps a gate and
+// word (6.5 ps the codes alone).  Narrow blocks stop paying where rows are long
+// for another reason: the sectors that a CTA has written a part of leave L2
+// before its next blocks fill them.  Measured (kernels, us, resident with the
+// fill beside it, and staged; all planes / codes alone): 5,300 gates that all
+// switch, 150 levels: 256 words 143 / 104 and 225 / 168, 1,024 words 481 / 342 and
+// 280 / 181, 2,048 words 952 / 674 and 306 / 199; 2,500 gates, 60 levels: 1,024
+// words 79 / 56 and 124 / 74, 2,048 words 145 / 104 and 137 / 83; 20,000 gates,
+// 3,367 not constant: 2,048 words 258 / 162 and 551 / 329, 8,192 words 1,838 / 1,532
+// and 1,904 / 1,207; 26,000 gates, 4,400 not constant: 1,024 words 282 / 185 and
+// 569 / 267, 4,955 words 4,320 and 2,498.
+bool resident_planes_pay(const ResidentShape &s, uint64_t W, uint32_t rows, uint64_t gates, uint32_t pieces) {
+    if (W > 1024ull * s.bw * s.bw) return false;
+    const double cells = (double)gates * W;
+    const double staged = rows == 3 ? 40.0 + 1.05 * pieces + 11e-6 * cells : 10.0 + 0.95 * pieces + 6.5e-6 * cells;
+    return 1.15 * (s.us + 5.0) <= staged;  // (and the fill's launch)
 }
 
 pdf_status build_plan(const NetPlan &n, const PlanOpts &o, LaunchPlan &pl) {

@@ -51,13 +51,23 @@ struct ResidentShape {
     uint32_t off_vt = 0, off_m = 0, off_bm = 0, off_mbar = 0;
     size_t smem = 0;
     double block_us = 0;  // modelled time of one column block
+    uint32_t words = 0;   // words an SM can take at a time, over all the widths that fit
+    double us = 0;        // modelled time of the walk
 };
 struct ResidentSizes {
     uint32_t n_gates = 0, n_levels = 0, image_bytes = 0;
     uint32_t sms = 0, regs = 0;
     size_t smem_block = 0, smem_sm = 0;
 };
-ResidentShape resident_shape(const ResidentSizes &z, uint64_t W);
+// rows: plane rows that it stores of every gate (0: none, lean walks; 2: codes; 3: and marks).
+ResidentShape resident_shape(const ResidentSizes &z, uint64_t W, uint32_t rows = 0);
+// Whether such a walk is the faster one, against the staged kernel's: of the
+// same netlist (up to resident_words), and (with rows, `gates` and `pieces` of
+// the whole netlist) of all gates.
+constexpr uint32_t kResidentWords = 8;  // words an SM has room for from which it always is
+uint64_t resident_words(const ResidentShape &s, uint32_t sms);
+bool resident_pays(const ResidentShape &s, uint64_t W, uint32_t sms);
+bool resident_planes_pay(const ResidentShape &s, uint64_t W, uint32_t rows, uint64_t gates, uint32_t pieces);
 
 struct LaunchPlan : PlanShape {
     std::vector<GateRec> recs;

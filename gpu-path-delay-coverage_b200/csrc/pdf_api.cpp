@@ -1325,8 +1325,16 @@ struct WsNeed {
         if (!k.resident && c->out_plan) with(c, pdf_circuit::resident_walk(*c->out_plan, W, out), W, need_planes);
         return with(c, k, W, need_planes);
     }
+    // every walk of a batch (sized without building the plan at the tile)
     WsNeed &batch(const pdf_circuit *c, uint64_t W) {
-        for (int i = 0; i < 4; i++) with(c, c->batch_walk(W, i & 1, i & 2), W, true);
+        const Plan &p = c->lean();
+        if (p.image) with(c, pdf_circuit::resident_walk(p, W, RES_LEAN), W, true);
+        Walk k;
+        k.p = &p;
+        for (uint32_t bw : {p.bw, c->tile_red.wanted ? c->tile_red.opts.bw : c->bw}) {
+            k.bw = bw;
+            with(c, k, W, true);
+        }
         return *this;
     }
 };

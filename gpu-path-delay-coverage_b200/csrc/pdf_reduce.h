@@ -103,9 +103,13 @@ inline NetFacts net_facts(const NetPlan &n, bool fixed) {
     f.observable.assign(G, 0);
     f.needed.assign(G, 0);
     std::vector<uint8_t> markable(G, 0);
+    // (constants come from killed gates and gates without fan-ins alone)
+    bool constants = false;
+    for (uint32_t g = 0; g < G && !constants; g++)
+        constants = (n.hdr[g] & RF_KILL) || (!n.nfi[g] && !(n.hdr[g] & RF_INPT));
     for (uint32_t g = 0; g < G; g++) {
         const uint32_t h = n.hdr[g], *fin = n.edges.data() + n.eoff[g];
-        f.value[g] = (int8_t)const_value(h, n.nfi[g], fin, f.value.data(), fixed);
+        if (constants) f.value[g] = (int8_t)const_value(h, n.nfi[g], fin, f.value.data(), fixed);
         if (f.value[g] >= 0) continue;
         bool m = h & RF_INPT;
         if (!m && (h & RF_MARKF0)) m = markable[fin[0]];
@@ -154,30 +158,39 @@ inline NetPlan reduce_net(const NetPlan &n, const NetFacts &f) {
     for (uint32_t l = 0; l < L; l++) r.level_off[l + 1] += r.level_off[l];
     // by level, then by kind (observable first, fan-in count, evaluation
     // flags), then by id: a counting sort by level, then one by kind within
-    // each level (a plain sort where the level is narrower than the buckets)
+    // each level (a plain sort where the level is much narrower than the buckets)
     constexpr uint32_t kKinds = 512;
     const auto kind = [&](uint32_t g) {
         const uint32_t h = n.hdr[g];
         return (f.observable[g] ? 0u : 256u) | std::min<uint32_t>(n.nfi[g], 4) << 5 |
                ((h >> 16) & 7u) << 2 | ((h & RF_XOR) ? 2u : 0u) | ((h & RF_OINV) ? 1u : 0u);
     };
+    struct Entry {
+        uint32_t g, kind;
+    };
     std::vector<uint32_t> at(r.level_off.begin(), r.level_off.end() - 1);
-    r.orig.assign(N, kNone);
+    std::vector<Entry> sorted(N, Entry{kNone, 0});
     for (uint32_t g = 0; g < G; g++)
-        if (f.needed[g]) r.orig[at[lvl[g]]++] = g;
-    std::vector<uint32_t> row, start;
+        if (f.needed[g]) sorted[at[lvl[g]]++] = Entry{g, kind(g)};
+    r.orig.assign(N, kNone);
+    uint32_t start[kKinds + 1];
     for (uint32_t l = 0; l < L; l++) {
-        uint32_t *o = r.orig.data() + r.level_off[l];
-        const uint32_t w = at[l] - r.level_off[l];
-        if (w < kKinds) {
-            std::stable_sort(o, o + w, [&](uint32_t x, uint32_t y) { return kind(x) < kind(y); });
+        const uint32_t o = r.level_off[l], w = at[l] - o;
+        Entry *e = sorted.data() + o;
+        if (w < 64) {  // (few of a kind apart: by insertion)
+            for (uint32_t i = 1; i < w; i++) {
+                const Entry x = e[i];
+                uint32_t k = i;
+                for (; k && e[k - 1].kind > x.kind; k--) e[k] = e[k - 1];
+                e[k] = x;
+            }
+            for (uint32_t i = 0; i < w; i++) r.orig[o + i] = e[i].g;
             continue;
         }
-        row.assign(o, o + w);
-        start.assign(kKinds + 1, 0);
-        for (uint32_t g : row) start[kind(g) + 1]++;
+        std::fill(start, start + kKinds + 1, 0u);
+        for (uint32_t i = 0; i < w; i++) start[e[i].kind + 1]++;
         for (uint32_t k = 0; k < kKinds; k++) start[k + 1] += start[k];
-        for (uint32_t g : row) o[start[kind(g)]++] = g;
+        for (uint32_t i = 0; i < w; i++) r.orig[o + start[e[i].kind]++] = e[i].g;
     }
     std::vector<uint32_t> id(G, kNone);
     for (uint32_t k = 0; k < N; k++)

@@ -692,8 +692,7 @@ namespace {
 constexpr uint64_t kWideLevel = 1024;
 
 // Column block of single calls over at most `words` words when the caller asked
-// for no tile: the widest of 1, 2 and 4 words that still gives every SM a CTA.
-// A walk is a chain of levels, whose steps are shorter with fewer words.
+// for no tile: the narrowest of 1, 2 and 4 words with at most one CTA per SM.  A walk is a chain of levels, whose steps are shorter with fewer words.
 // Measured (us; blocks of 1, 2, 4 words), four stage calls over 20,000 gates
 // without XOR: 96 words 329, 349, 388; 256 words 398, 348, 387; 384 words 660,
 // 432, 403; 45,000 gates FIXED: 96 words 2,101, 2,270, 2,429; 256 words 3,239,
@@ -993,7 +992,7 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
         if (reduced) c->red.mean_width = (uint32_t)mean_level(rnet);
         for (Plan *p : {&c->full, &c->red, &c->live, &c->tile_full.plan, &c->tile_red.plan}) {
             p->res.sms = (uint32_t)prop.multiProcessorCount;
-            p->res.regs = 64;  // its launch bound's
+            p->res.regs = kResidentRegs;  // its launch bound's
             p->res.smem_block = res_smem;
             p->res.smem_sm = (size_t)prop.sharedMemPerMultiprocessor;
         }

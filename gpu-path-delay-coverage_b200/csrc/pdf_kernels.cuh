@@ -235,7 +235,9 @@ cudaError_t launch_batch(const BatchLaunch &b, cudaStream_t st);
 
 // The resident forward kernel (pdf_resident.cu): threads per CTA at most, and
 // its launches.
-constexpr uint32_t kResidentThreads = 512;
+// CTAs of as many an SM at least, which bounds their registers (the walks are
+// shaped for them).
+constexpr uint32_t kResidentThreads = 512, kResidentCtas = 2, kResidentRegs = 65536 / (kResidentThreads * kResidentCtas);
 enum ResidentOut : int { RES_LEAN = 0, RES_PLANES = 1, RES_SIM = 2 };  // no planes; all three; V and T only
 cudaError_t launch_resident(const FwdArgs &a, int sem, int out, uint32_t bw, uint32_t ctas, uint32_t threads,
                             size_t smem, cudaStream_t st);

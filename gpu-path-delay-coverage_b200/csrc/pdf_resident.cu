@@ -275,7 +275,7 @@ __device__ __forceinline__ void resident_cta(const FwdArgs &a, const uint32_t ct
 }
 
 template <int BW, int SEM, int OUT>
-__global__ void __launch_bounds__(kResidentThreads) k_resident(const FwdArgs a) {
+__global__ void __launch_bounds__(kResidentThreads, kResidentCtas) k_resident(const FwdArgs a) {
     grid_trigger();
     resident_cta<BW, SEM, OUT>(a, blockIdx.x);
     grid_wait();
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kFillThreads) k_fill_planes(const int8_t *valu
 
 // The circuits of a batch whose netlists fit on chip.
 template <int BW, int SEM>
-__global__ void __launch_bounds__(kResidentThreads)
+__global__ void __launch_bounds__(kResidentThreads, kResidentCtas)
     k_batch_resident(const FwdArgs *args, const uint32_t *bpref, uint32_t n, BatchCtl *ctl, uint32_t blk0) {
     __shared__ FwdArgs s_a;
     __shared__ uint32_t s_blk;

@@ -3,7 +3,10 @@
 
 One gate-eval is one (vector pair x gate) through the whole pipeline:
 two-pattern simulation, robust marking, pruning, first-detect merge and
-exact path counting.  The default workload is the mixed-size batch (c4):
+exact path counting: pairs graded times gates of the netlist.  (Gates that no
+result depends on are not evaluated: the value says how fast netlists are
+graded, not how many gates were folded; the roofline counts what a pass has to
+read and write.)  The default workload is the mixed-size batch (c4):
 256 synthetic netlists of 500-200,000 gates (depth 20-150) with 1,024-65,536
 vector pairs each, graded in one batched pass per step (a CUDA graph of one
 forward launch per class of circuits, then the cover), beside the same
@@ -195,11 +198,38 @@ def profile_summary(name: str):
 
 
 def alg_bytes(nl, n_pairs: int) -> float:
-    """Algorithmic bytes of grading n_pairs pairs on netlist nl: the 2-bit
-    transition code and the 1-bit mark of every (net, pair), written once
-    (0.375 B per gate-eval), and the 2-bit codes of the primary inputs read
-    (0.25 B per PI and pair)."""
+    """Algorithmic bytes of grading n_pairs pairs on netlist nl with every
+    plane asked for: the 2-bit transition code and the 1-bit mark of every
+    (net, pair), written once (0.375 B per gate-eval), and the 2-bit codes of
+    the primary inputs read (0.25 B per PI and pair)."""
     return 0.375 * nl.n_gates * n_pairs + 0.25 * nl.n_pi * n_pairs
+
+
+def lean_bytes(nl, n_pairs: int) -> float:
+    """The same without planes, where a pass returns two first-pair ids per
+    net (4 B each) and a count: no code or mark of a net need leave the chip."""
+    return 8.0 * nl.n_gates + 0.25 * nl.n_pi * n_pairs
+
+
+FORWARD_KERNELS = ("k_batch_resident", "k_batch_forward_lanes", "k_batch_forward", "k_resident", "k_fill_planes", "k_wide",
+                   "k_forward_lanes", "k_forward")
+
+
+def own_kernels(torch, step) -> dict[str, int]:
+    """This library's kernels that one step launches, by name (traced once,
+    outside any timed region)."""
+    import re
+
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        step()
+        torch.cuda.synchronize()
+    out: dict[str, int] = {}
+    for e in prof.key_averages():
+        m = re.search(r"\b(k_[a-z_]+)\b", e.key)
+        if m:
+            out[m.group(1)] = out.get(m.group(1), 0) + e.count
+    return out
 
 
 def roofline(alg: float, kernel_ms: float, kernel: str, prof: dict | None, units: float,
@@ -565,17 +595,19 @@ def run_ours(args):
     value = units / (ms / 1e3)
     fwd_ms = prof_ms[0] / max(1, prof_calls)
     tile = c.info().tile_words
-    kname = "k_forward_lanes" if tile in LANE_TILES else "k_forward"
-    prof = profile_summary(f"{kname}_{args.workload}_tile{tile}") if not args.planes and args.segs == 1 and \
-        args.mark_mode == "robust" and not args.pairs else None
+    kernels = own_kernels(torch, step)
+    kname = " + ".join(k for k in FORWARD_KERNELS if k in kernels)
+    prof = profile_summary(f"{kname}_{args.workload}") if not args.planes and args.segs == 1 and \
+        args.mark_mode == "robust" and not args.pairs and not args.tile_words else None
     sm_count = torch.cuda.get_device_properties(local).multi_processor_count
     line = {
         "metric": "gate-evals/s", "value": value, "unit": "gate-evals/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "u32", "data": "synthetic (seeded)",
         "config": workload_config(P, args.workload, nl, n, args),
-        "roofline": dict(roofline(alg_bytes(nl, n), fwd_ms, f"{kname} (tile {tile} words)", prof, G * n,
-                                  sm_count, clocks.get("sm_mhz")), cover_ms=prof_ms[1] / max(1, prof_calls)),
+        "roofline": dict(roofline((alg_bytes if args.planes else lean_bytes)(nl, n), fwd_ms,
+                                  f"{kname} (tile {tile} words)", prof, G * n, sm_count, clocks.get("sm_mhz")),
+                         cover_ms=prof_ms[1] / max(1, prof_calls), kernels_per_step=kernels),
         "e2e": {"value": units / ((stream_ms or e2e_ms_mean) / 1e3), "unit": "gate-evals/s",
                 "h2d_bytes_per_step": int(2 * nl.n_pi * W * 4), "d2h_bytes_per_step": 64,
                 "mode": ("streamed: pinned host pairs copied on a second stream while the previous step "
@@ -584,8 +616,7 @@ def run_ours(args):
                          "count back" if dist else "one synchronous pdf_grade per step"),
                 "value_one_call_per_step": units / (e2e_ms_mean / 1e3),
                 "note": "one call per step: pdf_grade with the host pairs (H2D inside the call), then the next"},
-        # k_forward, k_active, k_cover; with segments k_forward, k_seg_merge, k_seg_first, k_cover
-        "gpu_launches": (4 if args.segs > 1 else 3) * args.steps,
+        "gpu_launches": sum(kernels.values()) * args.steps,
         "clocks": clocks,
         "result_stable": bool(totals_ok and stream_ok),
         "batch_count": job_total,
@@ -833,7 +864,8 @@ def run_batched(args):
     info = b.info()
     kernel_ms = sum(fwd_ms) / len(fwd_ms)
     sm_count = torch.cuda.get_device_properties(local).multi_processor_count
-    prof = profile_summary(f"k_batch_forward_c4_tile{tw}") if args.circuits == 256 else None
+    kernels = own_kernels(torch, lambda: b.run_async(stream))
+    prof = profile_summary(f"c4_tile{tw}") if args.circuits == 256 else None
     plain_best = min(plain_ms, plain_bt_ms, sweep_ms or float("inf"))
     line = {
         "metric": "gate-evals/s", "value": world * units / (ms / 1e3), "unit": "gate-evals/s", "n_gpus": world,
@@ -852,10 +884,11 @@ def run_batched(args):
                           "circuit's default tile, at the batch's tile, and each at the tile that graded "
                           "it fastest (every tile timed per circuit, 3 calls each); the fastest of these"},
         "batched_vs_plain": plain_best / ms,
-        "roofline": dict(roofline(sum(alg_bytes(nl, n) for nl, n in zip(nls, counts)), kernel_ms,
-                                  f"forward span of the pass (k_batch_forward{'_lanes' if tw in LANE_TILES else ''}, "
-                                  f"every class)", prof, units, sm_count, clocks.get("sm_mhz")),
-                         cover_ms=sum(cov_ms) / len(cov_ms)),
+        "roofline": dict(roofline(sum(lean_bytes(nl, n) for nl, n in zip(nls, counts)), kernel_ms,
+                                  "forward span of the pass (" +
+                                  ", ".join(k for k in FORWARD_KERNELS if k in kernels) + ", every class)", prof, units,
+                                  sm_count, clocks.get("sm_mhz")),
+                         cover_ms=sum(cov_ms) / len(cov_ms), kernels_per_pass=kernels),
         "e2e": {"value": world * units / (stream_ms / 1e3), "unit": "gate-evals/s",
                 "h2d_bytes_per_step": int(world * h2d), "d2h_bytes_per_step": 64 * len(jobs) * world,
                 "mode": "streamed: pinned host pairs of the next pass copied on a second stream while this "

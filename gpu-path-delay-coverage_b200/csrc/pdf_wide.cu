@@ -348,14 +348,21 @@ __device__ __forceinline__ uint32_t wide_gate(const FwdArgs &a, const WideArgs &
 
 // All CTAs of the (cooperative) grid; what each wrote before is visible after.
 // Bounded: false when the others did not come within `polls` (0: 2^22, seconds).
+__device__ __forceinline__ uint32_t acquire_u32(const uint32_t *p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ bool grid_sync(WideSync *s, uint32_t target, uint32_t polls) {
     __threadfence();
     atomicAdd(&s->arrived, 1u);
-    for (uint32_t i = 0, n = polls ? polls : 1u << 22; i < n; i++) {
-        uint32_t v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&s->arrived) : "memory");
-        if (v >= target) return true;
+    if (polls) {
+        for (uint32_t i = 0; i < polls; i++)
+            if (acquire_u32(&s->arrived) >= target) return true;
+        return false;
     }
+    for (uint32_t i = 0; i < (1u << 22); i++)
+        if (acquire_u32(&s->arrived) >= target) return true;
     return false;
 }
 

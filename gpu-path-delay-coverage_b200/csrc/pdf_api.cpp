@@ -1493,19 +1493,19 @@ pdf_status take_circuit_err(pdf_circuit *c, cudaStream_t cs) {
     return err_status(e);
 }
 
-// How many first-detecting pairs skip the cover's small table.  Up to one per
-// SM, the large table takes them side by side too, and those that would not fit
-// the small one are not walked twice; up to two where pairs mostly do not fit
-// (the FIXED non-robust table, netlists of 2^18 gates or more).  Measured (cover
-// kernels, us; through both tables and at once): 20,000 gates, 100 pairs 30 and
-// 29; 200,000 gates, 100 pairs 90 and 79; 1,000,000 gates, 32 pairs 459 and 211,
-// 256 pairs 591 and 485; FIXED non-robust, 20,000 gates, 32 pairs 211 and 139, 247
-// pairs 364 and 330, 477 pairs 565 and 585 (one table).  Where they fit, more
-// pairs than SMs are faster through the small one: FIXED robust, 60,000 gates,
-// 238 pairs 103 and 160.
+// How many first-detecting pairs skip the cover's small table: up to one per SM,
+// which the large table takes side by side too, where pairs often do not fit the
+// small one and would be walked twice (netlists of 2^16 gates or more); up to two
+// where they mostly do not (2^18 gates, the FIXED non-robust table).  Measured
+// (cover kernels, us; through both tables and at once): 200,000 gates, 100 pairs
+// 90 and 79; 1,000,000 gates, 32 pairs 459 and 211, 256 pairs 591 and 485; FIXED
+// non-robust, 20,000 gates, 32 pairs 211 and 139, 247 pairs 364 and 330, 477 pairs
+// 565 and 585 (one table).  Where they fit, the second pass is a launch too many:
+// 20,000 gates with segments, a whole call 196 and 200; FIXED robust, 60,000
+// gates, 238 pairs 103 and 160.
 uint32_t cover_few(const pdf_circuit *c, const Plan &p) {
-    const bool large = c->mark_mode == PDF_MARK_FIXED_NONROBUST || p.n_gates >= 1u << 18;
-    return (large ? 2 : 1) * c->cover_grid;
+    if (c->mark_mode == PDF_MARK_FIXED_NONROBUST || p.n_gates >= 1u << 18) return 2 * c->cover_grid;
+    return p.n_gates >= 1u << 16 ? c->cover_grid : 0;
 }
 
 CoverArgs base_cover(pdf_circuit *c, const Walk &k, Workspace &ws, const uint32_t *M, uint64_t ld, uint64_t n_pairs,

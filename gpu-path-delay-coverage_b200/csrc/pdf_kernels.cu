@@ -1271,7 +1271,11 @@ template <int TIER>
 __global__ void __launch_bounds__(kCoverThreads) k_cover(const CoverArgs a, uint32_t cap, uint32_t few) {
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr uint32_t CAND = TIER == 0 ? kCoverCandSmall : kCoverCand;
-    grid_trigger();
+    // The spill cover starts only once the CTAs of the large table are gone: on
+    // SMs still split for that table it would have next to no L1, which its walks
+    // over the netlist live on (335 pairs of 214,501 gates 302 ms, 266 so; 666
+    // pairs of 111,483 gates 99 and 71).
+    if (TIER == 0) grid_trigger();
     grid_wait();
     const bool direct = TIER == 0 || !a.mid_list;  // without a queue the large table takes every pair
     const uint32_t n_items = direct ? *a.active_count : a.acc->n_mid;
@@ -1387,6 +1391,7 @@ __global__ void __launch_bounds__(kCoverThreads) k_cover_lean(const CoverArgs a)
 // After k_cover: the pairs it queued, one per CTA at a time (CTA k uses
 // spill slot k); the last CTA closes the batch.
 __global__ void __launch_bounds__(kCoverThreads) k_cover_spill(const CoverArgs a) {
+    grid_wait();
     const uint32_t n_over = a.acc->n_over;
     if (!n_over) return;  // k_cover closed the batch
     for (uint32_t j = blockIdx.x; j < n_over; j += gridDim.x) spill_pair(a, a.over_list[j], spill_slot(a, blockIdx.x));
@@ -1847,11 +1852,7 @@ cudaError_t launch_cover(const CoverArgs &a, uint32_t grid, uint32_t threads, bo
     if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_cover<1>), smem)) != cudaSuccess) return e;
     e = launch_next(k_cover<1>, grid, threads, smem, st, a, a.hash_cap, 0u);
     if (e != cudaSuccess || !a.spill_slots) return e;
-    // A plain launch: started early it runs on SMs split for k_cover's tables, with
-    // next to no L1, which its walks over the netlist live on (335 pairs of 214,501
-    // gates 302 ms, 266 so; 666 pairs of 111,483 gates 99 and 71).
-    k_cover_spill<<<a.spill_slots, kCoverThreads, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_next(k_cover_spill, a.spill_slots, kCoverThreads, 0, st, a);
 }
 
 namespace {

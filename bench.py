@@ -405,7 +405,7 @@ def batch_config(members, args) -> dict:
             "gate_evals_per_pass": sum(nl.n_gates * n for nl, _, n in members),
             "mark_mode": MARK_MODES[args.mark_mode][1],
             "outputs": "path count and first-detect ids per circuit",
-            "l2": "flushed between timed steps (256 MiB write); the pass's planes (GBs) exceed L2"}
+            "l2": "flushed between timed steps (256 MiB write)"}
 
 
 def workload_config(P, name, nl, n_pairs, args=None) -> dict:

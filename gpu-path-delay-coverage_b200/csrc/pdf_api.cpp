@@ -688,11 +688,14 @@ namespace {
 // barriers (about 2 us a level).  Kernel times (us) at the thread-per-gate
 // kernel and at this one: 3,550 gates a level and 32,768 pairs with planes
 // 4,032 and 1,200; 1,500 a level and 65,536 pairs without 1,733 and 895; 308
-// a level and 32,768 pairs with planes 277 and 445.
+// a level and 32,768 pairs with planes 277 and 445.  Whole calls with planes
+// near the line: 1,108 gates a level (20 levels), 32 pairs 416 and 239, 65,536
+// pairs 1,517 and 753; 1,038 a level (40 levels) 545 and 291, 2,141 and 1,036.
 constexpr uint64_t kWideLevel = 1024;
 
 // Column block of single calls over at most `words` words when the caller asked
-// for no tile: the narrowest of 1, 2 and 4 words with at most one CTA per SM.  A walk is a chain of levels, whose steps are shorter with fewer words.
+// for no tile: the narrowest of 1, 2 and 4 words with at most one CTA per SM.
+// A walk is a chain of levels, whose steps are shorter with fewer words.
 // Measured (us; blocks of 1, 2, 4 words), four stage calls over 20,000 gates
 // without XOR: 96 words 329, 349, 388; 256 words 398, 348, 387; 384 words 660,
 // 432, 403; 45,000 gates FIXED: 96 words 2,101, 2,270, 2,429; 256 words 3,239,
@@ -872,8 +875,8 @@ extern "C" pdf_status pdf_circuit_create(const pdf_netlist *nl, const pdf_circui
     }
     pdf_status pst = PDF_OK;
     if (!other.valid()) pst = build_plan(net, po, full);
-    // The reduced netlist (single nets; segments are listed over every net),
-    // and the resident kernel's image of what a lean call walks.
+    // The reduced netlist (single nets only: a circuit with segments walks every
+    // gate), and the resident kernel's image of what a lean call walks.
     NetPlan rnet, lnet;
     ResidentImage image, limage;
     LaunchPlan live;
@@ -2125,7 +2128,8 @@ namespace {
 // one device block, which is reused when it is large enough.
 // up: the stream that uploads the control block, in order before the next
 // pass on it (the caller then must not rebind or destroy the batch before
-// that pass is done); null: uploaded and waited for here.
+// that pass is done); null: uploaded on a stream of the batch's own, which
+// the next pass waits for on the device.
 pdf_status batch_build(pdf_batch *b, const pdf_batch_job *jobs, uint32_t n_jobs, uint32_t flags,
                        cudaStream_t up = nullptr) {
     if (!jobs || !n_jobs || (flags & ~(uint32_t)(PDF_BATCH_APPEND | PDF_BATCH_NO_GRAPH))) return PDF_EINVAL;

@@ -15,7 +15,9 @@
 //
 // Measured (B200, kernel, us): a 20,000-gate circuit's 523 needed gates at
 // 32,768 pairs 45 -> 22; a 1M-gate circuit's at 65,536 pairs 125 -> 59; 7,000
-// gates that all switch at 3,776 pairs 92 -> 28.
+// gates that all switch at 3,776 pairs 92 -> 28.  The first and the last wait at
+// the levels' barriers most (7 and 14 warps of an issue; memory 1 to 2), issue 42 %
+// and 18 % active, DRAM at 1 % of its peak.
 //
 // With planes (OUT) it walks every gate that is not constant, all levels, and
 // stores codes as it finds them (20,000 gates x 32,768 pairs, 3,400 of them

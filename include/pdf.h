@@ -164,13 +164,19 @@ enum {
 typedef struct pdf_circuit_opts {
     int device;          /* CUDA device ordinal */
     int mark_mode;       /* PDF_MARK_* */
-    uint32_t max_pairs;  /* largest batch this circuit will grade (sizes scratch); 0 = 65536 */
+    uint32_t max_pairs;  /* largest batch this circuit will grade (the tile is chosen for it, and
+                            single calls over it; larger calls work and take the tile); 0 = 65536 */
     uint32_t tile_words; /* words (32 pairs) per CTA column block: 1, 2, 4, 8 (a thread per gate)
                             or 32, 64, 128 (the lane kernel: a warp per gate, 1, 2 or 4 words
                             per lane, for wide levels); 0 = chosen: a lane tile when max_pairs
                             gives >= 1 1,024-pair block per SM and the levels average >= 1,024
                             gates (the one with the least modelled time), else 8 when max_pairs
-                            gives >= 2 8-word CTAs per SM, else 4 */
+                            gives >= 2 8-word CTAs per SM, else 4.  The tile is that of batches,
+                            of the planes' row pitch and of the calls that no other kernel takes:
+                            a call over a netlist that fits on chip takes the resident kernel;
+                            where no tile was asked for, single calls on levels that average
+                            >= 1,024 gates take the wide kernel, and those over few pairs
+                            (max_pairs / 32 words, up to 2 words an SM) blocks of 1 or 2 words */
     uint32_t threads;    /* 0 = piece capacity + 64 (lane tiles: 1,024, or 512 at 128 words);
                             else threads per CTA: 64..1024, a multiple of 32, capped at the
                             lane tile's default; from 128 up, pieces of the thread-per-gate
